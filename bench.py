@@ -44,10 +44,6 @@ sys.path.insert(0, ROOT)
 
 N_ROWS, M_BITS, P_RANGE, SEED = 65536, 262144, (0.05, 0.5), 0x5EED2
 L2_BYTES = 126 * 1000 * 1000
-# DRAM bytes per launch of the tensor-core kernel on the 65536 x 262144 workload:
-# one ncu capture at 16384 x 262144 (10.710 GB read + 0.525 GB written), scaled
-# by the pairs ratio 16 (tiles, and the rows they re-read, grow with the pairs).
-TS_TRAFFIC_BENCH_WORKLOAD = 11.2358e9 * 16
 METRIC = "exact pairs/sec & ns/pair on 1 B200: learned-batched vs plain GPU vs CPU"
 
 
@@ -246,9 +242,23 @@ def tensor8_peak(device, size=8192, reps=10, loop_s=2.0):
     return res
 
 
-def tensor_peak_tops(device):
-    """(peak TOPS, source text) for the int8 tensor-core roofline."""
+def tensor_kernel(sb, kernel, bits):
+    """The kernel a contiguous call ran on: the tensor-core choices share the
+    4-bit kernel up to 2^24-bit rows."""
+    if kernel in (sb.KERNEL_MMA, sb.KERNEL_MMA_DB) and bits <= 1 << 24:
+        return "bb_f4_kernel"
+    return {sb.KERNEL_POPC: "bb_popc_kernel", sb.KERNEL_MMA: "bb_mma_ts_long_kernel",
+            sb.KERNEL_MMA_SS: "bb_mma_kernel", sb.KERNEL_MMA_DB: "bb_mma_ts2_long_kernel",
+            sb.KERNEL_MMA_2CTA: "bb_mma_2cta_kernel"}.get(kernel, "?")
+
+
+def tensor_peak_tops(device, bits4=True):
+    """(peak TOPS, source text) for the tensor-core roofline: the 4-bit kernel's
+    against four times the measured bf16 rate (the pipe's e2m1 rate), the 8-bit
+    kernels' against the largest of the measured 8-bit figures."""
     peaks, src = measured_peaks()
+    if bits4:
+        return 4.0 * peaks["bf16_tflops"], f"4 x bf16_tflops {src}: {4.0 * peaks['bf16_tflops']:.1f}"
     t8 = tensor8_peak(device)
     cands = {f"2 x bf16_tflops {src}": 2.0 * peaks["bf16_tflops"]}
     if t8.get("int8_tops"):
@@ -798,7 +808,7 @@ def triangle_row_sums(d_tri, n):
 def engine_roofline(eng, device):
     """Per STORM_t engine of the last call: device ms, the planner's
     prediction, and the engine's roofline -- the tensor cores against the
-    measured 8-bit tensor peak, the panel and the postings (bytes they must
+    4-bit tensor peak, the panel and the postings (bytes they must
     move) against the measured HBM bandwidth."""
     peaks, src = measured_peaks()
     tpk, _ = tensor_peak_tops(device)
@@ -809,7 +819,7 @@ def engine_roofline(eng, device):
         e = {"ms": round(ms, 3), "predicted_ms": round(pred, 3)}
         if ms > 0 and work > 0:
             if name == "tensor":
-                e.update({"tops_int8": work / (ms * 1e-3) / 1e12, "frac_of_tensor_peak": work / (ms * 1e-3) / 1e12 / tpk})
+                e.update({"tops": work / (ms * 1e-3) / 1e12, "frac_of_tensor_peak": work / (ms * 1e-3) / 1e12 / tpk})
             elif name in ("panel", "postings"):
                 gbs = work / (ms * 1e-3) / 1e9
                 e.update({"alg_bytes": work, "GBps": gbs, "frac_of_hbm": gbs / peaks["hbm_gbs"],
@@ -1047,9 +1057,8 @@ def config5a_full(sb, device, steps=3):
     res = {"workload": "200000 sites x 20000 haplotypes, P(k) ~ 1/k, 32-haplotype carrier blocks; "
                        "80 GB u32 triangle in HBM", "pairs_i_le_j": tri, "ms": round(k, 2),
            "pairs_per_s": tri / (k * 1e-3), "checksum_sum_i_lt_j": sums.pop() if len(sums) == 1 else None,
-           "kernel": {sb.KERNEL_POPC: "bb_popc_kernel", sb.KERNEL_MMA: "bb_mma_ts_kernel",
-                      sb.KERNEL_MMA_DB: "bb_mma_ts2_kernel"}.get(c.last_kernel(), "?"),
-           "roofline": {"achieved_tops_int8": tops, "peak": peak, "frac": tops / peak}}
+           "kernel": tensor_kernel(sb, c.last_kernel(), m),
+           "roofline": {"achieved_tops": tops, "peak": peak, "frac": tops / peak}}
     del out
     c.close()
     torch.cuda.empty_cache()
@@ -1076,7 +1085,7 @@ def autotune_config1(sb, device):
     tops = {nm: round(2.0 * 4096 * 4097 / 2 * 65536 / (t * 1e-3) / 1e12, 1) for nm, t in zip(names, times) if t > 0}
     return {"workload": "4096 rows x 65536 bits, Bernoulli(0.5)",
             "candidates_ms": {nm: round(t, 4) for nm, t in zip(names, times)},
-            "candidates_tops_int8": tops,
+            "candidates_tops": tops,
             "kept": names[cand.index((k, sched))] if (k, sched) in cand else f"kernel {k} schedule {sched}"}
 
 
@@ -1320,7 +1329,8 @@ def storm_t_forms(device, cpu_seconds=2.0, only=None):
     return out
 
 
-TENSOR_KERNELS = ("bb_mma_kernel", "bb_mma_ts_kernel", "bb_mma_ts2_kernel", "bb_mma_2cta_kernel")
+TENSOR_KERNELS = ("bb_f4_kernel", "bb_mma_kernel", "bb_mma_ts_long_kernel", "bb_mma_ts2_long_kernel",
+                  "bb_mma_2cta_kernel")
 
 
 def north_star_summary(line):
@@ -1342,9 +1352,9 @@ def north_star_summary(line):
 
     ns = {"headline_frac": r3(g(line, "roofline", "frac")), "headline_e2e_pairs_per_s": r3(g(line, "e2e", "value"))}
     at = line.get("autotune_config1")
-    if isinstance(at, dict) and "candidates_tops_int8" in at:
+    if isinstance(at, dict) and "candidates_tops" in at:
         peak = g(line, "roofline", "peak")
-        best = max(at["candidates_tops_int8"].values()) if at["candidates_tops_int8"] else None
+        best = max(at["candidates_tops"].values()) if at["candidates_tops"] else None
         ns["config1_best_tops"] = r3(best)
         ns["config1_frac"] = r3(best / peak) if best and peak else None
         ns["config1_kept"] = at.get("kept")
@@ -1489,9 +1499,7 @@ def run_b200_arm(args):
     elapsed_ms = sum(step_ms) if flush is not None else ev0.elapsed_time(ev1)
     elapsed_ms = max_over_ranks(elapsed_ms, dist, device)
     launches = args.steps * c.last_launches()
-    kernel_used = {sb.KERNEL_POPC: "bb_popc_kernel", sb.KERNEL_MMA: "bb_mma_ts_kernel",
-                   sb.KERNEL_MMA_SS: "bb_mma_kernel", sb.KERNEL_MMA_DB: "bb_mma_ts2_kernel",
-                   sb.KERNEL_MMA_2CTA: "bb_mma_2cta_kernel"}.get(c.last_kernel(), "?")
+    kernel_used = tensor_kernel(sb, c.last_kernel(), m)
     ms_per_step = elapsed_ms / args.steps
     value = world * tri / (ms_per_step / 1e3)
 
@@ -1573,16 +1581,13 @@ def run_b200_arm(args):
     # ---- roofline of the dominant kernel ----
     k_ms = statistics.median(kernel_ms)
     if kernel_used in TENSOR_KERNELS:
-        ops = 2.0 * tri * m                      # u8 MACs = pairs x row bits, 2 ops each
+        ops = 2.0 * tri * m                      # MACs = pairs x row bits, 2 ops each
         achieved = ops / (k_ms / 1e3) / 1e12
-        peak, peak_src = tensor_peak_tops(device)
-        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TOPS (int8)",
+        bits4 = kernel_used == "bb_f4_kernel"
+        peak, peak_src = tensor_peak_tops(device, bits4)
+        roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": f"TOPS ({'e2m1' if bits4 else 'int8'})",
                 "frac": achieved / peak, "peak_source": peak_src, "tensor8_measured": tensor8_peak(device),
                 "algorithmic": f"pairs(i<=j) x {m} bit-MACs x 2 ops", "traffic": args.traffic}
-        if args.traffic is None and (n, m) == (N_ROWS, M_BITS) and kernel_used == "bb_mma_ts_kernel":
-            roof["traffic"] = TS_TRAFFIC_BENCH_WORKLOAD
-            roof["traffic_source"] = ("dram__bytes_read.sum + dram__bytes_write.sum of one launch at 16384 x 262144 "
-                                      "(11.24 GB, profiles/bb_mma_ts_dram_16384x262144.md) x 16 (pairs ratio)")
     else:
         ops = 2.0 * tri * m
         achieved = ops / (k_ms / 1e3) / 1e12
@@ -1592,8 +1597,8 @@ def run_b200_arm(args):
     line = {
         "metric": METRIC, "value": value, "unit": "pairs/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_per_step, "ns_per_pair": 1e9 / (value / world),
-        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "u8 (tcgen05 kind::i8, s32 acc)"
-        if kernel_used in TENSOR_KERNELS else "u64 (AND + POPC)",
+        "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": "e2m1 (tcgen05 kind::mxf4, whole-number f32 acc)"
+        if kernel_used == "bb_f4_kernel" else "u8 (tcgen05 kind::i8, s32 acc)" if kernel_used in TENSOR_KERNELS else "u64 (AND + POPC)",
         "data": "synthetic (seeded Bernoulli rows generated on the GPU)",
         "config": {"workload": f"dense all-bitmap XX^T: {n} rows x {m} bits, p~U[0.05,0.5], u32 i<=j out",
                    "rows": n, "bits": m, "pairs_per_gpu": tri, "kernel": kernel_used, "schedule": args.schedule,

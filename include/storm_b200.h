@@ -80,11 +80,12 @@ typedef void (*STORM_tile_callback)(uint32_t i0, uint32_t j0, uint32_t nr, uint3
 #define STORM_B200_KERNEL_AUTO  0   /* MMA_DB for rows <= 2^17 bits, MMA up to
                                        2^27, POPC beyond                         */
 #define STORM_B200_KERNEL_POPC  1   /* CUDA-core AND + POPC tiles                  */
-#define STORM_B200_KERNEL_MMA   2   /* tcgen05 kind::i8, A operand in TMEM         */
+#define STORM_B200_KERNEL_MMA   2   /* tcgen05, A operand in TMEM: kind::mxf4 on CTA
+                                       pairs (256 x 256 tiles) for rows <= 2^24 bits,
+                                       kind::i8 (128 x 256 tiles) beyond         */
 #define STORM_B200_KERNEL_MMA_SS 3  /* tcgen05 kind::i8, both operands in smem     */
-#define STORM_B200_KERNEL_MMA_DB 4  /* tcgen05 kind::i8, A in TMEM, 128 x 192 tiles
-                                       with two accumulators drained by their own
-                                       warps while the next tile computes        */
+#define STORM_B200_KERNEL_MMA_DB 4  /* as MMA for rows <= 2^24 bits; beyond, kind::i8
+                                       with 128 x 192 tiles and two accumulators */
 #define STORM_B200_KERNEL_MMA_2CTA 5 /* tcgen05 kind::i8 on CTA pairs (cta_group::2):
                                        256 x 256 tiles, each CTA expanding half of
                                        the B rows                                */
@@ -115,8 +116,7 @@ int STORM_contig_set_kernel(STORM_contiguous_t* c, int kernel);
 int STORM_contig_set_schedule(STORM_contiguous_t* c, int schedule);
 /* Autotuner (no counterpart in the reference): times this container's own
  * all-pairs call on the GPU with each bitmap x bitmap kernel that is exact
- * for its row length -- tcgen05 with A in tensor memory (128 x 256 tiles,
- * then 128 x 192 double-buffered tiles), each under whole-tile and stream-K
+ * for its row length -- MMA, then MMA_DB, each under whole-tile and stream-K
  * schedules; tcgen05 with both operands in shared memory; CUDA-core POPC;
  * tcgen05 on CTA pairs (whole tiles) -- best of two calls each, and keeps
  * the fastest kernel and schedule for later calls.  times_ms (7 entries in
@@ -154,8 +154,8 @@ void* STORM_contig_stream(STORM_contiguous_t* c);
  * handle's stream) and how many kernels it launched. */
 float STORM_contig_last_kernel_ms(const STORM_contiguous_t* c);
 uint32_t STORM_contig_last_launches(const STORM_contiguous_t* c);
-/* Which kernel the last call ran (STORM_B200_KERNEL_POPC, _MMA, _MMA_SS or
- * _MMA_DB). */
+/* Which kernel choice the last call ran under (STORM_B200_KERNEL_POPC, _MMA,
+ * _MMA_SS, _MMA_DB or _MMA_2CTA; never _AUTO). */
 int STORM_contig_last_kernel(const STORM_contiguous_t* c);
 
 /* All pairs of rows that are already in device memory, into a device buffer,
@@ -174,8 +174,8 @@ int STORM_contig_last_kernel(const STORM_contiguous_t* c);
  * Runs the tensor-core kernel (row_bits <= 2^23) on `stream` (a
  * cudaStream_t; NULL = the default stream) and waits for that stream before
  * returning, so the counts and the sum are complete on return.  Its scratch
- * (status/sum words and a tile list of at most 32768 tiles of 128 x 256
- * pairs: n_rows up to 46080) is a 256 KiB array in the library that every
+ * (status/sum words and a tile list of 256 x 256 pairs: n_rows up to 46080)
+ * is a 127 KiB array in the library that every
  * GPU holding the library keeps until exit; larger problems return
  * STORM_B200_ELIMIT.  The first call on a device looks that array up (and
  * opts the kernel into its shared memory), so make the first call before any

@@ -92,7 +92,7 @@ __device__ __forceinline__ uint64_t ts_out_index(uint64_t n, uint64_t i, uint64_
     return a < b ? tri_index(n_out, a, b) : tri_index(n_out, b, a);
 }
 
-// Work schedule, identical in the three roles of a CTA. k_splits >= 1:
+// Work schedule, identical in every role of a worker (a CTA, or a CTA pair). k_splits >= 1:
 // whole tiles (or k_splits even K slices of each) dealt round robin over the
 // grid. k_splits == 0 (stream-K, data-parallel head): the first
 // W = floor(tiles / G) x G tiles go whole, round robin (G = grid); CTA c then
@@ -102,15 +102,18 @@ __device__ __forceinline__ uint64_t ts_out_index(uint64_t n, uint64_t i, uint64_
 // adds its partial counts into the output, which must be zeroed for the
 // tiles from W on; whole tiles store theirs.
 struct TsSched {
-    uint32_t nk, n_tiles, k_splits, it, whole = 0;
+    uint32_t nk, n_tiles, k_splits, it, grid, whole = 0;
     uint64_t pos = 0, end = 0;
     __device__ __forceinline__ TsSched(uint32_t nk_, uint32_t n_tiles_, uint32_t k_splits_)
-        : nk(nk_), n_tiles(n_tiles_), k_splits(k_splits_), it(blockIdx.x) {
+        : TsSched(nk_, n_tiles_, k_splits_, blockIdx.x, gridDim.x) {}
+    __device__ __forceinline__ TsSched(uint32_t nk_, uint32_t n_tiles_, uint32_t k_splits_, uint32_t worker,
+                                       uint32_t workers)
+        : nk(nk_), n_tiles(n_tiles_), k_splits(k_splits_), it(worker), grid(workers) {
         if (k_splits == 0) {
-            whole = (n_tiles / gridDim.x) * gridDim.x;
+            whole = (n_tiles / grid) * grid;
             const uint64_t S = (uint64_t)(n_tiles - whole) * nk;
-            pos = (uint64_t)whole * nk + S * blockIdx.x / gridDim.x;
-            end = (uint64_t)whole * nk + S * (blockIdx.x + 1) / gridDim.x;
+            pos = (uint64_t)whole * nk + S * worker / grid;
+            end = (uint64_t)whole * nk + S * (worker + 1) / grid;
         }
     }
     __device__ __forceinline__ bool next(uint32_t& t, uint32_t& kb0, uint32_t& kb1, bool& partial) {
@@ -120,7 +123,7 @@ struct TsSched {
                 kb0 = 0;
                 kb1 = nk;
                 partial = false;
-                it += gridDim.x;
+                it += grid;
                 return true;
             }
             if (pos >= end) return false;
@@ -138,7 +141,7 @@ struct TsSched {
         kb0 = (uint32_t)((uint64_t)nk * ks / k_splits);
         kb1 = (uint32_t)((uint64_t)nk * (ks + 1) / k_splits);
         partial = k_splits > 1;
-        it += gridDim.x;
+        it += grid;
         return true;
     }
 };
@@ -410,12 +413,6 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
 // k_splits: the work schedule (TsSched). 1 = whole tiles round robin;
 // > 1 = that many K slices per tile; 0 = stream-K. For any value but 1 the
 // partial counts are added into out with atomics (out zeroed beforehand).
-__global__ void __launch_bounds__(TS_THREADS, 1)
-bb_mma_ts_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
-                 uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags, uint32_t k_splits) {
-    ts_body<false, false>(X, n, w_pad, lay, tiles, n_tiles, out, flags, nullptr, 0, k_splits);
-}
-
 // Rows of 2^23 .. 2^27 bits: the 4-byte weight cycle keeps D = 8 x count < 2^31.
 __global__ void __launch_bounds__(TS_THREADS, 1)
 bb_mma_ts_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
@@ -427,13 +424,6 @@ bb_mma_ts_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad
 // Same kernel over a gathered subset of rows, writing into the triangle of
 // the full row set through row_map (the kernel layer's dense block).
 __global__ void __launch_bounds__(TS_THREADS, 1)
-bb_mma_ts_rows_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
-                      uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
-                      const uint32_t* __restrict__ row_map, uint64_t n_out, uint32_t k_splits) {
-    ts_body<true, false>(X, n, w_pad, lay, tiles, n_tiles, out, flags, row_map, n_out, k_splits);
-}
-
-__global__ void __launch_bounds__(TS_THREADS, 1)
 bb_mma_ts_rows_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay,
                            const uint2* __restrict__ tiles, uint32_t n_tiles, uint32_t* __restrict__ out,
                            DeviceFlags* __restrict__ flags, const uint32_t* __restrict__ row_map, uint64_t n_out,
@@ -442,12 +432,6 @@ bb_mma_ts_rows_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t 
 }
 
 // Thresholded form over contiguous rows (whole tiles round robin).
-__global__ void __launch_bounds__(TS_THREADS, 1)
-bb_mma_ts_thresh_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
-                        uint32_t n_tiles, DeviceFlags* __restrict__ flags, TsThresh th) {
-    ts_body<false, false, true>(X, n, w_pad, lay, tiles, n_tiles, nullptr, flags, nullptr, 0, 1u, th);
-}
-
 __global__ void __launch_bounds__(TS_THREADS, 1)
 bb_mma_ts_thresh_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay,
                              const uint2* __restrict__ tiles, uint32_t n_tiles, DeviceFlags* __restrict__ flags,

@@ -248,12 +248,6 @@ __device__ __forceinline__ void ts2_body(const uint64_t* __restrict__ X, uint32_
 }
 
 __global__ void __launch_bounds__(T2_THREADS, 1)
-bb_mma_ts2_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
-                  uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags, uint32_t k_splits) {
-    ts2_body<false>(X, n, w_pad, lay, tiles, n_tiles, out, flags, k_splits);
-}
-
-__global__ void __launch_bounds__(T2_THREADS, 1)
 bb_mma_ts2_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
                        uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
                        uint32_t k_splits) {

@@ -1838,6 +1838,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         const RowLayout lay{PANEL_PITCH, rows_alloc * PANEL_PITCH};
         d_panel.reserve(rows_alloc * panel_row_words(W));
         d_map.reserve(rows_alloc);
+        const uint32_t bm = rows_block_a((uint32_t)W);
         d_tiles.reserve((P / 128) * (2 * P / 256 + 1));
         const uint64_t npan = single ? 1 : (ne2 + P - 1) / P;
         auto is_q = [&](uint64_t global_row) { return global_row >= nd_pad; };
@@ -1863,19 +1864,19 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             if (is_q(gI)) break;                          // this and later panels are all tq
             expand(gI, mI, 0);
             std::vector<uint2> tri;
-            build_mma_tiles(tri, mI);                      // I x I triangle, tq x tq blocks left out
+            build_rows_tiles(tri, mI, (uint32_t)W);        // I x I triangle, tq x tq blocks left out
             tl.clear();
             for (const uint2& t : tri)
-                if (!(is_q(gI + (uint64_t)t.x * 128) && is_q(gI + (uint64_t)t.y * 256))) tl.push_back(t);
+                if (!(is_q(gI + (uint64_t)t.x * bm) && is_q(gI + (uint64_t)t.y * 256))) tl.push_back(t);
             tensor(mI);
             for (uint64_t J = I + 1; J < npan; ++J) {      // I x J rectangle (I is a full panel)
                 const uint64_t gJ = J * P, mJ = std::min<uint64_t>(P, ne2 - gJ);
                 expand(gJ, mJ, P);
                 tl.clear();
-                for (uint32_t bi = 0; bi < P / 128; ++bi) {
-                    if (is_q(gI + (uint64_t)bi * 128) && is_q(gJ)) continue;
+                for (uint32_t bi = 0; bi < P / bm; ++bi) {
+                    if (is_q(gI + (uint64_t)bi * bm) && is_q(gJ)) continue;
                     for (uint32_t bj = (uint32_t)(P / 256); bj < (uint32_t)((P + mJ + 255) / 256); ++bj)
-                        if (!(is_q(gI + (uint64_t)bi * 128) && is_q(gJ + (uint64_t)bj * 256 - P)))
+                        if (!(is_q(gI + (uint64_t)bi * bm) && is_q(gJ + (uint64_t)bj * 256 - P)))
                             tl.push_back(make_uint2(bi, bj));
                 }
                 tensor(P + mJ);

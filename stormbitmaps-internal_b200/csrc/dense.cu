@@ -5,6 +5,7 @@
 #include "bb_mma_ts.cuh"
 #include "bb_mma_ts2.cuh"
 #include "bb_mma_2cta.cuh"
+#include "bb_f4.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -42,13 +43,93 @@ static uint32_t ts_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t&
 
 constexpr uint64_t DB_AUTO_MAX_BITS = 1ull << 17;
 
+// The tensor-core kernel a row length runs on: up to 2^24 bits the 4-bit one
+// (its fp32 accumulator counts exactly that far), longer rows the 8-bit ones.
+// Measured on B200, 8-bit -> 4-bit (ms): 65536 x 2^18 bits 346 -> 177, 50000 x
+// 20000 18.5 -> 8.2, 4096 x 65536 0.45 -> 0.20, 100 x 1000 the same.
+static int exec_kind(int kind, uint64_t row_bits) {
+    return (kind == STORM_B200_KERNEL_MMA || kind == STORM_B200_KERNEL_MMA_DB) && row_bits <= F4_MAX_BITS ? KIND_F4
+                                                                                                           : kind;
+}
+
+// Schedule of the 4-bit kernel over `pairs` pairs of CTAs, as ts_schedule.
+static uint32_t f4_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t& pairs,
+                            int pref = STORM_B200_SCHED_AUTO) {
+    const uint32_t np = std::max(1, sms / 2);
+    const uint64_t nk = w_pad / F4_STAGE_WORDS;
+    const uint64_t waves = ((uint64_t)n_tiles + np - 1) / np;
+    const double fill = waves ? (double)n_tiles / (double)(waves * np) : 1.0;
+    const bool tiles = pref == STORM_B200_SCHED_TILES ||
+                       (pref == STORM_B200_SCHED_AUTO && (fill >= 0.985 || nk < 64));
+    if (tiles) {
+        pairs = std::min(n_tiles, np);
+        return 1;
+    }
+    pairs = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(np, (uint64_t)n_tiles * nk / 16));
+    return 0;
+}
+
+// Tensor map of device rows for the 4-bit kernel: 32-bit elements, boxes of
+// 512 bits x 128 rows with a 64-byte swizzle; row-major rows in two
+// dimensions (what lies past the row's words reads as zero), block-major
+// panels with the 1024-word block as the third.  blk_words: words per block,
+// 0 for row-major rows.
+static CUtensorMap f4_row_map(const uint64_t* X, uint64_t n, uint32_t w_pad, RowLayout lay, uint32_t* blk_words) {
+    typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                               const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (Encode)f;
+    }();
+    if (!encode) fail(STORM_B200_ECUDA, "cuTensorMapEncodeTiled is not available");
+    const bool blocked = lay.kstride != 1024;
+    *blk_words = blocked ? 1024u : 0u;
+    const cuuint64_t dims[3] = {blocked ? 2048u : 2ull * w_pad, n, blocked ? (w_pad + 1023u) / 1024u : 1u};
+    const cuuint64_t strides[2] = {lay.pitch * 8, blocked ? lay.kstride * 8 : lay.pitch * 8};
+    const cuuint32_t box[3] = {16, 128, 1}, one[3] = {1, 1, 1};
+    CUtensorMap m;
+    if (encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT32, 3, (void*)X, dims, strides, box, one,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        fail(STORM_B200_ECUDA, "tensor map of the rows");
+    return m;
+}
+
+// Launch of a kernel on `pairs` clusters of two CTAs.
+template <class... P, class... A>
+static cudaError_t launch_pairs(void (*kernel)(P...), uint32_t pairs, uint32_t threads, uint32_t smem, cudaStream_t st,
+                                A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * pairs, 1, 1);
+    cfg.blockDim = dim3(threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // Rows per A block and per B block of a kernel's tiles.
 uint64_t tile_rows_a(int kind) {
-    return kind == STORM_B200_KERNEL_POPC ? POPC_BM : kind == STORM_B200_KERNEL_MMA_2CTA ? C2_BM : MMA_BM;
+    return kind == STORM_B200_KERNEL_POPC       ? POPC_BM
+           : kind == KIND_F4                    ? F4_BM
+           : kind == STORM_B200_KERNEL_MMA_2CTA ? C2_BM
+                                                : MMA_BM;
 }
 uint64_t tile_rows_b(int kind) {
     return kind == STORM_B200_KERNEL_POPC     ? POPC_BM
            : kind == STORM_B200_KERNEL_MMA_DB ? T2_BN
+           : kind == KIND_F4                  ? F4_BN
            : kind == STORM_B200_KERNEL_MMA_2CTA ? C2_BN
                                                 : MMA_BN;
 }
@@ -60,7 +141,8 @@ void build_tiles(std::vector<uint2>& t, uint64_t n, int kind) {
     const uint64_t bm = tile_rows_a(kind), bn = tile_rows_b(kind);
     if (((n + bm - 1) / bm) * ((n + bn - 1) / bn) > 0xFFFFFFFFull)
         fail(STORM_B200_ELIMIT, "more than 2^32 tiles: split the rows into several containers");
-    if (kind == STORM_B200_KERNEL_MMA_2CTA) {
+    static_assert(F4_BM == C2_BM && F4_BN == C2_BN, "both pair kernels use 256 x 256 tiles");
+    if (kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4) {
         const uint64_t nb = (n + C2_BM - 1) / C2_BM;
         for (uint64_t bi = 0; bi < nb; ++bi)
             for (uint64_t bj = bi; bj < nb; ++bj) t.push_back(make_uint2((uint32_t)bi, (uint32_t)bj));
@@ -85,11 +167,8 @@ void build_tiles(std::vector<uint2>& t, uint64_t n, int kind) {
 int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStream_t st) {
     if (n > 0xFFFFFFFFull) fail(STORM_B200_ELIMIT, "more than 2^32 rows");
     int kind = kernel_pref;
-    // Automatic choice: rows of at most 2^17 bits (tiles of at most 512 K
-    // stages) take the double-buffered tensor-core kernel, whose drain of one
-    // tile overlaps the next tile's MMAs (measured on B200: 19 % faster at
-    // 20000-bit rows, 3 % at 65536, even at 2^18); longer rows up to 2^27
-    // bits the 128 x 256 kernel; past that the CUDA-core POPC kernel.
+    // Automatic choice: tensor cores up to 2^27-bit rows (both choices run the
+    // 4-bit kernel up to 2^24 bits and differ past it), CUDA-core POPC beyond.
     if (kind == STORM_B200_KERNEL_AUTO)
         kind = row_bits <= DB_AUTO_MAX_BITS    ? STORM_B200_KERNEL_MMA_DB
                : row_bits <= MMA_MAX_BITS_W4 ? STORM_B200_KERNEL_MMA
@@ -99,6 +178,8 @@ int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStr
         fail(STORM_B200_ELIMIT, "tensor-core kernel is exact only for rows of at most 2^27 bits");
     if (kind == STORM_B200_KERNEL_MMA_SS && row_bits > MMA_MAX_BITS)
         fail(STORM_B200_ELIMIT, "shared-memory tensor-core kernel is exact only for rows of at most 2^23 bits");
+    reported = kind;
+    kind = exec_kind(kind, row_bits);
     if (tiles_n != n || tiles_kind != kind) {
         build_tiles(h_tiles, n, kind);
         d_tiles.reserve(h_tiles.size());
@@ -118,12 +199,10 @@ int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStr
 // W = floor(tiles / grid) x grid on add into the output, and every one of them
 // has its A block at or past tile W's (the list is ordered by A block), so
 // zeroing the triangle from that block's first row on covers them.
-static_assert(T2_BM == MMA_BM, "both tensor-core tilings use 128-row A blocks");
-
 void DenseEngine::zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st) {
     const uint32_t whole = (n_tiles / grid) * grid;
     if (whole >= n_tiles) return;
-    const uint64_t r0 = (uint64_t)h_tiles[whole].x * MMA_BM;   // 128-row A blocks in both tensor-core tilings
+    const uint64_t r0 = (uint64_t)h_tiles[whole].x * tile_rows_a(tiles_kind);
     const uint64_t e0 = r0 * n - (r0 * (r0 - 1)) / 2;          // tri_index(n, r0, r0)
     SB_CUDA(cudaMemsetAsync(d_out + e0, 0, (tri_size(n) - e0) * sizeof(uint32_t), st));
 }
@@ -134,35 +213,35 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
     const int sms = require_device();
     if (count == 0) return;
     const RowLayout lay = row_major(dense_pitch(w_pad));
-    if (kind == STORM_B200_KERNEL_MMA) {
-        static std::atomic<uint64_t> done_a{0}, done_b{0};
-        smem_attr_once(bb_mma_ts_kernel, (int)TS_SMEM_BYTES, done_a);
-        smem_attr_once(bb_mma_ts_long_kernel, (int)TS_SMEM_BYTES, done_b);
-        // stream-K only for a launch over the whole tile list, whose output
-        // triangle can be zeroed first for the partial-count atomics
+    // stream-K only for a launch over the whole tile list, whose output
+    // triangle can be zeroed first for the partial-count atomics
+    const bool whole_list = t0 == 0 && count == n_tiles;
+    if (kind == KIND_F4) {
+        static std::atomic<uint64_t> done{0};
+        smem_attr_once(bb_f4_kernel, (int)F4_SMEM_BYTES, done);
+        uint32_t pairs = std::min<uint32_t>(count, (uint32_t)std::max(1, sms / 2));
+        const uint32_t ks = whole_list ? f4_schedule(count, sms, w_pad, pairs, schedule) : 1;
+        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, pairs, st);
+        uint32_t blk_words = 0;
+        const CUtensorMap map = f4_row_map(dX, n, w_pad, lay, &blk_words);
+        SB_CUDA(launch_pairs(bb_f4_kernel, pairs, F4_THREADS, F4_SMEM_BYTES, st, map, blk_words, n, w_pad,
+                             (const uint2*)(d_tiles.p + t0), count, d_out, d_flags.p, ks));
+    } else if (kind == STORM_B200_KERNEL_MMA) {
+        static std::atomic<uint64_t> done{0};
+        smem_attr_once(bb_mma_ts_long_kernel, (int)TS_SMEM_BYTES, done);
         uint32_t grid = count < (uint32_t)sms ? count : (uint32_t)sms;
-        const uint32_t ks = (t0 == 0 && count == n_tiles) ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
+        const uint32_t ks = whole_list ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
         if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, grid, st);
-        const uint32_t smem = (uint64_t)w_pad * 64 <= TS_COALESCE_MAX_BITS ? TS_SMEM_BYTES : TS_SMEM_BYTES_LEAN;
-        if ((uint64_t)w_pad * 64 <= MMA_MAX_BITS)
-            bb_mma_ts_kernel<<<grid, TS_THREADS, smem, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count, d_out, d_flags.p,
-                                                             ks);
-        else
-            bb_mma_ts_long_kernel<<<grid, TS_THREADS, smem, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count, d_out,
-                                                                  d_flags.p, ks);
+        bb_mma_ts_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
+                                                                            d_out, d_flags.p, ks);
     } else if (kind == STORM_B200_KERNEL_MMA_DB) {
-        static std::atomic<uint64_t> done_a{0}, done_b{0};
-        smem_attr_once(bb_mma_ts2_kernel, (int)T2_SMEM_BYTES, done_a);
-        smem_attr_once(bb_mma_ts2_long_kernel, (int)T2_SMEM_BYTES, done_b);
+        static std::atomic<uint64_t> done{0};
+        smem_attr_once(bb_mma_ts2_long_kernel, (int)T2_SMEM_BYTES, done);
         uint32_t grid = count < (uint32_t)sms ? count : (uint32_t)sms;
-        const uint32_t ks = (t0 == 0 && count == n_tiles) ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
+        const uint32_t ks = whole_list ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
         if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, grid, st);
-        if ((uint64_t)w_pad * 64 <= MMA_MAX_BITS)
-            bb_mma_ts2_kernel<<<grid, T2_THREADS, T2_SMEM_BYTES, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count, d_out,
-                                                                      d_flags.p, ks);
-        else
-            bb_mma_ts2_long_kernel<<<grid, T2_THREADS, T2_SMEM_BYTES, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
-                                                                           d_out, d_flags.p, ks);
+        bb_mma_ts2_long_kernel<<<grid, T2_THREADS, T2_SMEM_BYTES, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
+                                                                       d_out, d_flags.p, ks);
     } else if (kind == STORM_B200_KERNEL_MMA_2CTA) {
         // CTA pairs (clusters of 2), one per two SMs, whole tiles round robin
         static std::atomic<uint64_t> done_a{0}, done_b{0};
@@ -171,23 +250,9 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
         const uint32_t pairs = std::max<uint32_t>(1u, std::min<uint32_t>(count, (uint32_t)sms / 2));
         const uint32_t smem = (uint64_t)w_pad * 64 <= TS_COALESCE_MAX_BITS ? C2_SMEM_BYTES
                                                                           : C2_SMEM_BYTES - C2_EPI_BYTES;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * pairs, 1, 1);
-        cfg.blockDim = dim3(C2_THREADS, 1, 1);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
         const uint2* tl = d_tiles.p + t0;
-        if ((uint64_t)w_pad * 64 <= MMA_MAX_BITS)
-            SB_CUDA(cudaLaunchKernelEx(&cfg, bb_mma_2cta_kernel, dX, n, w_pad, lay, tl, count, d_out, d_flags.p));
-        else
-            SB_CUDA(cudaLaunchKernelEx(&cfg, bb_mma_2cta_long_kernel, dX, n, w_pad, lay, tl, count, d_out, d_flags.p));
+        SB_CUDA(launch_pairs((uint64_t)w_pad * 64 <= MMA_MAX_BITS ? bb_mma_2cta_kernel : bb_mma_2cta_long_kernel, pairs,
+                             C2_THREADS, smem, st, dX, n, w_pad, lay, tl, count, d_out, d_flags.p));
     } else if (kind == STORM_B200_KERNEL_MMA_SS) {
         static std::atomic<uint64_t> done{0};
         smem_attr_once(bb_mma_kernel, (int)MMA_SMEM_BYTES, done);
@@ -221,7 +286,7 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
     SB_CUDA(cudaStreamSynchronize(st));
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.launches = 1;
-    log.kernel = kind;
+    log.kernel = reported;
     if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
     return f.sum;
 }
@@ -326,7 +391,7 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
     const int sms = require_device();
     const uint64_t bm = tile_rows_a(kind), bn = tile_rows_b(kind);
     const uint32_t wave = kind == STORM_B200_KERNEL_POPC        ? 2u * (uint32_t)sms
-                          : kind == STORM_B200_KERNEL_MMA_2CTA ? (uint32_t)sms / 2
+                          : kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4 ? (uint32_t)std::max(1, sms / 2)
                                                                : (uint32_t)sms;
     const auto panels = host_panels(n_tiles, wave);
     // first tile of each A block (the list is ordered by A block)
@@ -378,7 +443,7 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
     SB_CUDA(cudaStreamSynchronize(copy_st));
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.launches = (uint32_t)panels.size();
-    log.kernel = kind;
+    log.kernel = reported;
     if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
     if (copied_from != 0) fail(STORM_B200_ECUDA, "panel schedule left rows uncopied");
     return f.sum;
@@ -400,7 +465,8 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
 // ===================================================================
 namespace sb200 {
 
-constexpr uint32_t NOALLOC_MAX_TILES = 32768;   // 256 KiB of (bi, bj) pairs: up to 46080 rows
+constexpr uint64_t NOALLOC_MAX_ROWS = 46080;
+constexpr uint32_t NOALLOC_MAX_TILES = (NOALLOC_MAX_ROWS / F4_BM) * (NOALLOC_MAX_ROWS / F4_BM + 1) / 2;
 
 struct NoAllocScratch {
     DeviceFlags flags;
@@ -409,15 +475,13 @@ struct NoAllocScratch {
 
 static __device__ __align__(256) NoAllocScratch g_noalloc_scratch;
 
-// One thread per A block row bi writes its tiles (bi, bj), bj >= bi / 2,
-// at offset bi * nbj - sum_{k < bi} floor(k / 2).
-__global__ void noalloc_tiles_kernel(NoAllocScratch* s, uint32_t nbi, uint32_t nbj) {
+// One thread per A block row bi writes its tiles (bi, bj), bj >= bi, at
+// offset bi * nb - bi (bi - 1) / 2.
+__global__ void noalloc_tiles_kernel(NoAllocScratch* s, uint32_t nb) {
     const uint32_t bi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (bi >= nbi) return;
-    const uint64_t m = bi / 2;
-    const uint64_t below = (bi % 2 == 0) ? m * (m - (m > 0 ? 1 : 0)) : m * m;
-    uint64_t t = (uint64_t)bi * nbj - below;
-    for (uint32_t bj = bi / 2; bj < nbj; ++bj, ++t) s->tiles[t] = make_uint2(bi, bj);
+    if (bi >= nb) return;
+    uint64_t t = (uint64_t)bi * nb - (uint64_t)bi * (bi - (bi > 0)) / 2;
+    for (uint32_t bj = bi; bj < nb; ++bj, ++t) s->tiles[t] = make_uint2(bi, bj);
 }
 
 }  // namespace sb200
@@ -435,10 +499,7 @@ extern "C" int STORM_contig_pairw_intersect_matrix_noalloc(const uint64_t* d_row
     if (row_bits > MMA_MAX_BITS) return STORM_B200_ELIMIT;
     const uint64_t need = n_rows * (n_rows + 1) / 2;
     if (d_out != NULL && out_len < need) return STORM_B200_ESIZE;
-    const uint32_t nbi = (uint32_t)((n_rows + TS_BM - 1) / TS_BM), nbj = (uint32_t)((n_rows + TS_BN - 1) / TS_BN);
-    uint64_t n_tiles = 0;
-    for (uint32_t bi = 0; bi < nbi; ++bi) n_tiles += nbj - bi / 2;
-    if (n_tiles > NOALLOC_MAX_TILES) return STORM_B200_ELIMIT;
+    if (n_rows > NOALLOC_MAX_ROWS) return STORM_B200_ELIMIT;
 
     // Once per device, with that device current: the device address of the
     // scratch array, and the kernel's shared-memory opt-in.
@@ -455,8 +516,8 @@ extern "C" int STORM_contig_pairw_intersect_matrix_noalloc(const uint64_t* d_row
                 return STORM_B200_ECUDA;
             void* p = nullptr;
             if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) return STORM_B200_ECUDA;
-            if (cudaFuncSetAttribute(bb_mma_ts_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)TS_SMEM_BYTES) != cudaSuccess)
+            if (cudaFuncSetAttribute(bb_f4_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)F4_SMEM_BYTES) != cudaSuccess)
                 return STORM_B200_ECUDA;
             scratch_of[dev] = p;
         }
@@ -469,15 +530,19 @@ extern "C" int STORM_contig_pairw_intersect_matrix_noalloc(const uint64_t* d_row
     if (cudaPeekAtLastError() != cudaSuccess) return STORM_B200_ECUDA;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (cudaMemsetAsync(&scratch->flags, 0, sizeof(DeviceFlags), st) != cudaSuccess) return STORM_B200_ECUDA;
-    noalloc_tiles_kernel<<<(nbi + 127) / 128, 128, 0, st>>>(scratch, nbi, nbj);
-    const uint32_t grid = n_tiles < (uint64_t)sms ? (uint32_t)n_tiles : (uint32_t)sms;
-    // The same epilogue rule as the allocating path: rows up to
-    // TS_COALESCE_MAX_BITS stage their counts through shared memory.
-    const uint32_t smem =
-        (uint64_t)row_pitch_words * 64 <= TS_COALESCE_MAX_BITS ? TS_SMEM_BYTES : TS_SMEM_BYTES_LEAN;
-    bb_mma_ts_kernel<<<grid, TS_THREADS, smem, st>>>(d_rows, (uint32_t)n_rows, row_pitch_words,
-                                                      row_major(row_pitch_words), scratch->tiles,
-                                                      (uint32_t)n_tiles, d_out, &scratch->flags, 1u);
+    const uint32_t nb = (uint32_t)((n_rows + F4_BM - 1) / F4_BM), n_pair_tiles = nb * (nb + 1) / 2;
+    noalloc_tiles_kernel<<<(nb + 127) / 128, 128, 0, st>>>(scratch, nb);
+    const uint32_t pairs = std::min<uint32_t>(n_pair_tiles, (uint32_t)std::max(1, sms / 2));
+    uint32_t blk_words = 0;
+    CUtensorMap map;
+    try {
+        map = f4_row_map(d_rows, n_rows, row_pitch_words, row_major(row_pitch_words), &blk_words);
+    } catch (const Status&) {
+        cudaStreamSynchronize(st);
+        return STORM_B200_ECUDA;
+    }
+    launch_pairs(bb_f4_kernel, pairs, F4_THREADS, F4_SMEM_BYTES, st, map, blk_words, (uint32_t)n_rows, row_pitch_words,
+                 (const uint2*)scratch->tiles, n_pair_tiles, d_out, &scratch->flags, 1u);
     if (cudaGetLastError() != cudaSuccess) {
         cudaStreamSynchronize(st);   // nothing already queued may still write d_out after the return
         return STORM_B200_ECUDA;
@@ -677,22 +742,27 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
     const int kind = prepare(n, row_bits, kernel_pref, st);
     SB_CUDA(cudaEventRecord(log.ev0, st));
     uint64_t found = 0;
-    if (kind == STORM_B200_KERNEL_MMA) {
-        static std::atomic<uint64_t> done_a{0}, done_b{0};
-        smem_attr_once(bb_mma_ts_thresh_kernel, (int)TS_SMEM_BYTES, done_a);
-        smem_attr_once(bb_mma_ts_thresh_long_kernel, (int)TS_SMEM_BYTES, done_b);
+    if (kind == STORM_B200_KERNEL_MMA || kind == KIND_F4) {
         SB_CUDA(cudaMemsetAsync(d_found.p, 0, sizeof(unsigned long long), st));
         row_popcount_kernel<<<(uint32_t)std::min<uint64_t>((n + 7) / 8, (uint64_t)sms * 16), 256, 0, st>>>(
             dX, n, w_pad, dense_pitch(w_pad), d_card.p);
         const TsThresh th{d_card.p, t, d_pairs, d_cnts, (unsigned long long)cap, d_found.p};
-        const uint32_t grid = n_tiles < (uint32_t)sms ? n_tiles : (uint32_t)sms;
         const RowLayout lay = row_major(dense_pitch(w_pad));
-        if ((uint64_t)w_pad * 64 <= MMA_MAX_BITS)
-            bb_mma_ts_thresh_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(dX, (uint32_t)n, w_pad, lay, d_tiles.p,
-                                                                                   n_tiles, d_flags.p, th);
-        else
+        if (kind == KIND_F4) {
+            static std::atomic<uint64_t> done{0};
+            smem_attr_once(bb_f4_thresh_kernel, (int)F4_SMEM_BYTES, done);
+            const uint32_t pairs = std::min<uint32_t>(n_tiles, (uint32_t)std::max(1, sms / 2));
+            uint32_t blk_words = 0;
+            const CUtensorMap map = f4_row_map(dX, n, w_pad, lay, &blk_words);
+            SB_CUDA(launch_pairs(bb_f4_thresh_kernel, pairs, F4_THREADS, F4_SMEM_BYTES, st, map, blk_words, (uint32_t)n,
+                                 w_pad, (const uint2*)d_tiles.p, n_tiles, d_flags.p, th));
+        } else {
+            static std::atomic<uint64_t> done{0};
+            smem_attr_once(bb_mma_ts_thresh_long_kernel, (int)TS_SMEM_BYTES, done);
+            const uint32_t grid = n_tiles < (uint32_t)sms ? n_tiles : (uint32_t)sms;
             bb_mma_ts_thresh_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(
                 dX, (uint32_t)n, w_pad, lay, d_tiles.p, n_tiles, d_flags.p, th);
+        }
         SB_CUDA(cudaGetLastError());
         unsigned long long h = 0;
         SB_CUDA(cudaMemcpyAsync(&h, d_found.p, sizeof(h), cudaMemcpyDeviceToHost, st));
@@ -710,7 +780,7 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
     SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
     SB_CUDA(cudaStreamSynchronize(st));
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
-    log.kernel = kind;
+    log.kernel = reported;
     if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
     if (sum) *sum = f.sum;
     return found;
@@ -724,29 +794,40 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
 // ===================================================================
 namespace sb200 {
 
-void build_mma_tiles(std::vector<uint2>& t, uint64_t n) { build_tiles(t, n, STORM_B200_KERNEL_MMA); }
+// Gathered rows of more than 2^24 bits: the 8-bit kernel.
+static bool rows_f4(uint32_t w_pad) { return (uint64_t)w_pad * 64 <= F4_MAX_BITS; }
+
+uint32_t rows_block_a(uint32_t w_pad) { return rows_f4(w_pad) ? F4_BM : MMA_BM; }
+
+void build_rows_tiles(std::vector<uint2>& t, uint64_t n, uint32_t w_pad) {
+    build_tiles(t, n, rows_f4(w_pad) ? KIND_F4 : STORM_B200_KERNEL_MMA);
+}
 
 void launch_ts_rows(const uint64_t* X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* tiles,
                     uint32_t n_tiles, uint32_t* out, DeviceFlags* flags, const uint32_t* row_map, uint64_t n_out, cudaStream_t st,
                     bool out_zeroed) {
     const int sms = require_device();
     if (n_tiles == 0) return;
-    static std::atomic<uint64_t> done_a{0}, done_b{0};
-    smem_attr_once(bb_mma_ts_rows_kernel, (int)TS_SMEM_BYTES, done_a);
-    smem_attr_once(bb_mma_ts_rows_long_kernel, (int)TS_SMEM_BYTES, done_b);
     if ((uint64_t)w_pad * 64 > MMA_MAX_BITS_W4) fail(STORM_B200_ELIMIT, "dense block rows longer than 2^27 bits");
     // With stream-K the partial counts are added into out, so the whole
     // triangle is zeroed first; the other phases write their own pairs after.
+    const bool f4 = rows_f4(w_pad);
     uint32_t grid = 0;
-    const uint32_t ks = ts_schedule(n_tiles, sms, w_pad, grid);
+    const uint32_t ks = f4 ? f4_schedule(n_tiles, sms, w_pad, grid) : ts_schedule(n_tiles, sms, w_pad, grid);
     if (ks != 1 && out && !out_zeroed) SB_CUDA(cudaMemsetAsync(out, 0, tri_size(n_out) * sizeof(uint32_t), st));
-    const uint32_t smem = (uint64_t)w_pad * 64 <= TS_COALESCE_MAX_BITS ? TS_SMEM_BYTES : TS_SMEM_BYTES_LEAN;
-    if ((uint64_t)w_pad * 64 <= MMA_MAX_BITS)
-        bb_mma_ts_rows_kernel<<<grid, TS_THREADS, smem, st>>>(X, n, w_pad, lay, tiles, n_tiles, out, flags, row_map, n_out,
-                                                              ks);
-    else
-        bb_mma_ts_rows_long_kernel<<<grid, TS_THREADS, smem, st>>>(X, n, w_pad, lay, tiles, n_tiles, out, flags, row_map,
-                                                                   n_out, ks);
+    if (f4) {
+        static std::atomic<uint64_t> done{0};
+        smem_attr_once(bb_f4_rows_kernel, (int)F4_SMEM_BYTES, done);
+        uint32_t blk_words = 0;
+        const CUtensorMap map = f4_row_map(X, n, w_pad, lay, &blk_words);
+        SB_CUDA(launch_pairs(bb_f4_rows_kernel, grid, F4_THREADS, F4_SMEM_BYTES, st, map, blk_words, n, w_pad, tiles,
+                             n_tiles, out, flags, ks, row_map, n_out));
+    } else {
+        static std::atomic<uint64_t> done{0};
+        smem_attr_once(bb_mma_ts_rows_long_kernel, (int)TS_SMEM_BYTES, done);
+        bb_mma_ts_rows_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(X, n, w_pad, lay, tiles, n_tiles, out,
+                                                                                flags, row_map, n_out, ks);
+    }
     SB_CUDA(cudaGetLastError());
 }
 

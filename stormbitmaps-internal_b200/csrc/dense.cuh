@@ -25,6 +25,7 @@ struct DenseEngine {
     DevBuf<uint2> d_tiles;
     uint64_t tiles_n = ~0ull;
     int tiles_kind = -1;
+    int reported = 0;   // the kernel choice a call reports (tiles_kind is what runs)
     uint32_t n_tiles = 0;
     DevBuf<DeviceFlags> d_flags;
     LaunchLog log;
@@ -80,10 +81,12 @@ struct DenseEngine {
 
 inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 
-// Tiles (bi, bj) of 128 x 256 pairs covering the triangle of n rows.
-void build_mma_tiles(std::vector<uint2>& t, uint64_t n);
-// The tile list of a bitmap x bitmap kernel (STORM_B200_KERNEL_*): 128 x 256
-// (tcgen05), 128 x 192 (double-buffered tcgen05) or 128 x 128 (POPC) tiles
+// The 4-bit tensor-core kernel (bb_f4.cuh), which MMA and MMA_DB run on up to
+// 2^24-bit rows; not a value of the interface.
+constexpr int KIND_F4 = 64;
+// The tile list of a bitmap x bitmap kernel (STORM_B200_KERNEL_*, KIND_F4):
+// 256 x 256 (CTA pairs), 128 x 256 (tcgen05), 128 x 192 (double-buffered
+// tcgen05) or 128 x 128 (POPC) tiles
 // covering every pair i <= j < n once, ordered by A block.
 void build_tiles(std::vector<uint2>& t, uint64_t n, int kind);
 // Rows per A block / per B block of a kernel's tiles.
@@ -97,6 +100,11 @@ std::vector<std::pair<uint32_t, uint32_t>> host_panels(uint32_t n_tiles, uint32_
 constexpr uint64_t TC_MAX_ROW_BITS = 1ull << 27;
 // ... and the shared-memory form (8-byte weight cycle only).
 constexpr uint64_t TC_SS_MAX_ROW_BITS = 1ull << 23;
+
+// Tiles of launch_ts_rows covering the triangle of n gathered rows of w_pad
+// words, and the rows of their A blocks (B blocks have 256).
+void build_rows_tiles(std::vector<uint2>& t, uint64_t n, uint32_t w_pad);
+uint32_t rows_block_a(uint32_t w_pad);
 
 // Tensor-core kernel over n gathered rows X (>= roundup(n, 256) rows of
 // w_pad words in layout `lay`); count (i, j) lands at the packed index of

@@ -585,7 +585,7 @@ static void rows_run(STORM_rows_t* r, int policy, uint32_t tile, int fixed_cell,
         r->d_dflags.reserve(1);
         if (r->dtiles_n != nd) {
             std::vector<uint2> tl;
-            build_mma_tiles(tl, nd);
+            build_rows_tiles(tl, nd, w_pad_d);
             r->d_dtiles.reserve(tl.size());
             SB_CUDA(cudaMemcpyAsync(r->d_dtiles.p, tl.data(), tl.size() * sizeof(uint2), cudaMemcpyHostToDevice, st));
             SB_CUDA(cudaStreamSynchronize(st));
