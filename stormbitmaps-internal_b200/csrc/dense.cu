@@ -164,7 +164,20 @@ void build_tiles(std::vector<uint2>& t, uint64_t n, int kind) {
     }
 }
 
-int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStream_t st) {
+// A 256 x 256 tile list in bands of F4_BAND A blocks, down each band's columns:
+// the tiles that run at one time then read about as many A blocks as B blocks
+// (8 + 9 for the 74 CTA pairs) instead of one A block and 74 B blocks, and the
+// rows they share come from L2.
+constexpr uint32_t F4_BAND = 8;
+
+static void band_tiles(std::vector<uint2>& t) {
+    std::stable_sort(t.begin(), t.end(), [](const uint2& a, const uint2& b) {
+        const uint32_t ba = a.x / F4_BAND, bb = b.x / F4_BAND;
+        return ba != bb ? ba < bb : a.y != b.y ? a.y < b.y : a.x < b.x;
+    });
+}
+
+int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, bool rows_in_order, cudaStream_t st) {
     if (n > 0xFFFFFFFFull) fail(STORM_B200_ELIMIT, "more than 2^32 rows");
     int kind = kernel_pref;
     // Automatic choice: tensor cores up to 2^27-bit rows (both choices run the
@@ -180,14 +193,17 @@ int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStr
         fail(STORM_B200_ELIMIT, "shared-memory tensor-core kernel is exact only for rows of at most 2^23 bits");
     reported = kind;
     kind = exec_kind(kind, row_bits);
-    if (tiles_n != n || tiles_kind != kind) {
+    const bool banded = kind == KIND_F4 && !rows_in_order;
+    if (tiles_n != n || tiles_kind != kind || tiles_banded != banded) {
         build_tiles(h_tiles, n, kind);
+        if (banded) band_tiles(h_tiles);
         d_tiles.reserve(h_tiles.size());
         SB_CUDA(cudaMemcpyAsync(d_tiles.p, h_tiles.data(), h_tiles.size() * sizeof(uint2), cudaMemcpyHostToDevice,
                                 st));
         n_tiles = (uint32_t)h_tiles.size();
         tiles_n = n;
         tiles_kind = kind;
+        tiles_banded = banded;
     }
     d_flags.reserve(1);
     SB_CUDA(cudaMemsetAsync(d_flags.p, 0, sizeof(DeviceFlags), st));
@@ -196,13 +212,14 @@ int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStr
 }
 
 // Stream-K over the whole cached list (TsSched, k_splits 0): tiles from
-// W = floor(tiles / grid) x grid on add into the output, and every one of them
-// has its A block at or past tile W's (the list is ordered by A block), so
-// zeroing the triangle from that block's first row on covers them.
+// W = floor(tiles / grid) x grid on add into the output: the triangle is zeroed
+// from the first row of the lowest A block among them.
 void DenseEngine::zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st) {
     const uint32_t whole = (n_tiles / grid) * grid;
     if (whole >= n_tiles) return;
-    const uint64_t r0 = (uint64_t)h_tiles[whole].x * tile_rows_a(tiles_kind);
+    uint32_t lowest = h_tiles[whole].x;
+    for (uint32_t t = whole; t < n_tiles; ++t) lowest = std::min(lowest, h_tiles[t].x);
+    const uint64_t r0 = (uint64_t)lowest * tile_rows_a(tiles_kind);
     const uint64_t e0 = r0 * n - (r0 * (r0 - 1)) / 2;          // tri_index(n, r0, r0)
     SB_CUDA(cudaMemsetAsync(d_out + e0, 0, (tri_size(n) - e0) * sizeof(uint32_t), st));
 }
@@ -277,7 +294,7 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
         log.last_ms = 0.f;
         return 0;
     }
-    const int kind = prepare(n, row_bits, kernel_pref, st);
+    const int kind = prepare(n, row_bits, kernel_pref, false, st);
     SB_CUDA(cudaEventRecord(log.ev0, st));
     launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
     SB_CUDA(cudaEventRecord(log.ev1, st));
@@ -335,7 +352,7 @@ uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad
         log.last_ms = 0.f;
         return 0;
     }
-    const int kind = prepare(n, row_bits, kernel_pref, st);
+    const int kind = prepare(n, row_bits, kernel_pref, true, st);
     return panels_to_host(dX, n, w_pad, kind, d_out, host_out, st, copy_st, 0);
 }
 
@@ -348,7 +365,7 @@ uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad,
         log.last_ms = 0.f;
         return 0;
     }
-    const int kind = prepare(n, row_bits, kernel_pref, st);
+    const int kind = prepare(n, row_bits, kernel_pref, true, st);
     // What the copies do not cover reads as zero: the row pitch's padding
     // words and the rows [n, n_pad) that whole 128 x 256 tiles read.
     const uint64_t n_pad = round_up(n, 256), pitch = dense_pitch(w_pad);
@@ -739,7 +756,7 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
     if ((kernel_pref == STORM_B200_KERNEL_AUTO || kernel_pref == STORM_B200_KERNEL_MMA_DB) &&
         row_bits <= MMA_MAX_BITS_W4)
         kernel_pref = STORM_B200_KERNEL_MMA;
-    const int kind = prepare(n, row_bits, kernel_pref, st);
+    const int kind = prepare(n, row_bits, kernel_pref, false, st);
     SB_CUDA(cudaEventRecord(log.ev0, st));
     uint64_t found = 0;
     if (kind == STORM_B200_KERNEL_MMA || kind == KIND_F4) {

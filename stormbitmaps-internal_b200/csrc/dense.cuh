@@ -25,6 +25,7 @@ struct DenseEngine {
     DevBuf<uint2> d_tiles;
     uint64_t tiles_n = ~0ull;
     int tiles_kind = -1;
+    bool tiles_banded = false;
     int reported = 0;   // the kernel choice a call reports (tiles_kind is what runs)
     uint32_t n_tiles = 0;
     DevBuf<DeviceFlags> d_flags;
@@ -69,7 +70,9 @@ struct DenseEngine {
     DevBuf<unsigned long long> d_found;
 
    private:
-    int prepare(uint64_t n, uint64_t row_bits, int kernel_pref, cudaStream_t st);
+    // rows_in_order: the tiles ordered by A block, as the host-output panels
+    // need them; otherwise in the order that suits L2.
+    int prepare(uint64_t n, uint64_t row_bits, int kernel_pref, bool rows_in_order, cudaStream_t st);
     void launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pad, uint32_t t0, uint32_t count,
                 uint32_t* d_out, cudaStream_t st);
     void zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st);
