@@ -6,6 +6,7 @@
 #include "bb_mma_ts2.cuh"
 #include "bb_mma_2cta.cuh"
 #include "bb_f4.cuh"
+#include "colsum.cuh"
 
 #include <algorithm>
 #include <mutex>
@@ -164,6 +165,14 @@ void build_tiles(std::vector<uint2>& t, uint64_t n, int kind) {
     }
 }
 
+// Automatic choice: tensor cores up to 2^27-bit rows (both choices run the
+// 4-bit kernel up to 2^24 bits and differ past it), CUDA-core POPC beyond.
+static int auto_kind(uint64_t row_bits) {
+    return row_bits <= DB_AUTO_MAX_BITS   ? STORM_B200_KERNEL_MMA_DB
+           : row_bits <= MMA_MAX_BITS_W4 ? STORM_B200_KERNEL_MMA
+                                         : STORM_B200_KERNEL_POPC;
+}
+
 // A 256 x 256 tile list in bands of F4_BAND A blocks, down each band's columns:
 // the tiles that run at one time then read about as many A blocks as B blocks
 // (8 + 9 for the 74 CTA pairs) instead of one A block and 74 B blocks, and the
@@ -180,12 +189,7 @@ static void band_tiles(std::vector<uint2>& t) {
 int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, bool rows_in_order, cudaStream_t st) {
     if (n > 0xFFFFFFFFull) fail(STORM_B200_ELIMIT, "more than 2^32 rows");
     int kind = kernel_pref;
-    // Automatic choice: tensor cores up to 2^27-bit rows (both choices run the
-    // 4-bit kernel up to 2^24 bits and differ past it), CUDA-core POPC beyond.
-    if (kind == STORM_B200_KERNEL_AUTO)
-        kind = row_bits <= DB_AUTO_MAX_BITS    ? STORM_B200_KERNEL_MMA_DB
-               : row_bits <= MMA_MAX_BITS_W4 ? STORM_B200_KERNEL_MMA
-                                             : STORM_B200_KERNEL_POPC;
+    if (kind == STORM_B200_KERNEL_AUTO) kind = auto_kind(row_bits);
     if ((kind == STORM_B200_KERNEL_MMA || kind == STORM_B200_KERNEL_MMA_DB || kind == STORM_B200_KERNEL_MMA_2CTA) &&
         row_bits > MMA_MAX_BITS_W4)
         fail(STORM_B200_ELIMIT, "tensor-core kernel is exact only for rows of at most 2^27 bits");
@@ -294,6 +298,8 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
         log.last_ms = 0.f;
         return 0;
     }
+    // The sum alone, no kernel asked for: from the columns' counts.
+    if (!d_out && kernel_pref == STORM_B200_KERNEL_AUTO) return run_sum(dX, n, w_pad, row_bits, st);
     const int kind = prepare(n, row_bits, kernel_pref, false, st);
     SB_CUDA(cudaEventRecord(log.ev0, st));
     launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
@@ -305,6 +311,40 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
     log.launches = 1;
     log.kernel = reported;
     if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
+    return f.sum;
+}
+
+uint64_t DenseEngine::run_sum(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, cudaStream_t st) {
+    const int sms = require_device();
+    const uint32_t strip = std::min<uint32_t>(w_pad, COLSUM_STRIP);
+    d_hist.reserve(64ull * strip);
+    d_flags.reserve(1);
+    log.ensure();
+    SB_CUDA(cudaMemsetAsync(d_flags.p, 0, sizeof(DeviceFlags), st));
+    SB_CUDA(cudaEventRecord(log.ev0, st));
+    log.launches = 0;
+    for (uint32_t w0 = 0; w0 < w_pad; w0 += strip) {
+        const uint32_t words = std::min(strip, w_pad - w0);
+        const uint32_t gx = (words + COLSUM_WORDS - 1) / COLSUM_WORDS;
+        // about four blocks per SM: enough loads in flight, while a block's
+        // fixed cost (the planes of 2048 columns into counts) stays below its rows'
+        const uint64_t splits = std::max<uint64_t>(1, (uint64_t)sms * 4 / gx);
+        const uint64_t per = std::min<uint64_t>(COLSUM_WARPS * COLSUM_WARP_ROWS,
+                                                round_up((n + splits - 1) / splits, 8 * COLSUM_WARPS));
+        SB_CUDA(cudaMemsetAsync(d_hist.p, 0, 64ull * words * sizeof(uint32_t), st));
+        column_counts_kernel<<<dim3(gx, (uint32_t)((n + per - 1) / per)), COLSUM_WARPS * 32, 0, st>>>(
+            dX, n, dense_pitch(w_pad), w0, words, per, d_hist.p);
+        pairs_of_counts_kernel<<<(uint32_t)std::min<uint64_t>((64ull * words + 255) / 256, (uint64_t)sms * 4), 256, 0,
+                                 st>>>(d_hist.p, 64ull * words, &d_flags.p->sum);
+        SB_CUDA(cudaGetLastError());
+        log.launches += 2;
+    }
+    SB_CUDA(cudaEventRecord(log.ev1, st));
+    DeviceFlags f;
+    SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
+    SB_CUDA(cudaStreamSynchronize(st));
+    SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
+    log.kernel = auto_kind(row_bits);
     return f.sum;
 }
 

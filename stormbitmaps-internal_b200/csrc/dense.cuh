@@ -38,7 +38,8 @@ struct DenseEngine {
     }
 
     // Returns the sum over i < j; writes the packed upper triangle to d_out
-    // when non-null.  `row_bits` is the logical row length (decides whether
+    // when non-null (a sum alone under the automatic kernel choice comes from
+    // the columns' counts, without a pair).  `row_bits` is the logical row length (decides whether
     // the exact tensor-core kernel applies).  Synchronous.
     uint64_t run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, uint32_t* d_out,
                  int kernel_pref, cudaStream_t st);
@@ -66,13 +67,14 @@ struct DenseEngine {
     uint64_t run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, int kernel_pref,
                            double t, uint2* d_pairs, uint32_t* d_cnts, uint64_t cap, uint64_t* sum,
                            cudaStream_t st);
-    DevBuf<uint32_t> d_card, d_scratch_tri;
+    DevBuf<uint32_t> d_card, d_scratch_tri, d_hist;
     DevBuf<unsigned long long> d_found;
 
    private:
     // rows_in_order: the tiles ordered by A block, as the host-output panels
     // need them; otherwise in the order that suits L2.
     int prepare(uint64_t n, uint64_t row_bits, int kernel_pref, bool rows_in_order, cudaStream_t st);
+    uint64_t run_sum(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, cudaStream_t st);
     void launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pad, uint32_t t0, uint32_t count,
                 uint32_t* d_out, cudaStream_t st);
     void zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st);
