@@ -27,10 +27,11 @@
 // bits x 128 rows, one per operand), warp 17 owns TMEM and, in the even CTA of
 // the pair, issues the MMAs, warps 18-25 drain the accumulator.  TMEM:
 // accumulator [0, 256), three A stages of 64 columns, scale factors at 480.
-// Rows of at most 65535 bits: the drain warps put their counts into shared
-// memory as 16-bit numbers, free the accumulator, and store them while the
-// next tile computes; longer rows store as they read (their tiles last long
-// enough).  Every wait is bounded (2 s), as in the other tensor-core kernels.
+// The drain warps put their counts into shared memory as 16-bit numbers, free
+// the accumulator, and store them while the next tile computes; a block that
+// holds a count past 65535 is read again and stored from tensor memory (its
+// tile lasts long enough).  Every wait is bounded (2 s), as in the other
+// tensor-core kernels.
 //
 // tiles[t] = (bi, bj): rows [256 bi, +256) x rows [256 bj, +256); CTA r of the
 // pair takes A rows 256 bi + 128 r .. and expands B rows 256 bj + 128 r ...
@@ -58,7 +59,6 @@ constexpr uint32_t F4_SMEM_BYTES = F4_OFF_CTL + 256 + 1024;
 constexpr int F4_B_WARP0 = 8, F4_TMA_WARP = 16, F4_MMA_WARP = 17, F4_EPI_WARP0 = 18;
 constexpr int F4_THREADS = (F4_EPI_WARP0 + (int)F4_EPI_WARPS) * 32;   // 832
 constexpr uint32_t F4_A_COL0 = 256, F4_SF_COL = 480;
-constexpr uint32_t F4_PACK_MAX_BITS = 65535;               // counts fit 16 bits
 // Longest K range one accumulator counts exactly (fp32 integers).
 constexpr uint64_t F4_MAX_BITS = 1ull << 24;
 static_assert(F4_SMEM_BYTES <= 232448, "shared memory of one CTA");
@@ -139,14 +139,14 @@ __device__ __forceinline__ uint4 f4_expand_b(uint32_t w) {
     return make_uint4((w << 2) & 0x44444444u, w & 0x22222222u, (w >> 2) & 0x11111111u, (w >> 1) & 0x44444444u);
 }
 
-template <bool kCluster>
+// CTA scope, as the arrivals (an acquire at cluster scope costs the MMA thread
+// 290 clocks a stage).
 __device__ __forceinline__ bool f4_wait(uint32_t bar, uint32_t parity, F4Ctl* ctl, DeviceFlags* flags, uint32_t site,
                                         bool drain = false) {
-    auto poll = [&]() { return kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-    if (poll()) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     const uint64_t t0 = globaltimer_ns();
     for (;;) {
-        if (poll()) return true;
+        if (mbar_try_wait(bar, parity)) return true;
         if (!drain && ctl->abort) return false;
         if (globaltimer_ns() - t0 > WAIT_LIMIT_NS) {
             atomicCAS(&flags->error, 0u, site);
@@ -164,70 +164,130 @@ struct F4Out {
     bool partial;                   // one K segment's share: added
 };
 
+// One count to its place: stored (how 1), added (how 2), or not at all (how 0
+// or !want).  Predicated, since the wanted lanes differ from row to row at the
+// diagonal and a branch per count costs more than the count.
+__device__ __forceinline__ void f4_put(uint32_t* dst, uint32_t v, bool want, uint32_t how) {
+    asm volatile(
+        "{\n\t.reg .pred st, ad;\n\t"
+        "setp.eq.u32 st, %2, 1;\n\t"
+        "setp.eq.u32 ad, %2, 2;\n\t"
+        "@st st.global.cs.u32 [%0], %1;\n\t"
+        "@ad red.global.add.u32 [%0], %1;\n\t}" ::"l"(dst),
+        "r"(v), "r"(want ? how : 0u)
+        : "memory");
+}
+
+// Stores a block of 32 rows x 32 NC columns from (i0, j0) on, 32 consecutive
+// counts of a row per instruction: at(rr, c) is this lane's count of row rr,
+// column 32 c + lane.  Returns its share of the sum over i < j.  The diagonal,
+// the last rows and row maps take a branch-free loop: the drain of a launch's
+// last tile is hidden by nothing, and with an index and a branch per count it
+// took 12 us (100 x 1000 bits: 23 -> 15 us of kernel).
+template <bool kRowMap, uint32_t NC, class At>
+__device__ __forceinline__ unsigned long long f4_emit(const F4Out& o, int lane, uint64_t i0, uint64_t j0, At at) {
+    if (i0 >= o.n || j0 >= o.n || i0 >= j0 + 32 * NC) return 0;
+    constexpr uint32_t RB = 8 / NC;                        // rows per batch: their counts are read before any store
+    const uint32_t rows = o.n - i0 < 32 ? (uint32_t)(o.n - i0) : 32u;
+    const uint32_t how = !o.out ? 0u : o.partial ? 2u : 1u;
+    // column col of row rr is wanted from the diagonal (lo) to the last row (cols)
+    const int32_t cols = o.n - j0 < 32 * NC ? (int32_t)(o.n - j0) : (int32_t)(32 * NC);
+    int32_t lo = (int64_t)i0 - (int64_t)j0 < -32 ? -32 : (int32_t)((int64_t)i0 - (int64_t)j0);
+    uint32_t s = 0;                                        // at most 128 counts of at most 2^24
+    // row maps: entry (a, b), a < b, is at base(a) + b, base(a) = tri_index(n, a, a) - a
+    auto base = [&](uint32_t a) { return tri_index(o.n_out, a, a) - a; };
+    uint32_t cm[NC], rm_l = ~0u;
+    uint64_t cb[NC], rb_l = 0;
+    // else: row i + 1 starts n - i entries after row i, one column later
+    uint64_t step = o.n - i0 - 1;
+    uint32_t* p = o.out + (tri_index(o.n, i0, i0) - i0 + j0 + lane);
+    if (!kRowMap && lo + 31 < 0 && cols == (int32_t)(32 * NC) && rows == 32 && how) {   // an inner block: no tests
+        if (how == 1) {
+#pragma unroll 4
+            for (uint32_t rr = 0; rr < 32; ++rr) {
+#pragma unroll
+                for (uint32_t c = 0; c < NC; ++c) {
+                    const uint32_t v = at(rr, c);
+                    __stcs(p + 32 * c, v);
+                    s += v;
+                }
+                p += step--;
+            }
+        } else {
+#pragma unroll 4
+            for (uint32_t rr = 0; rr < 32; ++rr) {
+#pragma unroll
+                for (uint32_t c = 0; c < NC; ++c) {
+                    const uint32_t v = at(rr, c);
+                    atomicAdd(p + 32 * c, v);
+                    s += v;
+                }
+                p += step--;
+            }
+        }
+        return s;
+    }
+    if (kRowMap) {
+#pragma unroll
+        for (uint32_t c = 0; c < NC; ++c) {
+            const int32_t col = (int32_t)(32 * c) + lane;
+            cm[c] = col < cols ? o.row_map[j0 + col] : ~0u;
+            cb[c] = cm[c] != ~0u ? base(cm[c]) : 0;
+        }
+        if (lane < (int)rows) rm_l = o.row_map[i0 + lane];
+        if (rm_l != ~0u) rb_l = base(rm_l);
+    }
+#pragma unroll 1
+    for (uint32_t r0 = 0; r0 < rows; r0 += RB) {
+        uint32_t v[RB][NC];
+#pragma unroll
+        for (uint32_t q = 0; q < RB; ++q)
+#pragma unroll
+            for (uint32_t c = 0; c < NC; ++c) v[q][c] = at(r0 + q, c);
+#pragma unroll
+        for (uint32_t q = 0; q < RB; ++q, ++lo) {
+            uint32_t rm = 0;
+            uint64_t rb = 0;
+            if (kRowMap) {
+                rm = __shfl_sync(0xffffffffu, rm_l, r0 + q);
+                rb = __shfl_sync(0xffffffffu, rb_l, r0 + q);
+            }
+            const bool row_ok = r0 + q < rows && (!kRowMap || rm != ~0u);
+#pragma unroll
+            for (uint32_t c = 0; c < NC; ++c) {
+                const int32_t col = (int32_t)(32 * c) + lane;
+                const bool want = row_ok && col >= lo && col < cols && (!kRowMap || cm[c] != ~0u);
+                uint32_t* dst = kRowMap ? o.out + (rm < cm[c] ? rb + cm[c] : cb[c] + rm) : p + 32 * c;
+                f4_put(dst, v[q][c], want, how);
+                s += want && col > lo ? v[q][c] : 0u;
+            }
+            p += step--;
+        }
+    }
+    return s;
+}
+
 // A 32 x 32 block of counts held lane = row i0 + lane, r[c] = column j0 + c:
-// through the warp's shared-memory block (16-byte chunks XOR-swizzled by row),
-// so that one store instruction writes 32 consecutive counts of one row.
-// Returns this lane's share of the sum over i < j.
+// through the warp's shared-memory block (16-byte chunks XOR-swizzled by row).
 template <bool kRowMap>
 __device__ __forceinline__ unsigned long long f4_store_block(const F4Out& o, uint32_t* buf, int lane, uint64_t i0,
                                                              uint64_t j0, const uint32_t (&r)[32]) {
-    if (i0 >= o.n || j0 >= o.n || i0 > j0 + 31) return 0;
 #pragma unroll
     for (uint32_t k = 0; k < 8; ++k)
         *reinterpret_cast<uint4*>(buf + lane * 32 + ((k ^ (lane & 7)) << 2)) =
             make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
     __syncwarp();
-    const uint64_t j = j0 + lane;
-    uint32_t s = 0;
-    unsigned long long local = 0;
-    auto at = [&](uint32_t rr) { return buf[rr * 32 + ((((uint32_t)lane >> 2) ^ (rr & 7)) << 2) + (lane & 3)]; };
-    if (!kRowMap && i0 + 31 < j0 && j0 + 31 < o.n) {       // every pair of the block is wanted
-        uint64_t step = o.n - i0 - 1;                      // row i + 1 starts n - i entries on, one column later
-        uint32_t* p = o.out ? o.out + (tri_index(o.n, i0, i0) - i0 + j) : nullptr;
-        if (!o.out) {
-#pragma unroll 8
-            for (uint32_t rr = 0; rr < 32; ++rr) s += at(rr);
-        } else if (!o.partial) {
-#pragma unroll 8
-            for (uint32_t rr = 0; rr < 32; ++rr) {
-                const uint32_t c = at(rr);
-                __stcs(p, c);
-                s += c;
-                p += step--;
-            }
-        } else {
-#pragma unroll 8
-            for (uint32_t rr = 0; rr < 32; ++rr) {
-                const uint32_t c = at(rr);
-                atomicAdd(p, c);
-                s += c;
-                p += step--;
-            }
-        }
-        local = s;
-    } else {
-#pragma unroll 2
-        for (uint32_t rr = 0; rr < 32; ++rr) {
-            const uint64_t i = i0 + rr;
-            const uint32_t c = at(rr);
-            if (i < o.n && j >= i && j < o.n && ts_mapped<kRowMap>(o.row_map, i, j)) {
-                if (o.out) {
-                    uint32_t* dst = o.out + ts_out_index<kRowMap>(o.n, i, j, o.row_map, o.n_out);
-                    if (o.partial) atomicAdd(dst, c);
-                    else *dst = c;
-                }
-                if (j > i) local += c;
-            }
-        }
-    }
+    const unsigned long long local = f4_emit<kRowMap, 1>(o, lane, i0, j0, [&](uint32_t rr, uint32_t) {
+        return buf[rr * 32 + ((((uint32_t)lane >> 2) ^ (rr & 7)) << 2) + (lane & 3)];
+    });
     __syncwarp();
     return local;
 }
 
-// Columns 32 c .. of a warp's 32 x 128 counts (fp32 whole numbers below 2^16,
-// lane = row) as 16-bit numbers, 256 bytes per row, 16-byte chunks XOR-swizzled
-// by row.  x + 2^23 holds x in its low bits.
-__device__ __forceinline__ void f4_pack_block(uint32_t* buf, int lane, uint32_t c, const uint32_t (&r)[32]) {
+// Columns 32 c .. of a warp's 32 x 128 counts (fp32 whole numbers, lane = row)
+// as 16-bit numbers, 256 bytes per row, 16-byte chunks XOR-swizzled by row.
+// x + 2^23 holds x in its low bits.  Returns the largest count.
+__device__ __forceinline__ float f4_pack_block(uint32_t* buf, int lane, uint32_t c, const uint32_t (&r)[32]) {
     uint32_t pk[16];
 #pragma unroll
     for (uint32_t k = 0; k < 16; ++k)
@@ -237,63 +297,22 @@ __device__ __forceinline__ void f4_pack_block(uint32_t* buf, int lane, uint32_t 
     for (uint32_t k = 0; k < 4; ++k)
         *reinterpret_cast<uint4*>(buf + lane * 64 + (((4 * c + k) ^ ((uint32_t)lane & 7u)) << 2)) =
             make_uint4(pk[4 * k], pk[4 * k + 1], pk[4 * k + 2], pk[4 * k + 3]);
+    float most = 0.0f;
+#pragma unroll
+    for (uint32_t k = 0; k < 32; ++k) most = fmaxf(most, __uint_as_float(r[k]));
+    return most;
 }
 
-// The packed 32 x 128 block to its places, 32 consecutive counts of a row per
-// store instruction; this lane's share of the sum over i < j.
+// The packed 32 x 128 block to its places.
 template <bool kRowMap>
 __device__ __forceinline__ unsigned long long f4_store_packed(const F4Out& o, const uint32_t* buf, int lane,
                                                               uint64_t i0, uint64_t j0) {
     __syncwarp();
     const uint16_t* h = reinterpret_cast<const uint16_t*>(buf);
-    auto at = [&](uint32_t rr, uint32_t c) {      // count of column 32 c + lane
+    const unsigned long long local = f4_emit<kRowMap, 4>(o, lane, i0, j0, [&](uint32_t rr, uint32_t c) {
         const uint32_t col = 32u * c + (uint32_t)lane;
         return (uint32_t)h[rr * 128 + (((col >> 3) ^ (rr & 7)) << 3) + (col & 7)];
-    };
-    unsigned long long local = 0;
-    if (!kRowMap && i0 + 31 < j0 && j0 + 127 < o.n) {          // every pair of the block is wanted
-        uint32_t s = 0;
-        uint64_t step = o.n - i0 - 1;                          // row i + 1 starts n - i entries on, one column later
-        uint32_t* p = o.out ? o.out + (tri_index(o.n, i0, i0) - i0 + j0 + lane) : nullptr;
-        if (!o.out) {
-#pragma unroll 4
-            for (uint32_t rr = 0; rr < 32; ++rr)
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) s += at(rr, c);
-        } else {
-#pragma unroll 4
-            for (uint32_t rr = 0; rr < 32; ++rr) {
-#pragma unroll
-                for (uint32_t c = 0; c < 4; ++c) {
-                    const uint32_t v = at(rr, c);
-                    if (o.partial) atomicAdd(p + 32 * c, v);
-                    else __stcs(p + 32 * c, v);
-                    s += v;
-                }
-                p += step--;
-            }
-        }
-        local = s;
-    } else if (i0 < o.n && j0 < o.n && i0 <= j0 + 127) {
-#pragma unroll 1
-        for (uint32_t rr = 0; rr < 32; ++rr) {
-            const uint64_t i = i0 + rr;
-            if (i >= o.n) break;
-#pragma unroll
-            for (uint32_t c = 0; c < 4; ++c) {
-                const uint64_t j = j0 + 32 * c + lane;
-                if (j >= i && j < o.n && ts_mapped<kRowMap>(o.row_map, i, j)) {
-                    const uint32_t v = at(rr, c);
-                    if (o.out) {
-                        uint32_t* dst = o.out + ts_out_index<kRowMap>(o.n, i, j, o.row_map, o.n_out);
-                        if (o.partial) atomicAdd(dst, v);
-                        else *dst = v;
-                    }
-                    if (j > i) local += v;
-                }
-            }
-        }
-    }
+    });
     __syncwarp();
     return local;
 }
@@ -364,7 +383,7 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
             const uint32_t g1 = g + (kb1 - kb0);
             for (uint32_t gs = g + ((g ^ grp) & 1u); gs < g1; gs += 2) {
                 const uint32_t slot = gs % F4_SLOTS, s = gs % F4_STAGES;
-                if (!f4_wait<false>(smem_u32(&ctl->raw_full[slot]), (gs / F4_SLOTS) & 1, ctl, flags, ERR_F4_RAW_FULL)) {
+                if (!f4_wait(smem_u32(&ctl->raw_full[slot]), (gs / F4_SLOTS) & 1, ctl, flags, ERR_F4_RAW_FULL)) {
                     ok = false;
                     break;
                 }
@@ -372,7 +391,7 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                 uint4 v[4];        // 64-byte swizzle: chunk q of row r lies at q ^ ((r / 2) % 4)
 #pragma unroll
                 for (uint32_t q = 0; q < 4; ++q) v[q] = lds128(src + ((q ^ ((row >> 1) & 3u)) << 4));
-                if (!f4_wait<true>(smem_u32(&ctl->empty[s]), ((gs / F4_STAGES) & 1) ^ 1, ctl, flags, ERR_F4_EMPTY)) {
+                if (!f4_wait(smem_u32(&ctl->empty[s]), ((gs / F4_STAGES) & 1) ^ 1, ctl, flags, ERR_F4_EMPTY)) {
                     ok = false;
                     break;
                 }
@@ -428,7 +447,7 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                 const uint32_t ra = tiles[t].x * F4_BM + 128u * rank, rb = tiles[t].y * F4_BN + 128u * rank;
                 for (uint32_t kb = kb0; kb < kb1; ++kb, ++u) {
                     const uint32_t slot = u % F4_SLOTS;
-                    if (!f4_wait<false>(smem_u32(&ctl->raw_empty[slot]), ((u / F4_SLOTS) & 1) ^ 1, ctl, flags,
+                    if (!f4_wait(smem_u32(&ctl->raw_empty[slot]), ((u / F4_SLOTS) & 1) ^ 1, ctl, flags,
                                         ERR_F4_TMA_EMPTY)) {
                         ok = false;
                         break;
@@ -445,7 +464,7 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
             }
             // No copy may still be in flight when the CTA ends, on an abort too.
             for (uint32_t k = u > F4_SLOTS ? u - F4_SLOTS : 0; k < u; ++k)
-                f4_wait<false>(smem_u32(&ctl->raw_full[k % F4_SLOTS]), (k / F4_SLOTS) & 1, ctl, flags,
+                f4_wait(smem_u32(&ctl->raw_full[k % F4_SLOTS]), (k / F4_SLOTS) & 1, ctl, flags,
                                ERR_F4_TMA_DRAIN, true);
         }
         __syncwarp();
@@ -457,11 +476,11 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                 const uint32_t idesc = f4_idesc(F4_BM, F4_BN);
                 bool ok = true;
                 for (; ok && sched.next(t, kb0, kb1, partial); ++tc) {
-                    if (!f4_wait<true>(smem_u32(&ctl->acc_empty), (tc & 1) ^ 1, ctl, flags, ERR_F4_ACCEMPTY)) break;
+                    if (!f4_wait(smem_u32(&ctl->acc_empty), (tc & 1) ^ 1, ctl, flags, ERR_F4_ACCEMPTY)) break;
                     tc_fence_after();
                     for (uint32_t kb = kb0; kb < kb1; ++kb, ++g) {
                         const uint32_t s = g % F4_STAGES;
-                        if (!f4_wait<true>(smem_u32(&ctl->full[s]), (g / F4_STAGES) & 1, ctl, flags, ERR_F4_FULL)) {
+                        if (!f4_wait(smem_u32(&ctl->full[s]), (g / F4_STAGES) & 1, ctl, flags, ERR_F4_FULL)) {
                             ok = false;
                             break;
                         }
@@ -483,7 +502,7 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                 issued = sched.next(t, kb0, kb1, partial);
             }
             // Both CTAs: the pair's MMAs have completed before tensor memory is freed.
-            if (issued) f4_wait<true>(smem_u32(&ctl->drain), 0, ctl, flags, ERR_F4_DRAIN, true);
+            if (issued) f4_wait(smem_u32(&ctl->drain), 0, ctl, flags, ERR_F4_DRAIN, true);
         }
         __syncwarp();
     } else {
@@ -493,23 +512,27 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
         const uint32_t lane_grp = (uint32_t)(warp & 3) * 32u, col0 = (e >> 2) * 128u;
         const uint32_t tacc = tmem_base + (lane_grp << 16) + col0;
         const uint32_t lead_acc_empty = mapa_shared(smem_u32(&ctl->acc_empty), 0);
-        const bool packed = !kThresh && (uint64_t)w_pad * 64 <= F4_PACK_MAX_BITS;
         F4Out o{out, n, n_out, row_map, false};
         unsigned long long total = 0;
         for (uint32_t tc = 0; sched.next(t, kb0, kb1, partial); ++tc) {
-            if (!f4_wait<true>(smem_u32(&ctl->acc_full), tc & 1, ctl, flags, ERR_F4_ACCFULL)) break;
+            if (!f4_wait(smem_u32(&ctl->acc_full), tc & 1, ctl, flags, ERR_F4_ACCFULL)) break;
             tc_fence_after();
             const uint64_t i0 = (uint64_t)tiles[t].x * F4_BM + 128u * rank + lane_grp;
             const uint64_t j0 = (uint64_t)tiles[t].y * F4_BN + col0;
             o.partial = partial;
+            bool packed = !kThresh;
             if (packed) {
+                float most = 0.0f;
 #pragma unroll 1
                 for (uint32_t c = 0; c < 4; ++c) {
                     uint32_t r[32];
                     tmem_ld_32x32b_x32(tacc + 32u * c, r);
                     tmem_ld_wait();
-                    f4_pack_block(buf, lane, c, r);
+                    most = fmaxf(most, f4_pack_block(buf, lane, c, r));
                 }
+                packed = !__any_sync(0xffffffffu, most >= 65536.0f);
+            }
+            if (packed) {
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_pair(lead_acc_empty);

@@ -53,7 +53,16 @@ static int exec_kind(int kind, uint64_t row_bits) {
                                                                                                            : kind;
 }
 
-// Schedule of the 4-bit kernel over `pairs` pairs of CTAs, as ts_schedule.
+constexpr uint32_t F4_MIN_SEG = 8;   // stages of a K segment at least
+
+// Schedule of the 4-bit kernel over `pairs` pairs of CTAs, as ts_schedule:
+// stream-K when the last wave would be under 98.5 % full and a tile has 64
+// stages (32768 bits), and whenever less than half of the pairs have a tile.
+// Measured on B200, whole tiles / stream-K (us of kernel): 78 tiles of 65536
+// bits 177 / 111, 136 tiles 175 / 175, 528 tiles 654 / 592, 136 tiles of
+// 20000 bits 71 / 77, 10 tiles of 20000 bits 47 / 26.  Segments of at least 8
+// stages: 3 tiles of 40 stages take 25 us so, 33 with 16 and 40 with 32; with
+// 4, 10 such tiles take 36 against 28.
 static uint32_t f4_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t& pairs,
                             int pref = STORM_B200_SCHED_AUTO) {
     const uint32_t np = std::max(1, sms / 2);
@@ -61,12 +70,12 @@ static uint32_t f4_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t&
     const uint64_t waves = ((uint64_t)n_tiles + np - 1) / np;
     const double fill = waves ? (double)n_tiles / (double)(waves * np) : 1.0;
     const bool tiles = pref == STORM_B200_SCHED_TILES ||
-                       (pref == STORM_B200_SCHED_AUTO && (fill >= 0.985 || nk < 64));
+                       (pref == STORM_B200_SCHED_AUTO && (fill >= 0.985 || nk < 64) && n_tiles * 2 > np);
     if (tiles) {
         pairs = std::min(n_tiles, np);
         return 1;
     }
-    pairs = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(np, (uint64_t)n_tiles * nk / 16));
+    pairs = (uint32_t)std::min<uint64_t>(np, std::max<uint64_t>(n_tiles, (uint64_t)n_tiles * nk / F4_MIN_SEG));
     return 0;
 }
 
