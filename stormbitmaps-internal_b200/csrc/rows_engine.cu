@@ -94,41 +94,65 @@ __device__ __forceinline__ void zone_set_range(unsigned long long* z, uint64_t c
     for (uint64_t cb = c0; cb <= c1; ++cb) atomicOr(&z[cb >> 6], 1ull << (cb & 63));
 }
 
-__global__ void __launch_bounds__(256)
+// A warp per row, rows side by side; the rows' occupancy words are OR-ed in
+// shared memory first and turned into coarse bins once per block, not once per
+// row (two 64-bit divisions per occupied bin: 2048 rows over 2^20 took 2.64 ms
+// with a block's rows one after another).  Universes past BZONE_OCC_WORDS
+// occupancy words convert row by row.
+constexpr uint32_t BZONE_THREADS = 1024;
+constexpr uint32_t BZONE_OCC_WORDS = 4096;   // occupancy words held per block (2^27 values)
+
+__global__ void __launch_bounds__(BZONE_THREADS)
 block_zone_kernel(RowsView v, const uint32_t* __restrict__ order, uint32_t n, uint32_t T,
                   uint64_t* __restrict__ out) {
     __shared__ unsigned long long z[BZONE_WORDS];
-    const uint32_t b = blockIdx.x;
+    __shared__ unsigned long long occ[BZONE_OCC_WORDS];
+    const uint32_t b = blockIdx.x, lane = threadIdx.x & 31;
     const uint32_t lo = b * T, hi = min(n, lo + T);
+    const bool fold = v.n_occ <= BZONE_OCC_WORDS;
     for (uint32_t k = threadIdx.x; k < BZONE_WORDS; k += blockDim.x) z[k] = 0ull;
+    if (fold)
+        for (uint32_t k = threadIdx.x; k < v.n_occ; k += blockDim.x) occ[k] = 0ull;
     __syncthreads();
     const uint64_t ubits = (uint64_t)v.nw * 64;
     const uint64_t nbins = BZONE_WORDS * 64;
     auto bin_of = [&](uint64_t x) { return x * nbins / ubits; };
-    for (uint32_t k = lo; k < hi; ++k) {
+    auto set_occ_word = [&](uint32_t w, uint64_t x) {
+        for (; x; x &= x - 1) {
+            const uint64_t bin = (uint64_t)w * 64 + (uint64_t)(__ffsll((long long)x) - 1);
+            const uint64_t first = bin * 512, last = min(first + 511, ubits - 1);
+            zone_set_range(z, bin_of(first), bin_of(last));
+        }
+    };
+    for (uint32_t k = lo + (threadIdx.x >> 5); k < hi; k += blockDim.x >> 5) {
         const uint32_t row = order[k];
         const RowMetaD& m = v.meta[row];
         if (m.card == 0) continue;
         const uint64_t s0 = v.s_off[row], len = v.s_off[row + 1] - s0;
         if (v.oc_off[row] != NONE) {
             const uint64_t* oc = v.oc + v.oc_off[row];
-            for (uint32_t w = threadIdx.x; w < v.n_occ; w += blockDim.x)
-                for (uint64_t x = oc[w]; x; x &= x - 1) {
-                    const uint64_t bin = (uint64_t)w * 64 + (uint64_t)(__ffsll((long long)x) - 1);
-                    const uint64_t first = bin * 512, last = min(first + 511, ubits - 1);
-                    zone_set_range(z, bin_of(first), bin_of(last));
-                }
+            for (uint32_t w = lane; w < v.n_occ; w += 32) {
+                const uint64_t x = oc[w];
+                if (!fold) set_occ_word(w, x);
+                else if (x & ~occ[w]) atomicOr(&occ[w], (unsigned long long)x);
+            }
         } else if (len <= ZONE_EXACT_MAX) {
-            for (uint64_t e = threadIdx.x; e < len; e += blockDim.x) {
+            for (uint64_t e = lane; e < len; e += 32) {
                 const uint64_t cb = bin_of(v.s_val[s0 + e]);
                 atomicOr(&z[cb >> 6], 1ull << (cb & 63));
             }
         } else {
             const uint64_t c0 = bin_of(m.first), c1 = bin_of(m.last);
-            for (uint64_t cb = c0 + threadIdx.x; cb <= c1; cb += blockDim.x) atomicOr(&z[cb >> 6], 1ull << (cb & 63));
+            for (uint64_t cb = c0 + lane; cb <= c1; cb += 32) atomicOr(&z[cb >> 6], 1ull << (cb & 63));
         }
     }
     __syncthreads();
+    if (fold) {
+        // a thread per occupancy bin
+        for (uint32_t q = threadIdx.x; q < v.n_occ * 64; q += blockDim.x)
+            if ((occ[q >> 6] >> (q & 63)) & 1ull) set_occ_word(q >> 6, 1ull << (q & 63));
+        __syncthreads();
+    }
     for (uint32_t k = threadIdx.x; k < BZONE_WORDS; k += blockDim.x) out[(uint64_t)b * BZONE_WORDS + k] = z[k];
 }
 
@@ -617,7 +641,7 @@ static void rows_run(STORM_rows_t* r, int policy, uint32_t tile, int fixed_cell,
     auto phases_1_2 = [&]() {
         SB_CUDA(cudaMemsetAsync(r->d_stats.p, 0, sizeof(RowsStatsDev), st));
         block_meta_kernel<<<(nb + 127) / 128, 128, 0, st>>>(c.v, c.order, n, T, r->d_bmeta.p, r->d_het.p);
-        if (zones) block_zone_kernel<<<nb, 256, 0, st>>>(c.v, c.order, n, T, r->d_bzone.p);
+        if (zones) block_zone_kernel<<<nb, BZONE_THREADS, 0, st>>>(c.v, c.order, n, T, r->d_bzone.p);
         select_tiles_kernel<<<(ntiles + 127) / 128, 128, 0, st>>>(
             r->d_bmeta.p, r->d_het.p, zones ? r->d_bzone.p : nullptr, nb,
             learned ? policy : (policy == STORM_POLICY_LEARNED ? STORM_POLICY_PERTILE : policy), fixed_cell, c.model,
