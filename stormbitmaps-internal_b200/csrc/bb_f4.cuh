@@ -546,25 +546,39 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
 #pragma unroll
                     for (uint32_t k = 0; k < 32; ++k) r[k] = __float2uint_rz(__uint_as_float(r[k]));
                     if constexpr (kThresh) {
-                        // whole tiles only (no partial segments); every lane
-                        // stays in the loop for the warp-aggregated appends
+                        // whole tiles only (no partial segments).  v / (ci + cj - v) >= t
+                        // needs v (1 + t) >= t (ci + cj): an fp32 test with 2^-16 to
+                        // spare picks the candidates, the exact one in double
+                        // precision decides them (nearly every pair fails the first).
                         const uint64_t i = i0 + lane, jb = j0 + 32u * c;
                         const bool row_ok = i < n;
-                        const double ci = row_ok ? (double)th.card[i] : 0.0;
+                        const uint32_t card_i = row_ok ? th.card[i] : 0u;
+                        const uint32_t card_j = jb + lane < n ? th.card[jb + lane] : 0u;
+                        const float tt = (float)th.t;
+                        const float ti = tt * (float)card_i, tj_own = tt * (float)card_j;
+                        const float scale = (1.0f + tt) * 1.0000153f;
+                        const int64_t q0 = (int64_t)i - (int64_t)jb, q1 = (int64_t)n - (int64_t)jb;   // i < j < n
+                        uint32_t cand = 0;
 #pragma unroll
                         for (int q = 0; q < 32; ++q) {
-                            const uint64_t j = jb + q;
-                            const uint32_t cnt = r[q];
-                            bool pass = false;
-                            if (row_ok && j > i && j < n) {
-                                total += cnt;
-                                if (cnt) {
-                                    const double un = ci + (double)th.card[j] - (double)cnt;
-                                    pass = un > 0.0 && (double)cnt / un >= th.t;
+                            const float tj = __shfl_sync(0xffffffffu, tj_own, q);
+                            const bool in = row_ok && q > q0 && q < q1 && r[q] != 0;
+                            if (in) total += r[q];
+                            if (in && (!(th.t > 0.0) || !((float)r[q] * scale < ti + tj))) cand |= 1u << q;
+                        }
+                        const uint32_t some = __reduce_or_sync(0xffffffffu, cand);
+                        if (some) {
+#pragma unroll
+                            for (int q = 0; q < 32; ++q) {
+                                if (!(some >> q & 1u)) continue;
+                                const uint32_t cj = __shfl_sync(0xffffffffu, card_j, q);
+                                bool pass = false;
+                                if (cand >> q & 1u) {
+                                    const double un = (double)card_i + (double)cj - (double)r[q];
+                                    pass = un > 0.0 && (double)r[q] / un >= th.t;
                                 }
-                            }
-                            const uint32_t m = __ballot_sync(0xffffffffu, pass);
-                            if (m) {
+                                const uint32_t m = __ballot_sync(0xffffffffu, pass);
+                                if (!m) continue;
                                 const int first = __ffs(m) - 1;
                                 unsigned long long b0 = 0;
                                 if (lane == first) b0 = atomicAdd(th.found, (unsigned long long)__popc(m));
@@ -572,8 +586,8 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                                 if (pass) {
                                     const unsigned long long k = b0 + __popc(m & ((1u << lane) - 1u));
                                     if (k < th.cap) {
-                                        th.pairs[k] = make_uint2((uint32_t)i, (uint32_t)j);
-                                        th.cnts[k] = cnt;
+                                        th.pairs[k] = make_uint2((uint32_t)i, (uint32_t)(jb + q));
+                                        th.cnts[k] = r[q];
                                     }
                                 }
                             }

@@ -774,15 +774,22 @@ int threshold_to_host(const uint2* d_pairs, const uint32_t* d_cnts, uint64_t fou
         SB_CUDA(cudaMemcpyAsync(ct.data(), d_cnts, m * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SB_CUDA(cudaStreamSynchronize(st));
     }
-    std::vector<uint64_t> idx(m);
-    for (uint64_t k = 0; k < m; ++k) idx[k] = k;
-    std::sort(idx.begin(), idx.end(), [&](uint64_t a, uint64_t b) {
-        return pr[a].x != pr[b].x ? pr[a].x < pr[b].x : pr[a].y < pr[b].y;
-    });
-    for (uint64_t k = 0; k < m; ++k) {
-        if (out_i) out_i[k] = pr[idx[k]].x;
-        if (out_j) out_j[k] = pr[idx[k]].y;
-        if (out_count) out_count[k] = ct[idx[k]];
+    // Ordered by (i, j): dealt to their rows, then each row's few sorted by j
+    // (a sort of all of them through an index took most of such a call).
+    uint32_t rows = 0;
+    for (uint64_t k = 0; k < m; ++k) rows = std::max(rows, pr[k].x + 1);
+    std::vector<uint64_t> at((uint64_t)rows + 1, 0);
+    for (uint64_t k = 0; k < m; ++k) ++at[pr[k].x + 1];
+    for (uint64_t r = 0; r < rows; ++r) at[r + 1] += at[r];
+    std::vector<uint64_t> hit(m);   // j << 32 | count
+    for (uint64_t k = 0; k < m; ++k) hit[at[pr[k].x]++] = (uint64_t)pr[k].y << 32 | ct[k];
+    for (uint64_t r = 0, k = 0; r < rows; ++r) {
+        std::sort(hit.begin() + k, hit.begin() + at[r]);   // at[r] is now the row's end
+        for (; k < at[r]; ++k) {
+            if (out_i) out_i[k] = (uint32_t)r;
+            if (out_j) out_j[k] = (uint32_t)(hit[k] >> 32);
+            if (out_count) out_count[k] = (uint32_t)hit[k];
+        }
     }
     return found > cap ? STORM_B200_ESIZE : 0;
 }
