@@ -676,10 +676,13 @@ __device__ __forceinline__ void tri_decode(uint64_t n, uint64_t p, uint64_t& i, 
 
 // Expands plain rows into contiguous bitmaps: local row r of X (W words,
 // W = 1024 x chunk slots, in layout `lay`: chunk slot s of row r -- one
-// 1024-word block -- at X + r x pitch + s x kstride) is row rows[r]. One CTA
-// per row, a warp per chunk slot: absent chunks and padding rows (~0) become
-// zeros, bitmap chunks are copied, list chunks are set bit by bit in a
-// shared-memory copy of the chunk and written out.
+// 1024-word block -- at X + r x pitch + s x kstride) is row rows[r]. A warp
+// per (row, chunk slot): absent chunks and padding rows (~0) become zeros,
+// bitmap chunks are copied, list chunks are set bit by bit in a shared-memory
+// copy of the chunk and written out. Bound: the 8 KiB written per item. A warp
+// finds its chunk by a 32-way search of the row's ids, with no chunk before it
+// in its way: with a CTA per row walking its slots one after another, 2048
+// rows of 2^24 values took 5.9 ms on B200.
 constexpr int EXPAND_WARPS = 4;
 
 // Expanded rows for the tensor cores are stored block-major: chunk slot s of
@@ -690,43 +693,92 @@ constexpr int EXPAND_WARPS = 4;
 constexpr uint64_t PANEL_PITCH = CHUNK_WORDS + 8;
 inline uint64_t panel_row_words(uint64_t W) { return W / CHUNK_WORDS * PANEL_PITCH; }
 
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+        if (lane >= d) x += y;
+    }
+    return x;
+}
+
+// Index of the first of n ascending ids that is >= x (warp-cooperative: 32
+// probes at a time).
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* __restrict__ ids, uint32_t n, uint32_t x, int lane) {
+    uint32_t lo = 0, len = n;              // the answer lies in [lo, lo + len]
+    while (len > 32) {
+        const uint32_t step = (len + 31) / 32;
+        const uint32_t at = lo + lane * step;
+        const uint32_t below = __popc(__ballot_sync(0xffffffffu, lane * step < len && ids[at] < x));
+        if (below == 0) return lo;
+        const uint32_t left = len - (below - 1) * step;
+        lo += (below - 1) * step;          // ids[lo] < x
+        len = left < step ? left : step;
+    }
+    return lo + __popc(__ballot_sync(0xffffffffu, lane < (int)len && ids[lo + lane] < x));
+}
+
+// Calls f(first entry, count) with up to eight consecutive entries of a list
+// (16-byte aligned) per lane, 256 per step of the warp.
+template <class F>
+__device__ __forceinline__ void warp_list8(const uint16_t* __restrict__ l, uint32_t nl, int lane, F f) {
+    for (uint32_t e0 = 0; e0 < nl; e0 += 256) {
+        const uint32_t e = e0 + 8 * lane;
+        uint16_t x[8];
+        if (e + 8 <= nl) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(l + e));
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = (uint16_t)(w[k / 2] >> (16 * (k & 1)));
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) x[k] = e + k < nl ? l[e + k] : (uint16_t)0;
+        }
+        f(x, e >= nl ? 0u : nl - e < 8 ? nl - e : 8u);
+    }
+}
+
 __global__ void __launch_bounds__(EXPAND_WARPS * 32)
 expand_rows_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t m, uint32_t W, RowLayout lay,
                    uint64_t* __restrict__ X) {
-    __shared__ __align__(16) unsigned long long chunk[EXPAND_WARPS][CHUNK_WORDS];
+    __shared__ __align__(16) uint32_t chunk[EXPAND_WARPS][2 * CHUNK_WORDS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t slots = W / CHUNK_WORDS;
-    for (uint32_t r = blockIdx.x; r < m; r += gridDim.x) {
+    const uint64_t items = (uint64_t)m * slots, nw = (uint64_t)gridDim.x * EXPAND_WARPS;
+    for (uint64_t it = (uint64_t)blockIdx.x * EXPAND_WARPS + warp; it < items; it += nw) {
+        const uint32_t r = (uint32_t)(it % m), s = (uint32_t)(it / m);
         const uint32_t row = rows[r];
-        uint64_t* dst_row = X + (uint64_t)r * lay.pitch;
-        const uint64_t c0 = row == ~0u ? 0 : v.row_off[row], c1 = row == ~0u ? 0 : v.row_off[row + 1];
-        uint64_t pos = c0;
-        for (uint32_t s = warp; s < slots; s += EXPAND_WARPS) {
-            while (pos < c1 && v.cid[pos] < s) ++pos;   // ids ascend: a forward walk
-            uint4* dst = reinterpret_cast<uint4*>(dst_row + (uint64_t)s * lay.kstride);
-            if (pos >= c1 || v.cid[pos] != s) {
-                for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = make_uint4(0, 0, 0, 0);
-                continue;
-            }
-            const uint32_t k = v.ckl[pos];
-            if (k & CK_BITMAP) {
-                const uint4* src = reinterpret_cast<const uint4*>(v.bm + v.coff[pos]);
-                for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = __ldg(src + q);
-            } else {
-                unsigned long long* cw = chunk[warp];
-                for (uint32_t q = lane; q < CHUNK_WORDS; q += 32) cw[q] = 0ull;
-                __syncwarp();
-                const uint16_t* l = v.lst + v.coff[pos];
-                const uint32_t nl = k & CK_LEN;
-                for (uint32_t e = lane; e < nl; e += 32) {
-                    const uint32_t x = l[e];
-                    atomicOr(&cw[x >> 6], 1ull << (x & 63));
-                }
-                __syncwarp();
-                const uint4* src = reinterpret_cast<const uint4*>(cw);
-                for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = src[q];
-                __syncwarp();
-            }
+        uint4* dst = reinterpret_cast<uint4*>(X + (uint64_t)r * lay.pitch + (uint64_t)s * lay.kstride);
+        uint64_t pos = 0;
+        bool have = false;
+        if (row != ~0u) {
+            const uint64_t c0 = v.row_off[row];
+            const uint32_t nc = (uint32_t)(v.row_off[row + 1] - c0);
+            const uint32_t q = nc == slots ? s : warp_lower_bound(v.cid + c0, nc, s, lane);
+            pos = c0 + q;
+            have = q < nc && v.cid[pos] == s;
+        }
+        if (!have) {
+            for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = make_uint4(0, 0, 0, 0);
+            continue;
+        }
+        const uint32_t k = v.ckl[pos];
+        if (k & CK_BITMAP) {
+            const uint4* src = reinterpret_cast<const uint4*>(v.bm + v.coff[pos]);
+            for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = __ldg(src + q);
+        } else {
+            uint32_t* cw = chunk[warp];
+            uint4* c4 = reinterpret_cast<uint4*>(cw);
+            for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) c4[q] = make_uint4(0, 0, 0, 0);
+            __syncwarp();
+            warp_list8(v.lst + v.coff[pos], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                    if (q < cnt) atomicOr(&cw[x[q] >> 5], 1u << (x[q] & 31));
+            });
+            __syncwarp();
+            for (uint32_t q = lane; q < CHUNK_WORDS / 2; q += 32) dst[q] = c4[q];
+            __syncwarp();
         }
     }
 }
@@ -797,29 +849,82 @@ chunk_pairs_kernel(ChunkView v, uint32_t mode, uint64_t n1, uint64_t n2, uint64_
 // ---- postings: pairs of plain rows without bitmap chunks ----------------
 // value of entry e of list chunk c: cid << 16 | entry (universe <= 2^27)
 
-// rows == nullptr: rows [0, nq). Bitmap chunks count every set bit (only the
-// rectangle sums send rows that have them).
-__global__ void postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq,
-                                     uint32_t* __restrict__ counts) {
+// A CTA per row, its warps over groups of `group` (1 .. 32) consecutive
+// chunks: f(value) for every list entry, g(chunk) -- warp-cooperative -- for
+// every bitmap chunk. Rows of long lists take group 1 (a warp per chunk, eight
+// entries per lane); rows of short ones (a chunk of a very sparse row holds a
+// handful of values) group 32, the warp walking the concatenated entries of 32
+// chunks, whose kinds and places it reads side by side. With a warp per row
+// and one chunk at a time, the 200 rows of a small container left the GPU idle
+// and 20000 rows of 6 values per chunk most lanes.
+constexpr uint32_t ROW_WALK_THREADS = 256;
+
+template <class F, class G>
+__device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint32_t group, F f, G g) {
     const int lane = threadIdx.x & 31;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nq; r += nw) {
-        const uint32_t row = rows ? rows[r] : r;
-        for (uint64_t c = v.row_off[row]; c < v.row_off[row + 1]; ++c) {
-            const uint32_t base = v.cid[c] << 16;
-            const uint32_t k = v.ckl[c];
+    const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
+    const uint32_t warps = blockDim.x >> 5;
+    if (group == 1) {
+        for (uint64_t c = c0 + (threadIdx.x >> 5); c < c1; c += warps) {
+            const uint32_t k = v.ckl[c], base = v.cid[c] << 16;
             if (k & CK_BITMAP) {
+                g(c);
+                continue;
+            }
+            warp_list8(v.lst + v.coff[c], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
+#pragma unroll
+                for (uint32_t q = 0; q < 8; ++q)
+                    if (q < cnt) f(base | x[q]);
+            });
+        }
+        return;
+    }
+    for (uint64_t cg = c0 + (uint64_t)(threadIdx.x >> 5) * group; cg < c1; cg += (uint64_t)warps * group) {
+        const uint64_t c = cg + lane;
+        const bool in = lane < (int)group && c < c1;
+        const uint32_t k = in ? v.ckl[c] : 0u;
+        const uint32_t base = in ? v.cid[c] << 16 : 0u;
+        const uint64_t off = in ? v.coff[c] : 0ull;
+        for (uint32_t bm = __ballot_sync(0xffffffffu, (k & CK_BITMAP) != 0); bm; bm &= bm - 1)
+            g(cg + (uint32_t)(__ffs(bm) - 1));
+        const uint32_t len = k & CK_BITMAP ? 0u : k & CK_LEN;
+        const uint32_t incl = warp_incl_scan(len, lane), excl = incl - len;
+        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            uint32_t o = 0;                // the last chunk of the group whose entries start at or before t
+#pragma unroll
+            for (uint32_t step = 16; step; step >>= 1)
+                if (__shfl_sync(0xffffffffu, excl, o + step) <= t) o += step;
+            const uint32_t e = t - __shfl_sync(0xffffffffu, excl, o), b = __shfl_sync(0xffffffffu, base, o);
+            const uint64_t at = __shfl_sync(0xffffffffu, off, o);
+            if (t < total) f(b | v.lst[at + e]);
+        }
+    }
+}
+
+// Chunks per group of row_walk for rows of `chunks` chunks holding `entries`
+// list entries in all: one from 48 entries a chunk on.
+static uint32_t walk_group(uint64_t chunks, uint64_t entries, bool bitmaps) {
+    return bitmaps || entries >= 48 * chunks ? 1u : 32u;
+}
+
+// rows == nullptr: rows [0, nq). Bitmap chunks count every set bit (only the
+// sums over pairs send rows that have them).
+__global__ void __launch_bounds__(ROW_WALK_THREADS)
+postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group,
+                     uint32_t* __restrict__ counts) {
+    const int lane = threadIdx.x & 31;
+    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x)
+        row_walk(
+            v, rows ? rows[r] : r, group, [&](uint32_t x) { atomicAdd(&counts[x], 1u); },
+            [&](uint64_t c) {
                 const uint64_t* wd = v.bm + v.coff[c];
+                const uint32_t base = v.cid[c] << 16;
                 for (uint32_t w = lane; w < CHUNK_WORDS; w += 32)
                     for (uint64_t x = wd[w]; x; x &= x - 1)
                         atomicAdd(&counts[base | (w << 6) | (uint32_t)__ffsll((long long)x) - 1u], 1u);
-            } else {
-                const uint16_t* l = v.lst + v.coff[c];
-                const uint32_t nl = k & CK_LEN;
-                for (uint32_t e = lane; e < nl; e += 32) atomicAdd(&counts[base | l[e]], 1u);
-            }
-        }
-    }
+            });
 }
 
 // sum over values of a[x] * b[x] into flags->sum: the rectangle sum of two
@@ -860,66 +965,83 @@ __global__ void postings_stats_kernel(const uint32_t* __restrict__ counts, uint6
     }
 }
 
-__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t x, int lane) {
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= d) x += y;
-    }
-    return x;
-}
-
 // Gives every value held by >= 2 rows a slot range in the postings array
 // (start) and, when `lists` is given, a list record; other values get
-// start = ~0. One atomic per warp per 32 values. (The run postings use it
-// for bins.)
-__global__ void postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t* __restrict__ start,
-                                      uint2* __restrict__ lists, PostingsStats* st) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t x0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; x0 < U; x0 += nw * 32) {
-        const uint64_t x = x0 + lane;
-        const uint32_t c = x < U ? counts[x] : 0u;
-        const bool want = c >= 2;
-        const uint32_t n_incl = warp_incl_scan(want ? c : 0u, lane);
-        const uint32_t b = __ballot_sync(0xffffffffu, want);
-        unsigned long long e0 = 0, l0 = 0;
-        if (lane == 31 && b) {
-            e0 = atomicAdd(&st->cursor[0], (unsigned long long)n_incl);
-            l0 = atomicAdd(&st->cursor[1], (unsigned long long)__popc(b));
+// start = ~0. A block takes 4096 values at a time and the two allocation
+// cursors once for all of them: one atomic per warp on the same two words took
+// 0.64 ms for 2^24 values (the counts and starts, 134 MB, cost 0.03). (The run
+// postings use it for bins.)
+constexpr uint32_t ALLOC_THREADS = 256, ALLOC_PER_THREAD = 16;
+
+__global__ void __launch_bounds__(ALLOC_THREADS)
+postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t* __restrict__ start,
+                      uint2* __restrict__ lists, PostingsStats* st) {
+    __shared__ uint32_t we[ALLOC_THREADS / 32], wl[ALLOC_THREADS / 32];
+    __shared__ unsigned long long e0s, l0s;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr uint32_t TILE = ALLOC_THREADS * ALLOC_PER_THREAD;
+    for (uint64_t x0 = (uint64_t)blockIdx.x * TILE; x0 < U; x0 += (uint64_t)gridDim.x * TILE) {
+        // value x0 + 512 warp + 32 k + lane: a warp's 16 groups of 32 in order
+        uint32_t c[ALLOC_PER_THREAD];
+        uint32_t e = 0, l = 0;
+        const uint64_t xw = x0 + (uint64_t)warp * 32 * ALLOC_PER_THREAD + lane;
+#pragma unroll
+        for (uint32_t k = 0; k < ALLOC_PER_THREAD; ++k) {
+            const uint64_t x = xw + 32 * k;
+            c[k] = x < U ? counts[x] : 0u;
+            e += c[k] >= 2 ? c[k] : 0u;
+            l += c[k] >= 2 ? 1u : 0u;
         }
-        e0 = __shfl_sync(0xffffffffu, e0, 31);
-        l0 = __shfl_sync(0xffffffffu, l0, 31);
-        if (x < U) {
-            if (want) {
-                const uint32_t s = (uint32_t)(e0 + n_incl - c);
+        const uint32_t ei = warp_incl_scan(e, lane), li = warp_incl_scan(l, lane);
+        if (lane == 31) {
+            we[warp] = ei;
+            wl[warp] = li;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t te = 0, tl = 0;
+            for (uint32_t k = 0; k < ALLOC_THREADS / 32; ++k) {
+                const uint32_t a = we[k], b = wl[k];
+                we[k] = te;
+                wl[k] = tl;
+                te += a;
+                tl += b;
+            }
+            e0s = tl ? atomicAdd(&st->cursor[0], (unsigned long long)te) : 0ull;
+            l0s = tl ? atomicAdd(&st->cursor[1], (unsigned long long)tl) : 0ull;
+        }
+        __syncthreads();
+        uint32_t s = (uint32_t)e0s + we[warp] + ei - e;      // list places of this thread's values
+        uint64_t q = l0s + wl[warp] + li - l;
+#pragma unroll
+        for (uint32_t k = 0; k < ALLOC_PER_THREAD; ++k) {
+            const uint64_t x = xw + 32 * k;
+            if (x >= U) continue;
+            if (c[k] >= 2) {
                 start[x] = s;
-                if (lists) lists[l0 + __popc(b & ((1u << lane) - 1u))] = make_uint2(s, c);
+                if (lists) lists[q] = make_uint2(s, c[k]);
+                s += c[k];
+                ++q;
             } else {
                 start[x] = ~0u;
             }
         }
+        __syncthreads();   // we, wl and the bases are read before the next tile's
     }
 }
 
 // Writes each Q row's position in the Q list (its local index) into the
 // lists of its values; start[x] advances to the end of x's list.
-__global__ void postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq,
-                                        uint32_t* __restrict__ start, uint32_t* __restrict__ post) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nq; r += nw) {
-        const uint32_t row = rows[r];
-        for (uint64_t c = v.row_off[row]; c < v.row_off[row + 1]; ++c) {
-            const uint32_t base = v.cid[c] << 16;
-            const uint16_t* l = v.lst + v.coff[c];
-            const uint32_t nl = v.ckl[c] & CK_LEN;
-            for (uint32_t e = lane; e < nl; e += 32) {
-                const uint32_t x = base | l[e];
+__global__ void __launch_bounds__(ROW_WALK_THREADS)
+postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group,
+                        uint32_t* __restrict__ start, uint32_t* __restrict__ post) {
+    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x)
+        row_walk(
+            v, rows[r], group,
+            [&](uint32_t x) {
                 if (start[x] != ~0u) post[atomicAdd(&start[x], 1u)] = r;
-            }
-        }
-    }
+            },
+            [](uint64_t) {});
 }
 
 // One increment per (pair of rows, shared value): thread per list for lists
@@ -1052,18 +1174,51 @@ __device__ __forceinline__ void run_bitmap_word(const uint64_t* wd, uint32_t nwc
     run_word_masks(x, cin, nin, wi, wlog, starts, lasts);
 }
 
-// Pieces per row and per bin; warp per row.
-__global__ void run_count_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
-                                 uint32_t* __restrict__ pieces, uint32_t* __restrict__ bins) {
+// A warp over a list chunk, eight entries per lane: f(value, starts, lasts)
+// per entry, in order of the lanes; `at` counts and the warp's running totals
+// are f's business. Entries of the neighbouring lanes decide a lane's first
+// and last one (run_pieces.cuh states the rules).
+template <class F>
+__device__ __forceinline__ void run_list_walk(const uint16_t* __restrict__ l, uint32_t nl, uint32_t wmask, int lane, F f) {
+    uint32_t carry = 0x10000u;             // the entry before the warp's first (none: nothing is its successor)
+    uint32_t e0 = 0;
+    warp_list8(l, nl, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
+        const uint32_t up = __shfl_up_sync(0xffffffffu, (uint32_t)x[7], 1);
+        const uint32_t dn = __shfl_down_sync(0xffffffffu, (uint32_t)x[0], 1);
+        const uint32_t before = lane ? up : carry;
+        const uint32_t e = e0 + 8 * lane;
+        const uint32_t after = e + 8 < nl ? (lane < 31 ? dn : (uint32_t)l[e + 8]) : 0x20000u;
+        uint32_t st = 0, la = 0;           // bit k: entry e + k starts / ends a piece
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            if (k >= cnt) continue;
+            const uint32_t v = x[k], p = k ? (uint32_t)x[k - 1] : before;
+            const uint32_t n = k + 1 < cnt ? (uint32_t)x[k < 7 ? k + 1 : 7] : after;
+            if (v != p + 1 || (v & wmask) == 0) st |= 1u << k;
+            if (n != v + 1 || ((v + 1) & wmask) == 0) la |= 1u << k;
+        }
+        f(x, st, la);
+        carry = __shfl_sync(0xffffffffu, (uint32_t)x[7], 31);
+        e0 += 256;
+    });
+}
+
+// Pieces per row, per chunk and per bin; CTA per row, a warp per chunk.
+__global__ void __launch_bounds__(ROW_WALK_THREADS)
+run_count_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
+                 uint32_t* __restrict__ pieces, uint32_t* __restrict__ chunk_pieces, uint32_t* __restrict__ bins) {
+    __shared__ uint32_t total;
     const int lane = threadIdx.x & 31;
     const uint32_t wmask = (1u << wlog) - 1u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nq; r += nw) {
+    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x) {
+        if (threadIdx.x == 0) total = 0;
+        __syncthreads();
         const uint32_t row = rows[r];
-        uint32_t cnt = 0;
-        for (uint64_t c = v.row_off[row]; c < v.row_off[row + 1]; ++c) {
+        const uint64_t c1 = v.row_off[row + 1];
+        for (uint64_t c = v.row_off[row] + (threadIdx.x >> 5); c < c1; c += ROW_WALK_THREADS / 32) {
             const uint32_t base = v.cid[c] << 16;
             const uint32_t k = v.ckl[c];
+            uint32_t cnt = 0;
             if (k & CK_BITMAP) {
                 const uint64_t* wd = v.bm + v.coff[c];
                 const uint32_t nwc = k & CK_LEN;
@@ -1076,17 +1231,23 @@ __global__ void run_count_kernel(ChunkView v, const uint32_t* __restrict__ rows,
                                   1u);
                 }
             } else {
-                const uint16_t* l = v.lst + v.coff[c];
-                const uint32_t nl = k & CK_LEN;
-                for (uint32_t e = lane; e < nl; e += 32)
-                    if (run_piece_start(l, e, wmask)) {
-                        ++cnt;
-                        atomicAdd(&bins[(base | l[e]) >> wlog], 1u);
-                    }
+                run_list_walk(v.lst + v.coff[c], k & CK_LEN, wmask, lane,
+                              [&](const uint16_t (&x)[8], uint32_t st, uint32_t) {
+                                  cnt += __popc(st);
+#pragma unroll
+                                  for (uint32_t q = 0; q < 8; ++q)
+                                      if (st >> q & 1u) atomicAdd(&bins[(base | x[q]) >> wlog], 1u);
+                              });
+            }
+            cnt = warp_sum_u32(cnt);
+            if (lane == 0) {
+                chunk_pieces[c] = cnt;
+                if (cnt) atomicAdd(&total, cnt);
             }
         }
-        cnt = warp_sum_u32(cnt);
-        if (lane == 0) pieces[r] = cnt;
+        __syncthreads();
+        if (threadIdx.x == 0) pieces[r] = total;
+        __syncthreads();
     }
 }
 
@@ -1111,20 +1272,50 @@ __global__ void run_stats_kernel(const uint32_t* __restrict__ bins, uint64_t nb,
 
 // The rows' pieces in row order: pieces[poff[r] + k] = (first value, end),
 // the k-th start and the k-th last value of the row paired by rank (list
-// entries, or set bits of bitmap chunks).
-__global__ void run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
-                                const uint64_t* __restrict__ poff, uint2* __restrict__ pieces) {
-    const int lane = threadIdx.x & 31;
+// entries, or set bits of bitmap chunks). A piece lies in one chunk, so the
+// pieces counted per chunk place every chunk's (a prefix over the row's at
+// most 2048 chunks), and a CTA's warps take the chunks side by side: with a
+// warp per row, 4000 rows of 51000 values took 1.24 ms, and counting 0.85.
+constexpr uint32_t RUN_MAX_CHUNKS = 2048;    // universe <= 2^27
+
+__global__ void __launch_bounds__(ROW_WALK_THREADS)
+run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
+                const uint64_t* __restrict__ poff, const uint32_t* __restrict__ chunk_pieces,
+                uint2* __restrict__ pieces) {
+    __shared__ uint32_t first[RUN_MAX_CHUNKS];
+    __shared__ uint32_t wsum[ROW_WALK_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t wmask = (1u << wlog) - 1u;
-    const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nq; r += nw) {
+    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x) {
         const uint32_t row = rows[r];
-        uint2* out = pieces + poff[r];
-        uint32_t ks = 0, kl = 0;
-        for (uint64_t c = v.row_off[row]; c < v.row_off[row + 1]; ++c) {
+        const uint64_t c0 = v.row_off[row];
+        const uint32_t nc = (uint32_t)(v.row_off[row + 1] - c0);
+        // first[k]: pieces of the chunks before chunk k
+        constexpr uint32_t PER = RUN_MAX_CHUNKS / ROW_WALK_THREADS;
+        uint32_t own[PER], sum = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < PER; ++q) {
+            const uint32_t k = threadIdx.x * PER + q;
+            own[q] = sum;
+            sum += k < nc ? chunk_pieces[c0 + k] : 0u;
+        }
+        const uint32_t incl = warp_incl_scan(sum, lane);
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        uint32_t before = incl - sum;
+        for (int w = 0; w < warp; ++w) before += wsum[w];
+#pragma unroll
+        for (uint32_t q = 0; q < PER; ++q) {
+            const uint32_t k = threadIdx.x * PER + q;
+            if (k < nc) first[k] = before + own[q];
+        }
+        __syncthreads();
+        for (uint32_t kc = warp; kc < nc; kc += ROW_WALK_THREADS / 32) {
+            const uint64_t c = c0 + kc;
             const uint32_t base = v.cid[c] << 16;
             const uint32_t k = v.ckl[c];
+            uint2* out = pieces + poff[r] + first[kc];
+            uint32_t ks = 0, kl = 0;
             if (k & CK_BITMAP) {
                 const uint64_t* wd = v.bm + v.coff[c];
                 const uint32_t nwc = k & CK_LEN;
@@ -1132,15 +1323,7 @@ __global__ void run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, 
                 for (uint32_t w0 = 0; w0 < nwc; w0 += 32) {
                     run_bitmap_word(wd, nwc, w0, lane, wlog, carry, starts, lasts);
                     const uint32_t ns = (uint32_t)__popcll(starts), nls = (uint32_t)__popcll(lasts);
-                    uint32_t xs = ns, xl = nls;   // inclusive scans over the lanes (words in order)
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t ys = __shfl_up_sync(0xffffffffu, xs, o), yl = __shfl_up_sync(0xffffffffu, xl, o);
-                        if (lane >= o) {
-                            xs += ys;
-                            xl += yl;
-                        }
-                    }
+                    const uint32_t xs = warp_incl_scan(ns, lane), xl = warp_incl_scan(nls, lane);
                     const uint32_t at = base + ((w0 + lane) << 6);
                     uint32_t j = ks + xs - ns;
                     for (uint64_t x = starts; x; x &= x - 1) out[j++].x = at + (uint32_t)(__ffsll((long long)x) - 1);
@@ -1150,21 +1333,24 @@ __global__ void run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, 
                     kl += __shfl_sync(0xffffffffu, xl, 31);
                 }
             } else {
-                const uint16_t* l = v.lst + v.coff[c];
-                const uint32_t nl = k & CK_LEN;
-                for (uint32_t e0 = 0; e0 < nl; e0 += 32) {
-                    const uint32_t e = e0 + lane;
-                    const bool in = e < nl;
-                    const bool st = in && run_piece_start(l, e, wmask);
-                    const bool la = in && run_piece_last(l, e, nl, wmask);
-                    const uint32_t bs = __ballot_sync(0xffffffffu, st), bl = __ballot_sync(0xffffffffu, la);
-                    if (st) out[ks + __popc(bs & lt)].x = base | l[e];
-                    if (la) out[kl + __popc(bl & lt)].y = (base | l[e]) + 1u;
-                    ks += __popc(bs);
-                    kl += __popc(bl);
-                }
+                run_list_walk(v.lst + v.coff[c], k & CK_LEN, wmask, lane,
+                              [&](const uint16_t (&x)[8], uint32_t st, uint32_t la) {
+                                  // ranks of the lane's starts and lasts, 16 bits each (a step holds 256 entries)
+                                  const uint32_t both = __popc(st) | (uint32_t)__popc(la) << 16;
+                                  const uint32_t inc = warp_incl_scan(both, lane), exc = inc - both;
+                                  uint32_t js = ks + (exc & 0xFFFFu), jl = kl + (exc >> 16);
+#pragma unroll
+                                  for (uint32_t q = 0; q < 8; ++q) {
+                                      if (st >> q & 1u) out[js++].x = base | x[q];
+                                      if (la >> q & 1u) out[jl++].y = (base | x[q]) + 1u;
+                                  }
+                                  const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+                                  ks += tot & 0xFFFFu;
+                                  kl += tot >> 16;
+                              });
             }
         }
+        __syncthreads();   // first is read before the next row's
     }
 }
 
@@ -1356,10 +1542,18 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             std::vector<uint32_t> second(n2);
             for (uint64_t r = 0; r < n2; ++r) second[r] = (uint32_t)(n1 + r);
             SB_CUDA(cudaMemcpyAsync(d_qrows.p, second.data(), n2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>((n1 + 7) / 8, (uint64_t)sms * 16), 256, 0, st>>>(
-                d.view(), nullptr, (uint32_t)n1, d_counts.p);
-            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>((n2 + 7) / 8, (uint64_t)sms * 16), 256, 0, st>>>(
-                d.view(), d_qrows.p, (uint32_t)n2, d_start.p);
+            uint64_t chunks = 0, entries = 0;
+            bool bitmaps = false;
+            for (const ChunkRowFacts& f : d.facts) {
+                chunks += f.chunks;
+                entries += f.list_entries;
+                bitmaps |= f.bitmap_chunks != 0;
+            }
+            const uint32_t group = walk_group(chunks, entries, bitmaps);
+            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>(n1, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
+                d.view(), nullptr, (uint32_t)n1, group, d_counts.p);
+            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>(n2, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
+                d.view(), d_qrows.p, (uint32_t)n2, group, d_start.p);
             counts_dot_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, d_start.p, U, d_flags.p);
             SB_CUDA(cudaGetLastError());
             launches += 3;
@@ -1403,6 +1597,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
 
     SB_CUDA(cudaEventRecord(log.ev0, st));
     PostingsStats ps{};
+    uint32_t q_group = 1;                                  // row_walk's group for the postings rows
     auto histogram = [&](const std::vector<uint32_t>& rows) {
         d_qrows.reserve(rows.size());
         SB_CUDA(cudaEventRecord(ev_hist0, st));
@@ -1411,8 +1606,17 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_counts.p, 0, U * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
-        const uint32_t gq = (uint32_t)std::min<uint64_t>((rows.size() + 7) / 8, (uint64_t)sms * 16);
-        postings_hist_kernel<<<gq, 256, 0, st>>>(d.view(), d_qrows.p, (uint32_t)rows.size(), d_counts.p);
+        uint64_t chunks = 0, entries = 0;
+        bool bitmaps = false;
+        for (uint32_t r : rows) {
+            chunks += d.facts[r].chunks;
+            entries += d.facts[r].list_entries;
+            bitmaps |= d.facts[r].bitmap_chunks != 0;
+        }
+        q_group = walk_group(chunks, entries, bitmaps);
+        const uint32_t gq = (uint32_t)std::min<uint64_t>(rows.size(), (uint64_t)sms * 64);
+        postings_hist_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)rows.size(), q_group,
+                                                             d_counts.p);
         postings_stats_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_pstats.p);
         SB_CUDA(cudaGetLastError());
         SB_CUDA(cudaEventRecord(ev_hist, st));
@@ -1456,8 +1660,10 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_rstats.reserve(2);
         SB_CUDA(cudaMemsetAsync(d_rbins.p, 0, n_bins * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_rstats.p, 0, 2 * sizeof(unsigned long long), st));
-        const uint32_t gq = (uint32_t)std::min<uint64_t>((q + 7) / 8, (uint64_t)sms * 16);
-        run_count_kernel<<<gq, 256, 0, st>>>(d.view(), d_qrows.p, (uint32_t)q, rwlog, d_rpieces.p, d_rbins.p);
+        d_cpieces.reserve(d.cid.n);
+        const uint32_t gq = (uint32_t)std::min<uint64_t>(q, (uint64_t)sms * 64);
+        run_count_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)q, rwlog, d_rpieces.p,
+                                                         d_cpieces.p, d_rbins.p);
         run_stats_kernel<<<sms * 8, 256, 0, st>>>(d_rbins.p, n_bins, d_rstats.p);
         SB_CUDA(cudaGetLastError());
         SB_CUDA(cudaEventRecord(ev_hist, st));
@@ -1579,7 +1785,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     };
     bool panel_plan = false;
     // The panel needs a block of expanded rows and its transpose in HBM.
-    const uint64_t panel_bytes = 2ull * PANEL_ROWS * W * sizeof(uint64_t);
+    const uint64_t panel_bytes = PANEL_ROWS * (W + panel_row_words(W)) * sizeof(uint64_t);
     auto panel_fits = [&]() {
         if (!facts_ok || panel_mode == 0 || U > PANEL_MAX_UNIVERSE) return false;
         size_t fr = 0, tot = 0;
@@ -1747,7 +1953,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // 256-row block is all H or all tq and the tq x tq blocks can be left out.
     // Panels of P rows when they do not all fit the budget.
     if (panel_plan) {
-        d_pX.reserve(PANEL_ROWS * W);
+        d_pX.reserve(PANEL_ROWS * panel_row_words(W));
         d_DT.reserve(PANEL_ROWS * W);
     }
     const uint64_t nd0 = dense.size();
@@ -1846,7 +2052,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         auto expand = [&](uint64_t first, uint64_t m, uint64_t slot) {
             SB_CUDA(cudaMemcpyAsync(d_map.p + slot, emap.data() + first, m * sizeof(uint32_t),
                                     cudaMemcpyHostToDevice, st));
-            const uint32_t grid = (uint32_t)std::min<uint64_t>(m, (uint64_t)sms * 16);
+            const uint32_t grid = (uint32_t)std::min<uint64_t>((m * slots + EXPAND_WARPS - 1) / EXPAND_WARPS,
+                                                               (uint64_t)sms * 64);
             expand_rows_kernel<<<grid, EXPAND_WARPS * 32, 0, st>>>(d.view(), d_map.p + slot, (uint32_t)m,
                                                                    (uint32_t)W, lay, d_panel.p + slot * lay.pitch);
             SB_CUDA(cudaGetLastError());
@@ -1962,9 +2169,10 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             const uint32_t prows = (uint32_t)std::min<uint64_t>(PANEL_ROWS, npw - b0);
             for (uint32_t t = 0; t < PANEL_ROWS; ++t) bmap[t] = t < prows ? h_perm[pw0 + b0 + t] : ~0u;
             SB_CUDA(cudaMemcpyAsync(d_pmap.p, bmap.data(), PANEL_ROWS * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            expand_rows_kernel<<<(uint32_t)std::min<uint64_t>(PANEL_ROWS, (uint64_t)sms * 16), EXPAND_WARPS * 32, 0,
-                                 st>>>(d.view(), d_pmap.p, PANEL_ROWS, (uint32_t)W, row_major(W), d_pX.p);
-            panel_transpose_kernel<<<(uint32_t)(W / PANEL_T_WORDS), 1024, PANEL_T_SMEM, st>>>(d_pX.p, W, d_DT.p);
+            const RowLayout play{PANEL_PITCH, PANEL_ROWS * PANEL_PITCH};   // block-major, as the tensor panels
+            expand_rows_kernel<<<(uint32_t)sms * 64, EXPAND_WARPS * 32, 0, st>>>(d.view(), d_pmap.p, PANEL_ROWS,
+                                                                                (uint32_t)W, play, d_pX.p);
+            panel_transpose_kernel<<<(uint32_t)(W / PANEL_T_WORDS), 1024, PANEL_T_SMEM, st>>>(d_pX.p, play, d_DT.p);
             SB_CUDA(cudaMemsetAsync(d_ctr.p, 0, sizeof(unsigned long long), st));
             const uint32_t ni = (uint32_t)items.size();
             uint32_t* scr = splits.empty() ? nullptr : d_pscratch.p;
@@ -2005,8 +2213,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
         const uint32_t gq = (uint32_t)std::min<uint64_t>((nq + 7) / 8, (uint64_t)sms * 16);
-        run_fill_kernel<<<gq, 256, 0, st>>>(d.view(), d_qrows.p, (uint32_t)nq, rwlog, d_rpoff.p, d_pieces.p);
-        postings_alloc_kernel<<<sms * 8, 256, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, d_pstats.p);
+        run_fill_kernel<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
+            d.view(), d_qrows.p, (uint32_t)nq, rwlog, d_rpoff.p, d_cpieces.p, d_pieces.p);
+        postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, d_pstats.p);
         run_scatter_kernel<<<gq, 256, 0, st>>>((uint32_t)nq, rwlog, d_rpoff.p, d_pieces.p, d_rstart.p, d_rlist.p);
         static std::atomic<uint64_t> done{0};
         smem_attr_once(run_sweep_kernel, (int)((POST_SWEEP_MAX_ROWS + RUN_SWEEP_BATCH + 1) * sizeof(uint32_t)), done);
@@ -2030,9 +2239,10 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             d_start.reserve(U);
             d_lists.reserve(ps.lists ? ps.lists : 1);
             d_post.reserve(ps.entries ? ps.entries : 1);
-            postings_alloc_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_start.p, d_lists.p, d_pstats.p);
-            const uint32_t gq = (uint32_t)std::min<uint64_t>((nq + 7) / 8, (uint64_t)sms * 16);
-            postings_scatter_kernel<<<gq, 256, 0, st>>>(d.view(), d_qrows.p, (uint32_t)nq, d_start.p, d_post.p);
+            postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_counts.p, U, d_start.p, d_lists.p, d_pstats.p);
+            const uint32_t gq = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64);
+            postings_scatter_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)nq, q_group,
+                                                                    d_start.p, d_post.p);
             if (sweep) {
                 static std::atomic<uint64_t> done{0};
                 smem_attr_once(postings_rows_kernel,

@@ -239,7 +239,7 @@ struct ChunkEngine {
     uint64_t last_panel_rows = 0, last_panel_queries = 0;
     int last_postings_form = -1;       // per-pair form of the last call's postings: 0 list by list,
                                        // 1 row sweep, 2 run sweep (-1: none)
-    DevBuf<uint32_t> d_rpieces, d_rbins, d_rstart;
+    DevBuf<uint32_t> d_rpieces, d_cpieces, d_rbins, d_rstart;
     DevBuf<uint64_t> d_rpoff;
     DevBuf<uint2> d_pieces, d_rlist;
     DevBuf<unsigned long long> d_rstats;

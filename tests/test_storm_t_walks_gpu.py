@@ -1,0 +1,105 @@
+"""The row walks of the chunked engine -- postings, run postings, expansion to
+bitmaps, transposed panel -- on rows at the edges of their groups: chunks of no
+more than a few values (walked 32 at a time) in rows of more and fewer than 32
+chunks, missing chunk ids, lists around multiples of 8 and 256 entries, runs
+across those steps and across bins. Whole numbers, equal to the oracle's."""
+import numpy as np
+import pytest
+
+import gen
+import oracle_lib as ol
+
+pytestmark = pytest.mark.gpu
+
+
+def _short(g):
+    """1 to 5 values in some of 70 chunks: groups of 32 chunks, the last one partial."""
+    sets = []
+    for r in range(150):
+        ids = np.flatnonzero(g.random(70) < (0.2, 0.9, 1.0)[r % 3])
+        v = [int(c) << 16 | int(x) for c in ids for x in g.integers(0, 40, size=int(g.integers(1, 6)))]
+        sets.append(np.unique(np.array(v, dtype=np.uint32)))
+    return sets
+
+
+def _lists(g):
+    """One to three chunks of 1 .. 4095 values, lengths around 8, 256 and 2048."""
+    sizes = (1, 7, 8, 9, 255, 256, 257, 263, 511, 513, 2047, 2048, 2049, 4095)
+    sets = []
+    for r in range(84):
+        v = [np.sort(g.choice(65536, size=sizes[(r + k) % len(sizes)], replace=False)) + (int(c) << 16)
+             for k, c in enumerate(np.sort(g.choice(9, size=1 + r % 3, replace=False)))]
+        sets.append(np.concatenate(v).astype(np.uint32))
+    return sets
+
+
+def _runs(g):
+    """Runs of 1 .. 700 values, adjacent ones and ones that end at a chunk's last value included."""
+    sets = []
+    for r in range(90):
+        v = [np.arange(s, s + int(g.integers(1, 700))) for s in g.integers(0, 5 * 65536 - 700, size=int(g.integers(1, 14)))]
+        v.append(np.arange(65536 - int(g.integers(1, 300)), 65536))
+        v.append(np.arange(65536, 65536 + int(g.integers(1, 300))))
+        sets.append(np.unique(np.concatenate(v)).astype(np.uint32))
+    return sets
+
+
+def _mixed(g):
+    """Bitmap chunks, long and short lists in the same rows, chunks missing."""
+    sets = []
+    for r in range(60):
+        v = []
+        for c in np.flatnonzero(g.random(40) < 0.5):
+            n = int((3, 300, 4095, 9000)[int(g.integers(0, 4))])
+            v.append(np.sort(g.choice(65536, size=n, replace=False)) + (int(c) << 16))
+        sets.append(np.concatenate(v).astype(np.uint32) if v else np.array([5], np.uint32))
+    return sets
+
+
+CORPORA = {"short": _short, "lists": _lists, "runs": _runs, "mixed": _mixed}
+# forced engines: postings list by list / row sweep / run sweep, transposed panel, tensor rows, the planner's choice
+MODES = ("lists", "rows", "runs", "panel", "tensor", "auto")
+
+
+@pytest.mark.parametrize("mode", MODES)
+@pytest.mark.parametrize("corpus", sorted(CORPORA))
+def test_walks_match_oracle(sb, corpus, mode):
+    sets = CORPORA[corpus](gen.rng(len(corpus) * 7 + 1))
+    vals, offs = gen.to_csr(sets)
+    want, ws = ol.sets_matrix(vals, offs)
+    s = sb.Storm()
+    s.add_rows(vals, offs)
+    if mode in ("lists", "rows", "runs"):
+        s.set_panel(0)
+        s.set_sparse_postings({"lists": 2, "rows": 3, "runs": 4}[mode])
+    elif mode == "panel":
+        s.set_panel(2)
+    elif mode == "tensor":
+        s.set_dense_block(1e-12)
+    got, total = s.matrix()
+    np.testing.assert_array_equal(got, want)
+    assert total == ws
+    assert s.pairw_intersect_cardinality() == ws
+    other = sb.Storm()
+    other.add_rows(vals, offs)
+    assert s.square(other) == 2 * ws + int(sum(len(v) for v in sets))
+    s.close()
+    other.close()
+
+
+@pytest.mark.parametrize("universe", (1 << 20, (1 << 27) + 12345, 1 << 30))
+def test_zone_maps_of_row_blocks(sb, universe):
+    """Kernel-layer blocks whose rows' occupancy is folded in shared memory and
+    (past 2^27 values) converted row by row: clustered rows, most tiles rejected."""
+    g = gen.rng(11)
+    sets = [np.unique((int(g.integers(0, 8)) * (universe // 8) + g.integers(0, 3000, size=600)).clip(max=universe - 1))
+            .astype(np.uint32) for _ in range(200)]
+    vals, offs = gen.to_csr(sets)
+    _, ws = ol.sets_matrix(vals, offs)
+    r = sb.StormRows(universe)
+    r.set_bitmap_budget(0)
+    for v in sets:
+        r.add(v)
+    assert r.allpairs_sum(sb.POLICY_PERTILE, 32)[0] == ws
+    assert r.allpairs_sum(sb.POLICY_PERTILE, 64)[0] == ws
+    r.close()
