@@ -227,7 +227,31 @@ void ChunkDev::upload(const ChunkPack& p, cudaStream_t st) {
     n_rows = p.rows();
     facts = p.facts;
     max_cid = p.max_cid;
+    order_rows();
     SB_CUDA(cudaStreamSynchronize(st));
+}
+
+// The planner wants the rows heaviest first on every call; the order belongs to
+// the rows and is made with their upload (a radix sort: 20000 rows in 0.1 ms; a
+// comparison sort per call took 1.1).
+void ChunkDev::order_rows() {
+    const uint64_t n = facts.size();
+    by_card.resize(n);
+    uint64_t most = 0;
+    for (uint64_t r = 0; r < n; ++r) {
+        by_card[r] = (uint32_t)r;
+        most = std::max(most, facts[r].card);
+    }
+    std::vector<uint32_t> other(n);
+    std::vector<uint64_t> at(2049);
+    for (int shift = 0; shift < 64 && most >> shift; shift += 11) {
+        std::fill(at.begin(), at.end(), 0);
+        auto digit = [&](uint32_t r) { return 2047 - (facts[r].card >> shift & 2047); };   // largest first
+        for (uint32_t r : by_card) ++at[digit(r) + 1];
+        for (uint64_t k = 0; k < 2048; ++k) at[k + 1] += at[k];
+        for (uint32_t r : by_card) other[at[digit(r)]++] = r;
+        by_card.swap(other);
+    }
 }
 
 PinnedStage::~PinnedStage() {
@@ -566,6 +590,7 @@ void ChunkDev::upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStre
         if (dup[r]) facts[r].plain = false;
         facts[r].runs = runs[r];
     }
+    order_rows();
 }
 
 void copy_to_host(uint32_t* out, const uint32_t* d_src, uint64_t count, cudaStream_t st, PinnedStage& stage) {
@@ -674,9 +699,9 @@ __device__ __forceinline__ void tri_decode(uint64_t n, uint64_t p, uint64_t& i, 
     j = p - S(i) + i;
 }
 
-// Expands plain rows into contiguous bitmaps: local row r of X (W words,
-// W = 1024 x chunk slots, in layout `lay`: chunk slot s of row r -- one
-// 1024-word block -- at X + r x pitch + s x kstride) is row rows[r]. A warp
+// Expands chunk slots [s0, s0 + ns) of plain rows (`slots` in all) into
+// contiguous bitmaps: local row r of X (in layout `lay`: chunk slot s0 + s of
+// row r -- one 1024-word block -- at X + r x pitch + s x kstride) is row rows[r]. A warp
 // per (row, chunk slot): absent chunks and padding rows (~0) become zeros,
 // bitmap chunks are copied, list chunks are set bit by bit in a shared-memory
 // copy of the chunk and written out. Bound: the 8 KiB written per item. A warp
@@ -739,16 +764,15 @@ __device__ __forceinline__ void warp_list8(const uint16_t* __restrict__ l, uint3
 }
 
 __global__ void __launch_bounds__(EXPAND_WARPS * 32)
-expand_rows_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t m, uint32_t W, RowLayout lay,
-                   uint64_t* __restrict__ X) {
+expand_rows_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t m, uint32_t s0, uint32_t ns, uint32_t slots,
+                   RowLayout lay, uint64_t* __restrict__ X) {
     __shared__ __align__(16) uint32_t chunk[EXPAND_WARPS][2 * CHUNK_WORDS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t slots = W / CHUNK_WORDS;
-    const uint64_t items = (uint64_t)m * slots, nw = (uint64_t)gridDim.x * EXPAND_WARPS;
+    const uint64_t items = (uint64_t)m * ns, nw = (uint64_t)gridDim.x * EXPAND_WARPS;
     for (uint64_t it = (uint64_t)blockIdx.x * EXPAND_WARPS + warp; it < items; it += nw) {
-        const uint32_t r = (uint32_t)(it % m), s = (uint32_t)(it / m);
+        const uint32_t r = (uint32_t)(it % m), sl = (uint32_t)(it / m), s = s0 + sl;
         const uint32_t row = rows[r];
-        uint4* dst = reinterpret_cast<uint4*>(X + (uint64_t)r * lay.pitch + (uint64_t)s * lay.kstride);
+        uint4* dst = reinterpret_cast<uint4*>(X + (uint64_t)r * lay.pitch + (uint64_t)sl * lay.kstride);
         uint64_t pos = 0;
         bool have = false;
         if (row != ~0u) {
@@ -849,82 +873,119 @@ chunk_pairs_kernel(ChunkView v, uint32_t mode, uint64_t n1, uint64_t n2, uint64_
 // ---- postings: pairs of plain rows without bitmap chunks ----------------
 // value of entry e of list chunk c: cid << 16 | entry (universe <= 2^27)
 
-// A CTA per row, its warps over groups of `group` (1 .. 32) consecutive
-// chunks: f(value) for every list entry, g(chunk) -- warp-cooperative -- for
-// every bitmap chunk. Rows of long lists take group 1 (a warp per chunk, eight
-// entries per lane); rows of short ones (a chunk of a very sparse row holds a
-// handful of values) group 32, the warp walking the concatenated entries of 32
-// chunks, whose kinds and places it reads side by side. With a warp per row
-// and one chunk at a time, the 200 rows of a small container left the GPU idle
-// and 20000 rows of 6 values per chunk most lanes.
-constexpr uint32_t ROW_WALK_THREADS = 256;
-
-template <class F, class G>
-__device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint32_t group, F f, G g) {
-    const int lane = threadIdx.x & 31;
-    const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
-    const uint32_t warps = blockDim.x >> 5;
+// Group `g0` .. of `group` (1 .. 32) consecutive chunks [cg, c1) of a row, one
+// warp: f(value) for every list entry, h(chunk) -- warp-cooperative -- for
+// every bitmap chunk. Long lists are walked one chunk at a time (group 1,
+// eight entries per lane); of short ones (a chunk of a very sparse row holds a
+// handful of values) the warp walks the concatenated entries of 32 chunks,
+// whose kinds and places it reads side by side.
+template <class F, class H>
+__device__ __forceinline__ void walk_group_chunks(const ChunkView& v, uint64_t cg, uint64_t c1, uint32_t group, int lane,
+                                                  F f, H h) {
     if (group == 1) {
-        for (uint64_t c = c0 + (threadIdx.x >> 5); c < c1; c += warps) {
-            const uint32_t k = v.ckl[c], base = v.cid[c] << 16;
-            if (k & CK_BITMAP) {
-                g(c);
-                continue;
-            }
-            warp_list8(v.lst + v.coff[c], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
-#pragma unroll
-                for (uint32_t q = 0; q < 8; ++q)
-                    if (q < cnt) f(base | x[q]);
-            });
+        const uint32_t k = v.ckl[cg], base = v.cid[cg] << 16;
+        if (k & CK_BITMAP) {
+            h(cg);
+            return;
         }
+        warp_list8(v.lst + v.coff[cg], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
+#pragma unroll
+            for (uint32_t q = 0; q < 8; ++q)
+                if (q < cnt) f(base | x[q]);
+        });
         return;
     }
-    for (uint64_t cg = c0 + (uint64_t)(threadIdx.x >> 5) * group; cg < c1; cg += (uint64_t)warps * group) {
-        const uint64_t c = cg + lane;
-        const bool in = lane < (int)group && c < c1;
-        const uint32_t k = in ? v.ckl[c] : 0u;
-        const uint32_t base = in ? v.cid[c] << 16 : 0u;
-        const uint64_t off = in ? v.coff[c] : 0ull;
-        for (uint32_t bm = __ballot_sync(0xffffffffu, (k & CK_BITMAP) != 0); bm; bm &= bm - 1)
-            g(cg + (uint32_t)(__ffs(bm) - 1));
-        const uint32_t len = k & CK_BITMAP ? 0u : k & CK_LEN;
-        const uint32_t incl = warp_incl_scan(len, lane), excl = incl - len;
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
-            const uint32_t t = t0 + lane;
-            uint32_t o = 0;                // the last chunk of the group whose entries start at or before t
+    const uint64_t c = cg + lane;
+    const bool in = lane < (int)group && c < c1;
+    const uint32_t k = in ? v.ckl[c] : 0u;
+    const uint32_t base = in ? v.cid[c] << 16 : 0u;
+    const uint64_t off = in ? v.coff[c] : 0ull;
+    for (uint32_t bm = __ballot_sync(0xffffffffu, (k & CK_BITMAP) != 0); bm; bm &= bm - 1)
+        h(cg + (uint32_t)(__ffs(bm) - 1));
+    const uint32_t len = k & CK_BITMAP ? 0u : k & CK_LEN;
+    const uint32_t incl = warp_incl_scan(len, lane), excl = incl - len;
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+        const uint32_t t = t0 + lane;
+        uint32_t o = 0;                    // the last chunk of the group whose entries start at or before t
 #pragma unroll
-            for (uint32_t step = 16; step; step >>= 1)
-                if (__shfl_sync(0xffffffffu, excl, o + step) <= t) o += step;
-            const uint32_t e = t - __shfl_sync(0xffffffffu, excl, o), b = __shfl_sync(0xffffffffu, base, o);
-            const uint64_t at = __shfl_sync(0xffffffffu, off, o);
-            if (t < total) f(b | v.lst[at + e]);
-        }
+        for (uint32_t step = 16; step; step >>= 1)
+            if (__shfl_sync(0xffffffffu, excl, o + step) <= t) o += step;
+        const uint32_t e = t - __shfl_sync(0xffffffffu, excl, o), b = __shfl_sync(0xffffffffu, base, o);
+        const uint64_t at = __shfl_sync(0xffffffffu, off, o);
+        if (t < total) f(b | v.lst[at + e]);
     }
 }
 
-// Chunks per group of row_walk for rows of `chunks` chunks holding `entries`
-// list entries in all: one from 48 entries a chunk on.
-static uint32_t walk_group(uint64_t chunks, uint64_t entries, bool bitmaps) {
-    return bitmaps || entries >= 48 * chunks ? 1u : 32u;
+// One row by a CTA: its warps take every eighth group of the row's chunks.
+constexpr uint32_t ROW_WALK_THREADS = 256;
+
+template <class F, class H>
+__device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint32_t group, F f, H h) {
+    const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
+    for (uint64_t cg = c0 + (uint64_t)(threadIdx.x >> 5) * group; cg < c1; cg += (uint64_t)(blockDim.x >> 5) * group)
+        walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, f, h);
 }
+
+// Every row, group by group: all rows' first groups, then all rows' second
+// ones (rows have at most `groups` each), so that the warps at work meet in one
+// part of the universe and what they update -- 4 bytes per value somewhere in
+// it -- stays in L2. With a warp (or CTA) per row, 200 mixed rows left the GPU
+// idle, and the places of 20000 rows' values (67 MB of cursors, 134 of
+// postings) were written from DRAM.  f(r, value), h(chunk).
+template <class F, class H>
+__device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __restrict__ rows, uint32_t nq,
+                                          uint32_t group, uint32_t groups, F f, H h) {
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, items = (uint64_t)nq * groups;
+    for (uint64_t it = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += nw) {
+        const uint32_t r = (uint32_t)(it % nq);
+        const uint32_t row = rows ? rows[r] : r;
+        const uint64_t cg = v.row_off[row] + it / nq * group, c1 = v.row_off[row + 1];
+        if (cg < c1)
+            walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, [&](uint32_t x) { f(r, x); }, h);
+    }
+}
+
+// How rows_walk and row_walk take a set of rows: chunks per group (one from 48
+// entries a chunk on, or with bitmap chunks) and groups of the longest row.
+struct WalkShape {
+    uint32_t group = 1, groups = 0;
+    template <class Facts>
+    void of(uint64_t n, Facts facts) {
+        uint64_t chunks = 0, entries = 0;
+        uint32_t most = 0;
+        bool bitmaps = false;
+        for (uint64_t k = 0; k < n; ++k) {
+            const ChunkRowFacts& f = facts(k);
+            chunks += f.chunks;
+            entries += f.list_entries;
+            bitmaps |= f.bitmap_chunks != 0;
+            most = std::max(most, f.chunks);
+        }
+        group = bitmaps || entries >= 48 * chunks ? 1u : 32u;
+        groups = (most + group - 1) / group;
+    }
+    uint32_t grid(uint64_t n, int sms) const {
+        return (uint32_t)std::max<uint64_t>(
+            1, std::min<uint64_t>((n * groups + ROW_WALK_THREADS / 32 - 1) / (ROW_WALK_THREADS / 32), (uint64_t)sms * 8));
+    }
+};
 
 // rows == nullptr: rows [0, nq). Bitmap chunks count every set bit (only the
 // sums over pairs send rows that have them).
 __global__ void __launch_bounds__(ROW_WALK_THREADS)
-postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group,
+postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
                      uint32_t* __restrict__ counts) {
     const int lane = threadIdx.x & 31;
-    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x)
-        row_walk(
-            v, rows ? rows[r] : r, group, [&](uint32_t x) { atomicAdd(&counts[x], 1u); },
-            [&](uint64_t c) {
-                const uint64_t* wd = v.bm + v.coff[c];
-                const uint32_t base = v.cid[c] << 16;
-                for (uint32_t w = lane; w < CHUNK_WORDS; w += 32)
-                    for (uint64_t x = wd[w]; x; x &= x - 1)
-                        atomicAdd(&counts[base | (w << 6) | (uint32_t)__ffsll((long long)x) - 1u], 1u);
-            });
+    rows_walk(
+        v, rows, nq, group, groups, [&](uint32_t, uint32_t x) { atomicAdd(&counts[x], 1u); },
+        [&](uint64_t c) {
+            const uint64_t* wd = v.bm + v.coff[c];
+            const uint32_t base = v.cid[c] << 16;
+            for (uint32_t w = lane; w < CHUNK_WORDS; w += 32)
+                for (uint64_t x = wd[w]; x; x &= x - 1)
+                    atomicAdd(&counts[base | (w << 6) | (uint32_t)__ffsll((long long)x) - 1u], 1u);
+        });
 }
 
 // sum over values of a[x] * b[x] into flags->sum: the rectangle sum of two
@@ -1033,15 +1094,16 @@ postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t*
 // Writes each Q row's position in the Q list (its local index) into the
 // lists of its values; start[x] advances to the end of x's list.
 __global__ void __launch_bounds__(ROW_WALK_THREADS)
-postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group,
+postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
                         uint32_t* __restrict__ start, uint32_t* __restrict__ post) {
-    for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x)
-        row_walk(
-            v, rows[r], group,
-            [&](uint32_t x) {
-                if (start[x] != ~0u) post[atomicAdd(&start[x], 1u)] = r;
-            },
-            [](uint64_t) {});
+    rows_walk(
+        v, rows, nq, group, groups,
+        [&](uint32_t r, uint32_t x) {
+            // a value of one row has start ~0, and its one row adds to it once
+            const uint32_t at = atomicAdd(&start[x], 1u);
+            if (at != ~0u) post[at] = r;
+        },
+        [](uint64_t) {});
 }
 
 // One increment per (pair of rows, shared value): thread per list for lists
@@ -1081,67 +1143,68 @@ __global__ void postings_pairs_kernel(const uint2* __restrict__ lists, uint64_t 
 // Row sweep: CTA per Q row a; for every value of a, the rows b > a on that
 // value's list get one shared-memory increment; then a's slice of the
 // triangle (its Q partners b > a and its diagonal) is written once, in
-// ascending order. The row's entries are split evenly over the threads (a
-// shared-memory prefix of its chunk lengths maps entry -> chunk), so rows of
-// one long chunk and rows of many short ones both keep every thread busy.
+// ascending order. Bound: the random reads of a value's count, end and list
+// (three sectors, from L2 in part), hidden by full SMs: counts of 16 bits
+// (kSmall, no row of more than 65535 values) let four CTAs share an SM.
 // Partners are counted for one block of local indices [pb0, pb0 + pbn) per
 // launch (at most POST_SWEEP_MAX_ROWS, the counters shared memory holds):
 // more postings rows take one launch per block, each reading a row's lists
 // again; the launch of block 0 writes the diagonal.
-// Shared memory: pbn counters, then up to POST_SWEEP_MAX_CHUNKS + 1 prefix
-// words. Lists hold local indices, list x is [end[x] - counts[x], end[x]).
-constexpr uint32_t POST_SWEEP_THREADS = 256;
-constexpr uint32_t POST_SWEEP_MAX_CHUNKS = 2048;  // universe <= 2^27
-constexpr uint32_t POST_SWEEP_MAX_ROWS = 51200;   // 200 KiB of counters + 8 KiB of prefix
+// Lists hold local indices, list x is [end[x] - counts[x], end[x]).
+constexpr uint32_t POST_SWEEP_THREADS = 256;      // run sweep
+constexpr uint32_t POST_ROWS_THREADS = 512;
+constexpr uint32_t POST_SWEEP_MAX_ROWS = 51200;   // 200 KiB of counters
 
-__global__ void __launch_bounds__(POST_SWEEP_THREADS)
-postings_rows_kernel(ChunkView v, const uint32_t* __restrict__ qrows, uint32_t nq, const uint32_t* __restrict__ counts,
-                     const uint32_t* __restrict__ end, const uint32_t* __restrict__ post, uint64_t n,
-                     uint32_t* __restrict__ out, uint32_t pb0, uint32_t pbn) {
+template <bool kSmall>
+__global__ void __launch_bounds__(POST_ROWS_THREADS)
+postings_rows_kernel(ChunkView v, const uint32_t* __restrict__ qrows, uint32_t nq, bool all_rows, uint32_t group,
+                     const uint32_t* __restrict__ counts, const uint32_t* __restrict__ end,
+                     const uint32_t* __restrict__ post, uint64_t n, uint32_t* __restrict__ out, uint32_t pb0,
+                     uint32_t pbn) {
     extern __shared__ uint32_t cnt[];
-    uint32_t* pref = cnt + pbn;                // pref[k] = entries of the row's chunks before chunk k
+    __shared__ uint32_t card;
     const uint32_t pb1 = pb0 + pbn;
+    const uint32_t words = kSmall ? (pbn + 1) / 2 : pbn;
     for (uint32_t a = blockIdx.x; a < nq; a += gridDim.x) {
         if (a + 1 >= pb1 && pb0 > 0) continue;     // no partner after a in this block, diagonal not here
         const uint32_t row = qrows[a];
-        const uint64_t c0 = v.row_off[row];
-        const uint32_t nc = (uint32_t)(v.row_off[row + 1] - c0);   // <= POST_SWEEP_MAX_CHUNKS (plain rows)
-        for (uint32_t b = threadIdx.x; b < pbn; b += blockDim.x) cnt[b] = 0;
-        if (threadIdx.x == 0) {
-            uint32_t acc = 0;
-            for (uint32_t k = 0; k < nc; ++k) {
-                pref[k] = acc;
-                acc += v.ckl[c0 + k] & CK_LEN;
-            }
-            pref[nc] = acc;
-        }
+        const uint32_t w0 = a + 1 <= pb0 ? 0u : kSmall ? (a + 1 - pb0) / 2 : a + 1 - pb0;
+        for (uint32_t b = w0 + threadIdx.x; b < words; b += blockDim.x) cnt[b] = 0;
+        if (threadIdx.x == 0) card = 0;
         __syncthreads();
-        const uint32_t total = pref[nc];
-        const uint32_t work = a + 1 < pb1 ? total : 0u;   // no partner in the block: the diagonal only
-        for (uint32_t e = threadIdx.x; e < work; e += blockDim.x) {
-            uint32_t lo = 0, hi = nc;              // last chunk k with pref[k] <= e
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (pref[mid] <= e) lo = mid;
-                else hi = mid;
-            }
-            const uint64_t c = c0 + lo;
-            const uint32_t x = (v.cid[c] << 16) | v.lst[v.coff[c] + (e - pref[lo])];
-            const uint32_t len = counts[x];
-            if (len < 2) continue;
-            const uint32_t e1 = end[x];
-            for (uint32_t k = e1 - len; k < e1; ++k) {
-                const uint32_t b = post[k];
-                if (b > a && b >= pb0 && b < pb1) atomicAdd(&cnt[b - pb0], 1u);
-            }
-        }
+        uint32_t mine = 0;
+        row_walk(
+            v, row, group,
+            [&](uint32_t x) {
+                ++mine;
+                const uint32_t len = counts[x], e1 = end[x];
+                if (len < 2) return;
+                for (uint32_t k = e1 - len; k < e1; k += 4) {
+                    uint32_t b[4];                 // read together: the increments between them would part the reads
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) b[q] = k + q < e1 ? __ldg(post + k + q) : 0u;
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) {
+                        if (b[q] <= a || b[q] < pb0 || b[q] >= pb1) continue;
+                        const uint32_t at = b[q] - pb0;
+                        if (kSmall) atomicAdd(&cnt[at >> 1], at & 1u ? 0x10000u : 1u);
+                        else atomicAdd(&cnt[at], 1u);
+                    }
+                }
+            },
+            [](uint64_t) {});
+        mine = warp_sum_u32(mine);
+        if ((threadIdx.x & 31) == 0 && mine) atomicAdd(&card, mine);
         __syncthreads();
         const uint64_t base = tri_index(n, row, row) - row;   // out index of (row, j) is base + j
+#pragma unroll 4
         for (uint32_t b = (a + 1 > pb0 ? a + 1 : pb0) + threadIdx.x; b < pb1; b += blockDim.x) {
-            const uint32_t gb = qrows[b];   // ascending: gb > row (the other order kept exact too)
-            out[gb > row ? base + gb : tri_index(n, gb, row)] = cnt[b - pb0];
+            const uint32_t gb = all_rows ? b : qrows[b];   // ascending: gb > row (the other order kept exact too)
+            const uint32_t q = b - pb0;
+            const uint32_t c = kSmall ? (cnt[q >> 1] >> (16 * (q & 1u))) & 0xFFFFu : cnt[q];
+            __stcs(out + (gb > row ? base + gb : tri_index(n, gb, row)), c);
         }
-        if (threadIdx.x == 0 && pb0 == 0) out[base + row] = total;
+        if (threadIdx.x == 0 && pb0 == 0) out[base + row] = card;
         __syncthreads();
     }
 }
@@ -1174,77 +1237,224 @@ __device__ __forceinline__ void run_bitmap_word(const uint64_t* wd, uint32_t nwc
     run_word_masks(x, cin, nin, wi, wlog, starts, lasts);
 }
 
-// A warp over a list chunk, eight entries per lane: f(value, starts, lasts)
-// per entry, in order of the lanes; `at` counts and the warp's running totals
-// are f's business. Entries of the neighbouring lanes decide a lane's first
-// and last one (run_pieces.cuh states the rules).
-template <class F>
-__device__ __forceinline__ void run_list_walk(const uint16_t* __restrict__ l, uint32_t nl, uint32_t wmask, int lane, F f) {
-    uint32_t carry = 0x10000u;             // the entry before the warp's first (none: nothing is its successor)
-    uint32_t e0 = 0;
-    warp_list8(l, nl, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
-        const uint32_t up = __shfl_up_sync(0xffffffffu, (uint32_t)x[7], 1);
-        const uint32_t dn = __shfl_down_sync(0xffffffffu, (uint32_t)x[0], 1);
-        const uint32_t before = lane ? up : carry;
-        const uint32_t e = e0 + 8 * lane;
-        const uint32_t after = e + 8 < nl ? (lane < 31 ? dn : (uint32_t)l[e + 8]) : 0x20000u;
-        uint32_t st = 0, la = 0;           // bit k: entry e + k starts / ends a piece
+// Eight consecutive entries of a strictly increasing list, two per word, with
+// the entry before them: bit k of the result says that entry k starts a piece
+// (run_pieces.cuh: after a gap, or at a bin's first value). Pairs of 16-bit
+// entries at a time.
+__device__ __forceinline__ uint32_t run_starts8(const uint32_t (&w)[4], uint32_t before, uint32_t wmask) {
+    uint32_t st = 0;
+    uint32_t prev = before << 16;          // entry -1 in the upper half
 #pragma unroll
-        for (uint32_t k = 0; k < 8; ++k) {
-            if (k >= cnt) continue;
-            const uint32_t v = x[k], p = k ? (uint32_t)x[k - 1] : before;
-            const uint32_t n = k + 1 < cnt ? (uint32_t)x[k < 7 ? k + 1 : 7] : after;
-            if (v != p + 1 || (v & wmask) == 0) st |= 1u << k;
-            if (n != v + 1 || ((v + 1) & wmask) == 0) la |= 1u << k;
-        }
-        f(x, st, la);
-        carry = __shfl_sync(0xffffffffu, (uint32_t)x[7], 31);
-        e0 += 256;
-    });
+    for (uint32_t q = 0; q < 4; ++q) {
+        const uint32_t pw = __byte_perm(prev, w[q], 0x5432);          // the entries before these two
+        const uint32_t gap = __vcmpne2(__vsub2(w[q], pw), 0x00010001u);
+        const uint32_t bin = __vcmpeq2(w[q] & (wmask | wmask << 16), 0u);
+        const uint32_t m = gap | bin;
+        st |= ((m & 1u) | (m >> 15 & 2u)) << (2 * q);
+        prev = w[q];
+    }
+    return st;
 }
 
-// Pieces per row, per chunk and per bin; CTA per row, a warp per chunk.
+// Entry k of eight packed ones.
+__device__ __forceinline__ uint32_t entry8(const uint32_t (&w)[4], uint32_t k) {
+    const uint32_t lo = k & 2u ? w[1] : w[0], hi = k & 2u ? w[3] : w[2];
+    return (k & 4u ? hi : lo) >> (16 * (k & 1u)) & 0xFFFFu;
+}
+
+// Eight entries of a list from e on (fewer at its end: zeros follow).
+__device__ __forceinline__ void list_load8(const uint16_t* __restrict__ l, uint32_t nl, uint32_t e, uint32_t (&w)[4]) {
+    if (e + 8 <= nl) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(l + e));
+        w[0] = v.x;
+        w[1] = v.y;
+        w[2] = v.z;
+        w[3] = v.w;
+    } else {
+#pragma unroll
+        for (uint32_t q = 0; q < 4; ++q) {
+            const uint32_t a = e + 2 * q < nl ? l[e + 2 * q] : 0u, b = e + 2 * q + 1 < nl ? l[e + 2 * q + 1] : 0u;
+            w[q] = a | b << 16;
+        }
+    }
+}
+
+// The list and bitmap chunks [c0, c1) of a row by one warp, in order: list
+// chunks in steps of 256 entries as f(chunk, its first value, step's entries w,
+// starts, lasts) with bits per entry, then done(chunk); bitmap chunks as
+// h(chunk). The kinds and places of 32 chunks are read side by side, and the
+// next step's entries -- of this chunk or the next one -- are on their way while
+// this one's are worked on (a chunk of a row of runs is a few hundred entries:
+// one or two steps, which their loads would make wait).
+template <class F, class D, class H>
+__device__ __forceinline__ void run_chunks(const ChunkView& v, uint64_t c0, uint64_t c1, uint32_t wmask, int lane, F f,
+                                           D done, H h) {
+    for (uint64_t cg = c0; cg < c1; cg += 32) {
+        const bool in = cg + lane < c1;
+        const uint32_t kk = in ? v.ckl[cg + lane] : 0u, bb = in ? v.cid[cg + lane] << 16 : 0u;
+        const uint64_t off = in ? v.coff[cg + lane] : 0ull;
+        const uint32_t m = (uint32_t)(c1 - cg < 32 ? c1 - cg : 32);
+        uint32_t nw[4] = {0, 0, 0, 0};
+        uint32_t k = __shfl_sync(0xffffffffu, kk, 0);
+        const uint16_t* l = v.lst + __shfl_sync(0xffffffffu, off, 0);
+        if (!(k & CK_BITMAP)) list_load8(l, k & CK_LEN, 8 * lane, nw);
+        for (uint32_t j = 0; j < m; ++j) {
+            const uint32_t base = __shfl_sync(0xffffffffu, bb, j);
+            // the chunk after this one
+            const uint32_t k2 = j + 1 < m ? __shfl_sync(0xffffffffu, kk, j + 1) : CK_BITMAP;
+            const uint16_t* l2 = v.lst + __shfl_sync(0xffffffffu, off, (j + 1) & 31);
+            const uint32_t nl = k & CK_BITMAP ? 0u : k & CK_LEN;
+            if (nl == 0 && !(k2 & CK_BITMAP)) list_load8(l2, k2 & CK_LEN, 8 * lane, nw);
+            if (k & CK_BITMAP) {
+                h(cg + j);
+            } else {
+                uint32_t carry = 0;
+                for (uint32_t e0 = 0; e0 < nl; e0 += 256) {
+                    const uint32_t e = e0 + 8 * lane;
+                    const uint32_t w[4] = {nw[0], nw[1], nw[2], nw[3]};
+                    if (e0 + 256 < nl) list_load8(l, nl, e + 256, nw);
+                    else if (!(k2 & CK_BITMAP)) list_load8(l2, k2 & CK_LEN, 8 * lane, nw);
+                    const uint32_t last = w[3] >> 16;
+                    const uint32_t up = __shfl_up_sync(0xffffffffu, last, 1);
+                    uint32_t st = run_starts8(w, lane ? up : carry, wmask);
+                    if (e == 0) st |= 1u;
+                    const uint32_t cnt = e >= nl ? 0u : nl - e < 8 ? nl - e : 8u;
+                    st &= (1u << cnt) - 1u;
+                    // an entry ends a piece where the next one starts one, or is not there
+                    uint32_t next = __shfl_down_sync(0xffffffffu, st, 1) & 1u;
+                    const uint32_t nx = __shfl_sync(0xffffffffu, nw[0], 0) & 0xFFFFu;   // the next step's first
+                    if (lane == 31) next = nx != last + 1 || (nx & wmask) == 0;
+                    uint32_t la = (st >> 1 | next << 7) & ((1u << cnt) - 1u);
+                    if (cnt && e + cnt == nl) la |= 1u << (cnt - 1);
+                    f(cg + j, base, w, st, la);
+                    carry = __shfl_sync(0xffffffffu, last, 31);
+                }
+                done(cg + j);
+            }
+            k = k2;
+            l = l2;
+        }
+    }
+}
+
+// The same chunks a lane per list chunk, for rows made of long runs: in a
+// strictly increasing list entry e + 1 follows entry e exactly where value minus
+// index stays the same, so a run's last entry is found by halving -- at once,
+// when the rest of the list is one run -- and the entries in between are never
+// read. g(lane's chunk index within the share's 32, chunk, base, first, last)
+// per run, by the lane that found it; list_done(chunk) once per lane and list
+// chunk; bitmap chunks as h(chunk), warp-cooperative. (256 entries per step of
+// a warp are 250 instructions to look at them all: 4000 rows of 51000 values in
+// runs of 256 took 323 us to count and 458 to fill.)
+template <class G, class D, class H>
+__device__ __forceinline__ void gallop_chunks(const ChunkView& v, uint64_t c0, uint64_t c1, int lane, G g, D list_done,
+                                              H h) {
+    for (uint64_t cg = c0; cg < c1; cg += 32) {
+        const uint64_t c = cg + lane;
+        const uint32_t k = c < c1 ? v.ckl[c] : 0u;
+        if (c < c1 && !(k & CK_BITMAP)) {
+            const uint16_t* l = v.lst + v.coff[c];
+            const uint32_t base = v.cid[c] << 16, nl = k & CK_LEN;
+            uint32_t e = 0;
+            const uint32_t end = nl ? l[nl - 1] : 0u;
+            while (e < nl) {
+                const uint32_t x = l[e];
+                uint32_t lo = e, last = x;                 // l[lo] = last is in x's run
+                if (end - x == nl - 1 - e) {
+                    lo = nl - 1;
+                    last = end;
+                } else {
+                    uint32_t hi = nl - 1;                  // l[hi] is not
+                    while (hi - lo > 1) {
+                        const uint32_t mid = (lo + hi) >> 1, y = l[mid];
+                        if (y - x == mid - e) {
+                            lo = mid;
+                            last = y;
+                        } else {
+                            hi = mid;
+                        }
+                    }
+                }
+                g(c, base, x, last);
+                e = lo + 1;
+            }
+            list_done(c);
+        }
+        __syncwarp();
+        for (uint32_t bm = __ballot_sync(0xffffffffu, (k & CK_BITMAP) != 0); bm; bm &= bm - 1)
+            h(cg + (uint32_t)(__ffs(bm) - 1));
+    }
+}
+
+// Mean run length (log2) from which the rows' lists are galloped through.
+constexpr uint32_t RUN_GALLOP_WLOG = 6;
+
+// A row's chunks dealt to the warps of its CTA in consecutive shares.
+__device__ __forceinline__ void warp_share(uint64_t c0, uint64_t c1, uint64_t& lo, uint64_t& hi) {
+    constexpr uint32_t WARPS = ROW_WALK_THREADS / 32;
+    const uint32_t warp = threadIdx.x >> 5;
+    lo = c0 + (c1 - c0) * warp / WARPS;
+    hi = c0 + (c1 - c0) * (warp + 1) / WARPS;
+}
+
+// Pieces per row, per chunk and per bin; CTA per row.
+template <bool kGallop>
 __global__ void __launch_bounds__(ROW_WALK_THREADS)
 run_count_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
                  uint32_t* __restrict__ pieces, uint32_t* __restrict__ chunk_pieces, uint32_t* __restrict__ bins) {
     __shared__ uint32_t total;
     const int lane = threadIdx.x & 31;
-    const uint32_t wmask = (1u << wlog) - 1u;
     for (uint32_t r = blockIdx.x; r < nq; r += gridDim.x) {
         if (threadIdx.x == 0) total = 0;
         __syncthreads();
         const uint32_t row = rows[r];
-        const uint64_t c1 = v.row_off[row + 1];
-        for (uint64_t c = v.row_off[row] + (threadIdx.x >> 5); c < c1; c += ROW_WALK_THREADS / 32) {
-            const uint32_t base = v.cid[c] << 16;
-            const uint32_t k = v.ckl[c];
-            uint32_t cnt = 0;
-            if (k & CK_BITMAP) {
-                const uint64_t* wd = v.bm + v.coff[c];
-                const uint32_t nwc = k & CK_LEN;
-                uint64_t carry = 0, starts, lasts;
-                for (uint32_t w0 = 0; w0 < nwc; w0 += 32) {
-                    run_bitmap_word(wd, nwc, w0, lane, wlog, carry, starts, lasts);
-                    cnt += __popcll(starts);
-                    for (uint64_t x = starts; x; x &= x - 1)
-                        atomicAdd(&bins[(base + ((w0 + lane) << 6) + (uint32_t)(__ffsll((long long)x) - 1)) >> wlog],
-                                  1u);
-                }
-            } else {
-                run_list_walk(v.lst + v.coff[c], k & CK_LEN, wmask, lane,
-                              [&](const uint16_t (&x)[8], uint32_t st, uint32_t) {
-                                  cnt += __popc(st);
-#pragma unroll
-                                  for (uint32_t q = 0; q < 8; ++q)
-                                      if (st >> q & 1u) atomicAdd(&bins[(base | x[q]) >> wlog], 1u);
-                              });
-            }
-            cnt = warp_sum_u32(cnt);
+        uint64_t lo, hi;
+        warp_share(v.row_off[row], v.row_off[row + 1], lo, hi);
+        uint32_t cnt = 0, mine = 0;
+        auto warp_done = [&](uint64_t c) {     // the warp's chunk
+            const uint32_t t = warp_sum_u32(cnt);
             if (lane == 0) {
-                chunk_pieces[c] = cnt;
-                if (cnt) atomicAdd(&total, cnt);
+                chunk_pieces[c] = t;
+                mine += t;
             }
+            cnt = 0;
+        };
+        auto bitmap = [&](uint64_t c) {
+            const uint64_t* wd = v.bm + v.coff[c];
+            const uint32_t nwc = v.ckl[c] & CK_LEN, base = v.cid[c] << 16;
+            uint64_t carry = 0, starts, lasts;
+            for (uint32_t w0 = 0; w0 < nwc; w0 += 32) {
+                run_bitmap_word(wd, nwc, w0, lane, wlog, carry, starts, lasts);
+                cnt += __popcll(starts);
+                for (uint64_t x = starts; x; x &= x - 1)
+                    atomicAdd(&bins[(base + ((w0 + lane) << 6) + (uint32_t)(__ffsll((long long)x) - 1)) >> wlog], 1u);
+            }
+            warp_done(c);
+        };
+        if constexpr (kGallop) {
+            gallop_chunks(
+                v, lo, hi, lane,
+                [&](uint64_t, uint32_t base, uint32_t first, uint32_t last) {
+                    const uint32_t b1 = (base | last) >> wlog;
+                    for (uint32_t b = (base | first) >> wlog; b <= b1; ++b, ++cnt) atomicAdd(&bins[b], 1u);
+                },
+                [&](uint64_t c) {              // the lane's own chunk
+                    chunk_pieces[c] = cnt;
+                    mine += cnt;
+                    cnt = 0;
+                },
+                bitmap);
+        } else {
+            run_chunks(
+                v, lo, hi, (1u << wlog) - 1u, lane,
+                [&](uint64_t, uint32_t base, const uint32_t (&w)[4], uint32_t st, uint32_t) {
+                    cnt += __popc(st);
+                    for (uint32_t m = st; m; m &= m - 1) atomicAdd(&bins[(base | entry8(w, __ffs(m) - 1)) >> wlog], 1u);
+                },
+                warp_done, bitmap);
         }
+        mine = warp_sum_u32(mine);
+        if (lane == 0 && mine) atomicAdd(&total, mine);
         __syncthreads();
         if (threadIdx.x == 0) pieces[r] = total;
         __syncthreads();
@@ -1278,6 +1488,7 @@ __global__ void run_stats_kernel(const uint32_t* __restrict__ bins, uint64_t nb,
 // warp per row, 4000 rows of 51000 values took 1.24 ms, and counting 0.85.
 constexpr uint32_t RUN_MAX_CHUNKS = 2048;    // universe <= 2^27
 
+template <bool kGallop>
 __global__ void __launch_bounds__(ROW_WALK_THREADS)
 run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t wlog,
                 const uint64_t* __restrict__ poff, const uint32_t* __restrict__ chunk_pieces,
@@ -1310,45 +1521,63 @@ run_fill_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uin
             if (k < nc) first[k] = before + own[q];
         }
         __syncthreads();
-        for (uint32_t kc = warp; kc < nc; kc += ROW_WALK_THREADS / 32) {
-            const uint64_t c = c0 + kc;
-            const uint32_t base = v.cid[c] << 16;
-            const uint32_t k = v.ckl[c];
-            uint2* out = pieces + poff[r] + first[kc];
+        uint64_t lo, hi;
+        warp_share(c0, c0 + nc, lo, hi);
+        uint2* const out0 = pieces + poff[r];
+        auto bitmap = [&](uint64_t c) {
+            uint2* out = out0 + first[c - c0];
+            const uint64_t* wd = v.bm + v.coff[c];
+            const uint32_t nwc = v.ckl[c] & CK_LEN, base = v.cid[c] << 16;
+            uint64_t carry = 0, starts, lasts;
             uint32_t ks = 0, kl = 0;
-            if (k & CK_BITMAP) {
-                const uint64_t* wd = v.bm + v.coff[c];
-                const uint32_t nwc = k & CK_LEN;
-                uint64_t carry = 0, starts, lasts;
-                for (uint32_t w0 = 0; w0 < nwc; w0 += 32) {
-                    run_bitmap_word(wd, nwc, w0, lane, wlog, carry, starts, lasts);
-                    const uint32_t ns = (uint32_t)__popcll(starts), nls = (uint32_t)__popcll(lasts);
-                    const uint32_t xs = warp_incl_scan(ns, lane), xl = warp_incl_scan(nls, lane);
-                    const uint32_t at = base + ((w0 + lane) << 6);
-                    uint32_t j = ks + xs - ns;
-                    for (uint64_t x = starts; x; x &= x - 1) out[j++].x = at + (uint32_t)(__ffsll((long long)x) - 1);
-                    j = kl + xl - nls;
-                    for (uint64_t x = lasts; x; x &= x - 1) out[j++].y = at + (uint32_t)__ffsll((long long)x);
-                    ks += __shfl_sync(0xffffffffu, xs, 31);
-                    kl += __shfl_sync(0xffffffffu, xl, 31);
-                }
-            } else {
-                run_list_walk(v.lst + v.coff[c], k & CK_LEN, wmask, lane,
-                              [&](const uint16_t (&x)[8], uint32_t st, uint32_t la) {
-                                  // ranks of the lane's starts and lasts, 16 bits each (a step holds 256 entries)
-                                  const uint32_t both = __popc(st) | (uint32_t)__popc(la) << 16;
-                                  const uint32_t inc = warp_incl_scan(both, lane), exc = inc - both;
-                                  uint32_t js = ks + (exc & 0xFFFFu), jl = kl + (exc >> 16);
-#pragma unroll
-                                  for (uint32_t q = 0; q < 8; ++q) {
-                                      if (st >> q & 1u) out[js++].x = base | x[q];
-                                      if (la >> q & 1u) out[jl++].y = (base | x[q]) + 1u;
-                                  }
-                                  const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
-                                  ks += tot & 0xFFFFu;
-                                  kl += tot >> 16;
-                              });
+            for (uint32_t w0 = 0; w0 < nwc; w0 += 32) {
+                run_bitmap_word(wd, nwc, w0, lane, wlog, carry, starts, lasts);
+                const uint32_t ns = (uint32_t)__popcll(starts), nls = (uint32_t)__popcll(lasts);
+                const uint32_t xs = warp_incl_scan(ns, lane), xl = warp_incl_scan(nls, lane);
+                const uint32_t word0 = base + ((w0 + lane) << 6);
+                uint32_t j = ks + xs - ns;
+                for (uint64_t x = starts; x; x &= x - 1) out[j++].x = word0 + (uint32_t)(__ffsll((long long)x) - 1);
+                j = kl + xl - nls;
+                for (uint64_t x = lasts; x; x &= x - 1) out[j++].y = word0 + (uint32_t)__ffsll((long long)x);
+                ks += __shfl_sync(0xffffffffu, xs, 31);
+                kl += __shfl_sync(0xffffffffu, xl, 31);
             }
+        };
+        if constexpr (kGallop) {
+            uint32_t j = 0;                // pieces of the lane's chunk so far
+            gallop_chunks(
+                v, lo, hi, lane,
+                [&](uint64_t c, uint32_t base, uint32_t from, uint32_t last) {
+                    uint2* out = out0 + first[c - c0];
+                    const uint32_t end = (base | last) + 1u;
+                    for (uint32_t s = base | from; s < end;) {
+                        const uint32_t next = (s | wmask) + 1u;        // the next bin
+                        out[j++] = make_uint2(s, next < end ? next : end);
+                        s = next;
+                    }
+                },
+                [&](uint64_t) { j = 0; }, bitmap);
+        } else {
+            uint64_t at = ~0ull;           // the chunk being walked
+            uint32_t ks = 0, kl = 0;       // its starts and lasts so far
+            run_chunks(
+                v, lo, hi, wmask, lane,
+                [&](uint64_t c, uint32_t base, const uint32_t (&w)[4], uint32_t st, uint32_t la) {
+                    if (c != at) ks = kl = 0;
+                    at = c;
+                    uint2* out = out0 + first[c - c0];
+                    // ranks of the lane's starts and lasts, 16 bits each (a step holds 256 entries)
+                    const uint32_t both = __popc(st) | (uint32_t)__popc(la) << 16;
+                    const uint32_t inc = warp_incl_scan(both, lane), exc = inc - both;
+                    uint32_t j = ks + (exc & 0xFFFFu);
+                    for (uint32_t m = st; m; m &= m - 1) out[j++].x = base | entry8(w, __ffs(m) - 1);
+                    j = kl + (exc >> 16);
+                    for (uint32_t m = la; m; m &= m - 1) out[j++].y = (base | entry8(w, __ffs(m) - 1)) + 1u;
+                    const uint32_t tot = __shfl_sync(0xffffffffu, inc, 31);
+                    ks += tot & 0xFFFFu;
+                    kl += tot >> 16;
+                },
+                [](uint64_t) {}, bitmap);
         }
         __syncthreads();   // first is read before the next row's
     }
@@ -1542,18 +1771,12 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             std::vector<uint32_t> second(n2);
             for (uint64_t r = 0; r < n2; ++r) second[r] = (uint32_t)(n1 + r);
             SB_CUDA(cudaMemcpyAsync(d_qrows.p, second.data(), n2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            uint64_t chunks = 0, entries = 0;
-            bool bitmaps = false;
-            for (const ChunkRowFacts& f : d.facts) {
-                chunks += f.chunks;
-                entries += f.list_entries;
-                bitmaps |= f.bitmap_chunks != 0;
-            }
-            const uint32_t group = walk_group(chunks, entries, bitmaps);
-            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>(n1, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
-                d.view(), nullptr, (uint32_t)n1, group, d_counts.p);
-            postings_hist_kernel<<<(uint32_t)std::min<uint64_t>(n2, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
-                d.view(), d_qrows.p, (uint32_t)n2, group, d_start.p);
+            WalkShape ws;
+            ws.of(n1 + n2, [&](uint64_t r) -> const ChunkRowFacts& { return d.facts[r]; });
+            postings_hist_kernel<<<ws.grid(n1, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), nullptr, (uint32_t)n1, ws.group,
+                                                                              ws.groups, d_counts.p);
+            postings_hist_kernel<<<ws.grid(n2, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)n2,
+                                                                              ws.group, ws.groups, d_start.p);
             counts_dot_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, d_start.p, U, d_flags.p);
             SB_CUDA(cudaGetLastError());
             launches += 3;
@@ -1597,7 +1820,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
 
     SB_CUDA(cudaEventRecord(log.ev0, st));
     PostingsStats ps{};
-    uint32_t q_group = 1;                                  // row_walk's group for the postings rows
+    WalkShape q_walk;                                      // of the postings rows
     auto histogram = [&](const std::vector<uint32_t>& rows) {
         d_qrows.reserve(rows.size());
         SB_CUDA(cudaEventRecord(ev_hist0, st));
@@ -1606,17 +1829,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_counts.p, 0, U * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
-        uint64_t chunks = 0, entries = 0;
-        bool bitmaps = false;
-        for (uint32_t r : rows) {
-            chunks += d.facts[r].chunks;
-            entries += d.facts[r].list_entries;
-            bitmaps |= d.facts[r].bitmap_chunks != 0;
-        }
-        q_group = walk_group(chunks, entries, bitmaps);
-        const uint32_t gq = (uint32_t)std::min<uint64_t>(rows.size(), (uint64_t)sms * 64);
-        postings_hist_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)rows.size(), q_group,
-                                                             d_counts.p);
+        q_walk.of(rows.size(), [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[rows[k]]; });
+        postings_hist_kernel<<<q_walk.grid(rows.size(), sms), ROW_WALK_THREADS, 0, st>>>(
+            d.view(), d_qrows.p, (uint32_t)rows.size(), q_walk.group, q_walk.groups, d_counts.p);
         postings_stats_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_pstats.p);
         SB_CUDA(cudaGetLastError());
         SB_CUDA(cudaEventRecord(ev_hist, st));
@@ -1662,7 +1877,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         SB_CUDA(cudaMemsetAsync(d_rstats.p, 0, 2 * sizeof(unsigned long long), st));
         d_cpieces.reserve(d.cid.n);
         const uint32_t gq = (uint32_t)std::min<uint64_t>(q, (uint64_t)sms * 64);
-        run_count_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)q, rwlog, d_rpieces.p,
+        auto count = rwlog >= RUN_GALLOP_WLOG ? run_count_kernel<true> : run_count_kernel<false>;
+        count<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)q, rwlog, d_rpieces.p,
                                                          d_cpieces.p, d_rbins.p);
         run_stats_kernel<<<sms * 8, 256, 0, st>>>(d_rbins.p, n_bins, d_rstats.p);
         SB_CUDA(cudaGetLastError());
@@ -1785,9 +2001,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     };
     bool panel_plan = false;
     // The panel needs a block of expanded rows and its transpose in HBM.
-    const uint64_t panel_bytes = PANEL_ROWS * (W + panel_row_words(W)) * sizeof(uint64_t);
+    const uint64_t px_words = PANEL_ROWS * panel_row_words(W);
+    const uint64_t panel_bytes = (PANEL_ROWS * W + px_words) * sizeof(uint64_t);
     auto panel_fits = [&]() {
         if (!facts_ok || panel_mode == 0 || U > PANEL_MAX_UNIVERSE) return false;
+        if (d_DT.n >= PANEL_ROWS * W && d_pX.n >= px_words) return true;   // it is there already
         size_t fr = 0, tot = 0;
         SB_CUDA(cudaMemGetInfo(&fr, &tot));
         return (double)panel_bytes < 0.5 * ((double)fr + (double)(d_pX.n + d_DT.n) * sizeof(uint64_t));
@@ -1823,10 +2041,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         // the top h rows H, the next m rows M, the rest L; every row with a
         // bitmap chunk in H u M.  The cheaper predicted plan runs.
         std::vector<uint32_t> pl;
-        for (uint32_t r = 0; r < n; ++r)
+        pl.reserve(n);
+        for (uint32_t r : d.by_card)
             if (d.facts[r].plain) pl.push_back(r);
-        std::stable_sort(pl.begin(), pl.end(),
-                         [&](uint32_t x, uint32_t y) { return d.facts[x].card > d.facts[y].card; });
         const uint64_t np = pl.size();
         std::vector<double> S1(np + 1, 0.0), S2(np + 1, 0.0), S3(np + 1, 0.0);
         uint64_t lb = 0;                                   // rows [0, lb) hold every bitmap-chunk row
@@ -1866,7 +2083,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         // Plan B over candidate cuts (h, m).
         uint64_t best_h = 0, best_m = 0;
         double best_b = -1.0;
-        if (postings_mode < 0 && panel_mode != 0 && panel_fits()) {
+        if (postings_mode < 0 && panel_mode != 0 && facts_ok && U <= PANEL_MAX_UNIVERSE) {
             std::vector<uint64_t> cand{0, lb, np};
             for (double x = 1.0; x < (double)np; x *= 1.12) cand.push_back((uint64_t)x);
             std::sort(cand.begin(), cand.end());
@@ -1892,17 +2109,21 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                 }
             }
         }
-        panel_plan = best_b >= 0 && (panel_mode > 0 || best_b < best_a);
+        // the free memory is asked for last: the query takes up to milliseconds
+        panel_plan = best_b >= 0 && (panel_mode > 0 || best_b < best_a) && panel_fits();
         std::vector<uint32_t> rest;
         if (panel_plan) {
             dense.assign(pl.begin(), pl.begin() + best_h);
             mrows.assign(pl.begin() + best_h, pl.begin() + best_h + best_m);
-            rest.assign(pl.begin() + best_h + best_m, pl.end());
         } else {
             dense.assign(pl.begin(), pl.begin() + best_k);
-            rest.assign(pl.begin() + best_k, pl.end());
         }
-        std::sort(rest.begin(), rest.end());               // stored order: ascending output writes
+        {                                                  // stored order: ascending output writes
+            std::vector<uint8_t> is_rest(n, 0);
+            for (uint64_t t = panel_plan ? best_h + best_m : best_k; t < np; ++t) is_rest[pl[t]] = 1;
+            for (uint32_t r = 0; r < n; ++r)
+                if (is_rest[r]) rest.push_back(r);
+        }
         if (rest.size() >= 2) {
             // The estimate assumes independent rows; correlated rows share
             // more. With the exact count, keep the postings only if they beat
@@ -1953,7 +2174,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // 256-row block is all H or all tq and the tq x tq blocks can be left out.
     // Panels of P rows when they do not all fit the budget.
     if (panel_plan) {
-        d_pX.reserve(PANEL_ROWS * panel_row_words(W));
+        d_pX.reserve(px_words);
         d_DT.reserve(PANEL_ROWS * W);
     }
     const uint64_t nd0 = dense.size();
@@ -1962,7 +2183,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     uint64_t P = 0;
     if (ne) {
         uint64_t budget = dense_budget_bytes;
-        if (!budget) {
+        if (!budget && d_panel.n >= round_up(ne, 256) * panel_row_words(W)) {
+            budget = d_panel.n * sizeof(uint64_t);   // they fit the buffer of an earlier call
+        } else if (!budget) {
             size_t fr = 0, tot = 0;
             SB_CUDA(cudaMemGetInfo(&fr, &tot));
             budget = (uint64_t)(0.6 * (double)(fr + d_panel.n * sizeof(uint64_t)));
@@ -2054,8 +2277,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                                     cudaMemcpyHostToDevice, st));
             const uint32_t grid = (uint32_t)std::min<uint64_t>((m * slots + EXPAND_WARPS - 1) / EXPAND_WARPS,
                                                                (uint64_t)sms * 64);
-            expand_rows_kernel<<<grid, EXPAND_WARPS * 32, 0, st>>>(d.view(), d_map.p + slot, (uint32_t)m,
-                                                                   (uint32_t)W, lay, d_panel.p + slot * lay.pitch);
+            expand_rows_kernel<<<grid, EXPAND_WARPS * 32, 0, st>>>(d.view(), d_map.p + slot, (uint32_t)m, 0u,
+                                                                   (uint32_t)slots, (uint32_t)slots, lay,
+                                                                   d_panel.p + slot * lay.pitch);
             SB_CUDA(cudaGetLastError());
             ++launches;
         };
@@ -2170,8 +2394,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             for (uint32_t t = 0; t < PANEL_ROWS; ++t) bmap[t] = t < prows ? h_perm[pw0 + b0 + t] : ~0u;
             SB_CUDA(cudaMemcpyAsync(d_pmap.p, bmap.data(), PANEL_ROWS * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
             const RowLayout play{PANEL_PITCH, PANEL_ROWS * PANEL_PITCH};   // block-major, as the tensor panels
-            expand_rows_kernel<<<(uint32_t)sms * 64, EXPAND_WARPS * 32, 0, st>>>(d.view(), d_pmap.p, PANEL_ROWS,
-                                                                                (uint32_t)W, play, d_pX.p);
+            expand_rows_kernel<<<(uint32_t)sms * 64, EXPAND_WARPS * 32, 0, st>>>(
+                d.view(), d_pmap.p, PANEL_ROWS, 0u, (uint32_t)slots, (uint32_t)slots, play, d_pX.p);
             panel_transpose_kernel<<<(uint32_t)(W / PANEL_T_WORDS), 1024, PANEL_T_SMEM, st>>>(d_pX.p, play, d_DT.p);
             SB_CUDA(cudaMemsetAsync(d_ctr.p, 0, sizeof(unsigned long long), st));
             const uint32_t ni = (uint32_t)items.size();
@@ -2213,7 +2437,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
         const uint32_t gq = (uint32_t)std::min<uint64_t>((nq + 7) / 8, (uint64_t)sms * 16);
-        run_fill_kernel<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
+        auto fill = rwlog >= RUN_GALLOP_WLOG ? run_fill_kernel<true> : run_fill_kernel<false>;
+        fill<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
             d.view(), d_qrows.p, (uint32_t)nq, rwlog, d_rpoff.p, d_cpieces.p, d_pieces.p);
         postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, d_pstats.p);
         run_scatter_kernel<<<gq, 256, 0, st>>>((uint32_t)nq, rwlog, d_rpoff.p, d_pieces.p, d_rstart.p, d_rlist.p);
@@ -2240,19 +2465,28 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             d_lists.reserve(ps.lists ? ps.lists : 1);
             d_post.reserve(ps.entries ? ps.entries : 1);
             postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_counts.p, U, d_start.p, d_lists.p, d_pstats.p);
-            const uint32_t gq = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64);
-            postings_scatter_kernel<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)nq, q_group,
-                                                                    d_start.p, d_post.p);
+            postings_scatter_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
+                d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_start.p, d_post.p);
             if (sweep) {
-                static std::atomic<uint64_t> done{0};
-                smem_attr_once(postings_rows_kernel,
-                               (int)((POST_SWEEP_MAX_ROWS + POST_SWEEP_MAX_CHUNKS + 1) * sizeof(uint32_t)), done);
-                const uint32_t gr = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 8);
+                uint64_t most = 0;
+                for (uint32_t r : qrows) most = std::max(most, d.facts[r].card);
+                const bool small = most <= 0xFFFF;   // a count is at most its row's values
+                static std::atomic<uint64_t> done_s{0}, done_l{0};
+                const int smem_max = (int)(POST_SWEEP_MAX_ROWS * sizeof(uint32_t));
+                smem_attr_once(postings_rows_kernel<true>, smem_max / 2, done_s);
+                smem_attr_once(postings_rows_kernel<false>, smem_max, done_l);
+                const uint32_t gr = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 16);
+                // a row's groups over all the warps of its CTA
+                const uint32_t warps = POST_ROWS_THREADS / 32, chunks = q_walk.group * q_walk.groups;
+                const uint32_t group =
+                    q_walk.group == 1 ? 1u : std::max(2u, std::min(32u, (chunks + warps - 1) / warps));
                 for (uint64_t pb0 = 0; pb0 < nq; pb0 += POST_SWEEP_MAX_ROWS) {
                     const uint32_t pbn = (uint32_t)std::min<uint64_t>(POST_SWEEP_MAX_ROWS, nq - pb0);
-                    const uint32_t smem = (uint32_t)((pbn + POST_SWEEP_MAX_CHUNKS + 1) * sizeof(uint32_t));
-                    postings_rows_kernel<<<gr, POST_SWEEP_THREADS, smem, st>>>(
-                        d.view(), d_qrows.p, (uint32_t)nq, d_counts.p, d_start.p, d_post.p, n, d_out, (uint32_t)pb0, pbn);
+                    const uint32_t smem = (uint32_t)(small ? (pbn + 1) / 2 : pbn) * sizeof(uint32_t);
+                    auto kernel = small ? postings_rows_kernel<true> : postings_rows_kernel<false>;
+                    kernel<<<gr, POST_ROWS_THREADS, smem, st>>>(d.view(), d_qrows.p, (uint32_t)nq, nq == n, group,
+                                                               d_counts.p, d_start.p, d_post.p, n, d_out, (uint32_t)pb0,
+                                                               pbn);
                     ++launches;
                 }
                 launches += 2;

@@ -139,6 +139,7 @@ struct ChunkDev {
     DevBuf<uint16_t> lst;
     uint64_t n_rows = 0;
     std::vector<ChunkRowFacts> facts;   // host copy of the per-row facts
+    std::vector<uint32_t> by_card;      // rows by value count, largest first (equal ones in stored order)
     uint32_t max_cid = 0;
     uint64_t payload_bytes = 0;         // bitmap and list bytes of the last upload
     void upload(const ChunkPack& p, cudaStream_t st);
@@ -152,6 +153,7 @@ struct ChunkDev {
     void upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStream_t st, PinnedStage& stage);
     DevBuf<uint8_t> d_row_dup;
     DevBuf<uint32_t> d_row_runs;
+    void order_rows();                  // by_card from the facts
     ChunkView view() const {
         return ChunkView{row_off.p, cid.p, ckl.p, coff.p, bm.p, lst.p};
     }
