@@ -874,7 +874,7 @@ chunk_pairs_kernel(ChunkView v, uint32_t mode, uint64_t n1, uint64_t n2, uint64_
 // value of entry e of list chunk c: cid << 16 | entry (universe <= 2^27)
 
 // Group `g0` .. of `group` (1 .. 32) consecutive chunks [cg, c1) of a row, one
-// warp: f(value) for every list entry, h(chunk) -- warp-cooperative -- for
+// warp: f(value, its place in the list pool) for every list entry, h(chunk) -- warp-cooperative -- for
 // every bitmap chunk. Long lists are walked one chunk at a time (group 1,
 // eight entries per lane); of short ones (a chunk of a very sparse row holds a
 // handful of values) the warp walks the concatenated entries of 32 chunks,
@@ -888,10 +888,12 @@ __device__ __forceinline__ void walk_group_chunks(const ChunkView& v, uint64_t c
             h(cg);
             return;
         }
+        uint64_t at = v.coff[cg] + 8 * lane;
         warp_list8(v.lst + v.coff[cg], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
 #pragma unroll
             for (uint32_t q = 0; q < 8; ++q)
-                if (q < cnt) f(base | x[q]);
+                if (q < cnt) f(base | x[q], at + q);
+            at += 256;
         });
         return;
     }
@@ -913,7 +915,7 @@ __device__ __forceinline__ void walk_group_chunks(const ChunkView& v, uint64_t c
             if (__shfl_sync(0xffffffffu, excl, o + step) <= t) o += step;
         const uint32_t e = t - __shfl_sync(0xffffffffu, excl, o), b = __shfl_sync(0xffffffffu, base, o);
         const uint64_t at = __shfl_sync(0xffffffffu, off, o);
-        if (t < total) f(b | v.lst[at + e]);
+        if (t < total) f(b | v.lst[at + e], at + e);
     }
 }
 
@@ -932,7 +934,7 @@ __device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint3
 // part of the universe and what they update -- 4 bytes per value somewhere in
 // it -- stays in L2. With a warp (or CTA) per row, 200 mixed rows left the GPU
 // idle, and the places of 20000 rows' values (67 MB of cursors, 134 of
-// postings) were written from DRAM.  f(r, value), h(chunk).
+// postings) were written from DRAM.  f(r, value, place), h(chunk).
 template <class F, class H>
 __device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __restrict__ rows, uint32_t nq,
                                           uint32_t group, uint32_t groups, F f, H h) {
@@ -942,7 +944,7 @@ __device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __
         const uint32_t row = rows ? rows[r] : r;
         const uint64_t cg = v.row_off[row] + it / nq * group, c1 = v.row_off[row + 1];
         if (cg < c1)
-            walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, [&](uint32_t x) { f(r, x); }, h);
+            walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, [&](uint32_t x, uint64_t at) { f(r, x, at); }, h);
     }
 }
 
@@ -978,7 +980,7 @@ postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq
                      uint32_t* __restrict__ counts) {
     const int lane = threadIdx.x & 31;
     rows_walk(
-        v, rows, nq, group, groups, [&](uint32_t, uint32_t x) { atomicAdd(&counts[x], 1u); },
+        v, rows, nq, group, groups, [&](uint32_t, uint32_t x, uint64_t) { atomicAdd(&counts[x], 1u); },
         [&](uint64_t c) {
             const uint64_t* wd = v.bm + v.coff[c];
             const uint32_t base = v.cid[c] << 16;
@@ -1028,7 +1030,8 @@ __global__ void postings_stats_kernel(const uint32_t* __restrict__ counts, uint6
 
 // Gives every value held by >= 2 rows a slot range in the postings array
 // (start) and, when `lists` is given, a list record; other values get
-// start = ~0. A block takes 4096 values at a time and the two allocation
+// start = ~0. With `heads` (16-bit lists) a list's length stands in front of
+// it. A block takes 4096 values at a time and the two allocation
 // cursors once for all of them: one atomic per warp on the same two words took
 // 0.64 ms for 2^24 values (the counts and starts, 134 MB, cost 0.03). (The run
 // postings use it for bins.)
@@ -1036,7 +1039,8 @@ constexpr uint32_t ALLOC_THREADS = 256, ALLOC_PER_THREAD = 16;
 
 __global__ void __launch_bounds__(ALLOC_THREADS)
 postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t* __restrict__ start,
-                      uint2* __restrict__ lists, PostingsStats* st) {
+                      uint2* __restrict__ lists, uint16_t* __restrict__ heads, PostingsStats* st) {
+    const uint32_t head = heads ? 1u : 0u;
     __shared__ uint32_t we[ALLOC_THREADS / 32], wl[ALLOC_THREADS / 32];
     __shared__ unsigned long long e0s, l0s;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1050,7 +1054,7 @@ postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t*
         for (uint32_t k = 0; k < ALLOC_PER_THREAD; ++k) {
             const uint64_t x = xw + 32 * k;
             c[k] = x < U ? counts[x] : 0u;
-            e += c[k] >= 2 ? c[k] : 0u;
+            e += c[k] >= 2 ? c[k] + head : 0u;
             l += c[k] >= 2 ? 1u : 0u;
         }
         const uint32_t ei = warp_incl_scan(e, lane), li = warp_incl_scan(l, lane);
@@ -1079,9 +1083,10 @@ postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t*
             const uint64_t x = xw + 32 * k;
             if (x >= U) continue;
             if (c[k] >= 2) {
-                start[x] = s;
+                if (heads) heads[s] = (uint16_t)c[k];
+                start[x] = s + head;
                 if (lists) lists[q] = make_uint2(s, c[k]);
-                s += c[k];
+                s += c[k] + head;
                 ++q;
             } else {
                 start[x] = ~0u;
@@ -1098,7 +1103,7 @@ postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t
                         uint32_t* __restrict__ start, uint32_t* __restrict__ post) {
     rows_walk(
         v, rows, nq, group, groups,
-        [&](uint32_t r, uint32_t x) {
+        [&](uint32_t r, uint32_t x, uint64_t) {
             // a value of one row has start ~0, and its one row adds to it once
             const uint32_t at = atomicAdd(&start[x], 1u);
             if (at != ~0u) post[at] = r;
@@ -1140,7 +1145,81 @@ __global__ void postings_pairs_kernel(const uint2* __restrict__ lists, uint64_t 
     }
 }
 
-// Row sweep: CTA per Q row a; for every value of a, the rows b > a on that
+// The lists of the 16-bit row sweep, each behind its length (heads of
+// postings_alloc_kernel): the rows' positions are written into them, counts[x]
+// counting down to the places, and place[p] becomes the list of the pool's
+// entry p (of its own value), so that the sweep finds a row's lists without
+// looking its values up.
+__global__ void __launch_bounds__(ROW_WALK_THREADS)
+postings_scatter16_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
+                          uint32_t* __restrict__ counts, const uint32_t* __restrict__ start,
+                          uint16_t* __restrict__ post, uint32_t* __restrict__ place) {
+    rows_walk(
+        v, rows, nq, group, groups,
+        [&](uint32_t r, uint32_t x, uint64_t at) {
+            const uint32_t s = start[x];
+            place[at] = s;
+            if (s != ~0u) post[s + atomicSub(&counts[x], 1u) - 1u] = (uint16_t)r;
+        },
+        [](uint64_t) {});
+}
+
+// Row sweep over 16-bit lists: CTA per Q row a. A row's entries lie together in
+// the list pool, so its lists' places are read in order, and a list -- its
+// length and members, two bytes each -- is one sector mostly: one random read
+// per value instead of three (count, end, members), from a third of the bytes.
+// Every list member b > a gets a shared-memory increment; then the row's slice
+// of the triangle is written once. At most 65535 rows of at most 65535 values:
+// members, lengths and counts fit 16 bits.
+constexpr uint32_t POST_ROWS_THREADS = 512;
+constexpr uint32_t POST16_MAX = 0xFFFF;
+
+__global__ void __launch_bounds__(POST_ROWS_THREADS)
+postings_rows16_kernel(ChunkView v, const uint32_t* __restrict__ qrows, uint32_t nq, bool all_rows,
+                       const uint32_t* __restrict__ place, const uint16_t* __restrict__ post, uint64_t n,
+                       uint32_t* __restrict__ out) {
+    extern __shared__ uint32_t cnt[];
+    __shared__ uint32_t card;
+    const uint32_t words = (nq + 1) / 2;
+    for (uint32_t a = blockIdx.x; a < nq; a += gridDim.x) {
+        const uint32_t row = qrows[a];
+        const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
+        for (uint32_t b = (a + 1) / 2 + threadIdx.x; b < words; b += blockDim.x) cnt[b] = 0;
+        if (threadIdx.x == 0) card = 0;
+        __syncthreads();
+        uint32_t mine = 0;
+        for (uint64_t c = c0 + threadIdx.x; c < c1; c += blockDim.x) mine += v.ckl[c] & CK_LEN;
+        if (mine) atomicAdd(&card, mine);
+        if (c1 > c0) {
+            const uint64_t p1 = v.coff[c1 - 1] + (v.ckl[c1 - 1] & CK_LEN);
+            for (uint64_t p = v.coff[c0] + threadIdx.x; p < p1; p += blockDim.x) {
+                const uint32_t s = place[p];
+                if (s == ~0u) continue;            // a value of this row alone, or between two lists
+                const uint32_t len = post[s - 1];
+                for (uint32_t k = 0; k < len; k += 4) {
+                    uint32_t b[4];                 // read together (the list is followed by at least 4 places)
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q) b[q] = post[s + k + q];
+#pragma unroll
+                    for (uint32_t q = 0; q < 4; ++q)
+                        if (k + q < len && b[q] > a) atomicAdd(&cnt[b[q] >> 1], b[q] & 1u ? 0x10000u : 1u);
+                }
+            }
+        }
+        __syncthreads();
+        const uint64_t base = tri_index(n, row, row) - row;   // out index of (row, j) is base + j
+#pragma unroll 4
+        for (uint32_t b = a + 1 + threadIdx.x; b < nq; b += blockDim.x) {
+            const uint32_t gb = all_rows ? b : qrows[b];      // ascending: gb > row (the other order kept exact too)
+            __stcs(out + (gb > row ? base + gb : tri_index(n, gb, row)), (cnt[b >> 1] >> (16 * (b & 1u))) & 0xFFFFu);
+        }
+        if (threadIdx.x == 0) out[base + row] = card;
+        __syncthreads();
+    }
+}
+
+// Row sweep of more rows, or longer ones: CTA per Q row a; for every value of
+// a, the rows b > a on that
 // value's list get one shared-memory increment; then a's slice of the
 // triangle (its Q partners b > a and its diagonal) is written once, in
 // ascending order. Bound: the random reads of a value's count, end and list
@@ -1152,7 +1231,6 @@ __global__ void postings_pairs_kernel(const uint2* __restrict__ lists, uint64_t 
 // again; the launch of block 0 writes the diagonal.
 // Lists hold local indices, list x is [end[x] - counts[x], end[x]).
 constexpr uint32_t POST_SWEEP_THREADS = 256;      // run sweep
-constexpr uint32_t POST_ROWS_THREADS = 512;
 constexpr uint32_t POST_SWEEP_MAX_ROWS = 51200;   // 200 KiB of counters
 
 template <bool kSmall>
@@ -1175,7 +1253,7 @@ postings_rows_kernel(ChunkView v, const uint32_t* __restrict__ qrows, uint32_t n
         uint32_t mine = 0;
         row_walk(
             v, row, group,
-            [&](uint32_t x) {
+            [&](uint32_t x, uint64_t) {
                 ++mine;
                 const uint32_t len = counts[x], e1 = end[x];
                 if (len < 2) return;
@@ -1932,26 +2010,39 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         return finish(q_sum);
     }
 
-    // Per-pair form of the postings: list by list into the output while the
-    // triangle fits in L2 (its atomics stay on chip), else the row sweep
-    // (partners counted in shared memory, each output written once).
-    const bool big_out = tri_size(n) * sizeof(uint32_t) > L2_BYTES_B200;
+    // Per-pair form of the postings: increments list by list into the output,
+    // or the row sweep (partners counted in shared memory, each output written
+    // once), whichever the constants say. Measured on B200, list by list / row
+    // sweep (ms, histogram and lists included): 4000 rows of 16777 values over
+    // 2^24 3.0 / 3.2, 6000 of 4194 over 2^22 1.2 / 1.3, 8000 of 16777 12.2 / 7.5,
+    // 20000 of 1678 2.8 / 1.8, 20000 of 5033 17.2 / 5.7, 20000 of 168 0.27 / 0.56.
+    const bool big_out = tri_size(n) * sizeof(uint32_t) > POST_L2_BYTES;
     const double c_list = big_out ? cost.ns_per_posting_pair_hbm : cost.ns_per_posting_pair;
     // The row sweeps count partners in blocks of POST_SWEEP_MAX_ROWS rows,
-    // reading each row's lists (or bins) once per block.
+    // reading each row's lists (or bins) once per block; up to POST16_MAX rows
+    // of value postings take one block.
     auto sweep_blocks = [&](uint64_t q) { return (double)((q + POST_SWEEP_MAX_ROWS - 1) / POST_SWEEP_MAX_ROWS); };
-    auto sweep_ns = [&](double incr, uint64_t q) {
-        return (double)q * (double)q * cost.ns_per_sweep_row_pair + incr * cost.ns_per_posting_sweep * sweep_blocks(q);
+    auto sweep_ns = [&](double incr, uint64_t q, double entries) {
+        const double reads = entries * cost.ns_per_sweep_entry + incr * cost.ns_per_posting_sweep;
+        return (double)q * (double)q * cost.ns_per_sweep_count + (q <= POST16_MAX ? reads : 3.0 * reads * sweep_blocks(q));
     };
-    auto sweep_form = [&](double incr, uint64_t q) {
+    auto sweep_form = [&](double incr, uint64_t q, double entries) {
         if (postings_mode == 2) return false;
-        return postings_mode == 3 || (big_out && sweep_ns(incr, q) < incr * c_list);
+        return postings_mode == 3 || sweep_ns(incr, q, entries) < incr * c_list;
     };
-    // ns of the postings for a set of q rows with incr increments (sums need
-    // only the histogram)
-    auto post_ns = [&](double incr, uint64_t q) {
-        const double per_pair = sweep_form(incr, q) ? sweep_ns(incr, q) : incr * c_list;
-        return (d_out ? per_pair : 0.0) + (double)U * cost.ns_per_universe_value;
+    // ns of the postings for a set of q rows of `entries` values with incr
+    // increments (sums need only the histogram)
+    auto post_ns = [&](double incr, uint64_t q, double entries) {
+        const double per_pair = sweep_form(incr, q, entries) ? sweep_ns(incr, q, entries) : incr * c_list;
+        return (d_out ? per_pair : 0.0) + entries * cost.ns_per_posting_entry + (double)U * cost.ns_per_universe_value;
+    };
+    // ns of the tensor cores for h rows among themselves and against m more:
+    // whole 256 x 256 tiles, and the rows' expansion
+    auto tensor_ns = [&](double h, double m) {
+        const double nb = std::ceil(h / 256.0), mb = std::ceil(m / 256.0);
+        return h <= 0.0 ? 0.0
+                        : tc_ns * 65536.0 * (nb * (nb + 1.0) / 2.0 + nb * mb) +
+                              (h + m) * (double)W * 8.0 * cost.ns_per_expand_byte;
     };
     // ns of the run sweep with `checks` entry reads for q rows (per pair only)
     auto run_ns = [&](double checks, uint64_t q) {
@@ -1967,6 +2058,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // estimate beats the value postings' and its exact count (the piece
     // histogram) beats `alt`, else the value postings on their exact count
     // (the value histogram).
+    auto values_of = [&](const std::vector<uint32_t>& rows) {
+        uint64_t c = 0;
+        for (uint32_t r : rows) c += d.facts[r].card;
+        return c;
+    };
     auto decide = [&](const std::vector<uint32_t>& rest, double alt) -> bool {
         const uint64_t q = rest.size();
         if (q < 2) return false;
@@ -1981,7 +2077,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                 C2 += (double)f.card * (double)f.card;
             }
             const double run_e = run_ns(P * P * RW / (double)U, q);
-            const double val_e = post_ns((C1 * C1 - C2) / (2.0 * (double)U), q);
+            const double val_e = post_ns((C1 * C1 - C2) / (2.0 * (double)U), q, C1);
             if (postings_mode == 4 || run_e < val_e || !lists_only) {
                 run_histogram(rest);
                 if (postings_mode == 4 || postings_mode == 1 || run_ns((double)run_checks, q) < alt) {
@@ -1993,7 +2089,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         }
         if (!lists_only) return false;
         ps = histogram(rest);
-        if (ps.entries < (1ull << 32) && (postings_mode > 0 || post_ns((double)ps.pairs, q) < alt)) {
+        if (ps.entries < (1ull << 32) && (postings_mode > 0 || post_ns((double)ps.pairs, q, (double)values_of(rest)) < alt)) {
             qrows = rest;
             return true;
         }
@@ -2060,7 +2156,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             const uint64_t q = np - from;
             if (q < 2) return 0.0;
             const double r1 = S1[np] - S1[from], r2 = S2[np] - S2[from];
-            double v = from >= lb ? post_ns((r1 * r1 - r2) / (2.0 * (double)U), q) : HUGE_VAL;
+            double v = from >= lb ? post_ns((r1 * r1 - r2) / (2.0 * (double)U), q, r1) : HUGE_VAL;
             if (run_ok(q)) {
                 const double P = S3[np] - S3[from];
                 v = std::min(v, run_ns(P * P * RW / (double)U, q));
@@ -2071,8 +2167,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         uint64_t best_k = lb;
         double best_a = -1.0;
         for (uint64_t k = 0; k <= np; ++k) {
-            const double kk = (double)k;
-            const double v = tc_ns * (kk * (kk - 1.0) / 2.0 + kk * (double)(np - k)) + post_est(k);
+            const double v = tensor_ns((double)k, (double)(np - k)) + post_est(k);
             if (best_a < 0 || v < best_a) {
                 best_a = v;
                 best_k = k;
@@ -2100,7 +2195,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                     const double panel = cost.ns_per_panel_value * (sl * nb + sm * (nbh + 0.5 * nbm + 0.5)) +
                                          cost.ns_per_panel_pair * (nl * (double)e + m * (m - 1.0) / 2.0 + m * hh) +
                                          nb * build_ns;
-                    const double v = tc_ns * hh * (hh - 1.0) / 2.0 + panel + post_est(e);
+                    const double v = tensor_ns(hh, 0.0) + panel + post_est(e);
                     if (best_b < 0 || v < best_b) {
                         best_b = v;
                         best_h = h;
@@ -2133,7 +2228,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             const double alt = panel_plan ? cost.ns_per_panel_value * (S1[np] - S1[np - rest.size()]) *
                                                 (0.5 * std::ceil(q / PANEL_ROWS) + 0.5) +
                                                 cost.ns_per_panel_pair * q * (q - 1.0) / 2.0
-                                          : tc_ns * (q * (q - 1.0) / 2.0);
+                                          : tensor_ns(q, 0.0);
             if (decide(rest, alt)) {
             } else if (panel_plan) {
                 mrows.insert(mrows.end(), rest.begin(), rest.end());
@@ -2222,7 +2317,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         if (!e) SB_CUDA(cudaEventCreate(&e));
     {
         const double dd = (double)nd, tqn = (double)tq.size();
-        last_engine_pred_ms[0] = 1e-6 * tc_ns * (dd * (dd + 1.0) / 2.0 + dd * tqn);
+        last_engine_pred_ms[0] = 1e-6 * tensor_ns(dd, tqn);
         last_engine_work[0] = 2.0 * (dd * (dd + 1.0) / 2.0 + dd * tqn) * (double)U;
         last_engine_work[1] = (double)(nc * n - (nc * (nc - 1)) / 2 * (nc ? 1 : 0));
         if (panel_plan && (nm || nd) && (nq + nm)) {
@@ -2246,7 +2341,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             last_engine_work[3] = 16.0 * pcs + 8.0 * (double)run_entries + 8.0 * (double)run_checks +
                                   4.0 * (double)nq * ((double)nq + 1.0) / 2.0 + 4.0 * (double)n_bins;
         } else if (nq) {
-            last_engine_pred_ms[3] = 1e-6 * post_ns((double)ps.pairs, nq);
+            last_engine_pred_ms[3] = 1e-6 * post_ns((double)ps.pairs, nq, (double)values_of(qrows));
             double vals = 0.0;
             for (uint32_t r : qrows) vals += (double)d.facts[r].card;
             last_engine_work[3] = 8.0 * vals + 8.0 * (double)ps.entries + 8.0 * (double)ps.pairs + 8.0 * (double)U;
@@ -2440,7 +2535,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         auto fill = rwlog >= RUN_GALLOP_WLOG ? run_fill_kernel<true> : run_fill_kernel<false>;
         fill<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
             d.view(), d_qrows.p, (uint32_t)nq, rwlog, d_rpoff.p, d_cpieces.p, d_pieces.p);
-        postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, d_pstats.p);
+        postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, nullptr, d_pstats.p);
         run_scatter_kernel<<<gq, 256, 0, st>>>((uint32_t)nq, rwlog, d_rpoff.p, d_pieces.p, d_rstart.p, d_rlist.p);
         static std::atomic<uint64_t> done{0};
         smem_attr_once(run_sweep_kernel, (int)((POST_SWEEP_MAX_ROWS + RUN_SWEEP_BATCH + 1) * sizeof(uint32_t)), done);
@@ -2458,45 +2553,73 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         last_postings_rows = nq;
     } else if (nq) {
         q_sum = ps.pairs;
-        const bool sweep = sweep_form((double)ps.pairs, nq);
+        const bool sweep = sweep_form((double)ps.pairs, nq, (double)values_of(qrows));
         last_postings_form = sweep ? 1 : 0;
         if (d_out) {
             d_start.reserve(U);
-            d_lists.reserve(ps.lists ? ps.lists : 1);
-            d_post.reserve(ps.entries ? ps.entries : 1);
-            postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_counts.p, U, d_start.p, d_lists.p, d_pstats.p);
-            postings_scatter_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
-                d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_start.p, d_post.p);
-            if (sweep) {
-                uint64_t most = 0;
-                for (uint32_t r : qrows) most = std::max(most, d.facts[r].card);
-                const bool small = most <= 0xFFFF;   // a count is at most its row's values
-                static std::atomic<uint64_t> done_s{0}, done_l{0};
-                const int smem_max = (int)(POST_SWEEP_MAX_ROWS * sizeof(uint32_t));
-                smem_attr_once(postings_rows_kernel<true>, smem_max / 2, done_s);
-                smem_attr_once(postings_rows_kernel<false>, smem_max, done_l);
-                const uint32_t gr = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 16);
-                // a row's groups over all the warps of its CTA
-                const uint32_t warps = POST_ROWS_THREADS / 32, chunks = q_walk.group * q_walk.groups;
-                const uint32_t group =
-                    q_walk.group == 1 ? 1u : std::max(2u, std::min(32u, (chunks + warps - 1) / warps));
-                for (uint64_t pb0 = 0; pb0 < nq; pb0 += POST_SWEEP_MAX_ROWS) {
-                    const uint32_t pbn = (uint32_t)std::min<uint64_t>(POST_SWEEP_MAX_ROWS, nq - pb0);
-                    const uint32_t smem = (uint32_t)(small ? (pbn + 1) / 2 : pbn) * sizeof(uint32_t);
-                    auto kernel = small ? postings_rows_kernel<true> : postings_rows_kernel<false>;
-                    kernel<<<gr, POST_ROWS_THREADS, smem, st>>>(d.view(), d_qrows.p, (uint32_t)nq, nq == n, group,
-                                                               d_counts.p, d_start.p, d_post.p, n, d_out, (uint32_t)pb0,
-                                                               pbn);
-                    ++launches;
+            uint64_t most = 0;
+            for (uint32_t r : qrows) most = std::max(most, d.facts[r].card);
+            bool sweep16 = sweep && nq <= POST16_MAX && most <= POST16_MAX && ps.entries + ps.lists < 0xFFFFFFFFull;
+            if (sweep16) {
+                try {
+                    d_post16.reserve(ps.entries + ps.lists + 8);
+                    d_place.reserve(d.lst.n);
+                } catch (const Status& e) {   // no room for the entries' lists: the sweep that looks them up
+                    if (e.code != STORM_B200_ENOMEM) throw;
+                    cudaGetLastError();
+                    sweep16 = false;
                 }
-                launches += 2;
+            }
+            if (!sweep16) {
+                if (!sweep) d_lists.reserve(ps.lists ? ps.lists : 1);
+                d_post.reserve(ps.entries ? ps.entries : 1);
+            }
+            postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_counts.p, U, d_start.p, sweep ? nullptr : d_lists.p,
+                                                                    sweep16 ? d_post16.p : nullptr, d_pstats.p);
+            if (sweep16) {
+                SB_CUDA(cudaMemsetAsync(d_place.p, 0xFF, d.lst.n * sizeof(uint32_t), st));
+                postings_scatter16_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
+                    d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_counts.p, d_start.p, d_post16.p,
+                    d_place.p);
+                static std::atomic<uint64_t> done16{0};
+                smem_attr_once(postings_rows16_kernel, (int)((POST16_MAX + 1) * sizeof(uint16_t)), done16);
+                postings_rows16_kernel<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 16), POST_ROWS_THREADS,
+                                         (nq + 1) / 2 * sizeof(uint32_t), st>>>(
+                    d.view(), d_qrows.p, (uint32_t)nq, nq == n, d_place.p, d_post16.p, n, d_out);
+                SB_CUDA(cudaGetLastError());
+                launches += 3;
             } else {
-                const uint32_t gp = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((ps.lists + 255) / 256,
-                                                                                       (uint64_t)sms * 16));
-                postings_pairs_kernel<<<gp, 256, 0, st>>>(d_lists.p, ps.lists, d_post.p, d_qrows.p, n, d_out);
-                postings_diag_kernel<<<(uint32_t)std::min<uint64_t>((nq + 255) / 256, (uint64_t)sms * 4), 256, 0,
-                                       st>>>(d.view(), d_qrows.p, (uint32_t)nq, n, d_out);
-                launches += 4;
+                postings_scatter_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
+                    d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_start.p, d_post.p);
+                if (sweep) {
+                    const bool small = most <= 0xFFFF;   // a count is at most its row's values
+                    static std::atomic<uint64_t> done_s{0}, done_l{0};
+                    const int smem_max = (int)(POST_SWEEP_MAX_ROWS * sizeof(uint32_t));
+                    smem_attr_once(postings_rows_kernel<true>, smem_max / 2, done_s);
+                    smem_attr_once(postings_rows_kernel<false>, smem_max, done_l);
+                    const uint32_t gr = (uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 16);
+                    // a row's groups over all the warps of its CTA
+                    const uint32_t warps = POST_ROWS_THREADS / 32, chunks = q_walk.group * q_walk.groups;
+                    const uint32_t group =
+                        q_walk.group == 1 ? 1u : std::max(2u, std::min(32u, (chunks + warps - 1) / warps));
+                    for (uint64_t pb0 = 0; pb0 < nq; pb0 += POST_SWEEP_MAX_ROWS) {
+                        const uint32_t pbn = (uint32_t)std::min<uint64_t>(POST_SWEEP_MAX_ROWS, nq - pb0);
+                        const uint32_t smem = (uint32_t)(small ? (pbn + 1) / 2 : pbn) * sizeof(uint32_t);
+                        auto kernel = small ? postings_rows_kernel<true> : postings_rows_kernel<false>;
+                        kernel<<<gr, POST_ROWS_THREADS, smem, st>>>(d.view(), d_qrows.p, (uint32_t)nq, nq == n, group,
+                                                                   d_counts.p, d_start.p, d_post.p, n, d_out, (uint32_t)pb0,
+                                                                   pbn);
+                        ++launches;
+                    }
+                    launches += 2;
+                } else {
+                    const uint32_t gp = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((ps.lists + 255) / 256,
+                                                                                           (uint64_t)sms * 16));
+                    postings_pairs_kernel<<<gp, 256, 0, st>>>(d_lists.p, ps.lists, d_post.p, d_qrows.p, n, d_out);
+                    postings_diag_kernel<<<(uint32_t)std::min<uint64_t>((nq + 255) / 256, (uint64_t)sms * 4), 256, 0,
+                                           st>>>(d.view(), d_qrows.p, (uint32_t)nq, n, d_out);
+                    launches += 4;
+                }
             }
             SB_CUDA(cudaGetLastError());
         }

@@ -200,15 +200,19 @@ enum PairMode : uint32_t {
 struct ChunkCostModel {
     double ns_per_shared_chunk = 0.086;
     double ns_per_lane_iteration = 0.0228;
-    double ns_per_tensor_bit = 0.7e-6;
-    double ns_per_posting_pair = 0.05;       // one (pair, shared value) increment, output in L2
-    double ns_per_posting_pair_hbm = 0.042;  // the same, output larger than L2
-    double ns_per_posting_sweep = 0.016;     // the same in the row sweep (shared memory)
-    double ns_per_sweep_row_pair = 0.0047;   // row sweep: clearing and writing, per (row, row)
-    double ns_per_universe_value = 2e-4;     // histogram clear + scan per universe value
-    double ns_per_panel_value = 0.05;        // transposed panel: one query value against one 2048-row block
+    double ns_per_tensor_bit = 0.3e-6;       // per bit of a pair in the tensor cores' 256 x 256 tiles
+    double ns_per_expand_byte = 1.0 / 2600.0;
+    double ns_per_posting_pair = 0.010;      // one (pair, shared value) increment, output in L2
+    double ns_per_posting_pair_hbm = 0.045;  // the same, output larger
+    double ns_per_posting_entry = 0.022;     // one value of a row counted and put into its list
+    double ns_per_posting_sweep = 0.0038;    // row sweep: one increment (shared memory)
+    double ns_per_sweep_entry = 0.016;       // row sweep: one value's list found
+    double ns_per_sweep_count = 0.0005;      // row sweep: clearing and writing, per (row, row)
+    double ns_per_sweep_row_pair = 0.0047;   // run sweep: the same
+    double ns_per_universe_value = 6e-3;     // histogram clear + scans per universe value
+    double ns_per_panel_value = 0.04;        // transposed panel: one query value against one 2048-row block
     double ns_per_panel_pair = 0.005;        // transposed panel: one count written
-    double ns_per_panel_byte = 1.0 / 6000.0; // transposed panel: expansion and transpose traffic
+    double ns_per_panel_byte = 1.0 / 4300.0; // transposed panel: expansion and transpose traffic
     double ns_per_run_check = 0.03;          // run sweep: one bin entry read against one piece
 };
 double chunk_self_pair_ns(const ChunkCostModel& m, const ChunkRowFacts& f, uint64_t slots);
@@ -225,6 +229,7 @@ constexpr double CHUNK_DENSE_AUTO = -1.0;
 // histogram: the sum over those pairs is sum_v C(rows holding v, 2).
 constexpr uint64_t POSTINGS_MAX_UNIVERSE = 1ull << 27;
 constexpr uint64_t L2_BYTES_B200 = 126ull << 20;
+constexpr uint64_t POST_L2_BYTES = 96ull << 20;   // outputs up to here take increments at L2's pace
 
 struct ChunkEngine {
     DevBuf<DeviceFlags> d_flags;
@@ -268,6 +273,8 @@ struct ChunkEngine {
     DevBuf<uint32_t> d_perm, d_map;
     DevBuf<uint32_t> d_qrows, d_counts, d_start, d_post;
     DevBuf<uint2> d_lists;
+    DevBuf<uint16_t> d_post16;
+    DevBuf<uint32_t> d_place;
     DevBuf<PostingsStats> d_pstats;
     DevBuf<uint64_t> d_panel;
     DevBuf<uint2> d_tiles;

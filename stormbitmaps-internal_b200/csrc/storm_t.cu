@@ -897,6 +897,7 @@ int STORM_calibrate(STORM_t* s, uint32_t sample_rows, double* out) {
         }
         ChunkCostModel& c = d->engine.cost;
         c.ns_per_tensor_bit *= scale[0];
+        c.ns_per_expand_byte *= scale[0];
         c.ns_per_panel_value *= scale[1];
         c.ns_per_panel_pair *= scale[1];
         c.ns_per_panel_byte *= scale[1];
@@ -906,6 +907,9 @@ int STORM_calibrate(STORM_t* s, uint32_t sample_rows, double* out) {
             c.ns_per_posting_pair *= scale[2];
             c.ns_per_posting_pair_hbm *= scale[2];
             c.ns_per_posting_sweep *= scale[2];
+            c.ns_per_posting_entry *= scale[2];
+            c.ns_per_sweep_entry *= scale[2];
+            c.ns_per_sweep_count *= scale[2];
         }
         c.ns_per_sweep_row_pair *= scale[2];
         if (out) {

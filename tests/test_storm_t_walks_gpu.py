@@ -103,3 +103,33 @@ def test_zone_maps_of_row_blocks(sb, universe):
     assert r.allpairs_sum(sb.POLICY_PERTILE, 32)[0] == ws
     assert r.allpairs_sum(sb.POLICY_PERTILE, 64)[0] == ws
     r.close()
+
+
+@pytest.mark.parametrize("n", (2, 511, 513, 3001))
+def test_row_sweep_in_16_bits(sb, n):
+    """The row sweep over 16-bit lists: values of one row and of all rows (the
+    longest list), empty rows, an odd number of counters, beside chunk-kernel
+    rows that leave gaps in the rows' order."""
+    g = gen.rng(n)
+    sets = [np.unique(np.concatenate([g.integers(0, 3 << 16, size=int(g.integers(0, 60))), [7, 70000]])).astype(np.uint32)
+            for _ in range(n)]
+    sets[0] = np.array([7, 70000, 123456], np.uint32)
+    if n > 2:
+        sets[n // 2] = np.zeros(0, np.uint32)
+    for dup in (False, True):
+        rows = list(sets)
+        if dup:
+            rows[n - 1] = np.sort(np.concatenate([rows[n - 1], rows[n - 1][:1]]))
+        vals, offs = gen.to_csr(rows)
+        want, ws = (ol.storm_matrix if dup else ol.sets_matrix)(vals, offs)
+        s = sb.Storm()
+        for v in rows:
+            s.add(v)
+        s.set_dense_block(0.0)
+        s.set_panel(0)
+        s.set_sparse_postings(3)
+        got, total = s.matrix()
+        strict = np.not_equal(*np.triu_indices(n))
+        np.testing.assert_array_equal(got[strict], want[strict])
+        assert total == ws
+        s.close()
