@@ -1866,9 +1866,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             d_out = keep;
         }
         SB_CUDA(cudaEventRecord(log.ev1, st));
-        DeviceFlags f;
-        SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-        SB_CUDA(cudaStreamSynchronize(st));
+        const DeviceFlags f = read_flags(d_flags.p, st);
         SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
         log.launches = launches;
         return f.sum;
@@ -1973,9 +1971,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     };
     auto finish = [&](uint64_t extra_sum) {
         SB_CUDA(cudaEventRecord(log.ev1, st));
-        DeviceFlags f;
-        SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-        SB_CUDA(cudaStreamSynchronize(st));
+        const DeviceFlags f = read_flags(d_flags.p, st);
         if (f.error) fail(STORM_B200_ETIMEOUT, "tensor-core dense block: a pipeline wait timed out");
         SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
         log.launches = launches;
@@ -2096,8 +2092,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         return false;
     };
     bool panel_plan = false;
-    // The panel needs a block of expanded rows and its transpose in HBM.
-    const uint64_t px_words = PANEL_ROWS * panel_row_words(W);
+    // The panel needs a transposed block and some of its rows expanded in HBM.
+    const uint64_t px_words = PANEL_ROWS * PANEL_PITCH * std::min<uint64_t>(slots, PANEL_X_SLOTS);
     const uint64_t panel_bytes = (PANEL_ROWS * W + px_words) * sizeof(uint64_t);
     auto panel_fits = [&]() {
         if (!facts_ok || panel_mode == 0 || U > PANEL_MAX_UNIVERSE) return false;
@@ -2488,10 +2484,20 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             const uint32_t prows = (uint32_t)std::min<uint64_t>(PANEL_ROWS, npw - b0);
             for (uint32_t t = 0; t < PANEL_ROWS; ++t) bmap[t] = t < prows ? h_perm[pw0 + b0 + t] : ~0u;
             SB_CUDA(cudaMemcpyAsync(d_pmap.p, bmap.data(), PANEL_ROWS * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            const RowLayout play{PANEL_PITCH, PANEL_ROWS * PANEL_PITCH};   // block-major, as the tensor panels
-            expand_rows_kernel<<<(uint32_t)sms * 64, EXPAND_WARPS * 32, 0, st>>>(
-                d.view(), d_pmap.p, PANEL_ROWS, 0u, (uint32_t)slots, (uint32_t)slots, play, d_pX.p);
-            panel_transpose_kernel<<<(uint32_t)(W / PANEL_T_WORDS), 1024, PANEL_T_SMEM, st>>>(d_pX.p, play, d_DT.p);
+            // PANEL_X_SLOTS chunk slots at a time, block-major as the tensor
+            // panels: the expanded rows of a whole block would take as much
+            // memory as the block itself, and its allocation 20 ms of a
+            // container's first call.
+            const RowLayout play{PANEL_PITCH, PANEL_ROWS * PANEL_PITCH};
+            for (uint32_t s0 = 0; s0 < slots; s0 += PANEL_X_SLOTS) {
+                const uint32_t ns = (uint32_t)std::min<uint64_t>(PANEL_X_SLOTS, slots - s0);
+                const uint32_t items = PANEL_ROWS * ns / EXPAND_WARPS;
+                expand_rows_kernel<<<std::min(items, (uint32_t)sms * 64), EXPAND_WARPS * 32, 0, st>>>(
+                    d.view(), d_pmap.p, PANEL_ROWS, s0, ns, (uint32_t)slots, play, d_pX.p);
+                panel_transpose_kernel<<<ns * CHUNK_WORDS / PANEL_T_WORDS, 1024, PANEL_T_SMEM, st>>>(
+                    d_pX.p, play, d_DT.p + (uint64_t)s0 * CHUNK_WORDS * 64 * PANEL_WORDS);
+                launches += 2;
+            }
             SB_CUDA(cudaMemsetAsync(d_ctr.p, 0, sizeof(unsigned long long), st));
             const uint32_t ni = (uint32_t)items.size();
             uint32_t* scr = splits.empty() ? nullptr : d_pscratch.p;
@@ -2504,7 +2510,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             else if (max_card < (1ull << 23)) SB_PANEL_QUERY(20);
             else SB_PANEL_QUERY(24);
 #undef SB_PANEL_QUERY
-            launches += 3;
+            launches += 1;
             if (scr && d_out) {
                 panel_reduce_kernel<<<(uint32_t)std::min<uint64_t>(splits.size(), (uint64_t)sms * 8), 256, 0, st>>>(
                     perm, d_splits.p, (uint32_t)splits.size(), pw0 + b0, prows, scr, n, d_out);

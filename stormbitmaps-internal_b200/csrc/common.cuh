@@ -117,6 +117,19 @@ struct DeviceFlags {
     unsigned long long sum;   // sum over i < j accumulated by the epilogues
 };
 
+// This thread's pinned place for the flags (or a pageable one where there is no
+// pinned memory), kept until the thread exits: a copy into pageable memory is
+// staged by the driver, which costs a small call more than its kernel's launch.
+DeviceFlags* flags_slot();
+
+// Waits for `st` and returns the flags left there by the work queued on it.
+inline DeviceFlags read_flags(const DeviceFlags* d, cudaStream_t st) {
+    DeviceFlags* h = flags_slot();
+    SB_CUDA(cudaMemcpyAsync(h, d, sizeof(*h), cudaMemcpyDeviceToHost, st));
+    SB_CUDA(cudaStreamSynchronize(st));
+    return *h;
+}
+
 inline uint64_t tri_size(uint64_t n) { return n * (n + 1) / 2; }
 
 // Raises a kernel's dynamic shared-memory limit once per device (the

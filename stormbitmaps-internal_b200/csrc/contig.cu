@@ -29,6 +29,7 @@ struct STORM_contiguous_s {
     uint64_t n_rows = 0;    // rows on the device + staged
     uint64_t dev_rows = 0;  // rows already in HBM
     uint64_t cap_rows = 0;  // HBM capacity in rows
+    uint64_t padded = 0;    // rows [padded, next multiple of 256) were zeroed and not written since (0: none were)
     std::vector<uint64_t> stage;   // rows added by STORM_contig_add, not yet in HBM
     sb200::DevBuf<uint64_t> d_rows;
     sb200::DevBuf<uint32_t> d_out;
@@ -82,6 +83,7 @@ static void contig_grow(STORM_contiguous_t* c, uint64_t rows) {
     c->d_rows.p = np;
     c->d_rows.n = cap * c->pitch;
     c->cap_rows = cap;
+    c->padded = 0;
 }
 
 // Append `rows` rows of `wpr` words from host memory into HBM (rows zero padded).
@@ -90,6 +92,7 @@ static void contig_append_device(STORM_contiguous_t* c, const uint64_t* host, ui
     contig_grow(c, c->dev_rows + rows);
     cudaStream_t st = contig_stream(c);
     uint64_t* dst = c->d_rows.p + c->dev_rows * c->pitch;
+    c->padded = 0;
     if (wpr != c->w_pad)
         SB_CUDA(cudaMemsetAsync(dst, 0, rows * c->pitch * sizeof(uint64_t), st));
     SB_CUDA(cudaMemcpy2DAsync(dst, c->pitch * sizeof(uint64_t), host, wpr * sizeof(uint64_t),
@@ -108,9 +111,11 @@ static void contig_flush(STORM_contiguous_t* c) {
     contig_grow(c, c->dev_rows ? c->dev_rows : 1);
     const uint64_t n_pad = round_up(std::max<uint64_t>(c->dev_rows, 1), 256);
     cudaStream_t st = contig_stream(c);
-    if (n_pad > c->dev_rows)
+    if (n_pad > c->dev_rows && (c->padded != c->dev_rows || c->dev_rows == 0)) {
         SB_CUDA(cudaMemsetAsync(c->d_rows.p + c->dev_rows * c->pitch, 0,
                                 (n_pad - c->dev_rows) * c->pitch * sizeof(uint64_t), st));
+        c->padded = c->dev_rows;
+    }
 }
 
 // Sum over i < j; packed triangle into d_out when non-null.
@@ -223,6 +228,7 @@ int STORM_contig_clear(STORM_contiguous_t* bitmap) {
     bitmap->stage.clear();
     bitmap->n_rows = 0;
     bitmap->dev_rows = 0;   // capacity is kept, as the reference keeps its vectors'
+    bitmap->padded = 0;
     set_last_status(0);
     return 1;
 }
@@ -359,6 +365,7 @@ int STORM_contig_pairw_intersect_matrix_from_host(STORM_contiguous_t* c, const u
         c->stage.clear();
         c->n_rows = 0;
         c->dev_rows = 0;
+        c->padded = 0;
         if (sum) *sum = 0;
         if (n_rows == 0) return 0;
         contig_grow(c, n_rows);

@@ -313,9 +313,7 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
     SB_CUDA(cudaEventRecord(log.ev0, st));
     launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
     SB_CUDA(cudaEventRecord(log.ev1, st));
-    DeviceFlags f;
-    SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-    SB_CUDA(cudaStreamSynchronize(st));
+    const DeviceFlags f = read_flags(d_flags.p, st);
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.launches = 1;
     log.kernel = reported;
@@ -349,9 +347,7 @@ uint64_t DenseEngine::run_sum(const uint64_t* dX, uint64_t n, uint32_t w_pad, ui
         log.launches += 2;
     }
     SB_CUDA(cudaEventRecord(log.ev1, st));
-    DeviceFlags f;
-    SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-    SB_CUDA(cudaStreamSynchronize(st));
+    const DeviceFlags f = read_flags(d_flags.p, st);
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.kernel = auto_kind(row_bits);
     return f.sum;
@@ -469,6 +465,23 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
         panel_ev.push_back(e);
     }
     SB_CUDA(cudaEventRecord(log.ev0, st));
+    if (panels.size() == 1 && chunk_rows == 0) {   // one launch: its copy follows on the same stream
+        launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
+        SB_CUDA(cudaEventRecord(log.ev1, st));
+        DeviceFlags f;
+        try {
+            SB_CUDA(cudaMemcpyAsync(host_out, d_out, tri_size(n) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+            f = read_flags(d_flags.p, st);
+        } catch (...) {
+            cudaStreamSynchronize(st);
+            throw;
+        }
+        SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
+        log.launches = 1;
+        log.kernel = reported;
+        if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
+        return f.sum;
+    }
     uint64_t copied_from = n;   // rows [copied_from, n) are on their way to the host
     try {
         for (size_t p = 0; p < panels.size(); ++p) {
@@ -503,9 +516,7 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
         throw;
     }
     SB_CUDA(cudaEventRecord(log.ev1, st));
-    DeviceFlags f;
-    SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-    SB_CUDA(cudaStreamSynchronize(st));
+    const DeviceFlags f = read_flags(d_flags.p, st);
     SB_CUDA(cudaStreamSynchronize(copy_st));
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.launches = (uint32_t)panels.size();
@@ -849,9 +860,7 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
         log.launches = 3;
     }
     SB_CUDA(cudaEventRecord(log.ev1, st));
-    DeviceFlags f;
-    SB_CUDA(cudaMemcpyAsync(&f, d_flags.p, sizeof(f), cudaMemcpyDeviceToHost, st));
-    SB_CUDA(cudaStreamSynchronize(st));
+    const DeviceFlags f = read_flags(d_flags.p, st);
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.kernel = reported;
     if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");

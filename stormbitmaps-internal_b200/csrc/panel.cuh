@@ -32,6 +32,7 @@ namespace sb200 {
 
 constexpr uint32_t PANEL_ROWS = 2048;                  // panel rows per block
 constexpr uint32_t PANEL_WORDS = PANEL_ROWS / 64;      // DT words per value
+constexpr uint32_t PANEL_X_SLOTS = 32;                 // chunk slots expanded at a time (541 MB)
 constexpr uint32_t PANEL_T_WORDS = 4;                  // row words per transpose CTA (256 values)
 constexpr uint32_t PANEL_Q_WARPS = 4;                  // warps per query CTA (33 KiB of shared memory)
 constexpr uint32_t PANEL_NO_VALUE = 0xFFFFFFFFu;
@@ -41,8 +42,9 @@ constexpr uint32_t PANEL_MAX_SLOTS = 8192;             // scratch slots of split
 
 // X: PANEL_ROWS expanded rows (rows past the block's end are zero),
 // block-major, so that the 2048 rows' words a CTA reads lie within 17 MB and
-// not on 2048 pages (row-major rows of 2^24 bits took 5.3 ms).  DT[v * PANEL_WORDS + w] bit r = bit v of row 64 w + r.  CTA: 32
-// warps, warp w transposes rows 64w .. 64w + 63 for PANEL_T_WORDS words: each
+// not on 2048 pages (row-major rows of 2^24 bits took 5.3 ms, these 1.9).
+// DT[v * PANEL_WORDS + w] bit r = bit v of row 64 w + r.  CTA: 32 warps, warp w
+// transposes rows 64w .. 64w + 63 for PANEL_T_WORDS words: each
 // 32 x 32 bit block (32 rows' 32-bit half-word, one per lane) is transposed
 // in registers by five butterfly stages (shfl_xor over lanes 16, 8, 4, 2, 1),
 // after which lane l holds bit l of that half-word across the 32 rows.  The
@@ -85,7 +87,7 @@ __global__ void __launch_bounds__(1024)
 panel_transpose_kernel(const uint64_t* __restrict__ X, RowLayout lay, uint64_t* __restrict__ DT) {
     extern __shared__ unsigned long long stage[];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint64_t k0 = (uint64_t)blockIdx.x * PANEL_T_WORDS;
+    const uint64_t k0 = (uint64_t)blockIdx.x * PANEL_T_WORDS;   // within X
     const uint64_t at = k0 / CHUNK_WORDS * lay.kstride + k0 % CHUNK_WORDS;
     const uint64_t* ra = X + (uint64_t)(64 * warp + lane) * lay.pitch + at;
     const uint64_t* rb = X + (uint64_t)(64 * warp + 32 + lane) * lay.pitch + at;

@@ -26,6 +26,24 @@ unsigned host_threads() {
     return n;
 }
 
+DeviceFlags* flags_slot() {
+    struct Slot {
+        DeviceFlags* pinned = nullptr;
+        DeviceFlags plain{};
+        Slot() {
+            if (cudaMallocHost((void**)&pinned, sizeof(DeviceFlags)) != cudaSuccess) {
+                cudaGetLastError();
+                pinned = nullptr;
+            }
+        }
+        ~Slot() {
+            if (pinned) cudaFreeHost(pinned);
+        }
+    };
+    static thread_local Slot slot;
+    return slot.pinned ? slot.pinned : &slot.plain;
+}
+
 int require_device() {
     int dev = 0;
     SB_CUDA(cudaGetDevice(&dev));
