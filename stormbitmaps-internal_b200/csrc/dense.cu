@@ -224,17 +224,23 @@ int DenseEngine::prepare(uint64_t n, uint64_t row_bits, int kernel_pref, bool ro
     return kind;
 }
 
-// Stream-K over the whole cached list (TsSched, k_splits 0): tiles from
-// W = floor(tiles / grid) x grid on add into the output: the triangle is zeroed
-// from the first row of the lowest A block among them.
-void DenseEngine::zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st) {
-    const uint32_t whole = (n_tiles / grid) * grid;
-    if (whole >= n_tiles) return;
-    uint32_t lowest = h_tiles[whole].x;
-    for (uint32_t t = whole; t < n_tiles; ++t) lowest = std::min(lowest, h_tiles[t].x);
-    const uint64_t r0 = (uint64_t)lowest * tile_rows_a(tiles_kind);
-    const uint64_t e0 = r0 * n - (r0 * (r0 - 1)) / 2;          // tri_index(n, r0, r0)
-    SB_CUDA(cudaMemsetAsync(d_out + e0, 0, (tri_size(n) - e0) * sizeof(uint32_t), st));
+// Stream-K over tiles [t0, t1) of the cached list, which hold every tile of
+// their A blocks (TsSched, k_splits 0): tiles from W = t0 + floor(tiles / grid)
+// x grid on add into the output: the triangle is zeroed from the first row of
+// the lowest A block among them to the last row of the highest.
+void DenseEngine::zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t t0, uint32_t t1, uint32_t grid,
+                                     cudaStream_t st) {
+    const uint32_t whole = t0 + (t1 - t0) / grid * grid;
+    if (whole >= t1) return;
+    uint32_t lowest = h_tiles[whole].x, highest = lowest;
+    for (uint32_t t = whole; t < t1; ++t) {
+        lowest = std::min(lowest, h_tiles[t].x);
+        highest = std::max(highest, h_tiles[t].x);
+    }
+    const uint64_t bm = tile_rows_a(tiles_kind);
+    const uint64_t r0 = lowest * bm, r1 = std::min<uint64_t>(n, (highest + 1) * bm);
+    auto start = [n](uint64_t r) { return r * n - r * (r - (r > 0)) / 2; };   // tri_index(n, r, r)
+    SB_CUDA(cudaMemsetAsync(d_out + start(r0), 0, (start(r1) - start(r0)) * sizeof(uint32_t), st));
 }
 
 // Tiles [t0, t0 + count) of the cached list.
@@ -243,15 +249,18 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
     const int sms = require_device();
     if (count == 0) return;
     const RowLayout lay = row_major(dense_pitch(w_pad));
-    // stream-K only for a launch over the whole tile list, whose output
-    // triangle can be zeroed first for the partial-count atomics
+    // stream-K only for a launch that holds every tile of its A blocks: its rows
+    // of the triangle can be zeroed first for the partial-count atomics
     const bool whole_list = t0 == 0 && count == n_tiles;
+    const bool whole_blocks = (t0 == 0 || h_tiles[t0 - 1].x != h_tiles[t0].x) &&
+                              (t0 + count == n_tiles || h_tiles[t0 + count].x != h_tiles[t0 + count - 1].x);
     if (kind == KIND_F4) {
         static std::atomic<uint64_t> done{0};
         smem_attr_once(bb_f4_kernel, (int)F4_SMEM_BYTES, done);
         uint32_t pairs = std::min<uint32_t>(count, (uint32_t)std::max(1, sms / 2));
-        const uint32_t ks = whole_list ? f4_schedule(count, sms, w_pad, pairs, schedule) : 1;
-        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, pairs, st);
+        const uint32_t ks =
+            whole_list || (whole_blocks && !tiles_banded) ? f4_schedule(count, sms, w_pad, pairs, schedule) : 1;
+        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, t0, t0 + count, pairs, st);
         uint32_t blk_words = 0;
         const CUtensorMap map = f4_row_map(dX, n, w_pad, lay, &blk_words);
         SB_CUDA(launch_pairs(bb_f4_kernel, pairs, F4_THREADS, F4_SMEM_BYTES, st, map, blk_words, n, w_pad,
@@ -261,7 +270,7 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
         smem_attr_once(bb_mma_ts_long_kernel, (int)TS_SMEM_BYTES, done);
         uint32_t grid = count < (uint32_t)sms ? count : (uint32_t)sms;
         const uint32_t ks = whole_list ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
-        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, grid, st);
+        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, t0, t0 + count, grid, st);
         bb_mma_ts_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
                                                                             d_out, d_flags.p, ks);
     } else if (kind == STORM_B200_KERNEL_MMA_DB) {
@@ -269,7 +278,7 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
         smem_attr_once(bb_mma_ts2_long_kernel, (int)T2_SMEM_BYTES, done);
         uint32_t grid = count < (uint32_t)sms ? count : (uint32_t)sms;
         const uint32_t ks = whole_list ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
-        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, grid, st);
+        if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, t0, t0 + count, grid, st);
         bb_mma_ts2_long_kernel<<<grid, T2_THREADS, T2_SMEM_BYTES, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
                                                                        d_out, d_flags.p, ks);
     } else if (kind == STORM_B200_KERNEL_MMA_2CTA) {
@@ -389,6 +398,59 @@ std::vector<std::pair<uint32_t, uint32_t>> host_panels(uint32_t n_tiles, uint32_
     return p;
 }
 
+// Rows of `wpr` words one after another to rows of w_pad words `pitch` apart,
+// the words past wpr zeroed. A warp per row; bound by HBM.
+__global__ void __launch_bounds__(256)
+repitch_rows_kernel(const uint64_t* __restrict__ src, uint32_t wpr, uint64_t* __restrict__ dst, uint64_t pitch,
+                    uint32_t w_pad, uint64_t rows) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t r = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += nw) {
+        const uint64_t* s = src + r * wpr;
+        uint64_t* d = dst + r * pitch;
+        for (uint32_t w = lane; w < w_pad; w += 32) d[w] = w < wpr ? __ldcs(s + w) : 0;
+    }
+}
+
+// Host rows into device rows `pitch` words apart: across the bus as they lie,
+// into `stage` (as many words as the host rows), and spread out on the device;
+// or, without `stage`, by a copy with two pitches, which is slow for short rows.
+void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_t* host, uint32_t wpr, uint64_t rows,
+                    uint64_t* stage, cudaStream_t st) {
+    if (rows == 0) return;
+    if (stage) {
+        SB_CUDA(cudaMemcpyAsync(stage, host, rows * wpr * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
+        repitch_rows_kernel<<<(uint32_t)std::min<uint64_t>((rows + 7) / 8, 1184), 256, 0, st>>>(stage, wpr, dst, pitch,
+                                                                                              w_pad, rows);
+        SB_CUDA(cudaGetLastError());
+        return;
+    }
+    if (wpr != w_pad)
+        SB_CUDA(cudaMemset2DAsync(dst + wpr, pitch * sizeof(uint64_t), 0, (w_pad - wpr) * sizeof(uint64_t), rows, st));
+    SB_CUDA(cudaMemcpy2DAsync(dst, pitch * sizeof(uint64_t), host, (size_t)wpr * sizeof(uint64_t),
+                              (size_t)wpr * sizeof(uint64_t), rows, cudaMemcpyHostToDevice, st));
+}
+
+// Panels of a host-output call. Where the tiles take long beside the copies
+// (more than 24 waves), host_panels: whole waves. Below, the copies do, and what
+// counts is that the copy back starts early and never waits: up to eight panels
+// of whole A blocks, equal in rows -- a fifth of the triangle is copied while the
+// second-last panel's rows come in -- of which each spreads over all SMs
+// (stream-K), and no more than one per 2 MiB that crosses the bus.
+std::vector<std::pair<uint32_t, uint32_t>> DenseEngine::host_plan(int kind, uint64_t n, uint64_t bus_bytes) const {
+    const int sms = require_device();
+    const uint32_t wave = kind == STORM_B200_KERNEL_POPC        ? 2u * (uint32_t)sms
+                          : kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4 ? (uint32_t)std::max(1, sms / 2)
+                                                               : (uint32_t)sms;
+    if (kind != KIND_F4 || n_tiles > 24 * wave) return host_panels(n_tiles, wave);
+    const uint32_t nb = (uint32_t)((n + F4_BM - 1) / F4_BM);
+    const uint32_t k = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({8, nb, bus_bytes >> 21}));
+    auto first = [nb](uint32_t b) { return (uint32_t)((uint64_t)b * nb - (uint64_t)b * (b - (b > 0)) / 2); };   // tile of block b
+    std::vector<std::pair<uint32_t, uint32_t>> p;
+    for (uint32_t q = k; q-- > 0;) p.emplace_back(first(nb * q / k), first(nb * (q + 1) / k));
+    return p;
+}
+
 uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits,
                                   uint32_t* d_out, uint32_t* host_out, int kernel_pref, cudaStream_t st,
                                   cudaStream_t copy_st) {
@@ -398,7 +460,8 @@ uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad
         return 0;
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
-    return panels_to_host(dX, n, w_pad, kind, d_out, host_out, st, copy_st, 0);
+    const auto panels = host_plan(kind, n, tri_size(n) * sizeof(uint32_t));
+    return panels_to_host(dX, n, w_pad, kind, panels, {}, d_out, host_out, st, copy_st);
 }
 
 uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits,
@@ -411,51 +474,62 @@ uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad,
         return 0;
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
-    // What the copies do not cover reads as zero: the row pitch's padding
-    // words and the rows [n, n_pad) that whole 128 x 256 tiles read.
+    const auto panels = host_plan(kind, n, tri_size(n) * sizeof(uint32_t) + n * host_wpr * sizeof(uint64_t));
+    const bool one = panels.size() == 1;             // everything on one stream
+    cudaStream_t in = one ? st : h2d_st;
+    // Rows [n, n_pad) read as zero: whole tiles read them.
     const uint64_t n_pad = round_up(n, 256), pitch = dense_pitch(w_pad);
-    if (host_wpr != w_pad)
-        SB_CUDA(cudaMemsetAsync(dX, 0, n_pad * pitch * sizeof(uint64_t), h2d_st));
-    else if (n_pad > n)
-        SB_CUDA(cudaMemsetAsync(dX + n * pitch, 0, (n_pad - n) * pitch * sizeof(uint64_t), h2d_st));
-    const uint64_t chunk_rows = round_up(std::max<uint64_t>(1, (n + 31) / 32), 128);
-    const uint64_t chunks = (n + chunk_rows - 1) / chunk_rows;
-    while (h2d_ev.size() < chunks) {
+    if (n_pad > n) SB_CUDA(cudaMemsetAsync(dX + n * pitch, 0, (n_pad - n) * pitch * sizeof(uint64_t), in));
+    uint64_t* stage = nullptr;
+    if (host_wpr < ROW_STAGE_WORDS && n * host_wpr * sizeof(uint64_t) <= ROW_STAGE_BYTES) {
+        d_stage.reserve(n * host_wpr);
+        stage = d_stage.p;
+    }
+    // Rows arrive last rows first: the bottom panels read only them. Chunks of
+    // whole panels where those are whole A blocks, else 32 equal ones; event c
+    // marks rows [arrive[c], n) (and the zeroing) as resident.
+    std::vector<uint64_t> arrive;
+    if (one) {
+        arrive.push_back(0);
+    } else if (kind == KIND_F4 && n_tiles <= 24u * (uint32_t)std::max(1, require_device() / 2)) {
+        for (const auto& q : panels) arrive.push_back((uint64_t)h_tiles[q.first].x * F4_BM);
+    } else {
+        const uint64_t chunk_rows = round_up(std::max<uint64_t>(1, (n + 31) / 32), 128);
+        for (uint64_t c = (n + chunk_rows - 1) / chunk_rows; c-- > 0;) arrive.push_back(c * chunk_rows);
+    }
+    while (h2d_ev.size() < arrive.size()) {
         cudaEvent_t e;
         SB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         h2d_ev.push_back(e);
     }
-    // Last rows first: the bottom panels read only them. Event c marks rows
-    // [c x chunk_rows, n) (and the zeroing) as resident.
-    for (uint64_t c = chunks; c-- > 0;) {
-        const uint64_t r0 = c * chunk_rows, r1 = std::min(n, r0 + chunk_rows);
-        SB_CUDA(cudaMemcpy2DAsync(dX + r0 * pitch, (size_t)pitch * sizeof(uint64_t), host_rows + r0 * host_wpr,
-                                  (size_t)host_wpr * sizeof(uint64_t), (size_t)host_wpr * sizeof(uint64_t),
-                                  r1 - r0, cudaMemcpyHostToDevice, h2d_st));
-        SB_CUDA(cudaEventRecord(h2d_ev[c], h2d_st));
-    }
     uint64_t s = 0;
     try {
-        s = panels_to_host(dX, n, w_pad, kind, d_out, host_out, st, copy_st, chunk_rows);
+        uint64_t r1 = n;
+        for (size_t c = 0; c < arrive.size(); ++c) {
+            const uint64_t r0 = arrive[c];
+            rows_to_device(dX + r0 * pitch, pitch, w_pad, host_rows + r0 * host_wpr, host_wpr, r1 - r0,
+                           stage ? stage + r0 * host_wpr : nullptr, in);
+            if (!one) SB_CUDA(cudaEventRecord(h2d_ev[c], in));
+            r1 = r0;
+        }
+        s = panels_to_host(dX, n, w_pad, kind, panels, one ? std::vector<uint64_t>{} : arrive, d_out, host_out, st,
+                           copy_st);
     } catch (...) {
-        cudaStreamSynchronize(h2d_st);   // no copy may still read the caller's rows after the return
+        cudaStreamSynchronize(in);   // no copy may still read the caller's rows after the return
         throw;
     }
-    SB_CUDA(cudaStreamSynchronize(h2d_st));
+    SB_CUDA(cudaStreamSynchronize(in));
     return s;
 }
 
-// chunk_rows != 0: rows arrive in chunks of chunk_rows on h2d_ev; each panel
-// waits for the chunk holding the lowest row its tiles read.
-uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, int kind, uint32_t* d_out,
-                                     uint32_t* host_out, cudaStream_t st, cudaStream_t copy_st,
-                                     uint64_t chunk_rows) {
-    const int sms = require_device();
+// arrive: rows [arrive[c], n) are resident once event h2d_ev[c] has passed
+// (descending; empty: all are); each panel waits for the lowest row its tiles
+// read.
+uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, int kind,
+                                     const std::vector<std::pair<uint32_t, uint32_t>>& panels,
+                                     const std::vector<uint64_t>& arrive, uint32_t* d_out, uint32_t* host_out,
+                                     cudaStream_t st, cudaStream_t copy_st) {
     const uint64_t bm = tile_rows_a(kind), bn = tile_rows_b(kind);
-    const uint32_t wave = kind == STORM_B200_KERNEL_POPC        ? 2u * (uint32_t)sms
-                          : kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4 ? (uint32_t)std::max(1, sms / 2)
-                                                               : (uint32_t)sms;
-    const auto panels = host_panels(n_tiles, wave);
     // first tile of each A block (the list is ordered by A block)
     std::vector<uint32_t> first_tile((size_t)h_tiles.back().x + 1, 0);
     for (uint32_t t = n_tiles; t-- > 0;) first_tile[h_tiles[t].x] = t;
@@ -465,35 +539,23 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
         panel_ev.push_back(e);
     }
     SB_CUDA(cudaEventRecord(log.ev0, st));
-    if (panels.size() == 1 && chunk_rows == 0) {   // one launch: its copy follows on the same stream
-        launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
-        SB_CUDA(cudaEventRecord(log.ev1, st));
-        DeviceFlags f;
-        try {
-            SB_CUDA(cudaMemcpyAsync(host_out, d_out, tri_size(n) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-            f = read_flags(d_flags.p, st);
-        } catch (...) {
-            cudaStreamSynchronize(st);
-            throw;
-        }
-        SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
-        log.launches = 1;
-        log.kernel = reported;
-        if (f.error) fail(STORM_B200_ETIMEOUT, "bitmap x bitmap kernel: bounded wait expired");
-        return f.sum;
-    }
+    cudaStream_t back = panels.size() == 1 ? st : copy_st;   // one launch: its copy follows on the same stream
     uint64_t copied_from = n;   // rows [copied_from, n) are on their way to the host
+    DeviceFlags f;
     try {
         for (size_t p = 0; p < panels.size(); ++p) {
             const uint32_t t0 = panels[p].first, t1 = panels[p].second;
-            if (chunk_rows) {
+            if (!arrive.empty()) {
                 uint64_t need = n;
                 for (uint32_t t = t0; t < t1; ++t)
                     need = std::min(need, std::min<uint64_t>(h_tiles[t].x * bm, h_tiles[t].y * bn));
-                SB_CUDA(cudaStreamWaitEvent(st, h2d_ev[need / chunk_rows], 0));
+                size_t c = 0;
+                while (c + 1 < arrive.size() && arrive[c] > need) ++c;
+                SB_CUDA(cudaStreamWaitEvent(st, h2d_ev[c], 0));
             }
             launch(kind, dX, (uint32_t)n, w_pad, t0, t1 - t0, d_out, st);
-            SB_CUDA(cudaEventRecord(panel_ev[p], st));
+            if (p + 1 == panels.size()) SB_CUDA(cudaEventRecord(log.ev1, st));
+            if (back != st) SB_CUDA(cudaEventRecord(panel_ev[p], st));
             // Every tile from t0 on is done: the A blocks whose first tile is at
             // or past t0 are complete, and their rows are contiguous in the
             // packed triangle.
@@ -503,21 +565,20 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
             if (r < copied_from) {
                 const uint64_t e0 = r * n - (r * (r - 1)) / 2;   // tri_index(n, r, r)
                 const uint64_t e1 = copied_from * n - (copied_from * (copied_from - 1)) / 2;
-                SB_CUDA(cudaStreamWaitEvent(copy_st, panel_ev[p], 0));
+                if (back != st) SB_CUDA(cudaStreamWaitEvent(back, panel_ev[p], 0));
                 SB_CUDA(cudaMemcpyAsync(host_out + e0, d_out + e0, (e1 - e0) * sizeof(uint32_t),
-                                        cudaMemcpyDeviceToHost, copy_st));
+                                        cudaMemcpyDeviceToHost, back));
                 copied_from = r;
             }
         }
+        f = read_flags(d_flags.p, st);
     } catch (...) {
         // no copy may still write the caller's buffer after the return
         cudaStreamSynchronize(st);
         cudaStreamSynchronize(copy_st);
         throw;
     }
-    SB_CUDA(cudaEventRecord(log.ev1, st));
-    const DeviceFlags f = read_flags(d_flags.p, st);
-    SB_CUDA(cudaStreamSynchronize(copy_st));
+    if (back != st) SB_CUDA(cudaStreamSynchronize(back));
     SB_CUDA(cudaEventElapsedTime(&log.last_ms, log.ev0, log.ev1));
     log.launches = (uint32_t)panels.size();
     log.kernel = reported;

@@ -17,6 +17,16 @@ namespace sb200 {
 // -> 46.4.  (256 bytes more was slower than none at 2^18: 395.1.)
 inline uint64_t dense_pitch(uint32_t w_pad) { return w_pad % 512 == 0 ? (uint64_t)w_pad + 8 : (uint64_t)w_pad; }
 
+// Host rows shorter than this, up to this size in all, cross the bus as they lie
+// and are spread out on the device (rows_to_device). Host to host on B200, copies
+// with two pitches / staged (ms): 12000 rows of 2504 bytes 6.64 / 5.37, 3000 of
+// them 0.94 / 0.55; 8192 of 8192 bytes 2.97 / 3.07, 16384 of them 10.44 / 10.63
+// (the spreading waits for a free SM).
+constexpr uint32_t ROW_STAGE_WORDS = 640;
+constexpr uint64_t ROW_STAGE_BYTES = 256ull << 20;
+void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_t* host, uint32_t wpr, uint64_t rows,
+                    uint64_t* stage, cudaStream_t st);
+
 // Device rows: X is [n_pad][dense_pitch(w_pad)] u64, of which each row's
 // first w_pad words are read (zero past the row's bits), n_pad % 256 == 0
 // and w_pad % 8 == 0.
@@ -68,6 +78,7 @@ struct DenseEngine {
                            double t, uint2* d_pairs, uint32_t* d_cnts, uint64_t cap, uint64_t* sum,
                            cudaStream_t st);
     DevBuf<uint32_t> d_card, d_scratch_tri, d_hist;
+    DevBuf<uint64_t> d_stage;   // host rows as they lie (up to ROW_STAGE_BYTES)
     DevBuf<unsigned long long> d_found;
 
    private:
@@ -77,9 +88,12 @@ struct DenseEngine {
     uint64_t run_sum(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, cudaStream_t st);
     void launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pad, uint32_t t0, uint32_t count,
                 uint32_t* d_out, cudaStream_t st);
-    void zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t grid, cudaStream_t st);
-    uint64_t panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, int kind, uint32_t* d_out,
-                            uint32_t* host_out, cudaStream_t st, cudaStream_t copy_st, uint64_t chunk_rows);
+    void zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t t0, uint32_t t1, uint32_t grid, cudaStream_t st);
+    std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint64_t bus_bytes) const;
+    uint64_t panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, int kind,
+                            const std::vector<std::pair<uint32_t, uint32_t>>& panels,
+                            const std::vector<uint64_t>& arrive, uint32_t* d_out, uint32_t* host_out, cudaStream_t st,
+                            cudaStream_t copy_st);
     std::vector<uint2> h_tiles;
     std::vector<cudaEvent_t> panel_ev, h2d_ev;
 };
