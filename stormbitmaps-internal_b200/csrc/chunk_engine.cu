@@ -2162,7 +2162,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         // Plan A: H = [0, k); the rows below k by postings.
         uint64_t best_k = lb;
         double best_a = -1.0;
-        for (uint64_t k = 0; k <= np; ++k) {
+        // H fills whole tiles: every 256th row, and the two ends
+        for (uint64_t k = 0; k <= np; k = k == np ? np + 1 : std::min(np, (k < lb && k + 256 > lb) ? lb : k / 256 * 256 + 256)) {
             const double v = tensor_ns((double)k, (double)(np - k)) + post_est(k);
             if (best_a < 0 || v < best_a) {
                 best_a = v;
@@ -2303,8 +2304,10 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_perm.reserve(n);
         SB_CUDA(cudaMemcpyAsync(d_perm.p, h_perm.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
         perm = d_perm.p;
-        // The tensor cores (stream-K) and the postings add into the triangle.
-        if (d_out) SB_CUDA(cudaMemsetAsync(d_out, 0, tri_size(n) * sizeof(uint32_t), st));
+        // The tensor cores (stream-K) and the list form add into the triangle;
+        // a row sweep over every row writes all of it.
+        const bool swept = nq == n && (use_run || sweep_form((double)ps.pairs, nq, (double)values_of(qrows)));
+        if (d_out && !swept) SB_CUDA(cudaMemsetAsync(d_out, 0, tri_size(n) * sizeof(uint32_t), st));
     }
 
     // ---- predicted device time of each engine for this plan

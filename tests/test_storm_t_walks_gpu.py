@@ -133,3 +133,36 @@ def test_row_sweep_in_16_bits(sb, n):
         np.testing.assert_array_equal(got[strict], want[strict])
         assert total == ws
         s.close()
+
+
+@pytest.mark.parametrize("n", (2, 300, 52000))
+def test_outputs_that_held_other_values(sb, n):
+    """Every entry of the triangle is written, whatever the buffer held: row
+    sweeps over all rows (no clear before them; past 65535 x 16 bits and one
+    block of counters too), the list form, and empty rows."""
+    import torch
+
+    g = gen.rng(n)
+    card = g.integers(0, 12, size=n) if n < 1000 else (np.arange(n) % 1000 == 0) * 9
+    base = g.integers(0, 1 << 18, size=n)
+    sets = [np.unique(base[r] % 3 * 70000 + g.integers(0, 50, size=int(card[r]))).astype(np.uint32) for r in range(n)]
+    if n > 1000:                                # one row past 16 bits, in list chunks: counters of 32 bits
+        sets[n - 1] = (np.arange(0, 65536, 17)[None, :] + (np.arange(20) << 16)[:, None]).ravel().astype(np.uint32)
+    vals, offs = gen.to_csr(sets)
+    out = torch.empty(n * (n + 1) // 2, dtype=torch.int32, device="cuda")
+    s = sb.Storm()
+    s.add_rows(vals, offs)
+    s.set_dense_block(0.0)
+    s.set_panel(0)
+    got = []
+    for mode in (2, 3, 4):
+        s.set_sparse_postings(mode)
+        out.fill_(-7)
+        s.matrix_device(out.data_ptr(), out.numel())
+        torch.cuda.synchronize()
+        got.append(out.clone())
+    s.close()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    if n < 1000:
+        want, _ = ol.sets_matrix(vals, offs)
+        np.testing.assert_array_equal(got[0].cpu().numpy().view(np.uint32), want)
