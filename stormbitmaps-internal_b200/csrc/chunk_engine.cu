@@ -950,11 +950,17 @@ __device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __
 
 // How rows_walk and row_walk take a set of rows: chunks per group (one from 48
 // entries a chunk on, or with bitmap chunks) and groups of the longest row.
+// Rows of few entries a chunk among which most entries lie in chunks of many
+// take groups of four: 32 such chunks are a long serial item for one warp
+// (3072 Zipf rows over 2^24, histogram to lists: 0.79 ms by 32, 0.59 by 8,
+// 0.58 by 4; 1094 over 2^23 0.32, 0.21, 0.20).
+constexpr uint32_t WALK_SKEW_GROUP = 4;
 struct WalkShape {
     uint32_t group = 1, groups = 0;
     template <class Facts>
     void of(uint64_t n, Facts facts) {
         uint64_t chunks = 0, entries = 0;
+        double spread = 0.0;                              // entries x (their row's entries per chunk)
         uint32_t most = 0;
         bool bitmaps = false;
         for (uint64_t k = 0; k < n; ++k) {
@@ -963,8 +969,9 @@ struct WalkShape {
             entries += f.list_entries;
             bitmaps |= f.bitmap_chunks != 0;
             most = std::max(most, f.chunks);
+            if (f.chunks) spread += (double)f.list_entries * (double)f.list_entries / (double)f.chunks;
         }
-        group = bitmaps || entries >= 48 * chunks ? 1u : 32u;
+        group = bitmaps || entries >= 48 * chunks ? 1u : spread >= 48.0 * (double)entries ? WALK_SKEW_GROUP : 32u;
         groups = (most + group - 1) / group;
     }
     uint32_t grid(uint64_t n, int sms) const {
@@ -1922,7 +1929,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // length of the plain list rows rounded to a power of two in [16, 32768]
     // (a run of length l spans about 1 + l / bin bins; the sweep's entry
     // reads, pieces^2 x bin / U for uniform rows, are least at bin = l).
-    uint32_t rwlog = 4;
+    uint32_t rwlog = 4, most_chunks = 0;
     if (facts_ok) {
         double sc = 0.0, sr = 0.0;
         for (uint64_t r = 0; r < n; ++r) {
@@ -1930,6 +1937,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             if (f.plain && f.bitmap_chunks == 0) {
                 sc += (double)f.card;
                 sr += (double)f.runs;
+                most_chunks = std::max(most_chunks, f.chunks);
             }
         }
         const double ml = sr > 0.0 ? sc / sr : 1.0;
@@ -2040,9 +2048,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                         : tc_ns * 65536.0 * (nb * (nb + 1.0) / 2.0 + nb * mb) +
                               (h + m) * (double)W * 8.0 * cost.ns_per_expand_byte;
     };
-    // ns of the run sweep with `checks` entry reads for q rows (per pair only)
-    auto run_ns = [&](double checks, uint64_t q) {
+    // ns of the run sweep with `checks` entry reads for q rows of `pieces`
+    // pieces (per pair only)
+    auto run_ns = [&](double checks, uint64_t q, double pieces) {
         return (double)q * (double)q * cost.ns_per_sweep_row_pair + checks * cost.ns_per_run_check * sweep_blocks(q) +
+               pieces * cost.ns_per_run_piece + (double)most_chunks * cost.ns_per_run_row_chunk +
                (double)n_bins * cost.ns_per_universe_value;
     };
     auto run_ok = [&](uint64_t q) {
@@ -2072,11 +2082,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                 C1 += (double)f.card;
                 C2 += (double)f.card * (double)f.card;
             }
-            const double run_e = run_ns(P * P * RW / (double)U, q);
+            const double run_e = run_ns(P * P * RW / (double)U, q, P);
             const double val_e = post_ns((C1 * C1 - C2) / (2.0 * (double)U), q, C1);
             if (postings_mode == 4 || run_e < val_e || !lists_only) {
                 run_histogram(rest);
-                if (postings_mode == 4 || postings_mode == 1 || run_ns((double)run_checks, q) < alt) {
+                if (postings_mode == 4 || postings_mode == 1 || run_ns((double)run_checks, q, P) < alt) {
                     use_run = true;
                     qrows = rest;
                     return true;
@@ -2092,15 +2102,30 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         return false;
     };
     bool panel_plan = false;
+    // The panel's blocks of `rows` panel rows: the bytes that expansion (written,
+    // read again) and transposed lines take, and what one query value costs
+    // against all of them, in units of a whole block (ns_per_panel_value): a
+    // narrow line reads in proportion to its width, the staging of the value
+    // does not shrink.
+    auto panel_last = [](uint64_t rows) { return rows ? (rows - 1) % PANEL_ROWS + 1 : 0; };
+    auto panel_bytes = [&](uint64_t rows) {
+        const double lines = (double)(rows - panel_last(rows)) + 64.0 * (rows ? panel_block_words(panel_last(rows)) : 0);
+        return (2.0 * (double)rows + lines) * (double)W * 8.0;
+    };
+    auto panel_blocks = [&](uint64_t rows) {
+        if (!rows) return 0.0;
+        const uint32_t pw = panel_block_words(panel_last(rows));
+        return (double)((rows - 1) / PANEL_ROWS) + (pw == 32 ? 1.0 : pw == 16 ? PANEL_HALF_COST : PANEL_QUARTER_COST);
+    };
     // The panel needs a transposed block and some of its rows expanded in HBM.
     const uint64_t px_words = PANEL_ROWS * PANEL_PITCH * std::min<uint64_t>(slots, PANEL_X_SLOTS);
-    const uint64_t panel_bytes = (PANEL_ROWS * W + px_words) * sizeof(uint64_t);
-    auto panel_fits = [&]() {
+    auto dt_words = [&](uint64_t rows) { return U * panel_block_words(rows); };   // of its widest block
+    auto panel_fits = [&](uint64_t rows) {
         if (!facts_ok || panel_mode == 0 || U > PANEL_MAX_UNIVERSE) return false;
-        if (d_DT.n >= PANEL_ROWS * W && d_pX.n >= px_words) return true;   // it is there already
+        if (d_DT.n >= dt_words(rows) && d_pX.n >= px_words) return true;   // it is there already
         size_t fr = 0, tot = 0;
         SB_CUDA(cudaMemGetInfo(&fr, &tot));
-        return (double)panel_bytes < 0.5 * ((double)fr + (double)(d_pX.n + d_DT.n) * sizeof(uint64_t));
+        return (double)((dt_words(rows) + px_words) * sizeof(uint64_t)) < 0.5 * ((double)fr + (double)(d_pX.n + d_DT.n) * sizeof(uint64_t));
     };
 
     if (panel_mode == 2 && facts_ok && U <= PANEL_MAX_UNIVERSE) {
@@ -2155,7 +2180,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             double v = from >= lb ? post_ns((r1 * r1 - r2) / (2.0 * (double)U), q, r1) : HUGE_VAL;
             if (run_ok(q)) {
                 const double P = S3[np] - S3[from];
-                v = std::min(v, run_ns(P * P * RW / (double)U, q));
+                v = std::min(v, run_ns(P * P * RW / (double)U, q, P));
             }
             return v;
         };
@@ -2172,27 +2197,32 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         }
         if (postings_mode == 4) best_k = 0;                // forced: every plain row to the run sweep
         else if (postings_mode > 0) best_k = lb;           // forced: every list row to the postings
+        // ns of the panel over the rows [0, e) (H the first h of them), queried by
+        // M among themselves and by all that follow
+        auto panel_ns = [&](uint64_t h, uint64_t e) {
+            const double m = (double)(e - h), hh = (double)h, nl = (double)(np - e), nb = panel_blocks(e);
+            const double sl = S1[np] - S1[e], sm = S1[e] - S1[h];
+            return cost.ns_per_panel_value * (sl * nb + sm * std::min(nb, (hh + 0.5 * m) / PANEL_ROWS + 0.5)) +
+                   cost.ns_per_panel_pair * (nl * (double)e + m * (m - 1.0) / 2.0 + m * hh) +
+                   cost.ns_per_panel_byte * panel_bytes(e) + cost.ns_panel_fixed;
+        };
         // Plan B over candidate cuts (h, m).
         uint64_t best_h = 0, best_m = 0;
         double best_b = -1.0;
         if (postings_mode < 0 && panel_mode != 0 && facts_ok && U <= PANEL_MAX_UNIVERSE) {
+            // cuts: every 12 %, and where the tensor tiles and the narrow blocks end
             std::vector<uint64_t> cand{0, lb, np};
             for (double x = 1.0; x < (double)np; x *= 1.12) cand.push_back((uint64_t)x);
+            for (uint64_t x = 256; x < np && x <= 2 * PANEL_ROWS; x += 256) cand.push_back(x);
             std::sort(cand.begin(), cand.end());
             cand.erase(std::unique(cand.begin(), cand.end()), cand.end());
-            const double build_ns = 3.0 * (double)PANEL_ROWS * (double)W * 8.0 * cost.ns_per_panel_byte;
-            for (uint64_t h : cand) {
-                for (uint64_t e : cand) {                  // e = h + m
-                    if (e < h || e > np || e == 0) continue;   // rows past e: postings (value or run form)
-                    if (panel_mode > 0 && e == h) continue;    // forced: some rows in M
-                    const double m = (double)(e - h), hh = (double)h, nl = (double)(np - e);
-                    const double nb = std::ceil((double)e / PANEL_ROWS);
-                    const double nbh = hh / PANEL_ROWS, nbm = m / PANEL_ROWS;
-                    const double sl = S1[np] - S1[e], sm = S1[e] - S1[h];
-                    const double panel = cost.ns_per_panel_value * (sl * nb + sm * (nbh + 0.5 * nbm + 0.5)) +
-                                         cost.ns_per_panel_pair * (nl * (double)e + m * (m - 1.0) / 2.0 + m * hh) +
-                                         nb * build_ns;
-                    const double v = tensor_ns(hh, 0.0) + panel + post_est(e);
+            for (uint64_t e : cand) {                      // e = h + m; rows past e: postings (value or run form)
+                if (e == 0 || e > np) continue;
+                const double rest_ns = post_est(e);
+                for (uint64_t h : cand) {
+                    if (h > e) break;
+                    if (panel_mode > 0 && e == h) break;   // forced: some rows in M
+                    const double v = tensor_ns((double)h, 0.0) + panel_ns(h, e) + rest_ns;
                     if (best_b < 0 || v < best_b) {
                         best_b = v;
                         best_h = h;
@@ -2201,8 +2231,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                 }
             }
         }
-        // the free memory is asked for last: the query takes up to milliseconds
-        panel_plan = best_b >= 0 && (panel_mode > 0 || best_b < best_a) && panel_fits();
+        // The estimates are within 10 % of the times where the plans are close.
+        // The free memory is asked for last: the query takes up to milliseconds.
+        panel_plan = best_b >= 0 && (panel_mode > 0 || best_b < 0.9 * best_a) && panel_fits(best_h + best_m);
         std::vector<uint32_t> rest;
         if (panel_plan) {
             dense.assign(pl.begin(), pl.begin() + best_h);
@@ -2219,21 +2250,20 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         if (rest.size() >= 2) {
             // The estimate assumes independent rows; correlated rows share
             // more. With the exact count, keep the postings only if they beat
-            // the alternative on these pairs: the panel (the rows queried
-            // against themselves) or the tensor cores.
-            const double q = (double)rest.size();
-            const double alt = panel_plan ? cost.ns_per_panel_value * (S1[np] - S1[np - rest.size()]) *
-                                                (0.5 * std::ceil(q / PANEL_ROWS) + 0.5) +
-                                                cost.ns_per_panel_pair * q * (q - 1.0) / 2.0
-                                          : tensor_ns(q, 0.0);
-            if (decide(rest, alt)) {
-            } else if (panel_plan) {
-                mrows.insert(mrows.end(), rest.begin(), rest.end());
-            } else {
-                dense.insert(dense.end(), rest.begin(), rest.end());
-            }
-        } else if (panel_plan) {
+            // the alternative on these pairs: the panel with these rows in it
+            // too (more lines, a wider block) or the tensor cores.
+            const double alt = panel_plan ? panel_ns(best_h, np) - panel_ns(best_h, best_h + best_m)
+                                          : tensor_ns((double)rest.size(), 0.0);
+            if (decide(rest, alt)) rest.clear();
+        }
+        if (panel_plan && !rest.empty()) {                 // they join the panel, or all go to the tensor cores
+            panel_plan = panel_mode > 0 || (tensor_ns((double)best_h, 0.0) + panel_ns(best_h, np) < tensor_ns((double)np, 0.0) &&
+                                            panel_fits(np));
             mrows.insert(mrows.end(), rest.begin(), rest.end());
+            if (!panel_plan) {
+                dense.insert(dense.end(), mrows.begin(), mrows.end());
+                mrows.clear();
+            }
         } else {
             dense.insert(dense.end(), rest.begin(), rest.end());
         }
@@ -2267,7 +2297,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // Panels of P rows when they do not all fit the budget.
     if (panel_plan) {
         d_pX.reserve(px_words);
-        d_DT.reserve(PANEL_ROWS * W);
+        d_DT.reserve(dt_words(mrows.size() + dense.size()));
     }
     const uint64_t nd0 = dense.size();
     const uint64_t nd_pad = round_up(nd0, 256);
@@ -2320,23 +2350,26 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         last_engine_work[0] = 2.0 * (dd * (dd + 1.0) / 2.0 + dd * tqn) * (double)U;
         last_engine_work[1] = (double)(nc * n - (nc * (nc - 1)) / 2 * (nc ? 1 : 0));
         if (panel_plan && (nm || nd) && (nq + nm)) {
-            const double npw = (double)(nm + nd), nb = std::ceil(npw / PANEL_ROWS);
-            double vb = 0.0, pairs = 0.0;
+            const uint64_t npw = nm + nd;
+            double vb = 0.0, lines = 0.0, pairs = 0.0;
             for (uint64_t w = nc; w < nc + nq + nm; ++w) {
-                const double after = (double)(n - 1 - w) < npw ? (double)(n - 1 - w) : npw;   // panel rows after it
-                vb += (double)d.facts[h_perm[w]].card * std::ceil(after / PANEL_ROWS);
-                pairs += after;
+                const uint64_t after = std::min<uint64_t>(n - 1 - w, npw);   // panel rows after it
+                const uint64_t skip = (npw - after) / PANEL_ROWS * PANEL_ROWS;   // in blocks it is not queried against
+                const double c = (double)d.facts[h_perm[w]].card;
+                vb += c * panel_blocks(npw - skip);
+                lines += c * 8.0 * (double)((npw - skip - panel_last(npw)) / 64 + panel_block_words(panel_last(npw)));
+                pairs += (double)after;
             }
             last_engine_pred_ms[2] = 1e-6 * (cost.ns_per_panel_value * vb + cost.ns_per_panel_pair * pairs +
-                                             nb * 3.0 * PANEL_ROWS * (double)W * 8.0 * cost.ns_per_panel_byte);
-            last_engine_work[2] = 256.0 * vb + 4.0 * pairs + nb * 3.0 * PANEL_ROWS * (double)W * 8.0;
+                                             panel_bytes(npw) * cost.ns_per_panel_byte);
+            last_engine_work[2] = lines + 4.0 * pairs + panel_bytes(npw);
         }
         if (nq && use_run) {
             // run sweep: the pieces (8 B each, written and read), the bin
             // entries each piece reads (8 B), 4 B per count of the slice
-            last_engine_pred_ms[3] = 1e-6 * run_ns((double)run_checks, nq);
             double pcs = 0.0;
             for (uint32_t k : h_rpieces) pcs += (double)k;
+            last_engine_pred_ms[3] = 1e-6 * run_ns((double)run_checks, nq, pcs);
             last_engine_work[3] = 16.0 * pcs + 8.0 * (double)run_entries + 8.0 * (double)run_checks +
                                   4.0 * (double)nq * ((double)nq + 1.0) / 2.0 + 4.0 * (double)n_bins;
         } else if (nq) {
@@ -2425,13 +2458,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         // PANEL_MIN_SEG values (the per-item epilogue costs about as much as
         // a few hundred values), and doubled until the split rows' scratch
         // slots fit PANEL_MAX_SLOTS.
-        uint64_t max_card = 0;
         double total = 0.0;
-        for (uint64_t w = nc; w < nc + nq + nm; ++w) {
-            const uint64_t c = d.facts[h_perm[w]].card;
-            max_card = std::max<uint64_t>(max_card, c);
-            total += (double)c;
-        }
+        for (uint64_t w = nc; w < nc + nq + nm; ++w) total += (double)d.facts[h_perm[w]].card;
         std::vector<PanelItem> items;
         std::vector<PanelSplit> splits;
         std::vector<double> weight;
@@ -2480,13 +2508,12 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                                     cudaMemcpyHostToDevice, st));
         }
         static std::atomic<uint64_t> t_done{0};
-        smem_attr_once(panel_transpose_kernel, (int)PANEL_T_SMEM, t_done);
-        std::vector<uint32_t> bmap(PANEL_ROWS);
-        const uint32_t qgrid = (uint32_t)sms * 8;
+        smem_attr_once(panel_transpose_kernel<32>, (int)panel_t_smem(32), t_done);
         for (uint64_t b0 = 0; b0 < npw; b0 += PANEL_ROWS) {
             const uint32_t prows = (uint32_t)std::min<uint64_t>(PANEL_ROWS, npw - b0);
-            for (uint32_t t = 0; t < PANEL_ROWS; ++t) bmap[t] = t < prows ? h_perm[pw0 + b0 + t] : ~0u;
-            SB_CUDA(cudaMemcpyAsync(d_pmap.p, bmap.data(), PANEL_ROWS * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
+            const uint32_t pw = panel_block_words(prows);
+            SB_CUDA(cudaMemcpyAsync(d_pmap.p, h_perm.data() + pw0 + b0, prows * sizeof(uint32_t), cudaMemcpyHostToDevice,
+                                    st));
             // PANEL_X_SLOTS chunk slots at a time, block-major as the tensor
             // panels: the expanded rows of a whole block would take as much
             // memory as the block itself, and its allocation 20 ms of a
@@ -2494,25 +2521,25 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             const RowLayout play{PANEL_PITCH, PANEL_ROWS * PANEL_PITCH};
             for (uint32_t s0 = 0; s0 < slots; s0 += PANEL_X_SLOTS) {
                 const uint32_t ns = (uint32_t)std::min<uint64_t>(PANEL_X_SLOTS, slots - s0);
-                const uint32_t items = PANEL_ROWS * ns / EXPAND_WARPS;
+                const uint32_t items = (prows * ns + EXPAND_WARPS - 1) / EXPAND_WARPS;
                 expand_rows_kernel<<<std::min(items, (uint32_t)sms * 64), EXPAND_WARPS * 32, 0, st>>>(
-                    d.view(), d_pmap.p, PANEL_ROWS, s0, ns, (uint32_t)slots, play, d_pX.p);
-                panel_transpose_kernel<<<ns * CHUNK_WORDS / PANEL_T_WORDS, 1024, PANEL_T_SMEM, st>>>(
-                    d_pX.p, play, d_DT.p + (uint64_t)s0 * CHUNK_WORDS * 64 * PANEL_WORDS);
+                    d.view(), d_pmap.p, prows, s0, ns, (uint32_t)slots, play, d_pX.p);
+                auto transpose = pw == 32 ? panel_transpose_kernel<32> : pw == 16 ? panel_transpose_kernel<16>
+                                                                                  : panel_transpose_kernel<8>;
+                transpose<<<ns * CHUNK_WORDS / PANEL_T_WORDS, pw * 32, panel_t_smem(pw), st>>>(
+                    d_pX.p, play, prows, d_DT.p + (uint64_t)s0 * CHUNK_WORDS * 64 * pw);
                 launches += 2;
             }
             SB_CUDA(cudaMemsetAsync(d_ctr.p, 0, sizeof(unsigned long long), st));
             const uint32_t ni = (uint32_t)items.size();
             uint32_t* scr = splits.empty() ? nullptr : d_pscratch.p;
-#define SB_PANEL_QUERY(NP)                                                                                      \
-    panel_query_kernel<NP><<<qgrid, PANEL_Q_WARPS * 32, 0, st>>>(d.view(), perm, d_items.p, ni, pw0 + b0, prows, \
-                                                                 d_DT.p, n, d_out, scr, d_flags.p, d_ctr.p)
-            if (max_card < (1ull << 11)) SB_PANEL_QUERY(8);
-            else if (max_card < (1ull << 15)) SB_PANEL_QUERY(12);
-            else if (max_card < (1ull << 19)) SB_PANEL_QUERY(16);
-            else if (max_card < (1ull << 23)) SB_PANEL_QUERY(20);
-            else SB_PANEL_QUERY(24);
-#undef SB_PANEL_QUERY
+            auto query = [&](auto kernel) {
+                kernel<<<(uint32_t)sms * (PANEL_Q_SMEM_SM / (panel_q_smem(pw) + 1024)), 32, panel_q_smem(pw), st>>>(d.view(), perm, d_items.p, ni, pw0 + b0, prows, d_DT.p, n,
+                                                             d_out, scr, d_flags.p, d_ctr.p);
+            };
+            if (pw == 32) query(panel_query_kernel<32>);
+            else if (pw == 16) query(panel_query_kernel<16>);
+            else query(panel_query_kernel<8>);
             launches += 1;
             if (scr && d_out) {
                 panel_reduce_kernel<<<(uint32_t)std::min<uint64_t>(splits.size(), (uint64_t)sms * 8), 256, 0, st>>>(

@@ -200,7 +200,7 @@ enum PairMode : uint32_t {
 struct ChunkCostModel {
     double ns_per_shared_chunk = 0.086;
     double ns_per_lane_iteration = 0.0228;
-    double ns_per_tensor_bit = 0.3e-6;       // per bit of a pair in the tensor cores' 256 x 256 tiles
+    double ns_per_tensor_bit = 0.255e-6;      // per bit of a pair in the tensor cores' 256 x 256 tiles
     double ns_per_expand_byte = 1.0 / 2600.0;
     double ns_per_posting_pair = 0.010;      // one (pair, shared value) increment, output in L2
     double ns_per_posting_pair_hbm = 0.045;  // the same, output larger
@@ -210,9 +210,12 @@ struct ChunkCostModel {
     double ns_per_sweep_count = 0.0005;      // row sweep: clearing and writing, per (row, row)
     double ns_per_sweep_row_pair = 0.0047;   // run sweep: the same
     double ns_per_universe_value = 6e-3;     // histogram clear + scans per universe value
-    double ns_per_panel_value = 0.04;        // transposed panel: one query value against one 2048-row block
+    double ns_per_panel_value = 0.036;       // transposed panel: one query value against one 2048-row block
     double ns_per_panel_pair = 0.005;        // transposed panel: one count written
     double ns_per_panel_byte = 1.0 / 4300.0; // transposed panel: expansion and transpose traffic
+    double ns_panel_fixed = 1e5;             // transposed panel: its launches' ramps, the last items of a query
+    double ns_per_run_row_chunk = 600.0;     // run sweep: the longest row, walked by one CTA, per chunk
+    double ns_per_run_piece = 0.08;          // run sweep: one piece counted, stored and put into its bin's list
     double ns_per_run_check = 0.03;          // run sweep: one bin entry read against one piece
 };
 double chunk_self_pair_ns(const ChunkCostModel& m, const ChunkRowFacts& f, uint64_t slots);

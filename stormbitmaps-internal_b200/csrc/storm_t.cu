@@ -903,6 +903,7 @@ int STORM_calibrate(STORM_t* s, uint32_t sample_rows, double* out) {
         c.ns_per_panel_byte *= scale[1];
         if (post_form == 2) {   // the postings ran as the run sweep: its constant
             c.ns_per_run_check *= scale[2];
+            c.ns_per_run_piece *= scale[2];
         } else {
             c.ns_per_posting_pair *= scale[2];
             c.ns_per_posting_pair_hbm *= scale[2];

@@ -166,3 +166,30 @@ def test_outputs_that_held_other_values(sb, n):
     if n < 1000:
         want, _ = ol.sets_matrix(vals, offs)
         np.testing.assert_array_equal(got[0].cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("n", (1, 512, 513, 1024, 1025, 2049))
+def test_panel_widths_and_counter_flushes(sb, n):
+    """Transposed blocks of 512, 1024 and 2048 rows (and one row in a second
+    block), queried by rows of fewer values than a batch, of more than the
+    counters hold between two flushes (2016 words), in one work item and in
+    several, lists and bitmap chunks in one row, chunks missing, empty rows."""
+    g = gen.rng(n)
+    sets = []
+    for r in range(n):
+        v = [g.integers(0, 1 << 22, size=int(g.integers(0, 40))), np.arange(r % 7, 50)]
+        if r % 64 == 1:
+            v.append(g.integers(0, 40 << 16, size=30000))          # list chunks, split into items
+        if r % 100 == 3:
+            v.append((5 << 16) + g.choice(65536, size=9000, replace=False))   # a bitmap chunk
+        sets.append(np.unique(np.concatenate(v)).astype(np.uint32))
+    sets[n // 2] = np.zeros(0, np.uint32)
+    vals, offs = gen.to_csr(sets)
+    want, ws = ol.sets_matrix(vals, offs)
+    s = sb.Storm()
+    s.add_rows(vals, offs)
+    s.set_panel(2)
+    got, total = s.matrix()
+    np.testing.assert_array_equal(got, want)
+    assert total == ws and s.last_panel_rows() in (0, n)
+    s.close()
