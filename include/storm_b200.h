@@ -271,11 +271,11 @@ uint64_t STORM_last_dense_panels(const STORM_t* s);
  * value -- pairs with nothing in common cost nothing.  mode -1 (default):
  * used when the exact increment count predicts less time than the chunk
  * kernel; 1: whenever rows qualify; 0: never.  Per-pair counts take one of
- * two forms: the increments go list by list into the output, or -- for
- * outputs larger than L2, and when predicted faster from the exact
- * increment count -- a row sweep counts each row's partners in shared
- * memory (in blocks of 51200 partner rows, reading the row's lists once per
- * block) and writes its slice once.  A third per-pair form indexes runs
+ * two forms: the increments go list by list into the output, or -- when
+ * predicted faster from the exact increment count -- a row sweep counts each
+ * row's partners in shared memory (up to 65535 rows of at most 65535 values
+ * at once, otherwise in blocks of 51200 partner rows, reading the row's lists
+ * once per block) and writes its slice once.  A third per-pair form indexes runs
  * instead of values: the universe is cut into bins of a power of two near
  * the rows' mean run
  * length, each row's maximal runs into pieces per bin, and a row sweep adds

@@ -48,6 +48,9 @@ constexpr uint32_t C2_B_STAGE_BYTES = C2_B_ATOM_BYTES * (TS_KBITS / 128);   // 3
 constexpr uint32_t C2_TMEM_COLS = 512;
 constexpr uint32_t C2_A_COL0 = 256;
 constexpr uint32_t C2_EPI_BYTES = 8 * 32 * 32 * 4;         // per epilogue warp: a 32 x 32 u32 block
+// Rows up to this many bits take the coalesced epilogue (the epilogue is a
+// larger share of a short tile); longer rows the lean launch.
+constexpr uint64_t C2_COALESCE_MAX_BITS = 1u << 17;
 constexpr uint32_t C2_SMEM_BYTES = C2_STAGES * C2_B_STAGE_BYTES + 1024 + 256 + C2_EPI_BYTES;
 constexpr uint32_t C2_WARPS_PER_SIDE = 8;                  // arrivals per CTA on full / acc_empty
 

@@ -1,12 +1,12 @@
 // bb_mma_ts.cuh -- B x B on tcgen05 with the A operand in tensor memory.
 //
-// Same arithmetic as bb_mma.cuh (u8 x u8 -> s32, A bytes weighted 2^(k mod 8),
-// B bytes 2^(7 - k mod 8), D = 128 |Xi & Xj|), different data movement: the
-// 128 rows of the A panel are expanded by their own threads straight into
-// TMEM with tcgen05.st (lane = row, four K bytes per 32-bit column), so only
-// the 256 B rows pass through shared memory.  Measured on the SS form, the
-// shared-memory pipe (expansion stores + the tensor core's operand reads)
-// was the bottleneck; this removes a third of that traffic.
+// For rows of 2^24 .. 2^27 bits, past what the 4-bit kernel's fp32 accumulator
+// counts exactly: u8 x u8 -> s32, A bytes weighted 2^(k mod 4) and B bytes
+// 2^(3 - k mod 4), D = 8 |Xi & Xj| < 2^31.  The 128 rows of the A panel are
+// expanded by their own threads straight into TMEM with tcgen05.st (lane = row,
+// four K bytes per 32-bit column), so only the 256 B rows pass through shared
+// memory, whose pipe bounds the kernel (expansion stores and the tensor core's
+// operand reads).
 //
 // Warp roles (416 threads): warps 0-3 expand A rows into TMEM, warps 4-11
 // expand B rows into the swizzled smem ring, warp 12 owns TMEM and issues
@@ -31,12 +31,7 @@ constexpr uint32_t TS_B_ATOM_BYTES = TS_BN * 128;          // one 128-byte K ato
 constexpr uint32_t TS_B_STAGE_BYTES = TS_B_ATOM_BYTES * (TS_KBITS / 128);
 constexpr uint32_t TS_TMEM_COLS = 512;
 constexpr uint32_t TS_A_COL0 = 256;
-constexpr uint32_t TS_EPI_BYTES = 8 * 32 * 32 * 4;         // per epilogue warp: a 32 x 32 u32 block
-constexpr uint32_t TS_SMEM_BYTES = TS_STAGES * TS_B_STAGE_BYTES + 1024 + 256 + TS_EPI_BYTES;
-constexpr uint32_t TS_SMEM_BYTES_LEAN = TS_STAGES * TS_B_STAGE_BYTES + 1024 + 256;
-// Rows up to this many bits take the coalesced epilogue (the epilogue is a
-// larger share of a short tile); longer rows the lean launch.
-constexpr uint64_t TS_COALESCE_MAX_BITS = 1u << 17;
+constexpr uint32_t TS_SMEM_BYTES = TS_STAGES * TS_B_STAGE_BYTES + 1024 + 256;
 
 struct TsCtl {
     uint64_t full[TS_STAGES];
@@ -160,7 +155,7 @@ struct TsThresh {
     unsigned long long* found;
 };
 
-template <bool kRowMap, bool kW4, bool kThresh = false>
+template <bool kRowMap, bool kThresh = false>
 __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay,
                                         const uint2* __restrict__ tiles, uint32_t n_tiles,
                                         uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
@@ -172,14 +167,6 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
     uint8_t* ring = ts_smem + pad;
     const uint32_t ring_addr = raw_addr + pad;
     TsCtl* ctl = reinterpret_cast<TsCtl*>(ring + TS_STAGES * TS_B_STAGE_BYTES);
-    uint32_t* epi = reinterpret_cast<uint32_t*>(ring + TS_STAGES * TS_B_STAGE_BYTES + 256);
-    // The launch decides the epilogue: with TS_SMEM_BYTES of dynamic shared
-    // memory the counts are staged through smem and stored coalesced; with
-    // TS_SMEM_BYTES_LEAN (no staging buffer, more L1 left for the loads that
-    // feed long rows) each lane stores its own row.
-    uint32_t dyn_smem;
-    asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dyn_smem));
-    const bool coalesced = !kThresh && dyn_smem >= TS_SMEM_BYTES;
 
     const int tid = threadIdx.x;
     const int warp = tid >> 5, lane = tid & 31;
@@ -236,8 +223,8 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         uint32_t r[32];
-                        expand_a64<kW4>(w[2 * h], r);
-                        expand_a64<kW4>(w[2 * h + 1], r + 16);
+                        expand_a64<true>(w[2 * h], r);
+                        expand_a64<true>(w[2 * h + 1], r + 16);
                         tmem_st_32x32b_x32(taddr + 32u * h, r);
                     }
                     tmem_st_wait();
@@ -247,8 +234,7 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         // word q covers K bytes [64q, 64q + 64): atom q/2, chunks 4(q%2)..
-                        expand_store<true, kW4>(b_stage + (q >> 1) * TS_B_ATOM_BYTES, prow, (uint32_t)(q & 1),
-                                                w[q]);
+                        expand_store<true, true>(b_stage + (q >> 1) * TS_B_ATOM_BYTES, prow, (uint32_t)(q & 1), w[q]);
                     }
                     fence_proxy_async_smem();
                 }
@@ -266,95 +252,61 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
             const uint32_t lane_grp = (uint32_t)(warp & 3) * 32u;
             const uint32_t col0 = (uint32_t)(warp >> 2) * 128u;
             unsigned long long local = 0;
-            if (coalesced) {
-                // Each 32 x 32 block goes through this warp's smem buffer
-                // (16-byte chunks XOR-swizzled by row) so that one store
-                // instruction writes 32 consecutive counts of one row.
-                uint32_t* buf = epi + warp * 1024;
+            // Each lane writes its own row.
+            const uint64_t i = i0 + lane_grp + lane;
+            const bool row_ok = i < n;
+            const uint64_t base = row_ok ? tri_index(n, i, i) - i : 0;
 #pragma unroll 1
-                for (uint32_t c = 0; c < 4; ++c) {
-                    uint32_t r[32];
-                    tmem_ld_32x32b_x32(tmem_base + (lane_grp << 16) + col0 + 32u * c, r);
-                    tmem_ld_wait();
+            for (uint32_t c = 0; c < 4; ++c) {
+                uint32_t r[32];
+                tmem_ld_32x32b_x32(tmem_base + (lane_grp << 16) + col0 + 32u * c, r);
+                tmem_ld_wait();
+                if constexpr (kThresh) {
+                    // whole tiles only (no partial segments); every lane
+                    // stays in the loop for the warp-aggregated appends
+                    const uint64_t jb = j0 + col0 + 32u * c;
+                    const double ci = row_ok ? (double)th.card[i] : 0.0;
 #pragma unroll
-                    for (uint32_t k = 0; k < 8; ++k)
-                        *reinterpret_cast<uint4*>(buf + lane * 32 + ((k ^ (lane & 7)) << 2)) =
-                            make_uint4(r[4 * k], r[4 * k + 1], r[4 * k + 2], r[4 * k + 3]);
-                    __syncwarp();
-                    const uint64_t j = j0 + col0 + 32u * c + lane;
-#pragma unroll 4
-                    for (uint32_t rr = 0; rr < 32; ++rr) {
-                        const uint64_t i = i0 + lane_grp + rr;
-                        const uint32_t cnt =
-                            buf[rr * 32 + ((((uint32_t)lane >> 2) ^ (rr & 7)) << 2) + (lane & 3)] >> (kW4 ? 3 : 7);
-                        if (i < n && j >= i && j < n && ts_mapped<kRowMap>(row_map, i, j)) {
+                    for (int e = 0; e < 32; ++e) {
+                        const uint64_t j = jb + e;
+                        const uint32_t cnt = r[e] >> 3;
+                        bool pass = false;
+                        if (row_ok && j > i && j < n) {
+                            local += cnt;
+                            if (cnt) {
+                                const double u = ci + (double)th.card[j] - (double)cnt;
+                                pass = u > 0.0 && (double)cnt / u >= th.t;
+                            }
+                        }
+                        const uint32_t m = __ballot_sync(0xffffffffu, pass);
+                        if (m) {
+                            const int leader = __ffs(m) - 1;
+                            unsigned long long b0 = 0;
+                            if (lane == leader) b0 = atomicAdd(th.found, (unsigned long long)__popc(m));
+                            b0 = __shfl_sync(0xffffffffu, b0, leader);
+                            if (pass) {
+                                const unsigned long long k = b0 + __popc(m & ((1u << lane) - 1u));
+                                if (k < th.cap) {
+                                    th.pairs[k] = make_uint2((uint32_t)i, (uint32_t)j);
+                                    th.cnts[k] = cnt;
+                                }
+                            }
+                        }
+                    }
+                } else if (row_ok) {
+                    const uint64_t jb = j0 + col0 + 32u * c;
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) {
+                        const uint64_t j = jb + e;
+                        const uint32_t cnt = r[e] >> 3;
+                        if (j >= i && j < n && ts_mapped<kRowMap>(row_map, i, j)) {
                             if (out) {
-                                uint32_t* dst = out + ts_out_index<kRowMap>(n, i, j, row_map, n_out);
-                                if (partial) atomicAdd(dst, cnt);   // one K segment's share
+                                uint32_t* dst = out + (kRowMap ? ts_out_index<true>(n, i, j, row_map, n_out)
+                                                               : base + j);
+                                if (partial) atomicAdd(dst, cnt);
                                 else *dst = cnt;
                             }
                             if (j > i) local += cnt;
-                        }
-                    }
-                    __syncwarp();
-                }
-            } else {
-                // Lean form (no staging buffer): each lane writes its own row.
-                const uint64_t i = i0 + lane_grp + lane;
-                const bool row_ok = i < n;
-                const uint64_t base = row_ok ? tri_index(n, i, i) - i : 0;
-#pragma unroll 1
-                for (uint32_t c = 0; c < 4; ++c) {
-                    uint32_t r[32];
-                    tmem_ld_32x32b_x32(tmem_base + (lane_grp << 16) + col0 + 32u * c, r);
-                    tmem_ld_wait();
-                    if constexpr (kThresh) {
-                        // whole tiles only (no partial segments); every lane
-                        // stays in the loop for the warp-aggregated appends
-                        const uint64_t jb = j0 + col0 + 32u * c;
-                        const double ci = row_ok ? (double)th.card[i] : 0.0;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) {
-                            const uint64_t j = jb + e;
-                            const uint32_t cnt = r[e] >> (kW4 ? 3 : 7);
-                            bool pass = false;
-                            if (row_ok && j > i && j < n) {
-                                local += cnt;
-                                if (cnt) {
-                                    const double u = ci + (double)th.card[j] - (double)cnt;
-                                    pass = u > 0.0 && (double)cnt / u >= th.t;
-                                }
-                            }
-                            const uint32_t m = __ballot_sync(0xffffffffu, pass);
-                            if (m) {
-                                const int leader = __ffs(m) - 1;
-                                unsigned long long b0 = 0;
-                                if (lane == leader) b0 = atomicAdd(th.found, (unsigned long long)__popc(m));
-                                b0 = __shfl_sync(0xffffffffu, b0, leader);
-                                if (pass) {
-                                    const unsigned long long k = b0 + __popc(m & ((1u << lane) - 1u));
-                                    if (k < th.cap) {
-                                        th.pairs[k] = make_uint2((uint32_t)i, (uint32_t)j);
-                                        th.cnts[k] = cnt;
-                                    }
-                                }
-                            }
-                        }
-                    } else if (row_ok) {
-                        const uint64_t jb = j0 + col0 + 32u * c;
-#pragma unroll
-                        for (int e = 0; e < 32; ++e) {
-                            const uint64_t j = jb + e;
-                            const uint32_t cnt = r[e] >> (kW4 ? 3 : 7);
-                            if (j >= i && j < n && ts_mapped<kRowMap>(row_map, i, j)) {
-                                if (out) {
-                                    uint32_t* dst = out + (kRowMap ? ts_out_index<true>(n, i, j, row_map, n_out)
-                                                                   : base + j);
-                                    if (partial) atomicAdd(dst, cnt);
-                                    else *dst = cnt;
-                                }
-                                if (j > i) local += cnt;
-                            }
                         }
                     }
                 }
@@ -413,12 +365,12 @@ __device__ __forceinline__ void ts_body(const uint64_t* __restrict__ X, uint32_t
 // k_splits: the work schedule (TsSched). 1 = whole tiles round robin;
 // > 1 = that many K slices per tile; 0 = stream-K. For any value but 1 the
 // partial counts are added into out with atomics (out zeroed beforehand).
-// Rows of 2^23 .. 2^27 bits: the 4-byte weight cycle keeps D = 8 x count < 2^31.
+// Rows of 2^24 .. 2^27 bits: the 4-byte weight cycle keeps D = 8 x count < 2^31.
 __global__ void __launch_bounds__(TS_THREADS, 1)
 bb_mma_ts_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
                       uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
                       uint32_t k_splits) {
-    ts_body<false, true>(X, n, w_pad, lay, tiles, n_tiles, out, flags, nullptr, 0, k_splits);
+    ts_body<false>(X, n, w_pad, lay, tiles, n_tiles, out, flags, nullptr, 0, k_splits);
 }
 
 // Same kernel over a gathered subset of rows, writing into the triangle of
@@ -428,7 +380,7 @@ bb_mma_ts_rows_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t 
                            const uint2* __restrict__ tiles, uint32_t n_tiles, uint32_t* __restrict__ out,
                            DeviceFlags* __restrict__ flags, const uint32_t* __restrict__ row_map, uint64_t n_out,
                            uint32_t k_splits) {
-    ts_body<true, true>(X, n, w_pad, lay, tiles, n_tiles, out, flags, row_map, n_out, k_splits);
+    ts_body<true>(X, n, w_pad, lay, tiles, n_tiles, out, flags, row_map, n_out, k_splits);
 }
 
 // Thresholded form over contiguous rows (whole tiles round robin).
@@ -436,7 +388,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
 bb_mma_ts_thresh_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay,
                              const uint2* __restrict__ tiles, uint32_t n_tiles, DeviceFlags* __restrict__ flags,
                              TsThresh th) {
-    ts_body<false, true, true>(X, n, w_pad, lay, tiles, n_tiles, nullptr, flags, nullptr, 0, 1u, th);
+    ts_body<false, true>(X, n, w_pad, lay, tiles, n_tiles, nullptr, flags, nullptr, 0, 1u, th);
 }
 
 }  // namespace sb200

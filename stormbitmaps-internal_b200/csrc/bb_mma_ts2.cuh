@@ -1,14 +1,12 @@
 // bb_mma_ts2.cuh -- the tcgen05 B x B kernel of bb_mma_ts.cuh with a
-// double-buffered accumulator, for short rows.
+// double-buffered accumulator (KERNEL_MMA_DB past 2^24 bits).
 //
-// Same arithmetic (u8 x u8 -> s32, A bytes weighted 2^(k mod 8) or 2^(k mod 4),
-// B bytes bit-reversed), same operand movement (A expanded into TMEM by its
+// Same arithmetic, same operand movement (A expanded into TMEM by its
 // own threads, B expanded into a 128-byte-swizzled smem ring), but the tile
 // is 128 x 192 pairs so that TMEM holds two accumulators: [0, 192) and
 // [256, 448), with the two A stages at [192, 256) and [448, 512). Dedicated
 // epilogue warps drain one accumulator while the MMAs fill the other, so a
-// tile boundary no longer stalls the tensor pipe -- the cost that dominates
-// when a tile has few K stages (rows of tens of thousands of bits).
+// tile boundary does not stall the tensor pipe.
 //
 // Warp roles (480 threads): warps 0-3 expand A rows into TMEM, warps 4-9
 // expand B rows into the ring, warp 10 owns TMEM and issues the MMAs, warps
@@ -61,7 +59,6 @@ __device__ __forceinline__ bool t2_wait(uint32_t bar, uint32_t parity, T2Ctl* ct
 
 // tiles[t] = (bi, bj): rows [128 bi, +128) x rows [192 bj, +192). Rows at or
 // past n read as zero (no padding needed beyond the rows' own buffer).
-template <bool kW4>
 __device__ __forceinline__ void ts2_body(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay,
                                          const uint2* __restrict__ tiles, uint32_t n_tiles,
                                          uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
@@ -132,8 +129,8 @@ __device__ __forceinline__ void ts2_body(const uint64_t* __restrict__ X, uint32_
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         uint32_t r[32];
-                        expand_a64<kW4>(w[2 * h], r);
-                        expand_a64<kW4>(w[2 * h + 1], r + 16);
+                        expand_a64<true>(w[2 * h], r);
+                        expand_a64<true>(w[2 * h + 1], r + 16);
                         tmem_st_32x32b_x32(taddr + 32u * h, r);
                     }
                     tmem_st_wait();
@@ -142,7 +139,7 @@ __device__ __forceinline__ void ts2_body(const uint64_t* __restrict__ X, uint32_
                     uint8_t* b_stage = ring + s * T2_B_STAGE_BYTES;
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
-                        expand_store<true, kW4>(b_stage + (q >> 1) * T2_B_ATOM_BYTES, prow, (uint32_t)(q & 1),
+                        expand_store<true, true>(b_stage + (q >> 1) * T2_B_ATOM_BYTES, prow, (uint32_t)(q & 1),
                                                 w[q]);
                     fence_proxy_async_smem();
                 }
@@ -221,7 +218,7 @@ __device__ __forceinline__ void ts2_body(const uint64_t* __restrict__ X, uint32_
                 for (uint32_t rr = 0; rr < 32; ++rr) {
                     const uint64_t i = i0 + lane_grp + rr;
                     const uint32_t cnt =
-                        buf[rr * 32 + ((((uint32_t)lane >> 2) ^ (rr & 7)) << 2) + (lane & 3)] >> (kW4 ? 3 : 7);
+                        buf[rr * 32 + ((((uint32_t)lane >> 2) ^ (rr & 7)) << 2) + (lane & 3)] >> 3;
                     if (i < n && j >= i && j < n) {
                         if (out) {
                             uint32_t* dst = out + tri_index(n, i, i) - i + j;
@@ -251,7 +248,7 @@ __global__ void __launch_bounds__(T2_THREADS, 1)
 bb_mma_ts2_long_kernel(const uint64_t* __restrict__ X, uint32_t n, uint32_t w_pad, RowLayout lay, const uint2* __restrict__ tiles,
                        uint32_t n_tiles, uint32_t* __restrict__ out, DeviceFlags* __restrict__ flags,
                        uint32_t k_splits) {
-    ts2_body<true>(X, n, w_pad, lay, tiles, n_tiles, out, flags, k_splits);
+    ts2_body(X, n, w_pad, lay, tiles, n_tiles, out, flags, k_splits);
 }
 
 }  // namespace sb200

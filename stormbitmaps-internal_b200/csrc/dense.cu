@@ -271,7 +271,7 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
         uint32_t grid = count < (uint32_t)sms ? count : (uint32_t)sms;
         const uint32_t ks = whole_list ? ts_schedule(count, sms, w_pad, grid, schedule) : 1;
         if (ks != 1 && d_out) zero_stream_k_rows(d_out, n, t0, t0 + count, grid, st);
-        bb_mma_ts_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
+        bb_mma_ts_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES, st>>>(dX, n, w_pad, lay, d_tiles.p + t0, count,
                                                                             d_out, d_flags.p, ks);
     } else if (kind == STORM_B200_KERNEL_MMA_DB) {
         static std::atomic<uint64_t> done{0};
@@ -287,7 +287,7 @@ void DenseEngine::launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pa
         smem_attr_once(bb_mma_2cta_kernel, (int)C2_SMEM_BYTES, done_a);
         smem_attr_once(bb_mma_2cta_long_kernel, (int)C2_SMEM_BYTES, done_b);
         const uint32_t pairs = std::max<uint32_t>(1u, std::min<uint32_t>(count, (uint32_t)sms / 2));
-        const uint32_t smem = (uint64_t)w_pad * 64 <= TS_COALESCE_MAX_BITS ? C2_SMEM_BYTES
+        const uint32_t smem = (uint64_t)w_pad * 64 <= C2_COALESCE_MAX_BITS ? C2_SMEM_BYTES
                                                                           : C2_SMEM_BYTES - C2_EPI_BYTES;
         const uint2* tl = d_tiles.p + t0;
         SB_CUDA(launch_pairs((uint64_t)w_pad * 64 <= MMA_MAX_BITS ? bb_mma_2cta_kernel : bb_mma_2cta_long_kernel, pairs,
@@ -905,7 +905,7 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
             static std::atomic<uint64_t> done{0};
             smem_attr_once(bb_mma_ts_thresh_long_kernel, (int)TS_SMEM_BYTES, done);
             const uint32_t grid = n_tiles < (uint32_t)sms ? n_tiles : (uint32_t)sms;
-            bb_mma_ts_thresh_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(
+            bb_mma_ts_thresh_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES, st>>>(
                 dX, (uint32_t)n, w_pad, lay, d_tiles.p, n_tiles, d_flags.p, th);
         }
         SB_CUDA(cudaGetLastError());
@@ -968,7 +968,7 @@ void launch_ts_rows(const uint64_t* X, uint32_t n, uint32_t w_pad, RowLayout lay
     } else {
         static std::atomic<uint64_t> done{0};
         smem_attr_once(bb_mma_ts_rows_long_kernel, (int)TS_SMEM_BYTES, done);
-        bb_mma_ts_rows_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES_LEAN, st>>>(X, n, w_pad, lay, tiles, n_tiles, out,
+        bb_mma_ts_rows_long_kernel<<<grid, TS_THREADS, TS_SMEM_BYTES, st>>>(X, n, w_pad, lay, tiles, n_tiles, out,
                                                                                 flags, row_map, n_out, ks);
     }
     SB_CUDA(cudaGetLastError());
