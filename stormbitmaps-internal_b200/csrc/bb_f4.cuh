@@ -538,6 +538,10 @@ __device__ __forceinline__ void f4_body(const CUtensorMap& map, uint32_t blk_wor
                 if (lane == 0) mbar_arrive_pair(lead_acc_empty);
                 total += f4_store_packed<kRowMap>(o, buf, lane, i0, j0);
             } else {
+                // The packed rows lie 64 words apart and f4_store_block's 32, so a
+                // lane's 32-bit counts go where another lane just put packed ones:
+                // those stores are ordered before them (a vote orders no memory).
+                __syncwarp();
 #pragma unroll 1
                 for (uint32_t c = 0; c < 4; ++c) {
                     uint32_t r[32];
