@@ -2595,17 +2595,10 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             d_start.reserve(U);
             uint64_t most = 0;
             for (uint32_t r : qrows) most = std::max(most, d.facts[r].card);
-            bool sweep16 = sweep && nq <= POST16_MAX && most <= POST16_MAX && ps.entries + ps.lists < 0xFFFFFFFFull;
-            if (sweep16) {
-                try {
-                    d_post16.reserve(ps.entries + ps.lists + 8);
-                    d_place.reserve(d.lst.n);
-                } catch (const Status& e) {   // no room for the entries' lists: the sweep that looks them up
-                    if (e.code != STORM_B200_ENOMEM) throw;
-                    cudaGetLastError();
-                    sweep16 = false;
-                }
-            }
+            // without room for the entries' lists: the sweep that looks them up
+            const bool sweep16 = sweep && nq <= POST16_MAX && most <= POST16_MAX &&
+                                 ps.entries + ps.lists < 0xFFFFFFFFull &&
+                                 reserve_both(d_post16, ps.entries + ps.lists + 8, d_place, d.lst.n);
             if (!sweep16) {
                 if (!sweep) d_lists.reserve(ps.lists ? ps.lists : 1);
                 d_post.reserve(ps.entries ? ps.entries : 1);

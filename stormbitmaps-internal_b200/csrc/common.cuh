@@ -90,7 +90,29 @@ struct DevBuf {
         SB_CUDA(cudaMalloc((void**)&p, count * sizeof(T)));
         n = count;
     }
+    // The same where a call can do without the buffer: false, and nothing held,
+    // when there is no room for it.
+    bool try_reserve(size_t count) {
+        try {
+            reserve(count);
+        } catch (const Status& e) {
+            if (e.code != STORM_B200_ENOMEM) throw;
+            cudaGetLastError();
+            return false;
+        }
+        return true;
+    }
 };
+
+// Both buffers or neither: what the first took is given back when there is no
+// room for the second, since the path that does without them needs the memory.
+template <class A, class B>
+bool reserve_both(DevBuf<A>& a, size_t na, DevBuf<B>& b, size_t nb) {
+    if (a.try_reserve(na) && b.try_reserve(nb)) return true;
+    a.release();
+    b.release();
+    return false;
+}
 
 // Per-launch bookkeeping a handle keeps for measurement.
 struct LaunchLog {

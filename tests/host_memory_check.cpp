@@ -1,0 +1,91 @@
+// Host-only check of what the library does when device memory runs out, on a
+// fake of the CUDA calls that hand memory out (no GPU, no CUDA runtime): a
+// budget of bytes, and a record of what is held. Built and run by
+// test_host_memory_cpu.py.
+#include <cstdio>
+#include <cstdlib>
+#include <map>
+
+#include "common.cuh"
+
+static int g_fail = 0;
+#define CHECK(c)                                             \
+    do {                                                     \
+        if (!(c)) {                                          \
+            std::printf("line %d: %s\n", __LINE__, #c);      \
+            ++g_fail;                                        \
+        }                                                    \
+    } while (0)
+
+static std::map<void*, size_t> g_held;
+static size_t g_used = 0, g_budget = 0;
+static cudaError_t g_error = cudaSuccess, g_refusal = cudaErrorMemoryAllocation;
+
+extern "C" {
+cudaError_t cudaMalloc(void** p, size_t bytes) {
+    if (g_used + bytes > g_budget) return g_error = g_refusal;
+    *p = std::malloc(bytes ? bytes : 1);
+    g_held[*p] = bytes;
+    g_used += bytes;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    CHECK(g_held.count(p));
+    g_used -= g_held[p];
+    g_held.erase(p);
+    std::free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaGetLastError(void) {
+    const cudaError_t e = g_error;
+    g_error = cudaSuccess;
+    return e;
+}
+const char* cudaGetErrorString(cudaError_t) { return "fake"; }
+}
+
+using namespace sb200;
+
+static void buffers_a_call_can_do_without() {
+    DevBuf<uint32_t> b;
+    g_budget = 400;
+    CHECK(b.try_reserve(100) && b.n == 100 && g_used == 400);
+    CHECK(b.try_reserve(50) && b.n == 100);                      // large enough as it is
+    CHECK(!b.try_reserve(101) && b.p == nullptr && b.n == 0 && g_used == 0);
+    CHECK(g_error == cudaSuccess);                               // nothing left for the next launch's check
+    g_refusal = cudaErrorUnknown;
+    bool threw = false;
+    try {
+        b.try_reserve(101);
+    } catch (const Status& e) {
+        threw = e.code == STORM_B200_ECUDA;
+    }
+    CHECK(threw);                                                // any other failure is one
+    g_refusal = cudaErrorMemoryAllocation;
+    g_error = cudaSuccess;
+}
+
+// The 16-bit row sweep's buffers (2 bytes per list place, 4 per list entry) and
+// then the look-up sweep's (4 per place), in memory that holds the first or the
+// third of them but not the first two.
+static void sweep_buffers() {
+    const size_t places = 1000, entries = 3000;
+    DevBuf<uint16_t> post16;
+    DevBuf<uint32_t> place, post;
+    g_budget = 5000;
+    CHECK(!reserve_both(post16, places, place, entries));
+    CHECK(g_used == 0 && post16.p == nullptr && place.p == nullptr);
+    post.reserve(places);                                        // would throw beside a kept post16
+    CHECK(post.n == places);
+    post.release();
+    g_budget = 14000;
+    CHECK(reserve_both(post16, places, place, entries) && g_used == 14000);
+}
+
+int main() {
+    buffers_a_call_can_do_without();
+    sweep_buffers();
+    CHECK(g_held.empty());
+    std::printf(g_fail ? "FAIL (%d)\n" : "ok\n", g_fail);
+    return g_fail ? 1 : 0;
+}
