@@ -480,11 +480,7 @@ uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad,
     // Rows [n, n_pad) read as zero: whole tiles read them.
     const uint64_t n_pad = round_up(n, 256), pitch = dense_pitch(w_pad);
     if (n_pad > n) SB_CUDA(cudaMemsetAsync(dX + n * pitch, 0, (n_pad - n) * pitch * sizeof(uint64_t), in));
-    uint64_t* stage = nullptr;
-    if (host_wpr < ROW_STAGE_WORDS && n * host_wpr * sizeof(uint64_t) <= ROW_STAGE_BYTES) {
-        d_stage.reserve(n * host_wpr);
-        stage = d_stage.p;
-    }
+    uint64_t* const stage = row_stage(d_stage, n, host_wpr);
     // Rows arrive last rows first: the bottom panels read only them. Chunks of
     // whole panels where those are whole A blocks, else 32 equal ones; event c
     // marks rows [arrive[c], n) (and the zeroing) as resident.

@@ -24,6 +24,13 @@ inline uint64_t dense_pitch(uint32_t w_pad) { return w_pad % 512 == 0 ? (uint64_
 // (the spreading waits for a free SM).
 constexpr uint32_t ROW_STAGE_WORDS = 640;
 constexpr uint64_t ROW_STAGE_BYTES = 256ull << 20;
+// Where `rows` host rows of wpr words are staged: null when they are not, also
+// when there is no memory for it.
+inline uint64_t* row_stage(DevBuf<uint64_t>& buf, uint64_t rows, uint32_t wpr) {
+    const uint64_t words = rows * wpr;
+    if (wpr >= ROW_STAGE_WORDS || words * sizeof(uint64_t) > ROW_STAGE_BYTES || !buf.try_reserve(words)) return nullptr;
+    return buf.p;
+}
 void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_t* host, uint32_t wpr, uint64_t rows,
                     uint64_t* stage, cudaStream_t st);
 

@@ -6,7 +6,7 @@
 #include <cstdlib>
 #include <map>
 
-#include "common.cuh"
+#include "dense.cuh"
 
 static int g_fail = 0;
 #define CHECK(c)                                             \
@@ -82,9 +82,21 @@ static void sweep_buffers() {
     CHECK(reserve_both(post16, places, place, entries) && g_used == 14000);
 }
 
+// Host rows cross the bus by way of a staging buffer, or without one.
+static void staged_rows() {
+    DevBuf<uint64_t> stage;
+    g_budget = 300 * 313 * 8 - 1;
+    CHECK(row_stage(stage, 300, 313) == nullptr && g_used == 0);
+    g_budget = 300 * 313 * 8;
+    CHECK(row_stage(stage, 300, 313) == stage.p && stage.p);
+    CHECK(row_stage(stage, 1, ROW_STAGE_WORDS) == nullptr);      // long rows: straight to their places
+    CHECK(row_stage(stage, ROW_STAGE_BYTES / 8 / 313 + 1, 313) == nullptr);
+}
+
 int main() {
     buffers_a_call_can_do_without();
     sweep_buffers();
+    staged_rows();
     CHECK(g_held.empty());
     std::printf(g_fail ? "FAIL (%d)\n" : "ok\n", g_fail);
     return g_fail ? 1 : 0;
