@@ -20,7 +20,15 @@ constexpr uint32_t COLSUM_WORDS = 32;          // row words per block (a warp's 
 constexpr uint32_t COLSUM_PLANES = 9;          // planes of weight 8 .. 2048: a warp counts at most 4095 rows
 constexpr uint64_t COLSUM_WARP_ROWS = 4088;
 constexpr uint32_t COLSUM_STRIP = 1u << 16;    // row words per histogram (2^22 columns, 16 MiB)
+constexpr uint64_t COLSUM_MAX_ROWS = 65535ull * COLSUM_WARPS * COLSUM_WARP_ROWS;   // a grid's blocks along the rows
 
+// Whether the sum over n rows can come from the columns' counts: `hist` then
+// holds a strip of them. Without room for it every pair is counted.
+inline bool colsum_room(DevBuf<uint32_t>& hist, uint64_t n, uint32_t w_pad) {
+    return n <= COLSUM_MAX_ROWS && hist.try_reserve(64ull * (w_pad < COLSUM_STRIP ? w_pad : COLSUM_STRIP));
+}
+
+#ifdef __CUDACC__
 __device__ __forceinline__ void csa(uint64_t& sum, uint64_t& carry, uint64_t a, uint64_t b, uint64_t c) {
     sum = a ^ b ^ c;
     carry = (a & b) | (c & (a ^ b));
@@ -88,5 +96,6 @@ pairs_of_counts_kernel(const uint32_t* __restrict__ hist, uint64_t columns, unsi
     s = warp_sum_u64(s);
     if ((threadIdx.x & 31) == 0 && s) atomicAdd(sum, s);
 }
+#endif
 
 }  // namespace sb200

@@ -317,7 +317,8 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
         return 0;
     }
     // The sum alone, no kernel asked for: from the columns' counts.
-    if (!d_out && kernel_pref == STORM_B200_KERNEL_AUTO) return run_sum(dX, n, w_pad, row_bits, st);
+    if (!d_out && kernel_pref == STORM_B200_KERNEL_AUTO && colsum_room(d_hist, n, w_pad))
+        return run_sum(dX, n, w_pad, row_bits, st);
     const int kind = prepare(n, row_bits, kernel_pref, false, st);
     SB_CUDA(cudaEventRecord(log.ev0, st));
     launch(kind, dX, (uint32_t)n, w_pad, 0, n_tiles, d_out, st);
@@ -333,7 +334,6 @@ uint64_t DenseEngine::run(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64
 uint64_t DenseEngine::run_sum(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits, cudaStream_t st) {
     const int sms = require_device();
     const uint32_t strip = std::min<uint32_t>(w_pad, COLSUM_STRIP);
-    d_hist.reserve(64ull * strip);
     d_flags.reserve(1);
     log.ensure();
     SB_CUDA(cudaMemsetAsync(d_flags.p, 0, sizeof(DeviceFlags), st));

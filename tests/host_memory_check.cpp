@@ -6,6 +6,7 @@
 #include <cstdlib>
 #include <map>
 
+#include "colsum.cuh"
 #include "dense.cuh"
 
 static int g_fail = 0;
@@ -93,10 +94,22 @@ static void staged_rows() {
     CHECK(row_stage(stage, ROW_STAGE_BYTES / 8 / 313 + 1, 313) == nullptr);
 }
 
+// The sum from the columns' counts, or (false) from every pair.
+static void column_counts() {
+    DevBuf<uint32_t> hist;
+    g_budget = 64 * 8 * 4;
+    CHECK(colsum_room(hist, 100, 8) && g_used == g_budget);
+    CHECK(!colsum_room(hist, 100, 16) && g_used == 0);
+    g_budget = 64ull * COLSUM_STRIP * 4;
+    CHECK(colsum_room(hist, COLSUM_MAX_ROWS, 1u << 20));         // longer rows take several strips
+    CHECK(!colsum_room(hist, COLSUM_MAX_ROWS + 1, 8));           // more blocks than a grid has
+}
+
 int main() {
     buffers_a_call_can_do_without();
     sweep_buffers();
     staged_rows();
+    column_counts();
     CHECK(g_held.empty());
     std::printf(g_fail ? "FAIL (%d)\n" : "ok\n", g_fail);
     return g_fail ? 1 : 0;
