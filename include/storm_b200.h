@@ -121,7 +121,8 @@ int STORM_contig_set_schedule(STORM_contiguous_t* c, int schedule);
  * tcgen05 on CTA pairs (whole tiles) -- best of two calls each, and keeps
  * the fastest kernel and schedule for later calls that give counts (the sum
  * alone stays on the columns' counts).  times_ms (7 entries in that order, -1
- * when skipped) and the choice are reported when non-NULL.
+ * when skipped; MMA_DB has MMA's times where the two run one kernel) and the
+ * choice are reported when non-NULL.
  * Counts do not depend on it. */
 int STORM_contig_autotune(STORM_contiguous_t* c, int* best_kernel, int* best_schedule, double* times_ms);
 /* Pack the rows into HBM now (otherwise done by the first all-pairs call). */

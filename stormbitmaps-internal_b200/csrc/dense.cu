@@ -53,6 +53,8 @@ static int exec_kind(int kind, uint64_t row_bits) {
                                                                                                            : kind;
 }
 
+bool same_kernel(int a, int b, uint64_t row_bits) { return exec_kind(a, row_bits) == exec_kind(b, row_bits); }
+
 constexpr uint32_t F4_MIN_SEG = 8;   // stages of a K segment at least
 
 // Schedule of the 4-bit kernel over `pairs` pairs of CTAs, as ts_schedule:

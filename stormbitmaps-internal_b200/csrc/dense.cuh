@@ -110,6 +110,8 @@ inline uint64_t round_up(uint64_t x, uint64_t m) { return (x + m - 1) / m * m; }
 // The 4-bit tensor-core kernel (bb_f4.cuh), which MMA and MMA_DB run on up to
 // 2^24-bit rows; not a value of the interface.
 constexpr int KIND_F4 = 64;
+// Whether two kernel choices run the same kernel on rows of this length.
+bool same_kernel(int a, int b, uint64_t row_bits);
 // The tile list of a bitmap x bitmap kernel (STORM_B200_KERNEL_*, KIND_F4):
 // 256 x 256 (CTA pairs), 128 x 256 (tcgen05), 128 x 192 (double-buffered
 // tcgen05) or 128 x 128 (POPC) tiles

@@ -1,4 +1,5 @@
-"""What the contiguous autotuner's choice is kept for: calls that write every
+"""The contiguous autotuner: two names of one kernel are one candidate, and
+what the choice is kept for: calls that write every
 pair's count, not the sum alone (two launches, from the columns' counts; a pair
 kernel takes one)."""
 import numpy as np
@@ -39,4 +40,16 @@ def test_autotune_without_rows_keeps_the_choice(sb):
     c.add_bitmaps(words)
     assert c.pairw_intersect_cardinality() == ol.contig_matrix(words)[1]
     assert c.last_launches() == 1 and c.last_kernel() == sb.KERNEL_MMA
+    c.close()
+
+
+@pytest.mark.parametrize("m", (5000, 65536))
+def test_one_kernel_under_two_names_is_timed_once(sb, m):
+    """MMA and MMA_DB share a kernel up to 2^24 bits: the same times, and a
+    choice between the two that noise has no part in (the first)."""
+    c, (want, ws) = _container(sb, 700, m)
+    k, _, times = c.autotune()
+    assert times[2] == times[0] > 0 and times[3] == times[1] > 0
+    assert k != sb.KERNEL_MMA_DB
+    assert c.matrix()[1] == ws
     c.close()
