@@ -11,6 +11,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <cstdlib>
 #include <new>
 #include <stdexcept>
 #include <atomic>
@@ -139,9 +140,31 @@ struct DeviceFlags {
     unsigned long long sum;   // sum over i < j accumulated by the epilogues
 };
 
-// This thread's pinned place for the flags (or a pageable one where there is no
-// pinned memory), kept until the thread exits: a copy into pageable memory is
-// staged by the driver, which costs a small call more than its kernel's launch.
+// Host memory of the library's own, registered with CUDA so that copies to it
+// are not staged by the driver. The page outlives what CUDA knows of it: after a
+// cudaDeviceReset (or where it cannot be registered at all) it is pageable memory
+// that a copy reaches all the same, where memory of cudaMallocHost would be gone
+// with its address still kept.
+struct RegisteredPage {
+    static constexpr size_t BYTES = 4096;    // whole pages: nothing else shares what is registered
+    void* p = nullptr;
+    RegisteredPage() {
+        p = std::aligned_alloc(BYTES, BYTES);
+        if (!p) fail(STORM_B200_ENOMEM, "host memory");
+        if (cudaHostRegister(p, BYTES, cudaHostRegisterPortable) != cudaSuccess) cudaGetLastError();
+    }
+    RegisteredPage(const RegisteredPage&) = delete;
+    RegisteredPage& operator=(const RegisteredPage&) = delete;
+    ~RegisteredPage() {
+        const cudaError_t e = cudaHostUnregister(p);
+        if (e != cudaSuccess) cudaGetLastError();
+        // still registered for all this can tell: the page stays
+        if (e == cudaSuccess || e == cudaErrorHostMemoryNotRegistered || e == cudaErrorInvalidValue) std::free(p);
+    }
+};
+
+// This thread's place for the flags, kept until the thread exits: a copy into
+// unregistered memory costs a small call more than its kernel's launch.
 DeviceFlags* flags_slot();
 
 // Waits for `st` and returns the flags left there by the work queued on it.

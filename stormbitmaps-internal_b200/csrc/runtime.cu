@@ -27,21 +27,8 @@ unsigned host_threads() {
 }
 
 DeviceFlags* flags_slot() {
-    struct Slot {
-        DeviceFlags* pinned = nullptr;
-        DeviceFlags plain{};
-        Slot() {
-            if (cudaMallocHost((void**)&pinned, sizeof(DeviceFlags)) != cudaSuccess) {
-                cudaGetLastError();
-                pinned = nullptr;
-            }
-        }
-        ~Slot() {
-            if (pinned) cudaFreeHost(pinned);
-        }
-    };
-    static thread_local Slot slot;
-    return slot.pinned ? slot.pinned : &slot.plain;
+    static thread_local RegisteredPage page;
+    return static_cast<DeviceFlags*>(page.p);
 }
 
 int require_device() {

@@ -4,7 +4,10 @@
 // test_host_memory_cpu.py.
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <map>
+#include <set>
+#include <thread>
 
 #include "colsum.cuh"
 #include "dense.cuh"
@@ -19,6 +22,7 @@ static int g_fail = 0;
     } while (0)
 
 static std::map<void*, size_t> g_held;
+static std::set<void*> g_registered;
 static size_t g_used = 0, g_budget = 0;
 static cudaError_t g_error = cudaSuccess, g_refusal = cudaErrorMemoryAllocation;
 
@@ -37,6 +41,23 @@ cudaError_t cudaFree(void* p) {
     std::free(p);
     return cudaSuccess;
 }
+// CUDA's own pinned memory goes with the device; registered memory is the caller's.
+cudaError_t cudaMallocHost(void** p, size_t bytes) { return cudaMalloc(p, bytes); }
+cudaError_t cudaFreeHost(void* p) { return cudaFree(p); }
+cudaError_t cudaHostRegister(void* p, size_t, unsigned int) {
+    if (g_budget == 0) return g_error = cudaErrorNotSupported;
+    g_registered.insert(p);
+    return cudaSuccess;
+}
+cudaError_t cudaHostUnregister(void* p) {
+    if (!g_registered.erase(p)) return g_error = cudaErrorHostMemoryNotRegistered;
+    return cudaSuccess;
+}
+cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t bytes, cudaMemcpyKind, cudaStream_t) {
+    std::memcpy(dst, src, bytes);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGetLastError(void) {
     const cudaError_t e = g_error;
     g_error = cudaSuccess;
@@ -44,6 +65,13 @@ cudaError_t cudaGetLastError(void) {
 }
 const char* cudaGetErrorString(cudaError_t) { return "fake"; }
 }
+
+namespace sb200 {
+DeviceFlags* flags_slot() {                                      // as runtime.cu keeps it
+    static thread_local RegisteredPage page;
+    return static_cast<DeviceFlags*>(page.p);
+}
+}  // namespace sb200
 
 using namespace sb200;
 
@@ -105,11 +133,36 @@ static void column_counts() {
     CHECK(!colsum_room(hist, COLSUM_MAX_ROWS + 1, 8));           // more blocks than a grid has
 }
 
+// A thread's place for the flags is the library's own memory: it holds through
+// a reset of the device, after which CUDA knows nothing of it and has handed its
+// own pinned memory to others, and goes with the thread.
+static void flags() {
+    for (size_t budget : {size_t(1) << 20, size_t(0)}) {         // registered, and where nothing can be
+        g_budget = budget;
+        std::thread([&] {
+            DeviceFlags on_device{0, 0, 42};
+            CHECK(read_flags(&on_device, nullptr).sum == 42);
+            CHECK(g_held.empty());                               // none of CUDA's memory is kept
+            CHECK(g_registered.size() == (budget ? 1u : 0u) && g_error == cudaSuccess);
+            g_registered.clear();                                // cudaDeviceReset
+            on_device.sum = 43;
+            CHECK(read_flags(&on_device, nullptr).sum == 43);
+        }).join();
+        g_budget = 1 << 20;
+        std::thread([] {
+            DeviceFlags on_device{0, 0, 44};
+            CHECK(read_flags(&on_device, nullptr).sum == 44 && g_registered.size() == 1);
+        }).join();
+        CHECK(g_registered.empty());
+    }
+}
+
 int main() {
     buffers_a_call_can_do_without();
     sweep_buffers();
     staged_rows();
     column_counts();
+    flags();
     CHECK(g_held.empty());
     std::printf(g_fail ? "FAIL (%d)\n" : "ok\n", g_fail);
     return g_fail ? 1 : 0;

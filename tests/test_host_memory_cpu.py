@@ -16,7 +16,7 @@ def test_out_of_memory_and_what_is_kept():
     out = os.path.join(ROOT, "_build", "host_memory_check")
     os.makedirs(out, exist_ok=True)
     exe = os.path.join(out, "host_memory_check")
-    subprocess.run([cxx, "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"), "-I", os.path.join(PKG, "csrc"),
+    subprocess.run([cxx, "-std=c++17", "-O1", "-pthread", "-I", os.path.join(ROOT, "include"), "-I", os.path.join(PKG, "csrc"),
                     "-I", "/usr/local/cuda/include", os.path.join(ROOT, "tests", "host_memory_check.cpp"), "-o", exe],
                    check=True, capture_output=True, text=True)
     r = subprocess.run([exe], capture_output=True, text=True, timeout=60)
