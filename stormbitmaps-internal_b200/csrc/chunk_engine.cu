@@ -11,6 +11,7 @@
 #include "list16_ref.cuh"
 #include "panel.cuh"
 #include "run_pieces.cuh"
+#include "walk_shape.cuh"
 
 namespace sb200 {
 
@@ -920,8 +921,6 @@ __device__ __forceinline__ void walk_group_chunks(const ChunkView& v, uint64_t c
 }
 
 // One row by a CTA: its warps take every eighth group of the row's chunks.
-constexpr uint32_t ROW_WALK_THREADS = 256;
-
 template <class F, class H>
 __device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint32_t group, F f, H h) {
     const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
@@ -929,71 +928,34 @@ __device__ __forceinline__ void row_walk(const ChunkView& v, uint32_t row, uint3
         walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, f, h);
 }
 
-// Every row, group by group: all rows' first groups, then all rows' second
-// ones (rows have at most `groups` each), so that the warps at work meet in one
-// part of the universe and what they update -- 4 bytes per value somewhere in
-// it -- stays in L2. With a warp (or CTA) per row, 200 mixed rows left the GPU
-// idle, and the places of 20000 rows' values (67 MB of cursors, 134 of
-// postings) were written from DRAM.  f(r, value, place), h(chunk).
+// Rows (all of the first w.n when `rows` is null) dealt to the grid's warps as
+// walk_shape.cuh says: f(index of the row, value, place), h(chunk).
 template <class F, class H>
-__device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __restrict__ rows, uint32_t nq,
-                                          uint32_t group, uint32_t groups, F f, H h) {
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, items = (uint64_t)nq * groups;
+__device__ __forceinline__ void rows_walk(const ChunkView& v, const uint32_t* __restrict__ rows, WalkShape::Dims w,
+                                          F f, H h) {
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5, items = w.items();
     for (uint64_t it = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < items; it += nw) {
-        const uint32_t r = (uint32_t)(it % nq);
+        const uint32_t r = w.row(it);
         const uint32_t row = rows ? rows[r] : r;
-        const uint64_t cg = v.row_off[row] + it / nq * group, c1 = v.row_off[row + 1];
-        if (cg < c1)
-            walk_group_chunks(v, cg, c1, group, threadIdx.x & 31, [&](uint32_t x, uint64_t at) { f(r, x, at); }, h);
+        const uint64_t c0 = v.row_off[row], c1 = v.row_off[row + 1];
+        for (uint32_t k = w.first_chunk(it); k < (uint32_t)(c1 - c0); k += w.step())
+            walk_group_chunks(v, c0 + k, c1, w.group, threadIdx.x & 31, [&](uint32_t x, uint64_t at) { f(r, x, at); }, h);
     }
 }
 
-// How rows_walk and row_walk take a set of rows: chunks per group (one from 48
-// entries a chunk on, or with bitmap chunks) and groups of the longest row.
-// Rows of few entries a chunk among which most entries lie in chunks of many
-// take groups of four: 32 such chunks are a long serial item for one warp
-// (3072 Zipf rows over 2^24, histogram to lists: 0.79 ms by 32, 0.59 by 8,
-// 0.58 by 4; 1094 over 2^23 0.32, 0.21, 0.20).
-constexpr uint32_t WALK_SKEW_GROUP = 4;
-struct WalkShape {
-    uint32_t group = 1, groups = 0;
-    template <class Facts>
-    void of(uint64_t n, Facts facts) {
-        uint64_t chunks = 0, entries = 0;
-        double spread = 0.0;                              // entries x (their row's entries per chunk)
-        uint32_t most = 0;
-        bool bitmaps = false;
-        for (uint64_t k = 0; k < n; ++k) {
-            const ChunkRowFacts& f = facts(k);
-            chunks += f.chunks;
-            entries += f.list_entries;
-            bitmaps |= f.bitmap_chunks != 0;
-            most = std::max(most, f.chunks);
-            if (f.chunks) spread += (double)f.list_entries * (double)f.list_entries / (double)f.chunks;
-        }
-        group = bitmaps || entries >= 48 * chunks ? 1u : spread >= 48.0 * (double)entries ? WALK_SKEW_GROUP : 32u;
-        groups = (most + group - 1) / group;
-    }
-    uint32_t grid(uint64_t n, int sms) const {
-        return (uint32_t)std::max<uint64_t>(
-            1, std::min<uint64_t>((n * groups + ROW_WALK_THREADS / 32 - 1) / (ROW_WALK_THREADS / 32), (uint64_t)sms * 8));
-    }
-};
-
-// rows == nullptr: rows [0, nq). Bitmap chunks count every set bit (only the
+// rows == nullptr: rows [0, w.n). Bitmap chunks count every set bit (only the
 // sums over pairs send rows that have them).
-__global__ void __launch_bounds__(ROW_WALK_THREADS)
-postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
-                     uint32_t* __restrict__ counts) {
+__global__ void __launch_bounds__(ROW_WALK_THREADS, ROW_WALK_BLOCKS)
+postings_hist_kernel(ChunkView v, const uint32_t* __restrict__ rows, WalkShape::Dims w, uint32_t* __restrict__ counts) {
     const int lane = threadIdx.x & 31;
     rows_walk(
-        v, rows, nq, group, groups, [&](uint32_t, uint32_t x, uint64_t) { atomicAdd(&counts[x], 1u); },
+        v, rows, w, [&](uint32_t, uint32_t x, uint64_t) { atomicAdd(&counts[x], 1u); },
         [&](uint64_t c) {
             const uint64_t* wd = v.bm + v.coff[c];
             const uint32_t base = v.cid[c] << 16;
-            for (uint32_t w = lane; w < CHUNK_WORDS; w += 32)
-                for (uint64_t x = wd[w]; x; x &= x - 1)
-                    atomicAdd(&counts[base | (w << 6) | (uint32_t)__ffsll((long long)x) - 1u], 1u);
+            for (uint32_t q = lane; q < CHUNK_WORDS; q += 32)
+                for (uint64_t x = wd[q]; x; x &= x - 1)
+                    atomicAdd(&counts[base | (q << 6) | (uint32_t)__ffsll((long long)x) - 1u], 1u);
         });
 }
 
@@ -1105,11 +1067,11 @@ postings_alloc_kernel(const uint32_t* __restrict__ counts, uint64_t U, uint32_t*
 
 // Writes each Q row's position in the Q list (its local index) into the
 // lists of its values; start[x] advances to the end of x's list.
-__global__ void __launch_bounds__(ROW_WALK_THREADS)
-postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
+__global__ void __launch_bounds__(ROW_WALK_THREADS, ROW_WALK_BLOCKS)
+postings_scatter_kernel(ChunkView v, const uint32_t* __restrict__ rows, WalkShape::Dims w,
                         uint32_t* __restrict__ start, uint32_t* __restrict__ post) {
     rows_walk(
-        v, rows, nq, group, groups,
+        v, rows, w,
         [&](uint32_t r, uint32_t x, uint64_t) {
             // a value of one row has start ~0, and its one row adds to it once
             const uint32_t at = atomicAdd(&start[x], 1u);
@@ -1157,12 +1119,12 @@ __global__ void postings_pairs_kernel(const uint2* __restrict__ lists, uint64_t 
 // counting down to the places, and place[p] becomes the list of the pool's
 // entry p (of its own value), so that the sweep finds a row's lists without
 // looking its values up.
-__global__ void __launch_bounds__(ROW_WALK_THREADS)
-postings_scatter16_kernel(ChunkView v, const uint32_t* __restrict__ rows, uint32_t nq, uint32_t group, uint32_t groups,
+__global__ void __launch_bounds__(ROW_WALK_THREADS, ROW_WALK_BLOCKS)
+postings_scatter16_kernel(ChunkView v, const uint32_t* __restrict__ rows, WalkShape::Dims w,
                           uint32_t* __restrict__ counts, const uint32_t* __restrict__ start,
                           uint16_t* __restrict__ post, uint32_t* __restrict__ place) {
     rows_walk(
-        v, rows, nq, group, groups,
+        v, rows, w,
         [&](uint32_t r, uint32_t x, uint64_t at) {
             const uint32_t s = start[x];
             place[at] = s;
@@ -1857,11 +1819,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             for (uint64_t r = 0; r < n2; ++r) second[r] = (uint32_t)(n1 + r);
             SB_CUDA(cudaMemcpyAsync(d_qrows.p, second.data(), n2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
             WalkShape ws;
-            ws.of(n1 + n2, [&](uint64_t r) -> const ChunkRowFacts& { return d.facts[r]; });
-            postings_hist_kernel<<<ws.grid(n1, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), nullptr, (uint32_t)n1, ws.group,
-                                                                              ws.groups, d_counts.p);
-            postings_hist_kernel<<<ws.grid(n2, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)n2,
-                                                                              ws.group, ws.groups, d_start.p);
+            for (const ChunkRowFacts& f : d.facts) ws.add(f);
+            ws.done();
+            postings_hist_kernel<<<ws.grid(n1, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), nullptr, ws.dims(n1), d_counts.p);
+            postings_hist_kernel<<<ws.grid(n2, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, ws.dims(n2),
+                                                                              d_start.p);
             counts_dot_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, d_start.p, U, d_flags.p);
             SB_CUDA(cudaGetLastError());
             launches += 3;
@@ -1904,7 +1866,13 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     SB_CUDA(cudaEventRecord(log.ev0, st));
     PostingsStats ps{};
     WalkShape q_walk;                                      // of the postings rows
-    auto histogram = [&](const std::vector<uint32_t>& rows) {
+    auto walk_of = [&](const std::vector<uint32_t>& rows) {
+        WalkShape w;
+        for (uint32_t r : rows) w.add(d.facts[r]);
+        w.done();
+        return w;
+    };
+    auto histogram = [&](const std::vector<uint32_t>& rows, const WalkShape& shape) {
         d_qrows.reserve(rows.size());
         SB_CUDA(cudaEventRecord(ev_hist0, st));
         SB_CUDA(cudaMemcpyAsync(d_qrows.p, rows.data(), rows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
@@ -1912,9 +1880,9 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_counts.p, 0, U * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
-        q_walk.of(rows.size(), [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[rows[k]]; });
+        q_walk = shape;
         postings_hist_kernel<<<q_walk.grid(rows.size(), sms), ROW_WALK_THREADS, 0, st>>>(
-            d.view(), d_qrows.p, (uint32_t)rows.size(), q_walk.group, q_walk.groups, d_counts.p);
+            d.view(), d_qrows.p, q_walk.dims(rows.size()), d_counts.p);
         postings_stats_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_pstats.p);
         SB_CUDA(cudaGetLastError());
         SB_CUDA(cudaEventRecord(ev_hist, st));
@@ -1992,11 +1960,16 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // chunk kernel.
     if (!d_out && post_ok) {
         std::vector<uint32_t> plain;
+        WalkShape shape;                                   // in the same pass: 10^6 rows' facts are 40 MB
         for (uint32_t r = 0; r < n; ++r)
-            if (d.facts[r].plain) plain.push_back(r);
+            if (d.facts[r].plain) {
+                plain.push_back(r);
+                shape.add(d.facts[r]);
+            }
+        shape.done();
         uint64_t q_sum = 0;
         if (plain.size() >= 2) {
-            q_sum = histogram(plain).pairs;
+            q_sum = histogram(plain, shape).pairs;
             last_postings_rows = plain.size();
         }
         const uint64_t nc = n - plain.size();
@@ -2094,7 +2067,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             }
         }
         if (!lists_only) return false;
-        ps = histogram(rest);
+        ps = histogram(rest, walk_of(rest));
         if (ps.entries < (1ull << 32) && (postings_mode > 0 || post_ns((double)ps.pairs, q, (double)values_of(rest)) < alt)) {
             qrows = rest;
             return true;
@@ -2608,8 +2581,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             if (sweep16) {
                 SB_CUDA(cudaMemsetAsync(d_place.p, 0xFF, d.lst.n * sizeof(uint32_t), st));
                 postings_scatter16_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
-                    d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_counts.p, d_start.p, d_post16.p,
-                    d_place.p);
+                    d.view(), d_qrows.p, q_walk.dims(nq), d_counts.p, d_start.p, d_post16.p, d_place.p);
                 static std::atomic<uint64_t> done16{0};
                 smem_attr_once(postings_rows16_kernel, (int)((POST16_MAX + 1) * sizeof(uint16_t)), done16);
                 postings_rows16_kernel<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 16), POST_ROWS_THREADS,
@@ -2619,7 +2591,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
                 launches += 3;
             } else {
                 postings_scatter_kernel<<<q_walk.grid(nq, sms), ROW_WALK_THREADS, 0, st>>>(
-                    d.view(), d_qrows.p, (uint32_t)nq, q_walk.group, q_walk.groups, d_start.p, d_post.p);
+                    d.view(), d_qrows.p, q_walk.dims(nq), d_start.p, d_post.p);
                 if (sweep) {
                     const bool small = most <= 0xFFFF;   // a count is at most its row's values
                     static std::atomic<uint64_t> done_s{0}, done_l{0};
