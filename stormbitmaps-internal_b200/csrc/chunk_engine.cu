@@ -227,20 +227,19 @@ void ChunkDev::upload(const ChunkPack& p, cudaStream_t st) {
     put(lst, p.lst, st);
     n_rows = p.rows();
     facts = p.facts;
+    by_card.rows_changed();
     max_cid = p.max_cid;
-    order_rows();
     SB_CUDA(cudaStreamSynchronize(st));
 }
 
-// The planner wants the rows heaviest first on every call; the order belongs to
-// the rows and is made with their upload (a radix sort: 20000 rows in 0.1 ms; a
-// comparison sort per call took 1.1).
-void ChunkDev::order_rows() {
+// A radix sort: 20000 rows in 0.1 ms, a comparison sort 1.1.
+const std::vector<uint32_t>& RowsByCard::of(const std::vector<ChunkRowFacts>& facts) {
+    if (made) return order;
     const uint64_t n = facts.size();
-    by_card.resize(n);
+    order.resize(n);
     uint64_t most = 0;
     for (uint64_t r = 0; r < n; ++r) {
-        by_card[r] = (uint32_t)r;
+        order[r] = (uint32_t)r;
         most = std::max(most, facts[r].card);
     }
     std::vector<uint32_t> other(n);
@@ -248,11 +247,13 @@ void ChunkDev::order_rows() {
     for (int shift = 0; shift < 64 && most >> shift; shift += 11) {
         std::fill(at.begin(), at.end(), 0);
         auto digit = [&](uint32_t r) { return 2047 - (facts[r].card >> shift & 2047); };   // largest first
-        for (uint32_t r : by_card) ++at[digit(r) + 1];
+        for (uint32_t r : order) ++at[digit(r) + 1];
         for (uint64_t k = 0; k < 2048; ++k) at[k + 1] += at[k];
-        for (uint32_t r : by_card) other[at[digit(r)]++] = r;
-        by_card.swap(other);
+        for (uint32_t r : order) other[at[digit(r)]++] = r;
+        order.swap(other);
     }
+    made = true;
+    return order;
 }
 
 PinnedStage::~PinnedStage() {
@@ -394,6 +395,7 @@ void ChunkDev::upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStre
     std::vector<uint64_t> c_base(n + 1, 0), b_base(n + 1, 0), l_base(n + 1, 0), w1(n + 1, 0);
     std::vector<uint32_t> row_max(n, 0);
     facts.assign(n, ChunkRowFacts{});
+    by_card.rows_changed();
     for (uint64_t r = 0; r < n; ++r) w1[r + 1] = w1[r] + 1 + live(r);
     parallel_rows(n, w1, hw, [&](uint64_t r0, uint64_t r1) {
         for (uint64_t r = r0; r < r1; ++r) {
@@ -591,7 +593,6 @@ void ChunkDev::upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStre
         if (dup[r]) facts[r].plain = false;
         facts[r].runs = runs[r];
     }
-    order_rows();
 }
 
 void copy_to_host(uint32_t* out, const uint32_t* d_src, uint64_t count, cudaStream_t st, PinnedStage& stage) {
@@ -2132,7 +2133,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         // bitmap chunk in H u M.  The cheaper predicted plan runs.
         std::vector<uint32_t> pl;
         pl.reserve(n);
-        for (uint32_t r : d.by_card)
+        for (uint32_t r : d.by_card.of(d.facts))
             if (d.facts[r].plain) pl.push_back(r);
         const uint64_t np = pl.size();
         std::vector<double> S1(np + 1, 0.0), S2(np + 1, 0.0), S3(np + 1, 0.0);

@@ -79,6 +79,20 @@ struct ChunkRowFacts {
     bool plain = true;
 };
 
+// Rows by value count, largest first (equal ones in stored order). The planner
+// of per-pair calls wants them on every call; the order belongs to the rows and
+// is kept from the first such call after an upload, since sums and single pairs
+// do without it.
+class RowsByCard {
+    std::vector<uint32_t> order;
+    bool made = false;
+
+   public:
+    void rows_changed() { made = false; }
+    bool is_made() const { return made; }
+    const std::vector<uint32_t>& of(const std::vector<ChunkRowFacts>& facts);
+};
+
 // Host staging of the packed layout, with the per-row facts and the largest
 // chunk id.
 struct ChunkPack {
@@ -139,7 +153,7 @@ struct ChunkDev {
     DevBuf<uint16_t> lst;
     uint64_t n_rows = 0;
     std::vector<ChunkRowFacts> facts;   // host copy of the per-row facts
-    std::vector<uint32_t> by_card;      // rows by value count, largest first (equal ones in stored order)
+    mutable RowsByCard by_card;         // of `facts`, for the per-pair plans
     uint32_t max_cid = 0;
     uint64_t payload_bytes = 0;         // bitmap and list bytes of the last upload
     void upload(const ChunkPack& p, cudaStream_t st);
@@ -153,7 +167,6 @@ struct ChunkDev {
     void upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStream_t st, PinnedStage& stage);
     DevBuf<uint8_t> d_row_dup;
     DevBuf<uint32_t> d_row_runs;
-    void order_rows();                  // by_card from the facts
     ChunkView view() const {
         return ChunkView{row_off.p, cid.p, ckl.p, coff.p, bm.p, lst.p};
     }
