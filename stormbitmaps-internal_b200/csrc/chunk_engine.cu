@@ -2231,8 +2231,8 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             if (decide(rest, alt)) rest.clear();
         }
         if (panel_plan && !rest.empty()) {                 // they join the panel, or all go to the tensor cores
-            panel_plan = panel_mode > 0 || (tensor_ns((double)best_h, 0.0) + panel_ns(best_h, np) < tensor_ns((double)np, 0.0) &&
-                                            panel_fits(np));
+            panel_plan = rows_join_panel(panel_mode > 0, tensor_ns((double)best_h, 0.0) + panel_ns(best_h, np),
+                                         tensor_ns((double)np, 0.0), [&] { return panel_fits(np); });
             mrows.insert(mrows.end(), rest.begin(), rest.end());
             if (!panel_plan) {
                 dense.insert(dense.end(), mrows.begin(), mrows.end());

@@ -236,6 +236,15 @@ double tensor_pair_ns(const ChunkCostModel& m, uint64_t slots);
 
 constexpr double CHUNK_DENSE_AUTO = -1.0;
 
+// Whether rows whose postings turned out dear join the panel, whose blocks they
+// widen, or all panel rows go to the tensor cores: by the times, or `forced`, but
+// in either case only where the wider blocks fit memory (asked last: the query
+// takes up to milliseconds).
+template <class Fits>
+bool rows_join_panel(bool forced, double panel_ns, double tensor_ns, Fits fits) {
+    return (forced || panel_ns < tensor_ns) && fits();
+}
+
 // Postings for the sparse rows (plain rows without bitmap chunks, outside the
 // dense block): a histogram of their values over the universe gives, per
 // value, the rows holding it; each pair of those rows gets one increment

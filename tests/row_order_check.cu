@@ -1,6 +1,8 @@
 // Host-only check of RowsByCard (chunk_engine.cuh): nothing is made before the
 // order is asked for, it is the stable one by value count, largest first, and it
-// is made again after the rows changed. Built and run by test_walk_cpu.py.
+// is made again after the rows changed. And of rows_join_panel: a panel that is
+// asked for by name needs its memory as one that is chosen. Built and run by
+// test_walk_cpu.py.
 #include <algorithm>
 #include <cstdio>
 #include <numeric>
@@ -35,6 +37,19 @@ int main() {
             fail += !same(d.by_card.of(d.facts), d.facts);
             fail += !d.by_card.is_made() || !same(d.by_card.of(d.facts), d.facts);
         }
+    int asked = 0;
+    auto fits = [&asked](bool answer) {
+        return [&asked, answer] {
+            ++asked;
+            return answer;
+        };
+    };
+    fail += sb200::rows_join_panel(true, 2.0, 1.0, fits(false));
+    fail += sb200::rows_join_panel(false, 1.0, 2.0, fits(false));
+    fail += !sb200::rows_join_panel(true, 2.0, 1.0, fits(true));
+    fail += !sb200::rows_join_panel(false, 1.0, 2.0, fits(true));
+    fail += asked != 4;
+    fail += sb200::rows_join_panel(false, 2.0, 1.0, fits(true)) || asked != 4;
     std::printf(fail ? "FAIL (%d)\n" : "ok\n", fail);
     return fail ? 1 : 0;
 }

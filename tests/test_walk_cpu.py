@@ -9,5 +9,6 @@ def test_walk_items(sb):
 
 def test_rows_by_value_count(sb):
     """The planner's order of the rows (tests/row_order_check.cu): made when it
-    is first asked for after an upload, not for the calls that do without it."""
+    is first asked for after an upload, not for the calls that do without it; and
+    the memory that a wider panel needs."""
     assert run_host_check("row_order_check").strip().endswith("ok")
