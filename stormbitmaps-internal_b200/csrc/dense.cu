@@ -190,7 +190,7 @@ static int auto_kind(uint64_t row_bits) {
 // rows they share come from L2.
 constexpr uint32_t F4_BAND = 8;
 
-static void band_tiles(std::vector<uint2>& t) {
+void band_tiles(std::vector<uint2>& t) {
     std::stable_sort(t.begin(), t.end(), [](const uint2& a, const uint2& b) {
         const uint32_t ba = a.x / F4_BAND, bb = b.x / F4_BAND;
         return ba != bb ? ba < bb : a.y != b.y ? a.y < b.y : a.x < b.x;
@@ -439,18 +439,42 @@ void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_
 // of whole A blocks, equal in rows -- a fifth of the triangle is copied while the
 // second-last panel's rows come in -- of which each spreads over all SMs
 // (stream-K), and no more than one per 2 MiB that crosses the bus.
-std::vector<std::pair<uint32_t, uint32_t>> DenseEngine::host_plan(int kind, uint64_t n, uint64_t bus_bytes) const {
-    const int sms = require_device();
+static bool panels_of_blocks(int kind, uint32_t n_tiles, int sms) {
+    return kind == KIND_F4 && n_tiles <= 24u * (uint32_t)std::max(1, sms / 2);
+}
+
+std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint32_t n_tiles, int sms,
+                                                     uint64_t bus_bytes) {
     const uint32_t wave = kind == STORM_B200_KERNEL_POPC        ? 2u * (uint32_t)sms
                           : kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4 ? (uint32_t)std::max(1, sms / 2)
                                                                : (uint32_t)sms;
-    if (kind != KIND_F4 || n_tiles > 24 * wave) return host_panels(n_tiles, wave);
+    if (!panels_of_blocks(kind, n_tiles, sms)) return host_panels(n_tiles, wave);
     const uint32_t nb = (uint32_t)((n + F4_BM - 1) / F4_BM);
     const uint32_t k = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({8, nb, bus_bytes >> 21}));
     auto first = [nb](uint32_t b) { return (uint32_t)((uint64_t)b * nb - (uint64_t)b * (b - (b > 0)) / 2); };   // tile of block b
     std::vector<std::pair<uint32_t, uint32_t>> p;
     for (uint32_t q = k; q-- > 0;) p.emplace_back(first(nb * q / k), first(nb * (q + 1) / k));
     return p;
+}
+
+std::vector<uint64_t> host_arrivals(int kind, uint64_t n, const std::vector<uint2>& tiles,
+                                    const std::vector<std::pair<uint32_t, uint32_t>>& panels, int sms) {
+    std::vector<uint64_t> arrive;
+    if (panels.size() == 1) {
+        arrive.push_back(0);
+    } else if (panels_of_blocks(kind, (uint32_t)tiles.size(), sms)) {
+        for (const auto& q : panels) arrive.push_back((uint64_t)tiles[q.first].x * F4_BM);
+    } else {
+        const uint64_t chunk_rows = round_up(std::max<uint64_t>(1, (n + 31) / 32), 128);
+        for (uint64_t c = (n + chunk_rows - 1) / chunk_rows; c-- > 0;) arrive.push_back(c * chunk_rows);
+    }
+    return arrive;
+}
+
+size_t arrival_of(const std::vector<uint64_t>& arrive, uint64_t row) {
+    size_t c = 0;
+    while (c + 1 < arrive.size() && arrive[c] > row) ++c;
+    return c;
 }
 
 uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits,
@@ -462,7 +486,7 @@ uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad
         return 0;
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
-    const auto panels = host_plan(kind, n, tri_size(n) * sizeof(uint32_t));
+    const auto panels = host_plan(kind, n, n_tiles, require_device(), tri_size(n) * sizeof(uint32_t));
     return panels_to_host(dX, n, w_pad, kind, panels, {}, d_out, host_out, st, copy_st);
 }
 
@@ -476,25 +500,16 @@ uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad,
         return 0;
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
-    const auto panels = host_plan(kind, n, tri_size(n) * sizeof(uint32_t) + n * host_wpr * sizeof(uint64_t));
+    const int sms = require_device();
+    const auto panels =
+        host_plan(kind, n, n_tiles, sms, tri_size(n) * sizeof(uint32_t) + n * host_wpr * sizeof(uint64_t));
     const bool one = panels.size() == 1;             // everything on one stream
     cudaStream_t in = one ? st : h2d_st;
     // Rows [n, n_pad) read as zero: whole tiles read them.
     const uint64_t n_pad = round_up(n, 256), pitch = dense_pitch(w_pad);
     if (n_pad > n) SB_CUDA(cudaMemsetAsync(dX + n * pitch, 0, (n_pad - n) * pitch * sizeof(uint64_t), in));
     uint64_t* const stage = row_stage(d_stage, n, host_wpr);
-    // Rows arrive last rows first: the bottom panels read only them. Chunks of
-    // whole panels where those are whole A blocks, else 32 equal ones; event c
-    // marks rows [arrive[c], n) (and the zeroing) as resident.
-    std::vector<uint64_t> arrive;
-    if (one) {
-        arrive.push_back(0);
-    } else if (kind == KIND_F4 && n_tiles <= 24u * (uint32_t)std::max(1, require_device() / 2)) {
-        for (const auto& q : panels) arrive.push_back((uint64_t)h_tiles[q.first].x * F4_BM);
-    } else {
-        const uint64_t chunk_rows = round_up(std::max<uint64_t>(1, (n + 31) / 32), 128);
-        for (uint64_t c = (n + chunk_rows - 1) / chunk_rows; c-- > 0;) arrive.push_back(c * chunk_rows);
-    }
+    const std::vector<uint64_t> arrive = host_arrivals(kind, n, h_tiles, panels, sms);
     while (h2d_ev.size() < arrive.size()) {
         cudaEvent_t e;
         SB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
@@ -547,9 +562,7 @@ uint64_t DenseEngine::panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_
                 uint64_t need = n;
                 for (uint32_t t = t0; t < t1; ++t)
                     need = std::min(need, std::min<uint64_t>(h_tiles[t].x * bm, h_tiles[t].y * bn));
-                size_t c = 0;
-                while (c + 1 < arrive.size() && arrive[c] > need) ++c;
-                SB_CUDA(cudaStreamWaitEvent(st, h2d_ev[c], 0));
+                SB_CUDA(cudaStreamWaitEvent(st, h2d_ev[arrival_of(arrive, need)], 0));
             }
             launch(kind, dX, (uint32_t)n, w_pad, t0, t1 - t0, d_out, st);
             if (p + 1 == panels.size()) SB_CUDA(cudaEventRecord(log.ev1, st));

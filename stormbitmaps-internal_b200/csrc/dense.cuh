@@ -96,7 +96,6 @@ struct DenseEngine {
     void launch(int kind, const uint64_t* dX, uint32_t n, uint32_t w_pad, uint32_t t0, uint32_t count,
                 uint32_t* d_out, cudaStream_t st);
     void zero_stream_k_rows(uint32_t* d_out, uint32_t n, uint32_t t0, uint32_t t1, uint32_t grid, cudaStream_t st);
-    std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint64_t bus_bytes) const;
     uint64_t panels_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, int kind,
                             const std::vector<std::pair<uint32_t, uint32_t>>& panels,
                             const std::vector<uint64_t>& arrive, uint32_t* d_out, uint32_t* host_out, cudaStream_t st,
@@ -124,6 +123,18 @@ uint64_t tile_rows_b(int kind);
 // order (the end of the list first), each a whole number of waves but the
 // last.
 std::vector<std::pair<uint32_t, uint32_t>> host_panels(uint32_t n_tiles, uint32_t wave);
+// The panels of a kernel's host-output call over n rows (n_tiles tiles in order
+// of A block), and how the rows of a host-to-host call arrive for them, last
+// rows first (the bottom panels read only them): rows [arrive[c], n) are
+// resident once part c is, in parts of whole panels where those are whole A
+// blocks, else in 32 equal ones. arrival_of: the part that a read of `row` waits for.
+std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint32_t n_tiles, int sms,
+                                                     uint64_t bus_bytes);
+std::vector<uint64_t> host_arrivals(int kind, uint64_t n, const std::vector<uint2>& tiles,
+                                    const std::vector<std::pair<uint32_t, uint32_t>>& panels, int sms);
+size_t arrival_of(const std::vector<uint64_t>& arrive, uint64_t row);
+// The pair kernels' tiles in the order that suits L2.
+void band_tiles(std::vector<uint2>& t);
 // Longest row the tensor-core kernels count exactly (4-byte weight cycle).
 constexpr uint64_t TC_MAX_ROW_BITS = 1ull << 27;
 // ... and the shared-memory form (8-byte weight cycle only).
