@@ -252,13 +252,19 @@ def tensor_kernel(sb, kernel, bits):
             sb.KERNEL_MMA_2CTA: "bb_mma_2cta_kernel"}.get(kernel, "?")
 
 
-def tensor_peak_tops(device, bits4=True):
+def tensor_peak_tops(device, bits4=True, sm_mhz=None):
     """(peak TOPS, source text) for the tensor-core roofline: the 4-bit kernel's
-    against four times the measured bf16 rate (the pipe's e2m1 rate), the 8-bit
-    kernels' against the largest of the measured 8-bit figures."""
+    against its pipe's rate at the clock of the timed region (without a sample,
+    the highest clock) -- a 256 x 256 tile of a CTA pair takes 1024 clocks per
+    512 bits (csrc/bb_f4.cuh), one pair per two SMs; the 8-bit kernels' against
+    the largest of the measured 8-bit figures."""
     peaks, src = measured_peaks()
     if bits4:
-        return 4.0 * peaks["bf16_tflops"], f"4 x bf16_tflops {src}: {4.0 * peaks['bf16_tflops']:.1f}"
+        import torch
+        pairs = torch.cuda.get_device_properties(device).multi_processor_count // 2
+        mhz = sm_mhz or peaks.get("sm_max_mhz", 1965.0)
+        return (2.0 * 256 * 256 * 512 / 1024 * pairs * mhz * 1e6 / 1e12,
+                f"kind::mxf4 pipe, {pairs} CTA pairs at {mhz:.0f} MHz ({'median sampled' if sm_mhz else 'highest'})")
     t8 = tensor8_peak(device)
     cands = {f"2 x bf16_tflops {src}": 2.0 * peaks["bf16_tflops"]}
     if t8.get("int8_tops"):
@@ -1335,7 +1341,7 @@ TENSOR_KERNELS = ("bb_f4_kernel", "bb_mma_kernel", "bb_mma_ts_long_kernel", "bb_
 
 def north_star_summary(line):
     """The figures the target names, compactly: the tensor-core kernel's
-    fraction of the measured 8-bit peak on the headline workload and on the
+    fraction of its pipe on the headline workload and on the
     4096 x 65536 configuration; learned-batched vs plain per-tile vs the
     reference CPU driver on the mixed-density corpus, with the selectors'
     regret; each full-size STORM_t configuration's device rate, CPU rate and
@@ -1580,13 +1586,15 @@ def run_b200_arm(args):
 
     # ---- roofline of the dominant kernel ----
     k_ms = statistics.median(kernel_ms)
+    line_clocks = clocks.summary()
     if kernel_used in TENSOR_KERNELS:
         ops = 2.0 * tri * m                      # MACs = pairs x row bits, 2 ops each
         achieved = ops / (k_ms / 1e3) / 1e12
         bits4 = kernel_used == "bb_f4_kernel"
-        peak, peak_src = tensor_peak_tops(device, bits4)
+        peak, peak_src = tensor_peak_tops(device, bits4, line_clocks["sm_mhz"])
         roof = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": f"TOPS ({'e2m1' if bits4 else 'int8'})",
-                "frac": achieved / peak, "peak_source": peak_src, "tensor8_measured": tensor8_peak(device),
+                "frac": achieved / peak, "peak_source": peak_src,
+                "of_measured_bf16": achieved / measured_peaks()[0]["bf16_tflops"], "tensor8_measured": tensor8_peak(device),
                 "algorithmic": f"pairs(i<=j) x {m} bit-MACs x 2 ops", "traffic": args.traffic}
     else:
         ops = 2.0 * tri * m
@@ -1610,7 +1618,7 @@ def run_b200_arm(args):
         "kernel_ms_median": k_ms,
         "gpu_launches": launches,
         "roofline": roof,
-        "clocks": clocks.summary(),
+        "clocks": line_clocks,
         "e2e": {"value": e2e_value, "unit": "pairs/s", "ms_per_step": e2e_step_ms,
                 "h2d_bytes_per_step": int(n * w * 8), "d2h_bytes_per_step": int(tri * 4),
                 "call": "STORM_contig_pairw_intersect_matrix_from_host (pinned host rows in, pinned host "
