@@ -23,6 +23,9 @@ rows of different ranks are independent, so there is no data-path
 collective ("scaling": "weak").  `--impl reference` times the reference's own
 CPU kernel (oracle/_ref, built from the reference sources) on the host cores,
 on a bounded row sample of the same workload, on rank 0 only.
+
+Rank 0 prints one JSON line, a few kilobytes; the characterisation forms of a
+one-GPU run go to a file (--forms-file), their summary to the line's end.
 """
 from __future__ import annotations
 
@@ -1339,7 +1342,7 @@ TENSOR_KERNELS = ("bb_f4_kernel", "bb_mma_kernel", "bb_mma_ts_long_kernel", "bb_
                   "bb_mma_2cta_kernel")
 
 
-def north_star_summary(line):
+def forms_summary(line):
     """The figures the target names, compactly: the tensor-core kernel's
     fraction of its pipe on the headline workload and on the
     4096 x 65536 configuration; learned-batched vs plain per-tile vs the
@@ -1397,6 +1400,23 @@ def north_star_summary(line):
         if regret:
             ns["storm_t_plan_regret"] = regret
     return ns
+
+
+def report(line, forms, path):
+    """The benchmark's own line, with the forms' summary last; the forms
+    themselves, tens of kilobytes that whoever reads the end of the output would
+    cut, go to the file `path`."""
+    line = dict(line)
+    if forms:
+        try:
+            os.makedirs(os.path.dirname(os.path.abspath(path)), exist_ok=True)
+            with open(path, "w") as f:
+                json.dump(forms, f, indent=1)
+            line["forms_file"] = os.path.relpath(path, ROOT)
+        except OSError as e:         # the line itself is never lost to it
+            line["forms_file"] = f"not written: {e}"
+    line["summary"] = forms_summary({**line, **forms})
+    return json.dumps(line)
 
 
 # ------------------------------------------------------------------ arms
@@ -1639,6 +1659,7 @@ def run_b200_arm(args):
                                     "sample": "oracle/_ref not built"}
     if thresh is not None:
         line["threshold_form"] = thresh
+    forms = {}
     if rank == 0 and world == 1 and args.forms:
         # Characterisation forms, each timed (wall seconds in form_seconds).
         # The default run keeps them to a few minutes: the STORM_t table keeps
@@ -1650,9 +1671,9 @@ def run_b200_arm(args):
         def form(key, fn):
             t1 = time.perf_counter()
             try:
-                line[key] = fn()
+                forms[key] = fn()
             except Exception as e:   # reported, never silently dropped
-                line[key] = {"error": f"{type(e).__name__}: {e}"}
+                forms[key] = {"error": f"{type(e).__name__}: {e}"}
             secs[key] = round(time.perf_counter() - t1, 1)
 
         form("mixed_density", lambda: mixed_density_forms(sb, device))
@@ -1663,10 +1684,9 @@ def run_b200_arm(args):
         form("storm_t_full", lambda: storm_t_full(device))
         form("autotune_config1", lambda: autotune_config1(sb, device))
         form("config5a_full", lambda: config5a_full(sb, device))
-        line["form_seconds"] = secs
+        forms["form_seconds"] = secs
     if rank == 0:
-        line["north_star"] = north_star_summary(line)   # last, so that the tail of the line keeps it
-        print(json.dumps(line), flush=True)
+        print(report(line, forms, args.forms_file), flush=True)
     if dist:
         dist.barrier()
         dist.destroy_process_group()
@@ -1691,6 +1711,8 @@ def main():
                     help="also the reduced-size STORM_t corpora and the whole density sweep (longer run)")
     ap.add_argument("--no-forms", dest="forms", action="store_false",
                     help="skip the mixed-density learned/plain/CPU comparison")
+    ap.add_argument("--forms-file", default=os.path.join(ROOT, "_build", "bench_forms.json"),
+                    help="where the forms' figures are written (the printed line has their summary)")
     ap.add_argument("--traffic", type=float, default=None,
                     help="dram bytes per launch of the dominant kernel from an ncu capture")
     ap.add_argument("--storm-t-case", default=None, choices=STORM_T_CASES,
