@@ -714,8 +714,8 @@ constexpr int EXPAND_WARPS = 4;
 
 // Expanded rows for the tensor cores are stored block-major: chunk slot s of
 // all the panel's rows together, rows PANEL_PITCH words (8 KiB + 64 bytes)
-// apart within it.  A tile's 384 rows at one K stage then lie in about 3 MiB
-// instead of on 384 pages of 2 MiB (rows of 2^24 bits row-major), and no two
+// apart within it.  A tile's 512 rows at one K stage then lie in about 4 MiB
+// instead of on 512 pages of 2 MiB (rows of 2^24 bits row-major), and no two
 // rows share a pitch that is a power of two.
 constexpr uint64_t PANEL_PITCH = CHUNK_WORDS + 8;
 inline uint64_t panel_row_words(uint64_t W) { return W / CHUNK_WORDS * PANEL_PITCH; }
@@ -1820,8 +1820,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             for (uint64_t r = 0; r < n2; ++r) second[r] = (uint32_t)(n1 + r);
             SB_CUDA(cudaMemcpyAsync(d_qrows.p, second.data(), n2 * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
             WalkShape ws;
-            for (const ChunkRowFacts& f : d.facts) ws.add(f);
-            ws.done();
+            ws.of(n1 + n2, [&](uint64_t r) -> const ChunkRowFacts& { return d.facts[r]; });
             postings_hist_kernel<<<ws.grid(n1, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), nullptr, ws.dims(n1), d_counts.p);
             postings_hist_kernel<<<ws.grid(n2, sms), ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, ws.dims(n2),
                                                                               d_start.p);
@@ -1867,13 +1866,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     SB_CUDA(cudaEventRecord(log.ev0, st));
     PostingsStats ps{};
     WalkShape q_walk;                                      // of the postings rows
-    auto walk_of = [&](const std::vector<uint32_t>& rows) {
-        WalkShape w;
-        for (uint32_t r : rows) w.add(d.facts[r]);
-        w.done();
-        return w;
-    };
-    auto histogram = [&](const std::vector<uint32_t>& rows, const WalkShape& shape) {
+    auto histogram = [&](const std::vector<uint32_t>& rows) {
         d_qrows.reserve(rows.size());
         SB_CUDA(cudaEventRecord(ev_hist0, st));
         SB_CUDA(cudaMemcpyAsync(d_qrows.p, rows.data(), rows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
@@ -1881,7 +1874,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_counts.p, 0, U * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
-        q_walk = shape;
+        q_walk.of(rows.size(), [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[rows[k]]; });
         postings_hist_kernel<<<q_walk.grid(rows.size(), sms), ROW_WALK_THREADS, 0, st>>>(
             d.view(), d_qrows.p, q_walk.dims(rows.size()), d_counts.p);
         postings_stats_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_pstats.p);
@@ -1961,16 +1954,11 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // chunk kernel.
     if (!d_out && post_ok) {
         std::vector<uint32_t> plain;
-        WalkShape shape;                                   // in the same pass: 10^6 rows' facts are 40 MB
         for (uint32_t r = 0; r < n; ++r)
-            if (d.facts[r].plain) {
-                plain.push_back(r);
-                shape.add(d.facts[r]);
-            }
-        shape.done();
+            if (d.facts[r].plain) plain.push_back(r);
         uint64_t q_sum = 0;
         if (plain.size() >= 2) {
-            q_sum = histogram(plain, shape).pairs;
+            q_sum = histogram(plain).pairs;
             last_postings_rows = plain.size();
         }
         const uint64_t nc = n - plain.size();
@@ -2068,7 +2056,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             }
         }
         if (!lists_only) return false;
-        ps = histogram(rest, walk_of(rest));
+        ps = histogram(rest);
         if (ps.entries < (1ull << 32) && (postings_mode > 0 || post_ns((double)ps.pairs, q, (double)values_of(rest)) < alt)) {
             qrows = rest;
             return true;

@@ -31,15 +31,20 @@ constexpr uint64_t WALK_SPARE_ITEMS = 1ull << 18;
 // nothing.
 struct WalkShape {
     uint32_t group = 1, groups = 0, lanes = 0;
-    void add(const ChunkRowFacts& f) {
-        ++n;
-        chunks += f.chunks;
-        entries += f.list_entries;
-        bitmaps |= f.bitmap_chunks != 0;
-        most = std::max(most, f.chunks);
-        if (f.chunks) spread += (double)f.list_entries * (double)f.list_entries / (double)f.chunks;
-    }
-    void done() {                                         // every row added
+    template <class Facts>
+    void of(uint64_t n, Facts facts) {
+        uint64_t chunks = 0, entries = 0;
+        double spread = 0.0;                              // entries x (their row's entries per chunk)
+        uint32_t most = 0;
+        bool bitmaps = false;
+        for (uint64_t k = 0; k < n; ++k) {
+            const ChunkRowFacts& f = facts(k);
+            chunks += f.chunks;
+            entries += f.list_entries;
+            bitmaps |= f.bitmap_chunks != 0;
+            most = std::max(most, f.chunks);
+            if (f.chunks) spread += (double)f.list_entries * (double)f.list_entries / (double)f.chunks;
+        }
         group = bitmaps || entries >= 48 * chunks ? 1u : spread >= 48.0 * (double)entries ? WALK_SKEW_GROUP : 32u;
         groups = (most + group - 1) / group;
         lanes = (uint32_t)std::min<uint64_t>(groups, n ? (chunks / group + n + WALK_SPARE_ITEMS) / n : 0);
@@ -58,12 +63,6 @@ struct WalkShape {
         __host__ __device__ uint32_t step() const { return lanes * group; }
     };
     Dims dims(uint64_t n) const { return Dims{(uint32_t)n, group, lanes}; }
-
-   private:
-    uint64_t n = 0, chunks = 0, entries = 0;
-    double spread = 0.0;                                  // entries x (their row's entries per chunk)
-    uint32_t most = 0;
-    bool bitmaps = false;
 };
 
 }  // namespace sb200

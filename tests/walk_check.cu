@@ -13,8 +13,7 @@ static void check(const char* name, const std::vector<sb200::ChunkRowFacts>& row
     using namespace sb200;
     const uint64_t n = rows.size();
     WalkShape s;
-    for (const ChunkRowFacts& f : rows) s.add(f);
-    s.done();
+    s.of(n, [&](uint64_t k) -> const ChunkRowFacts& { return rows[k]; });
     const WalkShape::Dims w = s.dims(n);
     std::vector<std::vector<uint8_t>> seen(n);
     uint64_t groups = 0;
