@@ -157,7 +157,9 @@ void* STORM_contig_stream(STORM_contiguous_t* c);
 float STORM_contig_last_kernel_ms(const STORM_contiguous_t* c);
 uint32_t STORM_contig_last_launches(const STORM_contiguous_t* c);
 /* Which kernel choice the last call ran under (STORM_B200_KERNEL_POPC, _MMA,
- * _MMA_SS, _MMA_DB or _MMA_2CTA; never _AUTO). */
+ * _MMA_SS, _MMA_DB or _MMA_2CTA; never _AUTO). Up to 2^24-bit rows _MMA and
+ * _MMA_DB are one kernel; a sum alone under _AUTO, which comes from the columns'
+ * counts, reports the choice that calls with counts get for that row length. */
 int STORM_contig_last_kernel(const STORM_contiguous_t* c);
 
 /* All pairs of rows that are already in device memory, into a device buffer,
@@ -321,8 +323,8 @@ uint64_t STORM_last_panel_rows(const STORM_t* s);
  * tensor cores, the chunk kernel, the transposed panel and the postings
  * (with their histogram); out12[4..7]: the planner's predicted ms for the
  * work it gave each (0 for the chunk kernel, which it does not price);
- * out12[8..11]: that work -- tensor cores in int8 operations (2 x pairs x
- * universe bits), chunk kernel in pairs, panel and postings in the bytes
+ * out12[8..11]: that work -- tensor cores in multiplications and
+ * additions (2 x pairs x universe bits), chunk kernel in pairs, panel and postings in the bytes
  * they must move (panel: a 256-byte transposed line per query value and
  * 2048-row block, the expanded and transposed blocks, 4 bytes per count;
  * postings: 8 bytes per value, per list entry and per increment, and the

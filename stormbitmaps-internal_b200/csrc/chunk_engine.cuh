@@ -280,9 +280,9 @@ struct ChunkEngine {
     // (events between the engines on the stream) and the cost model's
     // prediction for the work it gave each.
     double last_engine_ms[4] = {0, 0, 0, 0}, last_engine_pred_ms[4] = {0, 0, 0, 0};
-    // ... and the algorithmic work of each: tensor cores in int8 operations
-    // (2 x pairs x universe bits), chunk kernel in pairs, the panel and the
-    // postings in bytes they must move (panel: one 256-byte transposed line
+    // ... and the algorithmic work of each: tensor cores in multiplications and
+    // additions (2 x pairs x universe bits), chunk kernel in pairs, the panel
+    // and the postings in bytes they must move (panel: one 256-byte transposed line
     // per query value and block, the expanded and transposed blocks, 4 bytes
     // per count written; postings: the histogram and list entries, 8 bytes
     // per increment -- a read and a write of its count).

@@ -1,7 +1,9 @@
 // colsum.cuh -- the sum over all pairs of dense rows without a pair.
 //
 // sum_{i<j} |Xi & Xj| = sum_v C(n_v, 2), n_v = the rows holding column v, so a
-// call that wants only the sum reads the rows once.  Bound: HBM (the rows).
+// call that wants only the sum reads the rows once.  What it cannot do without is
+// that read; what bounds it is the chain of each warp's few steps (eight loads,
+// then their adders) and the unpacking of its planes, at a third of HBM's rate.
 // A warp reads 32 consecutive words of a row (256 bytes); each thread counts
 // its 64 columns over the warp's rows in bit-sliced planes: eight rows go
 // through carry-save adders into ones / twos / fours and a carry of weight 8

@@ -13,27 +13,20 @@
 
 namespace sb200 {
 
-// Work schedule of the tensor-core kernel (TsSched in bb_mma_ts.cuh): whole
-// tiles round robin when the last wave is nearly full (>= 98.5 %) or a tile
-// has fewer than 128 K stages (32768 bits: shorter tiles lose more to the
-// extra segment boundaries and partial-tile atomics than they gain); else
-// stream-K over the (tile, K stage) space, at least 32 stages per CTA.
-// Measured on B200: 272 tiles (1.8 waves) of 2^18-bit rows run 8 % faster
-// under stream-K, 136 tiles 1.9x, 1088 tiles (92 % fill) 7 %, 4160 tiles
-// (97 % fill) 3 %; 2176 tiles (98 % fill) of 2^16-bit rows 3 % slower, and
-// 80-stage tiles (20000-bit rows) 7 % slower. Those figures are for stream-K
-// over every tile; the kernels now run the first floor(tiles / grid) waves
-// as whole tiles and stream-K only the rest (TsSched), which measured faster
-// still on B200 (double-buffered kernel: 50000 x 20000 bits 7 %, 16384 x
-// 262144 5 %, 4096 x 65536 1 %) with counts unchanged. Returns the kernel's
+// Work schedule of the 8-bit tensor-core kernels (TsSched in bb_mma_ts.cuh),
+// rows of more than 2^24 bits: whole tiles round robin when the last wave is
+// nearly full (>= 98.5 %), else the first floor(tiles / grid) waves as whole
+// tiles and stream-K over the (tile, K stage) space of the rest, at least 32
+// stages per CTA. The line was measured at 2^18-bit rows (B200, stream-K over
+// every tile): 136 tiles 1.9x faster, 272 8 %, 1088 (92 % fill) 7 %, 4160 (97 %)
+// 3 %; longer rows only make a segment's fixed cost smaller. Returns the kernel's
 // k_splits argument (1 or 0) and sets the grid.
 static uint32_t ts_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t& grid,
                             int pref = STORM_B200_SCHED_AUTO) {
     const uint64_t nk = w_pad / (TS_KBITS / 64);
     const uint64_t waves = ((uint64_t)n_tiles + sms - 1) / sms;
     const double fill = waves ? (double)n_tiles / (double)(waves * (uint64_t)sms) : 1.0;
-    const bool tiles = pref == STORM_B200_SCHED_TILES ||
-                       (pref == STORM_B200_SCHED_AUTO && (fill >= 0.985 || nk < 128));
+    const bool tiles = pref == STORM_B200_SCHED_TILES || (pref == STORM_B200_SCHED_AUTO && fill >= 0.985);
     if (tiles) {
         grid = n_tiles < (uint32_t)sms ? n_tiles : (uint32_t)sms;
         return 1;
@@ -41,8 +34,6 @@ static uint32_t ts_schedule(uint32_t n_tiles, int sms, uint32_t w_pad, uint32_t&
     grid = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sms, (uint64_t)n_tiles * nk / 32));
     return 0;
 }
-
-constexpr uint64_t DB_AUTO_MAX_BITS = 1ull << 17;
 
 // The tensor-core kernel a row length runs on: up to 2^24 bits the 4-bit one
 // (its fp32 accumulator counts exactly that far), longer rows the 8-bit ones.
@@ -176,8 +167,11 @@ void build_tiles(std::vector<uint2>& t, uint64_t n, int kind) {
     }
 }
 
-// Automatic choice: tensor cores up to 2^27-bit rows (both choices run the
-// 4-bit kernel up to 2^24 bits and differ past it), CUDA-core POPC beyond.
+// Automatic choice: tensor cores up to 2^27-bit rows, CUDA-core POPC beyond. Both
+// tensor-core names run the 4-bit kernel up to 2^24 bits; which of them a call
+// reports there changes at 2^17.
+constexpr uint64_t DB_AUTO_MAX_BITS = 1ull << 17;
+
 static int auto_kind(uint64_t row_bits) {
     return row_bits <= DB_AUTO_MAX_BITS   ? STORM_B200_KERNEL_MMA_DB
            : row_bits <= MMA_MAX_BITS_W4 ? STORM_B200_KERNEL_MMA
@@ -642,7 +636,7 @@ extern "C" int STORM_contig_pairw_intersect_matrix_noalloc(const uint64_t* d_row
     using namespace sb200;
     if (d_rows == NULL) return STORM_B200_EVALUES;
     if (n_rows == 0 || n_rows > 0xFFFFFFFFull) return STORM_B200_EARG;
-    if ((uintptr_t)d_rows % 32 != 0) return STORM_B200_EARG;   // the kernel reads rows 32 bytes at a time
+    if ((uintptr_t)d_rows % 32 != 0) return STORM_B200_EARG;   // the call's contract; TMA itself wants 16
     if (row_pitch_words == 0 || row_pitch_words % 8 != 0 || (uint64_t)row_pitch_words * 64 < row_bits)
         return STORM_B200_EARG;
     if (row_bits > MMA_MAX_BITS) return STORM_B200_ELIMIT;
@@ -889,9 +883,8 @@ uint64_t DenseEngine::run_threshold(const uint64_t* dX, uint64_t n, uint32_t w_p
         if (sum) *sum = 0;
         return 0;
     }
-    // The thresholded form has its filter fused into the 128 x 256 tensor-core
-    // kernel's drain; the double-buffered kernel has none, so rows it would
-    // take go to the fused one.
+    // The filter is fused into the drain of the 4-bit kernel and, past 2^24 bits,
+    // of MMA's 8-bit one; MMA_DB's has none, so rows it would take go to MMA's.
     if ((kernel_pref == STORM_B200_KERNEL_AUTO || kernel_pref == STORM_B200_KERNEL_MMA_DB) &&
         row_bits <= MMA_MAX_BITS_W4)
         kernel_pref = STORM_B200_KERNEL_MMA;

@@ -10,9 +10,9 @@ namespace sb200 {
 
 // Row pitch (words) of the dense engine's device rows of w_pad words: a
 // pitch that is a multiple of 4 KiB gets 64 bytes more.  With a power-of-two
-// pitch the same K stage of the 384 rows a tile reads falls on the same
-// memory partitions, and their loads queue there; measured on B200 with the
-// tensor-core kernel (ms, same rows): 65536 x 2^18 bits 368.6 -> 353.8,
+// pitch the same K stage of the rows a tile reads falls on the same
+// memory partitions, and their loads queue there; measured on B200 with an
+// 8-bit tensor-core kernel (128 x 256 tiles; ms, same rows): 65536 x 2^18 bits 368.6 -> 353.8,
 // 16384 x 2^18 23.7 -> 21.6, 4096 x 2^16 0.484 -> 0.468, 4096 x 2^23 48.2
 // -> 46.4.  (256 bytes more was slower than none at 2^18: 395.1.)
 inline uint64_t dense_pitch(uint32_t w_pad) { return w_pad % 512 == 0 ? (uint64_t)w_pad + 8 : (uint64_t)w_pad; }
