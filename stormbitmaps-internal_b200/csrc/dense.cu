@@ -408,9 +408,8 @@ repitch_rows_kernel(const uint64_t* __restrict__ src, uint32_t wpr, uint64_t* __
     }
 }
 
-// Host rows into device rows `pitch` words apart: across the bus as they lie,
-// into `stage` (as many words as the host rows), and spread out on the device;
-// or, without `stage`, by a copy with two pitches, which is slow for short rows.
+// Host rows into device rows `pitch` words apart (dense.cuh says which way they
+// take): `stage` holds as many words as the host rows, or is null.
 void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_t* host, uint32_t wpr, uint64_t rows,
                     uint64_t* stage, cudaStream_t st) {
     if (rows == 0) return;
@@ -419,6 +418,10 @@ void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_
         repitch_rows_kernel<<<(uint32_t)std::min<uint64_t>((rows + 7) / 8, 1184), 256, 0, st>>>(stage, wpr, dst, pitch,
                                                                                               w_pad, rows);
         SB_CUDA(cudaGetLastError());
+        return;
+    }
+    if (wpr == pitch) {
+        SB_CUDA(cudaMemcpyAsync(dst, host, rows * wpr * sizeof(uint64_t), cudaMemcpyHostToDevice, st));
         return;
     }
     if (wpr != w_pad)

@@ -17,18 +17,23 @@ namespace sb200 {
 // -> 46.4.  (256 bytes more was slower than none at 2^18: 395.1.)
 inline uint64_t dense_pitch(uint32_t w_pad) { return w_pad % 512 == 0 ? (uint64_t)w_pad + 8 : (uint64_t)w_pad; }
 
-// Host rows shorter than this, up to this size in all, cross the bus as they lie
-// and are spread out on the device (rows_to_device). Host to host on B200, copies
-// with two pitches / staged (ms): 12000 rows of 2504 bytes 6.64 / 5.37, 3000 of
-// them 0.94 / 0.55; 8192 of 8192 bytes 2.97 / 3.07, 16384 of them 10.44 / 10.63
-// (the spreading waits for a free SM).
+// How host rows get to their places. Rows that already lie a pitch apart: one
+// copy. Others by a copy with two pitches, or, where that is slow -- short rows of
+// no multiple of 64 bytes, up to this size in all -- across the bus as they lie and
+// spread out on the device (rows_to_device). Host to host on B200, two pitches /
+// staged (ms, 8192 rows but where noted): 504 bytes 3.20 / 2.50 (2000 rows 0.42 /
+// 0.24), 2504 bytes 3.43 / 2.60 (0.70 / 0.65), 5600 bytes 3.44 / 2.82 (0.88 /
+// 0.87), 8168 bytes 3.57 / 3.05 (0.94 / 0.97; 300 rows 0.13 / 0.20), 32744 bytes
+// 6.40 / 6.80; of multiples of 4 KiB, which the pitch is 64 bytes longer than,
+// 4096 bytes 2.68 / 2.71, 8192 2.96 / 3.03, 16384 3.79 / 4.02.
 constexpr uint32_t ROW_STAGE_WORDS = 640;
 constexpr uint64_t ROW_STAGE_BYTES = 256ull << 20;
 // Where `rows` host rows of wpr words are staged: null when they are not, also
 // when there is no memory for it.
 inline uint64_t* row_stage(DevBuf<uint64_t>& buf, uint64_t rows, uint32_t wpr) {
     const uint64_t words = rows * wpr;
-    if (wpr >= ROW_STAGE_WORDS || words * sizeof(uint64_t) > ROW_STAGE_BYTES || !buf.try_reserve(words)) return nullptr;
+    if (wpr % 8 == 0 || wpr >= ROW_STAGE_WORDS || words * sizeof(uint64_t) > ROW_STAGE_BYTES || !buf.try_reserve(words))
+        return nullptr;
     return buf.p;
 }
 void rows_to_device(uint64_t* dst, uint64_t pitch, uint32_t w_pad, const uint64_t* host, uint32_t wpr, uint64_t rows,

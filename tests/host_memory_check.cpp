@@ -118,7 +118,9 @@ static void staged_rows() {
     CHECK(row_stage(stage, 300, 313) == nullptr && g_used == 0);
     g_budget = 300 * 313 * 8;
     CHECK(row_stage(stage, 300, 313) == stage.p && stage.p);
-    CHECK(row_stage(stage, 1, ROW_STAGE_WORDS) == nullptr);      // long rows: straight to their places
+    CHECK(row_stage(stage, 1, ROW_STAGE_WORDS + 1) == nullptr);  // long rows: straight to their places
+    for (uint32_t wpr : {8u, 64u, 312u, 400u, 512u, 632u})       // and rows of whole 64 bytes, whatever their length
+        CHECK(row_stage(stage, 1, wpr) == nullptr);
     CHECK(row_stage(stage, ROW_STAGE_BYTES / 8 / 313 + 1, 313) == nullptr);
 }
 

@@ -1,5 +1,6 @@
-"""Host rows that go to their places by copies with two pitches (640 words and
-more, as shorter ones do when there is no memory to stage them): ragged lengths,
+"""The ways host rows take to their places: one copy where they lie a pitch apart,
+copies with two pitches (640 words and more, as shorter ones when there is no
+memory to stage them; multiples of 512 words), and staged ones; ragged lengths,
 repeated calls on one container, few rows and several panels."""
 import numpy as np
 import pytest
@@ -10,8 +11,8 @@ import oracle_lib as ol
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("words", (639, 640, 641, 1023, 1024))
-def test_matrix_from_host_long_rows(sb, words):
+@pytest.mark.parametrize("words", (1, 7, 8, 9, 64, 312, 313, 512, 639, 640, 641, 1023, 1024))
+def test_matrix_from_host_row_lengths(sb, words):
     m = 64 * words - 7
     c = sb.StormContig(m)
     for n, seed in ((1100, 81), (3, 82), (300, 83)):
