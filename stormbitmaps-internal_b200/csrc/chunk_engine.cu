@@ -877,8 +877,8 @@ chunk_pairs_kernel(ChunkView v, uint32_t mode, uint64_t n1, uint64_t n2, uint64_
 
 // Group `g0` .. of `group` (1 .. 32) consecutive chunks [cg, c1) of a row, one
 // warp: f(value, its place in the list pool) for every list entry, h(chunk) -- warp-cooperative -- for
-// every bitmap chunk. Long lists are walked one chunk at a time (group 1,
-// eight entries per lane); of short ones (a chunk of a very sparse row holds a
+// every bitmap chunk. Long lists are walked one chunk at a time (group 1), eight
+// entries of each lane read together (walk_entry); of short ones (a chunk of a very sparse row holds a
 // handful of values) the warp walks the concatenated entries of 32 chunks,
 // whose kinds and places it reads side by side.
 template <class F, class H>
@@ -890,13 +890,21 @@ __device__ __forceinline__ void walk_group_chunks(const ChunkView& v, uint64_t c
             h(cg);
             return;
         }
-        uint64_t at = v.coff[cg] + 8 * lane;
-        warp_list8(v.lst + v.coff[cg], k & CK_LEN, lane, [&](const uint16_t (&x)[8], uint32_t cnt) {
+        const uint64_t off = v.coff[cg];
+        const uint32_t nl = k & CK_LEN;
+        for (uint32_t e0 = 0; e0 < nl; e0 += WALK_STEP) {
+            uint16_t x[WALK_STEP / 32];
 #pragma unroll
-            for (uint32_t q = 0; q < 8; ++q)
-                if (q < cnt) f(base | x[q], at + q);
-            at += 256;
-        });
+            for (uint32_t q = 0; q < WALK_STEP / 32; ++q) {
+                const uint32_t e = e0 + walk_entry(q, lane);
+                x[q] = e < nl ? v.lst[off + e] : (uint16_t)0;
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < WALK_STEP / 32; ++q) {
+                const uint32_t e = e0 + walk_entry(q, lane);
+                if (e < nl) f(base | x[q], off + e);
+            }
+        }
         return;
     }
     const uint64_t c = cg + lane;

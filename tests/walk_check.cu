@@ -1,5 +1,6 @@
 // Host-only check of walk_shape.cuh: the items of a walk take every chunk of
-// every row once, in the row's order within an item, and there are no more than
+// every row once, in the row's order within an item; its entries in coalesced
+// steps; and there are no more than
 // one per group of chunks and row and a constant beside them, whatever the longest row.
 // Built and run by test_walk_cpu.py.
 #include <cstdio>
@@ -49,7 +50,28 @@ static sb200::ChunkRowFacts row(uint32_t chunks, uint64_t per_chunk, uint32_t bi
     return f;
 }
 
+// A step takes 256 entries once, and 32 in a row at a time: a run's values then
+// lie in the fewest sectors (eight counters each) at every update.
+static void check_step() {
+    std::vector<int> seen(sb200::WALK_STEP, 0);
+    for (uint32_t q = 0; q < sb200::WALK_STEP / 32; ++q) {
+        std::vector<uint8_t> sector(sb200::WALK_STEP / 8, 0);
+        int sectors = 0;
+        for (uint32_t lane = 0; lane < 32; ++lane) {
+            const uint32_t e = sb200::walk_entry(q, lane);
+            if (e < sb200::WALK_STEP) ++seen[e];
+            if (e < sb200::WALK_STEP && !sector[e / 8]++) ++sectors;
+        }
+        if (sectors != 4) {
+            std::printf("update %u of a step touches %d sectors\n", q, sectors);
+            ++g_fail;
+        }
+    }
+    for (int s : seen) g_fail += s != 1;
+}
+
 int main() {
+    check_step();
     using Rows = std::vector<sb200::ChunkRowFacts>;
     check("no rows", {});
     check("empty rows", Rows(5));
