@@ -11,7 +11,6 @@
 #include "list16_ref.cuh"
 #include "panel.cuh"
 #include "run_pieces.cuh"
-#include "walk_shape.cuh"
 
 namespace sb200 {
 
@@ -227,7 +226,7 @@ void ChunkDev::upload(const ChunkPack& p, cudaStream_t st) {
     put(lst, p.lst, st);
     n_rows = p.rows();
     facts = p.facts;
-    by_card.rows_changed();
+    rows_changed();
     max_cid = p.max_cid;
     SB_CUDA(cudaStreamSynchronize(st));
 }
@@ -395,7 +394,7 @@ void ChunkDev::upload_rows(const STORM_bitmap_cont_t* rows, uint64_t n, cudaStre
     std::vector<uint64_t> c_base(n + 1, 0), b_base(n + 1, 0), l_base(n + 1, 0), w1(n + 1, 0);
     std::vector<uint32_t> row_max(n, 0);
     facts.assign(n, ChunkRowFacts{});
-    by_card.rows_changed();
+    rows_changed();
     for (uint64_t r = 0; r < n; ++r) w1[r + 1] = w1[r] + 1 + live(r);
     parallel_rows(n, w1, hw, [&](uint64_t r0, uint64_t r1) {
         for (uint64_t r = r0; r < r1; ++r) {
@@ -1874,7 +1873,12 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     SB_CUDA(cudaEventRecord(log.ev0, st));
     PostingsStats ps{};
     WalkShape q_walk;                                      // of the postings rows
-    auto histogram = [&](const std::vector<uint32_t>& rows) {
+    auto walk_of = [&](const std::vector<uint32_t>& rows) {
+        WalkShape w;
+        w.of(rows.size(), [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[rows[k]]; });
+        return w;
+    };
+    auto histogram = [&](const std::vector<uint32_t>& rows, const WalkShape& shape) {
         d_qrows.reserve(rows.size());
         SB_CUDA(cudaEventRecord(ev_hist0, st));
         SB_CUDA(cudaMemcpyAsync(d_qrows.p, rows.data(), rows.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
@@ -1882,7 +1886,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_counts.p, 0, U * sizeof(uint32_t), st));
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
-        q_walk.of(rows.size(), [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[rows[k]]; });
+        q_walk = shape;
         postings_hist_kernel<<<q_walk.grid(rows.size(), sms), ROW_WALK_THREADS, 0, st>>>(
             d.view(), d_qrows.p, q_walk.dims(rows.size()), d_counts.p);
         postings_stats_kernel<<<sms * 8, 256, 0, st>>>(d_counts.p, U, d_pstats.p);
@@ -1966,7 +1970,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             if (d.facts[r].plain) plain.push_back(r);
         uint64_t q_sum = 0;
         if (plain.size() >= 2) {
-            q_sum = histogram(plain).pairs;
+            q_sum = histogram(plain, d.plain_walk.of(plain, d.facts)).pairs;
             last_postings_rows = plain.size();
         }
         const uint64_t nc = n - plain.size();
@@ -2064,7 +2068,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
             }
         }
         if (!lists_only) return false;
-        ps = histogram(rest);
+        ps = histogram(rest, walk_of(rest));
         if (ps.entries < (1ull << 32) && (postings_mode > 0 || post_ns((double)ps.pairs, q, (double)values_of(rest)) < alt)) {
             qrows = rest;
             return true;

@@ -8,9 +8,9 @@
 // places of 20000 rows' values (67 MB of cursors, 134 of postings) were written
 // from DRAM.
 #pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
 #include <algorithm>
-
-#include "chunk_engine.cuh"
 
 namespace sb200 {
 
@@ -46,7 +46,7 @@ struct WalkShape {
         uint32_t most = 0;
         bool bitmaps = false;
         for (uint64_t k = 0; k < n; ++k) {
-            const ChunkRowFacts& f = facts(k);
+            const auto& f = facts(k);                     // ChunkRowFacts (chunk_engine.cuh)
             chunks += f.chunks;
             entries += f.list_entries;
             bitmaps |= f.bitmap_chunks != 0;

@@ -37,6 +37,22 @@ int main() {
             fail += !same(d.by_card.of(d.facts), d.facts);
             fail += !d.by_card.is_made() || !same(d.by_card.of(d.facts), d.facts);
         }
+    // the sums' walk of all plain rows, the same way
+    for (uint32_t n : {3u, 5000u}) {
+        std::vector<uint32_t> plain(n);
+        std::iota(plain.begin(), plain.end(), 0u);
+        d.facts.assign(n, ChunkRowFacts{});
+        for (auto& f : d.facts) f.chunks = 40, f.list_entries = n;
+        d.rows_changed();
+        fail += d.plain_walk.is_made() || d.by_card.is_made();
+        sb200::WalkShape want;
+        want.of(n, [&](uint64_t k) -> const ChunkRowFacts& { return d.facts[k]; });
+        for (int call = 0; call < 2; ++call) {
+            const sb200::WalkShape& got = d.plain_walk.of(plain, d.facts);
+            fail += got.group != want.group || got.groups != want.groups || got.lanes != want.lanes;
+            fail += !d.plain_walk.is_made();
+        }
+    }
     int asked = 0;
     auto fits = [&asked](bool answer) {
         return [&asked, answer] {

@@ -6,7 +6,7 @@
 #include <cstdio>
 #include <vector>
 
-#include "walk_shape.cuh"
+#include "chunk_engine.cuh"
 
 static int g_fail = 0;
 
