@@ -440,14 +440,18 @@ static bool panels_of_blocks(int kind, uint32_t n_tiles, int sms) {
     return kind == KIND_F4 && n_tiles <= 24u * (uint32_t)std::max(1, sms / 2);
 }
 
+// A copy into pageable memory blocks the host until it is done, so that panels
+// would run one after the other with nothing beside them: there one panel (3000 x
+// 20032 bits into pageable memory, eight panels / one: 1.47 / 1.10 ms, rows from
+// the host too 2.00 / 1.55; 8000 rows 7.5 / 7.1 and 8.4 / 8.1).
 std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint32_t n_tiles, int sms,
-                                                     uint64_t bus_bytes) {
+                                                     uint64_t bus_bytes, bool pinned_out) {
     const uint32_t wave = kind == STORM_B200_KERNEL_POPC        ? 2u * (uint32_t)sms
                           : kind == STORM_B200_KERNEL_MMA_2CTA || kind == KIND_F4 ? (uint32_t)std::max(1, sms / 2)
                                                                : (uint32_t)sms;
     if (!panels_of_blocks(kind, n_tiles, sms)) return host_panels(n_tiles, wave);
     const uint32_t nb = (uint32_t)((n + F4_BM - 1) / F4_BM);
-    const uint32_t k = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({8, nb, bus_bytes >> 21}));
+    const uint32_t k = pinned_out ? (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>({8, nb, bus_bytes >> 21})) : 1u;
     auto first = [nb](uint32_t b) { return (uint32_t)((uint64_t)b * nb - (uint64_t)b * (b - (b > 0)) / 2); };   // tile of block b
     std::vector<std::pair<uint32_t, uint32_t>> p;
     for (uint32_t q = k; q-- > 0;) p.emplace_back(first(nb * q / k), first(nb * (q + 1) / k));
@@ -474,6 +478,15 @@ size_t arrival_of(const std::vector<uint64_t>& arrive, uint64_t row) {
     return c;
 }
 
+// Whether copies to this host memory run beside the host (asked where a call may
+// take more than one panel: from 4 MiB on the bus).
+static bool pinned(const void* p) {
+    cudaPointerAttributes a{};
+    const bool known = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type != cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return known;
+}
+
 uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad, uint64_t row_bits,
                                   uint32_t* d_out, uint32_t* host_out, int kernel_pref, cudaStream_t st,
                                   cudaStream_t copy_st) {
@@ -483,7 +496,8 @@ uint64_t DenseEngine::run_to_host(const uint64_t* dX, uint64_t n, uint32_t w_pad
         return 0;
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
-    const auto panels = host_plan(kind, n, n_tiles, require_device(), tri_size(n) * sizeof(uint32_t));
+    const uint64_t bus_bytes = tri_size(n) * sizeof(uint32_t);
+    const auto panels = host_plan(kind, n, n_tiles, require_device(), bus_bytes, bus_bytes < (2u << 21) || pinned(host_out));
     return panels_to_host(dX, n, w_pad, kind, panels, {}, d_out, host_out, st, copy_st);
 }
 
@@ -498,8 +512,8 @@ uint64_t DenseEngine::run_host_to_host(uint64_t* dX, uint64_t n, uint32_t w_pad,
     }
     const int kind = prepare(n, row_bits, kernel_pref, true, st);
     const int sms = require_device();
-    const auto panels =
-        host_plan(kind, n, n_tiles, sms, tri_size(n) * sizeof(uint32_t) + n * host_wpr * sizeof(uint64_t));
+    const uint64_t bus_bytes = tri_size(n) * sizeof(uint32_t) + n * host_wpr * sizeof(uint64_t);
+    const auto panels = host_plan(kind, n, n_tiles, sms, bus_bytes, bus_bytes < (2u << 21) || pinned(host_out));
     const bool one = panels.size() == 1;             // everything on one stream
     cudaStream_t in = one ? st : h2d_st;
     // Rows [n, n_pad) read as zero: whole tiles read them.

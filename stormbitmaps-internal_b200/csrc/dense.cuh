@@ -134,7 +134,7 @@ std::vector<std::pair<uint32_t, uint32_t>> host_panels(uint32_t n_tiles, uint32_
 // resident once part c is, in parts of whole panels where those are whole A
 // blocks, else in 32 equal ones. arrival_of: the part that a read of `row` waits for.
 std::vector<std::pair<uint32_t, uint32_t>> host_plan(int kind, uint64_t n, uint32_t n_tiles, int sms,
-                                                     uint64_t bus_bytes);
+                                                     uint64_t bus_bytes, bool pinned_out);
 std::vector<uint64_t> host_arrivals(int kind, uint64_t n, const std::vector<uint2>& tiles,
                                     const std::vector<std::pair<uint32_t, uint32_t>>& panels, int sms);
 size_t arrival_of(const std::vector<uint64_t>& arrive, uint64_t row);

@@ -50,11 +50,13 @@ static void check_cover(int kind, uint64_t n) {
     }
 }
 
-static void check_plan(int kind, uint64_t n, int sms, uint64_t bus_bytes) {
+static void check_plan(int kind, uint64_t n, int sms, uint64_t bus_bytes, bool pinned) {
     std::vector<uint2> t;
     build_tiles(t, n, kind);
     const uint64_t bm = tile_rows_a(kind), bn = tile_rows_b(kind);
-    const auto panels = host_plan(kind, n, (uint32_t)t.size(), sms, bus_bytes);
+    const auto panels = host_plan(kind, n, (uint32_t)t.size(), sms, bus_bytes, pinned);
+    // pageable memory: no panels where they would be whole A blocks for the copies' sake
+    CHECK(pinned || kind != KIND_F4 || t.size() > 24u * std::max(1, sms / 2) || panels.size() == 1, n);
     const auto arrive = host_arrivals(kind, n, t, panels, sms);
     CHECK(!panels.empty() && !arrive.empty() && arrive.back() == 0 && arrive[0] < n, n);
     for (size_t c = 1; c < arrive.size(); ++c) CHECK(arrive[c] < arrive[c - 1], n);   // each row once, in one part
@@ -89,7 +91,8 @@ int main() {
         for (uint64_t n : {1ull, 256ull, 257ull, 700ull, 2000ull, 4097ull, 9000ull, 15000ull, 15104ull, 15105ull, 16000ull,
                            30000ull})
             for (int sms : {1, 2, 147, 148})
-                for (uint64_t mib : {0ull, 1ull, 5ull, 1000ull}) check_plan(kind, n, sms, mib << 20);
+                for (uint64_t mib : {0ull, 1ull, 5ull, 1000ull})
+                    for (bool pinned : {true, false}) check_plan(kind, n, sms, mib << 20, pinned);
     std::printf(g_fail ? "FAIL (%d)\n" : "ok\n", g_fail);
     return g_fail ? 1 : 0;
 }
