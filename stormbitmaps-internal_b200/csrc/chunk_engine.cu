@@ -1441,9 +1441,6 @@ __device__ __forceinline__ void gallop_chunks(const ChunkView& v, uint64_t c0, u
     }
 }
 
-// Mean run length (log2) from which the rows' lists are galloped through.
-constexpr uint32_t RUN_GALLOP_WLOG = 6;
-
 // A row's chunks dealt to the warps of its CTA in consecutive shares.
 __device__ __forceinline__ void warp_share(uint64_t c0, uint64_t c1, uint64_t& lo, uint64_t& hi) {
     constexpr uint32_t WARPS = ROW_WALK_THREADS / 32;
@@ -1904,18 +1901,22 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
     // (a run of length l spans about 1 + l / bin bins; the sweep's entry
     // reads, pieces^2 x bin / U for uniform rows, are least at bin = l).
     uint32_t rwlog = 4, most_chunks = 0;
+    bool run_gallop = false;
     if (facts_ok) {
         double sc = 0.0, sr = 0.0;
+        uint64_t chunks = 0;
         for (uint64_t r = 0; r < n; ++r) {
             const ChunkRowFacts& f = d.facts[r];
             if (f.plain && f.bitmap_chunks == 0) {
                 sc += (double)f.card;
                 sr += (double)f.runs;
                 most_chunks = std::max(most_chunks, f.chunks);
+                chunks += f.chunks;
             }
         }
         const double ml = sr > 0.0 ? sc / sr : 1.0;
         rwlog = (uint32_t)std::min(15.0, std::max(4.0, std::round(std::log2(std::max(ml, 1.0)))));
+        run_gallop = run_walk_gallops(rwlog, sc, (double)chunks);
     }
     const double RW = (double)(1u << rwlog);
     const uint64_t n_bins = U >> rwlog;
@@ -1935,7 +1936,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         SB_CUDA(cudaMemsetAsync(d_rstats.p, 0, 2 * sizeof(unsigned long long), st));
         d_cpieces.reserve(d.cid.n);
         const uint32_t gq = (uint32_t)std::min<uint64_t>(q, (uint64_t)sms * 64);
-        auto count = rwlog >= RUN_GALLOP_WLOG ? run_count_kernel<true> : run_count_kernel<false>;
+        auto count = run_gallop ? run_count_kernel<true> : run_count_kernel<false>;
         count<<<gq, ROW_WALK_THREADS, 0, st>>>(d.view(), d_qrows.p, (uint32_t)q, rwlog, d_rpieces.p,
                                                          d_cpieces.p, d_rbins.p);
         run_stats_kernel<<<sms * 8, 256, 0, st>>>(d_rbins.p, n_bins, d_rstats.p);
@@ -2542,7 +2543,7 @@ uint64_t ChunkEngine::run(const ChunkDev& d, PairMode mode, uint64_t n1, uint64_
         d_pstats.reserve(1);
         SB_CUDA(cudaMemsetAsync(d_pstats.p, 0, sizeof(PostingsStats), st));
         const uint32_t gq = (uint32_t)std::min<uint64_t>((nq + 7) / 8, (uint64_t)sms * 16);
-        auto fill = rwlog >= RUN_GALLOP_WLOG ? run_fill_kernel<true> : run_fill_kernel<false>;
+        auto fill = run_gallop ? run_fill_kernel<true> : run_fill_kernel<false>;
         fill<<<(uint32_t)std::min<uint64_t>(nq, (uint64_t)sms * 64), ROW_WALK_THREADS, 0, st>>>(
             d.view(), d_qrows.p, (uint32_t)nq, rwlog, d_rpoff.p, d_cpieces.p, d_pieces.p);
         postings_alloc_kernel<<<sms * 8, ALLOC_THREADS, 0, st>>>(d_rbins.p, n_bins, d_rstart.p, nullptr, nullptr, d_pstats.p);

@@ -28,6 +28,15 @@ constexpr uint32_t WALK_SKEW_GROUP = 4;
 constexpr uint32_t WALK_STEP = 256;
 __host__ __device__ inline uint32_t walk_entry(uint32_t q, uint32_t lane) { return 32 * q + lane; }
 
+// How the run postings go through rows' lists: a lane per chunk that gallops from
+// run to run, from a mean run length of 2^6 on (wlog) and for short lists, where a
+// warp looking at 256 entries at a time has a few to look at (run form forced, ms,
+// 256 entries / galloping: 20000 rows of 168 values over 2^24 3.45 / 2.01, 4000 of
+// 839 over 2^22 0.94 / 0.78, 300 of 671 over 2^26 0.30 / 0.15).
+inline bool run_walk_gallops(uint32_t wlog, double entries, double chunks) {
+    return wlog >= 6 || entries < 48.0 * chunks;
+}
+
 // Items of a walk beside one per row and one per group that there is: some find
 // no chunk, more leave less of a long row to one warp.
 constexpr uint64_t WALK_SPARE_ITEMS = 1ull << 18;

@@ -72,6 +72,11 @@ static void check_step() {
 
 int main() {
     check_step();
+    // the run postings gallop where runs are long, and where lists are short whatever the runs
+    for (uint32_t wlog = 4; wlog <= 15; ++wlog) {
+        g_fail += sb200::run_walk_gallops(wlog, 480000.0, 10000.0) != (wlog >= 6);
+        g_fail += !sb200::run_walk_gallops(wlog, 479999.0, 10000.0) || !sb200::run_walk_gallops(wlog, 12000.0, 10000.0);
+    }
     using Rows = std::vector<sb200::ChunkRowFacts>;
     check("no rows", {});
     check("empty rows", Rows(5));
