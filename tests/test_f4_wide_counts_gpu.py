@@ -54,3 +54,26 @@ def test_gathered_blocks_past_16_bits(sb):
     np.testing.assert_array_equal(got, want)
     assert total == ws and s.last_dense()[0] == n
     s.close()
+
+
+@pytest.mark.parametrize("m", (1 << 24, (1 << 24) - 4097))
+def test_large_counts_of_random_rows(sb, m):
+    """Counts near 2^24 that grow by irregular steps all the way (dense random
+    rows), whole tiles and K segments added up: every step of the fp32 counts is
+    a whole number below 2^24, exact."""
+    w = (m + 63) // 64
+    g = gen.rng(m)
+    words = ~(g.integers(0, 1 << 64, size=(9, w), dtype=np.uint64) & g.integers(0, 1 << 64, size=(9, w), dtype=np.uint64)
+              & g.integers(0, 1 << 64, size=(9, w), dtype=np.uint64) & g.integers(0, 1 << 64, size=(9, w), dtype=np.uint64))
+    words[3] |= ~np.uint64(0)                                    # a full row: counts equal the others' sizes
+    if m % 64:
+        words[:, -1] &= np.uint64((1 << (m % 64)) - 1)
+    want, ws = ol.contig_matrix(words)
+    for sched in (sb.SCHED_TILES, sb.SCHED_STREAM_K):
+        c = sb.StormContig(m)
+        c.set_schedule(sched)
+        c.add_bitmaps(words)
+        got, s = c.matrix()
+        np.testing.assert_array_equal(got, want, err_msg=str(sched))
+        assert s == ws
+        c.close()
